@@ -22,92 +22,158 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 // |weight| descending, followed by the empty slots in their original order;
 // then every non-empty slot with |w| < threshold is zeroed in place.
 // Here a 256-thread block stages 32 neurons' slots in shared memory with
-// coalesced row loads, each warp ranks one neuron's 128 slots at a time
-// (lane L holds slots L, L+32, L+64, L+96), scatters them to their ranks,
-// prunes, and the block writes the rows back coalesced.
+// coalesced row loads; each warp sorts four neurons at once, 128 keys
+// (32768 - |w|, slot) of each in registers, 4 a lane, by a bitonic network
+// whose merges start with a reflected exchange (every exchange then leaves the
+// smaller key at the lower position, so in-register exchanges are a bare
+// min and max).  Keys are distinct, so the network is stable.  The sorted
+// slots are gathered while still staged by slot, then the staging area is
+// rewritten by neuron and the block writes the rows back coalesced.
+// Bound by the network's 60 shuffles and ~300 ALU instructions a neuron: 630 us
+// at 1,009,091 neurons (1.8 GB moved, 2.9 TB/s), against 3,827 us for ranking
+// each key against the 127 others (256 shuffles, 512 compares a neuron).
 // ---------------------------------------------------------------------------
 constexpr int kSortNeurons = 32;
+constexpr int kSortPer = 4;   // neurons a warp sorts at once (8 warps x 4 = 32)
+
+struct SortIn {
+  uint32_t tg[AXC_MAX_DENDRITES][kSortNeurons + 1];
+  int16_t wt[AXC_MAX_DENDRITES][kSortNeurons + 2];
+  uint8_t tm[AXC_MAX_DENDRITES][kSortNeurons + 4];
+};
+// By neuron: ranks 4l..4l+3 are one chunk, chunk l of neuron c at l ^ c, so that
+// the row-wise reads (one rank of 32 neurons) meet 32, 16 and 32 banks; the four
+// targets of a chunk are rotated by c / 8 for the same reason.
+struct SortOut {
+  uint4 tg[kSortNeurons][32];
+  uint2 wt[kSortNeurons][32];
+  uint32_t tm[kSortNeurons][32];
+};
+union SortStage {
+  SortIn in;
+  SortOut out;
+};
+
+// One exchange of the network over the warp's 128 keys (position 4 * lane + r)
+// with the partner lane ^ m: register r meets the partner's R(r).
+template <bool REFLECT>
+__device__ __forceinline__ void sort_exchange(uint32_t (&k)[kSortPer][4], uint32_t m, bool low) {
+#pragma unroll
+  for (int e = 0; e < kSortPer; e++) {
+    uint32_t o[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) o[r] = __shfl_xor_sync(kFull, k[e][REFLECT ? 3 - r : r], m);
+#pragma unroll
+    for (int r = 0; r < 4; r++) k[e][r] = low ? min(k[e][r], o[r]) : max(k[e][r], o[r]);
+  }
+}
+
+__device__ __forceinline__ void sort_pair(uint32_t& a, uint32_t& b) {
+  const uint32_t lo = min(a, b), hi = max(a, b);
+  a = lo;
+  b = hi;
+}
+
+__device__ __forceinline__ void sort_in_lane(uint32_t (&k)[kSortPer][4]) {   // strides 2, 1
+#pragma unroll
+  for (int e = 0; e < kSortPer; e++) {
+    sort_pair(k[e][0], k[e][2]);
+    sort_pair(k[e][1], k[e][3]);
+    sort_pair(k[e][0], k[e][1]);
+    sort_pair(k[e][2], k[e][3]);
+  }
+}
 
 __global__ void __launch_bounds__(256) k_sort_and_prune(ShardVramPtrs v, uint32_t N, int16_t prune_threshold) {
-  __shared__ uint32_t s_tg[AXC_MAX_DENDRITES][kSortNeurons + 1];
-  __shared__ int16_t s_wt[AXC_MAX_DENDRITES][kSortNeurons + 1];
-  __shared__ uint8_t s_tm[AXC_MAX_DENDRITES][kSortNeurons + 1];
+  __shared__ __align__(16) SortStage st;
   const uint32_t n0 = blockIdx.x * kSortNeurons;
   const uint32_t col = threadIdx.x & 31, row0 = threadIdx.x >> 5;
+  const uint32_t n = n0 + col;
+#pragma unroll 4
   for (uint32_t r = row0; r < AXC_MAX_DENDRITES; r += 8) {
-    const uint32_t n = n0 + col;
     uint32_t t = 0; int16_t w = 0; uint8_t m = 0;
     if (n < N) {
       const size_t idx = (size_t)r * N + n;
-      t = v.dendrite_targets[idx];
-      w = v.dendrite_weights[idx];
-      m = v.dendrite_timers[idx];
+      t = __ldcs(v.dendrite_targets + idx);
+      w = __ldcs(v.dendrite_weights + idx);
+      m = __ldcs(v.dendrite_timers + idx);
     }
-    s_tg[r][col] = t; s_wt[r][col] = w; s_tm[r][col] = m;
+    st.in.tg[r][col] = t; st.in.wt[r][col] = w; st.in.tm[r][col] = m;
   }
   if (threadIdx.x < kSortNeurons && n0 + threadIdx.x < N) v.soma_flags[n0 + threadIdx.x] &= 0xF1;  // :456-458
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t c = warp; c < kSortNeurons; c += 8) {
-    uint32_t tg[4]; int16_t wt[4]; uint8_t tm[4]; int32_t aw[4]; bool ne[4];
+  uint32_t key[kSortPer][4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const uint32_t q = lane + 32 * j;
-      tg[j] = s_tg[q][c]; wt[j] = s_wt[q][c]; tm[j] = s_tm[q][c];
-      aw[j] = wt[j] >= 0 ? wt[j] : -wt[j];
-      ne[j] = tg[j] != 0;
+  for (int e = 0; e < kSortPer; e++) {
+    const uint32_t c = warp * kSortPer + e;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {   // any start order will do: the slot is part of the key
+      const uint32_t q = lane + 32u * r;
+      const int32_t w = st.in.wt[q][c];
+      const uint32_t aw = (uint32_t)(w >= 0 ? w : -w);
+      // an empty slot sorts after every |w| (0..32768)
+      key[e][r] = ((st.in.tg[q][c] != 0u ? 32768u - aw : 0x10000u) << 7) | q;
     }
-    uint32_t bal[4], nonempty = 0;
+  }
+  // merges of 2 and 4 inside a lane, then 8..128 across lanes
 #pragma unroll
-    for (int j = 0; j < 4; j++) { bal[j] = __ballot_sync(kFull, ne[j]); nonempty += __popc(bal[j]); }
-    uint32_t rank[4];
+  for (int e = 0; e < kSortPer; e++) {
+    sort_pair(key[e][0], key[e][1]);
+    sort_pair(key[e][2], key[e][3]);
+    sort_pair(key[e][0], key[e][3]);
+    sort_pair(key[e][1], key[e][2]);
+    sort_pair(key[e][0], key[e][1]);
+    sort_pair(key[e][2], key[e][3]);
+  }
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      // empties: after all non-empty slots, in original order
-      uint32_t before = 0;
+  for (uint32_t m = 1; m < 32; m *= 2) {   // blocks of 8m keys: 2m lanes
+    sort_exchange<true>(key, 2 * m - 1, (lane & m) == 0);
 #pragma unroll
-      for (int jj = 0; jj < 4; jj++) {
-        const uint32_t eb = ~bal[jj];
-        if (jj < j) before += __popc(eb);
-        else if (jj == j) before += __popc(eb & ((1u << lane) - 1u));
-      }
-      rank[j] = nonempty + before;
+    for (uint32_t s = m / 2; s > 0; s /= 2) sort_exchange<false>(key, s, (lane & s) == 0);
+    sort_in_lane(key);
+  }
+  uint32_t tg[kSortPer][4];
+  uint32_t wt[kSortPer][2], tm[kSortPer];
+#pragma unroll
+  for (int e = 0; e < kSortPer; e++) {
+    const uint32_t c = warp * kSortPer + e;
+    wt[e][0] = wt[e][1] = tm[e] = 0;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const uint32_t q = key[e][r] & 127u, inv = key[e][r] >> 7;
+      // pruned (:498-506): a live slot with |w| = 32768 - inv below the threshold
+      const bool cut = inv <= 32768u && 32768 - (int32_t)inv < (int32_t)prune_threshold;
+      const uint32_t t = st.in.tg[q][c];
+      const uint32_t w = (uint16_t)st.in.wt[q][c], m = st.in.tm[q][c];
+      tg[e][r] = cut ? 0u : t;
+      wt[e][r >> 1] |= (cut ? 0u : w) << (16 * (r & 1));
+      tm[e] |= (cut ? 0u : m) << (8 * r);
     }
-    uint32_t cnt[4] = {0, 0, 0, 0};
-    for (int src = 0; src < 32; src++) {
-#pragma unroll
-      for (int jj = 0; jj < 4; jj++) {
-        const int32_t oa = __shfl_sync(kFull, aw[jj], src);
-        const bool one = __shfl_sync(kFull, ne[jj], src);
-        const uint32_t oq = (uint32_t)src + 32u * jj;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const uint32_t q = lane + 32u * j;
-          cnt[j] += (one && (oa > aw[j] || (oa == aw[j] && oq < q))) ? 1u : 0u;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (ne[j]) rank[j] = cnt[j];
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      uint32_t t = tg[j]; int16_t w = wt[j]; uint8_t m = tm[j];
-      if (t != 0 && aw[j] < (int32_t)prune_threshold) { t = 0; w = 0; m = 0; }   // :498-506
-      s_tg[rank[j]][c] = t; s_wt[rank[j]][c] = w; s_tm[rank[j]][c] = m;
-    }
-    __syncwarp();
   }
   __syncthreads();
+#pragma unroll
+  for (int e = 0; e < kSortPer; e++) {
+    const uint32_t c = warp * kSortPer + e, ch = lane ^ c, rot = c >> 3;
+    // word j of the chunk holds rank (j - rot) & 3
+    const uint32_t a0 = tg[e][0], a1 = tg[e][1], a2 = tg[e][2], a3 = tg[e][3];
+    uint4 o = make_uint4(a0, a1, a2, a3);
+    if (rot == 1) o = make_uint4(a3, a0, a1, a2);
+    else if (rot == 2) o = make_uint4(a2, a3, a0, a1);
+    else if (rot == 3) o = make_uint4(a1, a2, a3, a0);
+    st.out.tg[c][ch] = o;
+    st.out.wt[c][ch] = make_uint2(wt[e][0], wt[e][1]);
+    st.out.tm[c][ch] = tm[e];
+  }
+  __syncthreads();
+  if (n >= N) return;
+#pragma unroll 4
   for (uint32_t r = row0; r < AXC_MAX_DENDRITES; r += 8) {
-    const uint32_t n = n0 + col;
-    if (n < N) {
-      const size_t idx = (size_t)r * N + n;
-      v.dendrite_targets[idx] = s_tg[r][col];
-      v.dendrite_weights[idx] = s_wt[r][col];
-      v.dendrite_timers[idx] = s_tm[r][col];
-    }
+    const uint32_t ch = (r >> 2) ^ col, j = r & 3u;
+    const size_t idx = (size_t)r * N + n;
+    v.dendrite_targets[idx] = reinterpret_cast<const uint32_t*>(&st.out.tg[col][ch])[(j + (col >> 3)) & 3u];
+    v.dendrite_weights[idx] = reinterpret_cast<const int16_t*>(&st.out.wt[col][ch])[j];
+    v.dendrite_timers[idx] = reinterpret_cast<const uint8_t*>(&st.out.tm[col][ch])[j];
   }
 }
 

@@ -127,3 +127,26 @@ def test_extract_telemetry_and_last_spikes(gpu):
         assert np.array_equal(vram.last_spikes(), ref)
     finally:
         lib.gpu_free(d_ids)
+
+
+@pytest.mark.parametrize("n,slots", [(4, 1), (28, 128), (36, 127), (100, 3), (128, 0)])
+def test_sort_and_prune_edges(gpu, n, slots):
+    """Neuron counts off the kernel's 32-neuron blocks, full and nearly empty rows, ties, both ends of the weights."""
+    from axicor_gb300.formats import state_blob_size
+
+    rng = np.random.default_rng(n)
+    state = np.zeros(state_blob_size(n), np.uint8)
+    sv = StateView(state, n)
+    sv.targets[:slots] = rng.integers(1, 1 << 31, size=(slots, n))
+    sv.weights[:] = rng.choice(np.array([-32768, -32767, -400, -1, 0, 1, 400, 32767], np.int16), size=(128, n))
+    sv.targets[rng.random((128, n)) < 0.1] = 0
+    sv.dendrite_timers[:] = rng.integers(0, 256, size=(128, n), dtype=np.uint8)
+    for threshold in (-5, 0, 1, 401, 32767):
+        vram = S.VramState(n, 32)
+        vram.upload_state(state)
+        N.lib().launch_sort_and_prune(C.byref(vram.ptrs), n, threshold)
+        N.lib().gpu_device_synchronize()
+        h = state.copy()
+        oracle.sort_and_prune(h, np.zeros(256, np.uint32), n, threshold)
+        assert np.array_equal(vram.download_state(), h), threshold
+        vram.free()
