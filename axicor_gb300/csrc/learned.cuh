@@ -741,15 +741,23 @@ __global__ void __launch_bounds__(128) k_learn_predict(LearnDev L, const __nv_bf
 }
 
 // ---------------------------------------------------------------------------
-// MLP training: one block of 4 warps per 16 samples, on the tensor cores.
-// Forward: warp p computes the hidden units 32p .. 32p + 31 of the 16 samples
-// (mlp_group_sum); the output is (((G0 + G1) + (G2 + G3)) + b2) + x[kResidF],
-// as in inference.  Loss: mean squared error over the minibatch (count
-// samples, 1/count).  Backward: dy = 2 (y - t) / count; gw2[u] and gb1[u] in
-// FP32 (rows g, then g + 8, then over g by xor 4, 8, 16); dh[s][u] = dy[s] w2[u]
-// where the pre-activation is positive, rounded to BF16 for the W1 gradient
-// G1 = dh^T x, 16 units x 8 features per MMA over the 16 samples.  Each block
-// writes its partial gradient; k_mlp_reduce sums them in block order.
+// MLP training: a block of 4 warps takes groups of 16 samples, on the tensor
+// cores.  Forward: warp p computes the hidden units 32p .. 32p + 31 of the 16
+// samples (mlp_group_sum); the output is (((G0 + G1) + (G2 + G3)) + b2) +
+// x[kResidF], as in inference.  Loss: mean squared error over the minibatch
+// (count samples, 1/count).  Backward: dy = 2 (y - t) / count; gw2[u] and
+// gb1[u] in FP32 (rows g, then g + 8); dh[s][u] = dy[s] w2[u] where the
+// pre-activation is positive, rounded to BF16 for the W1 gradient G1 = dh^T x,
+// 16 units x 8 features per MMA over the 16 samples.  A block takes the groups
+// blockIdx, blockIdx + gridDim, ... and adds each group's gradient to its own in
+// registers (FP32, in that order; the next group's samples are loaded while a
+// group is computed); after the last, gw2 and gb1 are summed over g (xor 4, 8,
+// 16) and the block writes one partial gradient; k_mlp_reduce sums the
+// partials in block order.  The grid is bounded (kGradBlocks), so a large count
+// costs no more partials: at 100,000 samples a block a group wrote and re-read
+// 211 MB of them (gradient 115 us + reduction 262 us; the whole
+// axc_mlp_loss_grad call 755 us with its allocations, 86 us now, bound by the
+// latency of a block's 14 groups one after another).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) k_mlp_grad(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ X,
                                                   const float* __restrict__ Yt, const uint32_t* __restrict__ idx,
@@ -760,64 +768,118 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const __nv_bfloat16* __restric
   __shared__ float ysum[4][16];
   __shared__ float s_dy[16], s_loss[16], s_x8[16];
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, q = lane & 3u;
-  const uint32_t s0 = blockIdx.x * 16u;
-  const uint32_t ns = min(16u, count - s0);
-  for (uint32_t i = threadIdx.x; i < 16u * kFeat; i += 128u) {
-    const uint32_t r = i / kFeat, f = i % kFeat;
-    float v = 0.f;
-    if (r < ns) v = X[(size_t)(idx ? idx[s0 + r] : s0 + r) * kFeat + f];
-    const __nv_bfloat16 bv = __float2bfloat16_rn(v);
-    xs[r][f] = bv;
-    xt[f][r] = bv;
-    if (f == kResidF) s_x8[r] = __bfloat162float(bv);
-  }
-  __syncthreads();
-  uint32_t a[4][4];
+  const uint32_t groups = (count + 15u) / 16u;
+  float gw1[2][8][4], gw2[4][2], gb1[4][2];
 #pragma unroll
-  for (int ks = 0; ks < 4; ks++) {
-    a[ks][0] = ld_bf16x2(&xs[g][16 * ks + 2 * q]);
-    a[ks][1] = ld_bf16x2(&xs[g + 8][16 * ks + 2 * q]);
-    a[ks][2] = ld_bf16x2(&xs[g][16 * ks + 8 + 2 * q]);
-    a[ks][3] = ld_bf16x2(&xs[g + 8][16 * ks + 8 + 2 * q]);
-  }
-  float acc[4][4];   // pre-activations of units 32w + 8nt + 2q (+1), rows g and g + 8
-  float sg8;
-  const float sg = mlp_group_sum(wb, a, w, &sg8, acc);
-  if (q == 0) {
-    ysum[w][g] = sg;
-    ysum[w][g + 8] = sg8;
-  }
-  __syncthreads();
-  if (threadIdx.x < 16) {
-    const uint32_t r = threadIdx.x;
-    const float y = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ysum[0][r], ysum[1][r]), __fadd_rn(ysum[2][r], ysum[3][r])),
-                                        __bfloat162float(wb[kOffB2])),
-                              s_x8[r]);
-    float dy = 0.f, lr = 0.f;
-    if (r < ns) {
-      const float d = __fsub_rn(y, Yt[idx ? idx[s0 + r] : s0 + r]);
-      dy = __fmul_rn(__fmul_rn(2.f, d), inv_count);
-      lr = __fmul_rn(__fmul_rn(d, d), inv_count);
+  for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+    for (int nf = 0; nf < 8; nf++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) gw1[mt][nf][e] = 0.f;
+#pragma unroll
+  for (int nt = 0; nt < 4; nt++) gw2[nt][0] = gw2[nt][1] = gb1[nt][0] = gb1[nt][1] = 0.f;
+  float gb2 = 0.f, loss = 0.f;   // thread 0
+  // sample r = 2i + threadIdx / 64, feature f = threadIdx % 64 of a group
+  const uint32_t xf = threadIdx.x & 63u, xr = threadIdx.x >> 6;
+  float xn[8], yn = 0.f;
+  const auto load = [&](uint32_t s0) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint32_t sm = s0 + 2u * i + xr;
+      xn[i] = sm < count ? X[(size_t)(idx ? idx[sm] : sm) * kFeat + xf] : 0.f;
     }
-    s_dy[r] = dy;
-    s_loss[r] = lr;
-  }
-  __syncthreads();
-  const float dyg = s_dy[g], dyg8 = s_dy[g + 8];
-  float gw2[4][2], gb1[4][2];
-#pragma unroll
-  for (int nt = 0; nt < 4; nt++) {
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const uint32_t u = 32u * w + 8u * nt + 2u * q + j;
-      const float w2u = __bfloat162float(wb[kOffW2 + u]);
-      const float ag = acc[nt][j], ag8 = acc[nt][2 + j];
-      gw2[nt][j] = __fadd_rn(__fmul_rn(dyg, bf16r(fmaxf(ag, 0.f))), __fmul_rn(dyg8, bf16r(fmaxf(ag8, 0.f))));
-      const float dhg = ag > 0.f ? __fmul_rn(dyg, w2u) : 0.f, dhg8 = ag8 > 0.f ? __fmul_rn(dyg8, w2u) : 0.f;
-      gb1[nt][j] = __fadd_rn(dhg, dhg8);
-      dht[u][g] = __float2bfloat16_rn(dhg);
-      dht[u][g + 8] = __float2bfloat16_rn(dhg8);
+    if (threadIdx.x < 16) {
+      const uint32_t sm = s0 + threadIdx.x;
+      yn = sm < count ? Yt[idx ? idx[sm] : sm] : 0.f;
     }
+  };
+  uint32_t gi = blockIdx.x;
+  if (gi < groups) load(gi * 16u);
+  for (; gi < groups; gi += gridDim.x) {
+    const uint32_t ns = min(16u, count - gi * 16u);
+    const float yt = yn;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint32_t r = 2u * i + xr;
+      const __nv_bfloat16 bv = __float2bfloat16_rn(xn[i]);
+      xs[r][xf] = bv;
+      xt[xf][r] = bv;
+      if (xf == kResidF) s_x8[r] = __bfloat162float(bv);
+    }
+    __syncthreads();
+    if (gi + gridDim.x < groups) load((gi + gridDim.x) * 16u);
+    uint32_t a[4][4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ks++) {
+      a[ks][0] = ld_bf16x2(&xs[g][16 * ks + 2 * q]);
+      a[ks][1] = ld_bf16x2(&xs[g + 8][16 * ks + 2 * q]);
+      a[ks][2] = ld_bf16x2(&xs[g][16 * ks + 8 + 2 * q]);
+      a[ks][3] = ld_bf16x2(&xs[g + 8][16 * ks + 8 + 2 * q]);
+    }
+    float acc[4][4];   // pre-activations of units 32w + 8nt + 2q (+1), rows g and g + 8
+    float sg8;
+    const float sg = mlp_group_sum(wb, a, w, &sg8, acc);
+    if (q == 0) {
+      ysum[w][g] = sg;
+      ysum[w][g + 8] = sg8;
+    }
+    __syncthreads();
+    if (threadIdx.x < 16) {
+      const uint32_t r = threadIdx.x;
+      const float y =
+          __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ysum[0][r], ysum[1][r]), __fadd_rn(ysum[2][r], ysum[3][r])),
+                              __bfloat162float(wb[kOffB2])),
+                    s_x8[r]);
+      float dy = 0.f, lr = 0.f;
+      if (r < ns) {
+        const float d = __fsub_rn(y, yt);
+        dy = __fmul_rn(__fmul_rn(2.f, d), inv_count);
+        lr = __fmul_rn(__fmul_rn(d, d), inv_count);
+      }
+      s_dy[r] = dy;
+      s_loss[r] = lr;
+    }
+    __syncthreads();
+    const float dyg = s_dy[g], dyg8 = s_dy[g + 8];
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const uint32_t u = 32u * w + 8u * nt + 2u * q + j;
+        const float w2u = __bfloat162float(wb[kOffW2 + u]);
+        const float ag = acc[nt][j], ag8 = acc[nt][2 + j];
+        const float g2 = __fadd_rn(__fmul_rn(dyg, bf16r(fmaxf(ag, 0.f))), __fmul_rn(dyg8, bf16r(fmaxf(ag8, 0.f))));
+        const float dhg = ag > 0.f ? __fmul_rn(dyg, w2u) : 0.f, dhg8 = ag8 > 0.f ? __fmul_rn(dyg8, w2u) : 0.f;
+        gw2[nt][j] = __fadd_rn(gw2[nt][j], g2);
+        gb1[nt][j] = __fadd_rn(gb1[nt][j], __fadd_rn(dhg, dhg8));
+        dht[u][g] = __float2bfloat16_rn(dhg);
+        dht[u][g + 8] = __float2bfloat16_rn(dhg8);
+      }
+    }
+    if (threadIdx.x == 0) {
+      float b2 = 0.f, l = 0.f;
+      for (int r = 0; r < 16; r++) {
+        b2 = __fadd_rn(b2, s_dy[r]);
+        l = __fadd_rn(l, s_loss[r]);
+      }
+      gb2 = __fadd_rn(gb2, b2);
+      loss = __fadd_rn(loss, l);
+    }
+    __syncwarp();   // a warp reads only its own units of dht
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++) {
+      const uint32_t ub = 32u * w + 16u * mt;
+      const uint32_t am[4] = {ld_bf16x2(&dht[ub + g][2 * q]), ld_bf16x2(&dht[ub + g + 8][2 * q]),
+                              ld_bf16x2(&dht[ub + g][8 + 2 * q]), ld_bf16x2(&dht[ub + g + 8][8 + 2 * q])};
+#pragma unroll
+      for (int nf = 0; nf < 8; nf++) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16_16816(d, am, ld_bf16x2(&xt[8 * nf + g][2 * q]), ld_bf16x2(&xt[8 * nf + g][8 + 2 * q]));
+#pragma unroll
+        for (int e = 0; e < 4; e++) gw1[mt][nf][e] = __fadd_rn(gw1[mt][nf][e], d[e]);
+      }
+    }
+    __syncthreads();   // xs, xt, s_dy are free for the next group
   }
 #pragma unroll
   for (int nt = 0; nt < 4; nt++) {
@@ -830,22 +892,17 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const __nv_bfloat16* __restric
       }
     }
   }
-  __syncthreads();
   float* Pp = partial + (size_t)blockIdx.x * (kParams + 1);
 #pragma unroll
   for (int mt = 0; mt < 2; mt++) {
     const uint32_t ub = 32u * w + 16u * mt;
-    const uint32_t am[4] = {ld_bf16x2(&dht[ub + g][2 * q]), ld_bf16x2(&dht[ub + g + 8][2 * q]),
-                            ld_bf16x2(&dht[ub + g][8 + 2 * q]), ld_bf16x2(&dht[ub + g + 8][8 + 2 * q])};
 #pragma unroll
     for (int nf = 0; nf < 8; nf++) {
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_bf16_16816(d, am, ld_bf16x2(&xt[8 * nf + g][2 * q]), ld_bf16x2(&xt[8 * nf + g][8 + 2 * q]));
       const uint32_t f = 8u * nf + 2u * q;
-      Pp[(size_t)(ub + g) * kFeat + f] = d[0];
-      Pp[(size_t)(ub + g) * kFeat + f + 1] = d[1];
-      Pp[(size_t)(ub + g + 8) * kFeat + f] = d[2];
-      Pp[(size_t)(ub + g + 8) * kFeat + f + 1] = d[3];
+      Pp[(size_t)(ub + g) * kFeat + f] = gw1[mt][nf][0];
+      Pp[(size_t)(ub + g) * kFeat + f + 1] = gw1[mt][nf][1];
+      Pp[(size_t)(ub + g + 8) * kFeat + f] = gw1[mt][nf][2];
+      Pp[(size_t)(ub + g + 8) * kFeat + f + 1] = gw1[mt][nf][3];
     }
   }
   if (g == 0) {
@@ -860,23 +917,29 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const __nv_bfloat16* __restric
     }
   }
   if (threadIdx.x == 0) {
-    float gb2 = 0.f, loss = 0.f;
-    for (int r = 0; r < 16; r++) {
-      gb2 = __fadd_rn(gb2, s_dy[r]);
-      loss = __fadd_rn(loss, s_loss[r]);
-    }
     Pp[kOffB2] = gb2;
     Pp[kParams] = loss;
   }
 }
 
-__global__ void __launch_bounds__(256) k_mlp_reduce(const float* __restrict__ partial, uint32_t nb,
-                                                    float* __restrict__ grad) {
+// grad[p] (p < kParams) and *loss: the partials added in block order, 16 loads
+// in flight a thread.
+__global__ void __launch_bounds__(64) k_mlp_reduce(const float* __restrict__ partial, uint32_t nb,
+                                                   float* __restrict__ grad, float* __restrict__ loss) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p > kParams) return;
   float s = 0.f;
-  for (uint32_t b = 0; b < nb; b++) s = __fadd_rn(s, partial[(size_t)b * (kParams + 1) + p]);
-  grad[p] = s;
+  uint32_t b = 0;
+  for (; b + 16 <= nb; b += 16) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __ldg(partial + (size_t)(b + i) * (kParams + 1) + p);
+#pragma unroll
+    for (int i = 0; i < 16; i++) s = __fadd_rn(s, v[i]);
+  }
+  for (; b < nb; b++) s = __fadd_rn(s, __ldg(partial + (size_t)b * (kParams + 1) + p));
+  if (p < kParams) grad[p] = s;
+  else if (loss) *loss = s;
 }
 
 __global__ void __launch_bounds__(256) k_mlp_to_bf16(const float* __restrict__ master, __nv_bfloat16* __restrict__ wb) {
@@ -922,6 +985,7 @@ __global__ void __launch_bounds__(128) k_mlp_predict(const __nv_bfloat16* __rest
 #include <cstddef>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <tuple>
 #include <vector>
 
@@ -931,6 +995,52 @@ namespace {
 // After chunks on the plain graph the features history is stale: the next
 // learned tick plans without the previous tick's features (no prediction, dense).
 __global__ void k_learn_resume(LearnCtl* c) { c->feat_done = 0; }
+
+// Blocks of the gradient kernel for `count` samples: a group of kGradPer samples
+// each up to three blocks per SM, beyond that several groups a block.
+static uint32_t grad_blocks(uint32_t count) {
+  return std::min(count / kGradPer + (count % kGradPer != 0), 3u * (uint32_t)sm_count());
+}
+
+// Scratch of one stand-alone MLP call, in the order of its stream, from a pool
+// of this library's own per device that keeps at most kMlpPoolKeep bytes between
+// calls (a cudaMalloc and cudaFree pair a call cost ten times the kernels at a
+// few thousand samples).  Threads and streams share the pool safely: the runtime
+// orders reuse.
+constexpr uint64_t kMlpPoolKeep = 32u << 20;
+static cudaError_t mlp_scratch(char** out, size_t bytes, cudaStream_t st) {
+  constexpr int kDevs = 64;
+  static std::mutex mu;
+  static cudaMemPool_t pools[kDevs] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kDevs) return cudaErrorInvalidDevice;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pools[dev]) {
+      cudaMemPoolProps pr = {};
+      pr.allocType = cudaMemAllocationTypePinned;
+      pr.location.type = cudaMemLocationTypeDevice;
+      pr.location.id = dev;
+      e = cudaMemPoolCreate(&pool, &pr);
+      uint64_t keep = kMlpPoolKeep;
+      if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) return e;
+      pools[dev] = pool;
+    }
+    pool = pools[dev];
+  }
+  return cudaMallocFromPoolAsync(reinterpret_cast<void**>(out), bytes, pool, st);
+}
+
+static void launch_mlp_grad(const __nv_bfloat16* wb, const float* X, const float* Y, const uint32_t* idx,
+                            uint32_t count, float* partial, float* grad, float* loss, cudaStream_t st) {
+  const uint32_t nb = grad_blocks(count);
+  k_mlp_grad<<<nb, 128, 0, st>>>(wb, X, Y, idx, count, 1.f / (float)count, partial);
+  k_mlp_reduce<<<(kParams + 1 + 63) / 64, 64, 0, st>>>(partial, nb, grad, loss);
+}
 
 constexpr uint32_t kGateChunks = 64;   // chunks on the plain graph after a dense-only probe, at most
 
@@ -1505,8 +1615,7 @@ int32_t axc_learned_train(void* handle, uint32_t epochs, uint32_t batch, float l
   if (e != cudaSuccess) return (int32_t)e;
   const uint32_t nval = n / 10, ntr = n - nval;
   if (ntr == 0) return (int32_t)cudaErrorInvalidValue;
-  const uint32_t maxb = std::max((std::min(batch, ntr) + kGradPer - 1) / kGradPer, (nval + kGradPer - 1) / kGradPer);
-  e = learned_partial(*L, std::max(maxb, 1u));
+  e = learned_partial(*L, std::max({grad_blocks(std::min(batch, ntr)), grad_blocks(nval), 1u}));
   if (e != cudaSuccess) return (int32_t)e;
   std::vector<uint32_t> order(ntr);
   for (uint32_t i = 0; i < ntr; i++) order[i] = i;
@@ -1518,9 +1627,7 @@ int32_t axc_learned_train(void* handle, uint32_t epochs, uint32_t batch, float l
     uint32_t steps = 0;
     for (uint32_t b0 = 0; b0 < ntr && e == cudaSuccess; b0 += batch) {
       const uint32_t cnt = std::min(batch, ntr - b0);
-      const uint32_t nb = (cnt + kGradPer - 1) / kGradPer;
-      k_mlp_grad<<<nb, 128, 0, st>>>(L->wb, L->X, L->Y, L->idx + b0, cnt, 1.f / (float)cnt, L->partial);
-      k_mlp_reduce<<<(kParams + 1 + 255) / 256, 256, 0, st>>>(L->partial, nb, L->grad);
+      launch_mlp_grad(L->wb, L->X, L->Y, L->idx + b0, cnt, L->partial, L->grad, L->grad + kParams, st);
       L->adam_step++;
       const float c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)L->adam_step)));
       const float c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)L->adam_step)));
@@ -1537,10 +1644,8 @@ int32_t axc_learned_train(void* handle, uint32_t epochs, uint32_t batch, float l
   if (e == cudaSuccess && out_val) {
     *out_val = 0.f;
     if (nval) {
-      const uint32_t nb = (nval + kGradPer - 1) / kGradPer;
-      k_mlp_grad<<<nb, 128, 0, st>>>(L->wb, L->X + (size_t)ntr * kFeat, L->Y + ntr, nullptr, nval,
-                                     1.f / (float)nval, L->partial);
-      k_mlp_reduce<<<(kParams + 1 + 255) / 256, 256, 0, st>>>(L->partial, nb, L->grad);
+      launch_mlp_grad(L->wb, L->X + (size_t)ntr * kFeat, L->Y + ntr, nullptr, nval, L->partial, L->grad,
+                      L->grad + kParams, st);
       e = cudaMemcpyAsync(out_val, L->grad + kParams, 4, cudaMemcpyDeviceToHost, st);
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
@@ -1565,40 +1670,32 @@ int32_t axc_mlp_loss_grad(const float* d_params, const float* d_x, const float* 
                           float* d_loss, void* stream_v) {
   if (!d_params || !d_x || !d_y || !d_grad || count == 0) return (int32_t)cudaErrorInvalidValue;
   cudaStream_t st = static_cast<cudaStream_t>(stream_v);
-  const uint32_t nb = (count + kGradPer - 1) / kGradPer;
-  __nv_bfloat16* wb = nullptr;
-  float *partial = nullptr, *grad = nullptr;
-  cudaError_t e = cudaMalloc(&wb, (size_t)kParams * 2);
-  if (e == cudaSuccess) e = cudaMalloc(&partial, (size_t)nb * (kParams + 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&grad, ((size_t)kParams + 1) * 4);
-  if (e == cudaSuccess) {
-    k_mlp_to_bf16<<<(kParams + 255) / 256, 256, 0, st>>>(d_params, wb);
-    k_mlp_grad<<<nb, 128, 0, st>>>(wb, d_x, d_y, nullptr, count, 1.f / (float)count, partial);
-    k_mlp_reduce<<<(kParams + 1 + 255) / 256, 256, 0, st>>>(partial, nb, grad);
-    e = cudaMemcpyAsync(d_grad, grad, (size_t)kParams * 4, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess && d_loss) e = cudaMemcpyAsync(d_loss, grad + kParams, 4, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  }
-  if (wb) cudaFree(wb);
-  if (partial) cudaFree(partial);
-  if (grad) cudaFree(grad);
-  return (int32_t)e;
+  const size_t wb_bytes = ((size_t)kParams * 2 + 255) & ~size_t(255);
+  char* base = nullptr;
+  cudaError_t e = mlp_scratch(&base, wb_bytes + (size_t)grad_blocks(count) * (kParams + 1) * 4, st);
+  if (e != cudaSuccess) return (int32_t)e;
+  __nv_bfloat16* wb = reinterpret_cast<__nv_bfloat16*>(base);
+  k_mlp_to_bf16<<<(kParams + 255) / 256, 256, 0, st>>>(d_params, wb);
+  launch_mlp_grad(wb, d_x, d_y, nullptr, count, reinterpret_cast<float*>(base + wb_bytes), d_grad, d_loss, st);
+  e = cudaFreeAsync(base, st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  return (int32_t)(e != cudaSuccess ? e : es);
 }
 
 int32_t axc_mlp_predict(const float* d_params, const float* d_x, uint32_t count, float* d_out, void* stream_v) {
   if (!d_params || !d_x || !d_out) return (int32_t)cudaErrorInvalidValue;
   if (count == 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream_v);
-  __nv_bfloat16* wb = nullptr;
-  cudaError_t e = cudaMalloc(&wb, (size_t)kParams * 2);
-  if (e == cudaSuccess) {
-    k_mlp_to_bf16<<<(kParams + 255) / 256, 256, 0, st>>>(d_params, wb);
-    k_mlp_predict<<<std::min((count + 15u) / 16u, 8192u), 128, 0, st>>>(wb, d_x, count, d_out);
-    e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = cudaGetLastError();
-  }
-  if (wb) cudaFree(wb);
-  return (int32_t)e;
+  char* base = nullptr;
+  cudaError_t e = mlp_scratch(&base, (size_t)kParams * 2, st);
+  if (e != cudaSuccess) return (int32_t)e;
+  __nv_bfloat16* wb = reinterpret_cast<__nv_bfloat16*>(base);
+  k_mlp_to_bf16<<<(kParams + 255) / 256, 256, 0, st>>>(d_params, wb);
+  k_mlp_predict<<<std::min((count + 15u) / 16u, 8192u), 128, 0, st>>>(wb, d_x, count, d_out);
+  e = cudaFreeAsync(base, st);
+  cudaError_t es = cudaStreamSynchronize(st);
+  if (es == cudaSuccess) es = cudaGetLastError();
+  return (int32_t)(e != cudaSuccess ? e : es);
 }
 
 }  // extern "C"

@@ -244,3 +244,18 @@ def test_gate_follows_the_brain_from_dense_to_sparse(gpu):
         b.check(*b.oracle(ticks), "gated and ungated chunks")
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("count", [1, 16, 17, 7296, 7297, 9001])
+def test_mlp_gradient_over_group_counts(gpu, count):
+    """One group, a ragged last group, and counts where the bounded grid gives some blocks several groups of 16
+    (from 3 blocks x 152 SMs x 16 = 7,296 samples); the tolerances of test_mlp_gradient_matches_oracle."""
+    rng = np.random.Generator(np.random.PCG64(count))
+    p = M.init_params(9)
+    x = rng.uniform(0, 1, (count, M.FEATURES)).astype(np.float32)
+    t = rng.uniform(0, 1, count).astype(np.float32)
+    loss, g = L.mlp_loss_grad(p, x, t)
+    lo, go = M.loss_grad(p, x, t)
+    assert loss == pytest.approx(lo, rel=1e-5)
+    assert np.abs(g - go).max() <= 2e-3 * np.abs(go).max()
+    assert np.linalg.norm(g - go) <= 1e-3 * np.linalg.norm(go)
