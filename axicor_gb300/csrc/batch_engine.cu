@@ -47,11 +47,14 @@ struct GraphCache {
 
 // Per batch, before its graph: the tick base and dopamine the captured kernels
 // read, and (row engine) whether the batch lays its row copy out anew.
-__global__ void k_set_batch_ctl(ShardCtl* ctl, uint32_t tick_base, int32_t dopamine, uint32_t rows, uint32_t force,
-                                uint32_t ticks) {
-  ctl->tick_base = tick_base;
-  ctl->dopamine = dopamine;
-  if (rows) layout_decide(ctl, force, ticks);
+__global__ void __launch_bounds__(512) k_set_batch_ctl(ShardCtl* ctl, uint32_t tick_base, int32_t dopamine,
+                                                      uint32_t rows, uint32_t force, uint32_t ticks,
+                                                      const uint32_t* lit, uint32_t A) {
+  if (threadIdx.x == 0) {
+    ctl->tick_base = tick_base;
+    ctl->dopamine = dopamine;
+  }
+  if (rows) layout_decide(ctl, force, ticks, lit, A);
 }
 
 cudaError_t ensure_counts(ShardScratch& s, uint32_t batch, bool* realloc, cudaStream_t stream) {
@@ -149,7 +152,8 @@ cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* ou
   else
     e = cudaMemsetAsync(s->batch_counts, 0, (size_t)b.ticks * 4, stream);
   if (e != cudaSuccess) return e;
-  k_set_batch_ctl<<<1, 1, 0, stream>>>(s->ctl, b.tick_base, (int32_t)b.dopamine, rows, force ? 1u : 0u, b.ticks);
+  k_set_batch_ctl<<<1, 512, 0, stream>>>(s->ctl, b.tick_base, (int32_t)b.dopamine, rows, force ? 1u : 0u, b.ticks,
+                                         rows ? s->rows->lit : nullptr, b.total_axons);
   // burst-counter reset before the batch (shard.rs:71)
   e = launch_reset_burst(*b.vram, b.padded_n, stream);
   if (e != cudaSuccess) return e;
@@ -279,7 +283,7 @@ extern "C" int32_t axc_profile_ticks(const ShardVramPtrs* vram, uint32_t padded_
       old->execs.clear();
     }
     cudaMemsetAsync(s->batch_counts, 0, (size_t)ticks * 4, st);
-    k_set_batch_ctl<<<1, 1, 0, st>>>(s->ctl, tick0, (int32_t)dopamine, 0u, 1u, ticks);   // layouts its own
+    k_set_batch_ctl<<<1, 32, 0, st>>>(s->ctl, tick0, (int32_t)dopamine, 0u, 1u, ticks, nullptr, 0u);   // layouts its own
     e = launch_rows_begin(*vram, *s, padded_n, total_axons, st);
     if (e != cudaSuccess) return (int32_t)e;
   }

@@ -37,7 +37,8 @@ struct ShardCtl {
   int32_t dopamine;       // batch mode: dopamine of the batch
   uint32_t fix_count;     // row engine: GSOP slots deferred to the fix-up stage
   uint32_t fix_overflow;  // row engine: the fix-up list overflowed, rescan the spikers
-  uint32_t eval_count[2]; // row engine: non-refractory neurons listed in tick k (slot k & 1)
+  uint32_t eval_act[2][2]; // row engine, tick k (slot k & 1): [0] non-refractory neurons listed, [1] axons with a
+                           // head on a segment of the batch (8-byte aligned pairs: one atomic adds both)
   uint32_t row_smax;      // row engine: longest row (slots before the first empty) of the batch
   uint32_t seg_max;       // row engine: largest segment of a live slot in the batch
   unsigned long long row_sum;  // row engine: checksum of the batch's targets (slot order)
@@ -50,7 +51,35 @@ struct ShardCtl {
   uint32_t lay_now;       // row engine: this batch lays the row copy out anew (layout_decide)
   uint32_t lay_since;     // row engine: ticks since the last layout
   uint32_t lay_every;     // row engine: ticks between layouts while the lit-sum criterion holds
+  uint32_t lay_wait;      // row engine: ticks a layout must last while it does not hold
+  uint32_t lay_lit;       // row engine: fully-lit axons when the layout was made
+  uint32_t pad4;
+  unsigned long long lay_pfx;     // row engine: pfx_total of the layout before the current one
+  unsigned long long gsop_same[2];  // row engine: 4-slot groups the 8-lane pass's GSOP visited and left as they
+                                    // were, and all it visited, since the last decision
+  uint32_t mixed_len;     // row engine: a neuron with slots has another signal_propagation_length than pmax
+  uint32_t streak;        // row engine: consecutive ticks that the sparse form could have run (sparse_tick)
+  uint32_t idx_ok;        // row engine: an inverted index was built (it holds while idx_sum == lay_sum)
   uint32_t pad3;
+  unsigned long long lay_sum, idx_sum;  // row engine: checksum of the rows' targets by position; the index's rows'
+  const uint32_t* ix_off; // inverted index of the rows (RowIndex)
+  const uint16_t* ix_seg;
+  const uint32_t* ix_ent;
+};
+
+// Inverted index of the row copy: per axon the row slots that target it
+// (n * 128 + row position), those of one segment together, for the sparse
+// form of a tick (row_engine.cuh).  The learned engine's: allocated when its
+// brain first turns quiet (4 bytes a slot; the batch and per-tick paths
+// allocate nothing beyond the row copy).
+struct RowIndex {
+  void* base = nullptr;
+  uint32_t* off = nullptr;  // [A+1] first entry of an axon
+  uint32_t* cur = nullptr;  // [A] fill cursor (build)
+  uint32_t* bsum = nullptr; // scan block sums (build)
+  uint16_t* seg = nullptr;  // [A][32] entries of an axon before segment s (s = 31: all segments >= 31);
+                            // kSegUnsorted in [0]: too many entries, unsorted
+  uint32_t* ent = nullptr;  // [live slots]
 };
 
 // Neuron-major copy of the dendrites used by the batch engine for the length
@@ -66,6 +95,9 @@ struct RowCache {
   uint32_t* eval = nullptr; // [N] non-refractory neurons of the tick
   uint32_t* fix = nullptr;  // [kFixCap] deferred GSOP slots (n*128 + slot)
   uint32_t* lit = nullptr;  // [A/32+1] fully-lit axons of the tick, one bit each
+  uint32_t* live = nullptr; // [A/32+1] axons with a head on a segment of the batch this tick, one bit each
+  uint32_t* evb = nullptr;  // [N/32+1] neurons evaluated this tick, one bit each
+  int32_t* acc = nullptr;   // [N] input current of the sparse form (zero between ticks)
   uint32_t* gs_n = nullptr; // [N] spikers with 1..8 slots GSOP may move (a thread each)
   uint32_t* gd_n = nullptr; // [N] spikers with more (8 lanes each)
   uint4* amask = nullptr;   // [N] row positions (bit q) whose weights GSOP may move (set at batch start)
@@ -74,6 +106,8 @@ struct RowCache {
   uint32_t* wcnt = nullptr; // [2][kMaxUpdateWarps] spikers each warp of the update pass listed (gs_n, gd_n)
   int2* lsum = nullptr;     // [N] x: wrapping sum of the row's lit-sum weights, y: row positions before them
   uint32_t* xlit = nullptr; // [A/32+1] axons taken as fully lit when the row layout was made
+  RowIndex ix;
+  bool ix_failed = false;   // no room for the index: not tried again
   uint8_t* posmap = nullptr;  // [N][128] row position of each columnar slot (learned engine only; own allocation)
 };
 
@@ -90,7 +124,7 @@ struct ShardScratch {
   ShardCtl* ctl = nullptr;
   uint32_t* batch_counts = nullptr;  // [batch_cap] per-tick network spike counts
   uint32_t batch_cap = 0;
-  uint32_t* h_counts_pinned = nullptr;  // pinned staging for batch_counts / tick_base
+  uint32_t* h_counts_pinned = nullptr;  // pinned: [0] the device asks for an inverted index (RowIndex)
   void* graph_cache = nullptr;          // batch engine graphs (batch_engine.cu)
   RowCache* rows = nullptr;             // batch engine neuron-major dendrites
   // Per-tick entry point (cu_step_day_phase): its row cache lives across calls.
@@ -129,22 +163,55 @@ inline bool batch_rows_force(ShardScratch& s) {
 
 #ifdef __CUDACC__
 // The device's layout decision for the next `ticks` ticks of a batch (one
-// thread, before the batch): a new layout when forced, while the current one
-// misses the lit-sum criterion (at most an eighth of the live slots outside
-// the lit-sum groups: the weights are still freezing, or the axons taken as
-// fully lit were not yet), and otherwise every lay_every ticks, doubling from
-// kBatchRelayoutMin to kBatchRelayoutMax.  The layout kernels of the batch
+// block, before the batch; lit: the last tick's fully-lit bitmap of A axons).
+// A new layout when forced; every lay_every ticks, doubling from
+// kBatchRelayoutMin to kBatchRelayoutMax, while the current one meets the
+// lit-sum criterion (at most an eighth of the live slots outside the lit-sum
+// groups); while it does not, when it could do better: a tenth more axons are
+// fully lit than when it was made, or an eighth of the 4-slot groups that GSOP
+// visited since the last decision no longer moved (the weights froze), but at
+// most every lay_wait ticks, doubling from 16 while the new layouts gain less
+// than a tenth, and at least every kBatchRelayoutMax.  A brain whose weights
+// never freeze, or that is quiet, so keeps its layout instead of paying for
+// one each batch (1.5 ms at 1.5M neurons).  The layout kernels of the batch
 // return at once when lay_now is 0.
-__device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint32_t ticks) {
+__device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint32_t ticks, const uint32_t* lit,
+                                              uint32_t A) {
+  __shared__ uint32_t s_lit;
   const bool met = c->slot_total > 0 && c->pfx_total * 8ull <= c->slot_total;
-  const bool build = force || !met || c->lay_since >= c->lay_every;
+  uint32_t n = 0;
+  if (threadIdx.x == 0) s_lit = 0;
+  __syncthreads();
+  if (force || !met) {
+    for (uint32_t i = threadIdx.x; i < (A + 31) / 32; i += blockDim.x) n += __popc(lit[i]);
+    n = __reduce_add_sync(0xFFFFFFFFu, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&s_lit, n);
+  }
+  __syncthreads();
+  if (threadIdx.x) return;
+  bool build = force;
+  if (!force && met) {
+    build = c->lay_since >= c->lay_every;
+  } else if (!force) {
+    const bool froze = c->gsop_same[0] > 0 && c->gsop_same[0] * 8ull >= c->gsop_same[1];
+    const bool grew = (unsigned long long)s_lit * 10ull > (unsigned long long)c->lay_lit * 11ull;
+    // (the sparse form reads no more than the movable slots of a few spikers: its rows stay)
+    build = (c->lay_since >= kBatchRelayoutMax && c->streak == 0u) ||
+            (c->lay_since >= c->lay_wait && (froze || grew) && c->slot_total > 0);
+  }
+  if (build && (force || !met)) c->lay_lit = s_lit;
+  // the last layout left a tenth fewer slots outside the groups than the one before
+  const bool paid = c->pfx_total * 10ull < c->lay_pfx * 9ull;
   if (build) {
     const uint32_t twice = 2u * c->lay_every;
     c->lay_every = (force || !met || c->lay_every < kBatchRelayoutMin) ? kBatchRelayoutMin
                    : twice < kBatchRelayoutMax                          ? twice
                                                                         : kBatchRelayoutMax;
+    c->lay_wait = (force || met) ? 0u : (paid || c->lay_wait < 16u) ? 16u : min(2u * c->lay_wait, kBatchRelayoutMax);
+    c->lay_pfx = c->pfx_total;
     c->lay_since = 0;
   }
+  c->gsop_same[0] = c->gsop_same[1] = 0;
   c->lay_since += ticks;
   c->lay_now = build ? 1u : 0u;
 }
@@ -168,7 +235,18 @@ cudaError_t rows_posmap(ShardScratch& s, cudaStream_t stream);
 cudaError_t launch_rows_begin(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, cudaStream_t stream,
                               bool row_sum = false, bool permute = true, bool with_posmap = true,
                               bool conditional = false);
+// The device's layout decision outside a batch's control kernel (per-tick calls).
+cudaError_t launch_rows_decide(ShardScratch& s, uint32_t A, bool force, uint32_t ticks, cudaStream_t stream);
 cudaError_t launch_rows_end(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, cudaStream_t stream);
+
+// Before a learned chunk of a shard with rows, on its stream: when the device
+// asked for an inverted index, lays the rows out if the device's decision says
+// so (as the chunk's own conditional layout would) and builds the index; else
+// nothing.
+cudaError_t rows_index_wish(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, cudaStream_t stream,
+                            bool row_sum = false, bool with_posmap = true);
+// The pinned word the device asks through.
+cudaError_t rows_wish_alloc(ShardScratch& s);
 
 // Tries of the update pass's first wait for its staged bitmap; returns the previous value.
 uint32_t set_first_wait_limit(uint32_t tries);
@@ -210,6 +288,7 @@ struct TickArgs {
   uint32_t k;                 // tick index inside the batch
   bool rows;                  // use the neuron-major row engine (batch mode only)
   uint32_t fix_cap;           // row engine: deferred-GSOP list capacity (<= kFixCap)
+  bool index;                 // row engine: the tick may run its sparse form (the learned engine's plain graph)
   bool defer_push;            // row engine: leave this tick's soma pushes to the next tick's prologue
                               // (never on the last tick of a batch)
 };

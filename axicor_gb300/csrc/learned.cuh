@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) k_learn_scatter(LearnDev L, uint32_t T, c
                                                        int32_t* __restrict__ acc, ShardCtl* __restrict__ sc) {
   LearnCtl& c = *L.ctl;
   if (blockIdx.x == 0 && threadIdx.x == 0 && c.mode == 1u) c.stat[c.overflow ? kStOverflow : kStSparse]++;
-  if (c.mode != 1u || c.overflow) return;
+  if (c.mode != 1u || c.overflow || index_ok(sc)) return;   // with the rows' index: sparse_hits
   __shared__ uint32_t s_prop[16];
   __shared__ uint32_t s_pmax;
   extern __shared__ uint32_t s_pre[];   // [T+1] prefix of the tiles' active-axon counts
@@ -409,12 +409,12 @@ __global__ void __launch_bounds__(256) k_learn_update(ShardVramPtrs P, LearnDev 
                                                       uint32_t* __restrict__ wcnt, ShardCtl* __restrict__ ctl,
                                                       uint32_t k) {
   LearnCtl& c = *L.ctl;
-  if (c.mode != 1u || c.overflow) return;
+  if (c.mode != 1u || c.overflow || index_ok(ctl)) return;
   __shared__ VariantParameters lut[16];
   lut_to_smem(lut);
   __syncthreads();
   const uint32_t tick = ctl->tick_base + k;
-  const uint32_t ecount = ctl->eval_count[k & 1];
+  const uint32_t ecount = ctl->eval_act[k & 1][0];
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1055,10 +1055,12 @@ static_assert(kGateSnapBytes == sizeof(GateSnap::before), "GateSnap mirrors Shar
 
 // Per chunk, before its graph: tick base, dopamine, and whether the chunk lays
 // its rows out anew (always on learned chunks: force).
-__global__ void k_learn_set_ctl(ShardCtl* ctl, uint32_t tick_base, int32_t dopamine, uint32_t force, uint32_t ticks) {
+__global__ void __launch_bounds__(512) k_learn_set_ctl(ShardCtl* ctl, uint32_t tick_base, int32_t dopamine,
+                                                      uint32_t force, uint32_t ticks, const uint32_t* lit,
+                                                      uint32_t A) {
   ctl->tick_base = tick_base;
   ctl->dopamine = dopamine;
-  layout_decide(ctl, force, ticks);
+  layout_decide(ctl, force, ticks, lit, A);
 }
 
 // splitmix64: seeded parameter init and minibatch order, identical on every host.
@@ -1216,10 +1218,9 @@ static void learned_update_forms(Learned& L, ShardScratch& s, uint32_t k, cudaSt
   const uint32_t fix_cap = kFixCap;
   // dense: the plain engine's passes on the movable-first rows, GSOP inside them
   // (the 8-lane pass, or the lit-sum form when its lit set held)
-  launch_rows_update<true>(L.v, s, N, A, k, fix_cap, L.ctl, st);
-  k_rows_update_lsum<false><<<kLsumBlocks * sms, 256, 0, st>>>(L.v, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend,
-                                                               r.fix, s.ctl, k, fix_cap, r.lit, r.lfz, r.lsum,
-                                                               ColWT{}, L.ctl);
+  launch_rows_update<true>(L.v, s, N, A, k, fix_cap, L.ctl, st, ColWT{}, false, true);
+  launch_rows_lsum(L.v, s, A, k, fix_cap, L.ctl, st);
+  launch_rows_sparse(L.v, s, N, A, k, fix_cap, L.ctl, st);
   // sparse: the axon-driven gather, GLIF, and GSOP of the spikers it listed
   k_learn_scatter<<<8 * sms, 256, ((size_t)L.T + 1) * 4, st>>>(D, L.T, L.inv, L.inv_seg, r.mask2, r.rw, r.posmap,
                                                                 L.v.soma_flags, L.v.axon_heads, A, L.acc, s.ctl);
@@ -1245,10 +1246,11 @@ static cudaError_t learned_tick(Learned& L, ShardScratch& s, uint32_t k, bool la
     k_rows_prologue<true><<<(G + 255) / 256, 256, 0, st>>>(L.v.axon_heads, A, L.v_seg, bits_k, L.voff,
                                                            bits_k ? L.nv : 0u, s.incoming, nullptr, k, r.mask2,
                                                            r.mult, L.v.soma_flags, L.v.timers, N, r.eval, s.ctl,
-                                                           raise, r.lit, D, k > 0 ? s.pend : nullptr, r.xlit);
+                                                           raise, r.lit, D, k > 0 ? s.pend : nullptr, r.xlit,
+                                                           r.live, r.evb);
   learned_update_forms(L, s, k, st);
   k_rows_fixup<<<2 * sms, 256, 0, st>>>(L.v, N, A, r.rt, r.rw, r.cnt, r.mask2, s.pend, r.eval, r.fix, s.ctl, k,
-                                        nullptr, nullptr, 0, ColWT{});
+                                        nullptr, nullptr, 0, ColWT{}, (volatile uint32_t*)s.h_counts_pinned);
   // soma pushes: by the next tick's prologue within a graph, here on its last tick
   if (last)
     k_rows_push<<<2 * sms, 256, 0, st>>>(L.v.axon_heads, L.v.soma_to_axon, A, s.pend, r.eval, L.v.soma_flags, N,
@@ -1431,6 +1433,7 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
   if (!s) return (int32_t)e;
   e = rows_alloc(*s, L->N, L->A, true, st);
   if (e == cudaSuccess) e = rows_posmap(*s, st);
+  if (e == cudaSuccess) e = rows_wish_alloc(*s);
   if (e != cudaSuccess) return (int32_t)e;
   s->tick_rows_valid.store(false);   // this run's rows replace the per-tick entry point's
   if (L->rows_base != s->rows->base) {
@@ -1475,6 +1478,7 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
         a.rows = true;
         a.defer_push = k + 1 < tpg;
         a.fix_cap = kFixCap;
+        a.index = true;
         le = launch_tick(L->v, *s, a, L->capture);
       } else {
         le = learned_tick(*L, *s, k, k + 1 == tpg, kind == 1, L->capture);
@@ -1523,8 +1527,10 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
         e = cudaMemsetAsync(L->stage + (size_t)have * L->words, 0, (size_t)(tpg + 1 - have) * L->words * 4, st);
       if (e != cudaSuccess) break;
     }
-    k_learn_set_ctl<<<1, 1, 0, st>>>(s->ctl, L->tick_base + t0, (int32_t)L->dopamine, force ? 1u : 0u, tpg);
-    e = launch_reset_burst(L->v, L->N, st);
+    k_learn_set_ctl<<<1, 512, 0, st>>>(s->ctl, L->tick_base + t0, (int32_t)L->dopamine, force ? 1u : 0u, tpg,
+                                       s->rows->lit, L->A);
+    e = rows_index_wish(L->v, *s, L->N, L->A, st, true, true);
+    if (e == cudaSuccess) e = launch_reset_burst(L->v, L->N, st);
     unsigned long long picked0 = 0, picked1 = 0;
     const size_t picked_at = offsetof(LearnCtl, stat) + kStSparsePicked * sizeof(unsigned long long);
     if (e == cudaSuccess && gate_on && !gated)

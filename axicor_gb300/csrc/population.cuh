@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(256) k_pop_begin(PopBrain* __restrict__ brains
     b.pmax = pmax_of(b.lut);
     b.ctl->row_smax = 0;
     b.ctl->seg_max = 0;
-    b.ctl->eval_count[0] = 0;
-    b.ctl->eval_count[1] = 0;
+    b.ctl->eval_act[0][0] = 0;
+    b.ctl->eval_act[1][0] = 0;
     b.mask2[b.A] = make_uint2(0u, 0x80000000u);
   }
   for (uint32_t a = threadIdx.x; a < b.A; a += blockDim.x) b.mult[a] = 0;
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(256) k_pop_prologue(const PopBrain* __restrict
   if (threadIdx.x == 0) {
     uint32_t tot = 0;
     for (int q = 0; q < 8; q++) { const uint32_t c = s_warp[q]; s_warp[q] = tot; tot += c; }
-    s_base = tot ? atomicAdd(&b.ctl->eval_count[k & 1], tot) : 0u;
+    s_base = tot ? atomicAdd(&b.ctl->eval_act[k & 1][0], tot) : 0u;
   }
   __syncthreads();
   if (ev) b.eval[s_base + s_warp[w] + __popc(ballot & ((1u << lane) - 1u))] = i;
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(1024) k_pop_chunks(const PopBrain* __restrict_
   const uint32_t per = (count + 1023) / 1024;
   const uint32_t b0 = threadIdx.x * per;
   uint32_t s = 0;
-  for (uint32_t b = b0; b < min(b0 + per, count); b++) s += (brains[b].ctl->eval_count[k & 1] + chunk - 1) / chunk;
+  for (uint32_t b = b0; b < min(b0 + per, count); b++) s += (brains[b].ctl->eval_act[k & 1][0] + chunk - 1) / chunk;
   part[threadIdx.x] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(1024) k_pop_chunks(const PopBrain* __restrict_
   __syncthreads();
   uint32_t pos = part[threadIdx.x];
   for (uint32_t b = b0; b < min(b0 + per, count); b++) {
-    const uint32_t e = brains[b].ctl->eval_count[k & 1];
+    const uint32_t e = brains[b].ctl->eval_act[k & 1][0];
     for (uint32_t st = 0; st < e; st += chunk) chunks[pos++] = make_uint2(b, st);
   }
 }
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256, 3) k_pop_update(const PopBrain* __restric
     const bool use_lit = (A >> 5) + 1 <= lit_cap;
     const uint32_t seg_hi = min(b.ctl->seg_max, 30u);   // lit bits cover segments 1..seg_hi
     const uint32_t tick = b.tick_base + pctl->tick0 + k;
-    const uint32_t ecount = min(b.ctl->eval_count[k & 1] - cd.y, chunk);
+    const uint32_t ecount = min(b.ctl->eval_act[k & 1][0] - cd.y, chunk);
     const uint32_t smax = b.ctl->row_smax;
     for (uint32_t off = warp * G; off < ecount; off += 8 * G) {
       const uint32_t idx = off + grp;
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(256) k_pop_fixup(const PopBrain* __restrict__ 
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   // the next tick's lists (the slot was last used two ticks ago)
-  for (uint32_t b = tid; b < count; b += stride) brains[b].ctl->eval_count[(k + 1) & 1] = 0;
+  for (uint32_t b = tid; b < count; b += stride) brains[b].ctl->eval_act[(k + 1) & 1][0] = 0;
   if (nfix == 0 && !overflow) return;
   if (!overflow) {
     for (uint32_t i = tid; i < nfix; i += stride) {
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(256) k_pop_fixup(const PopBrain* __restrict__ 
     const uint2 cd = chunks[ci];
     const PopBrain& b = brains[cd.x];
     const uint32_t li = rem / kRowStride, q = rem % kRowStride;
-    if (cd.y + li >= b.ctl->eval_count[k & 1]) continue;
+    if (cd.y + li >= b.ctl->eval_act[k & 1][0]) continue;
     const uint32_t n = b.eval[cd.y + li];
     if (!(b.P.soma_flags[n] & 1) || q >= (b.cnt[n] & 0xFFu)) continue;
     const uint32_t r = n * kRowStride + q;
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(256) k_pop_push(const PopBrain* __restrict__ b
     const uint2 cd = chunks[w / chunk];
     const PopBrain& b = brains[cd.x];
     const uint32_t li = cd.y + w % chunk;
-    if (li >= b.ctl->eval_count[k & 1]) continue;
+    if (li >= b.ctl->eval_act[k & 1][0]) continue;
     const uint32_t n = b.eval[li];
     if (!(b.P.soma_flags[n] & 1)) continue;
     const uint32_t ax = b.P.soma_to_axon[n];
@@ -597,8 +597,8 @@ __global__ void k_pop_next_graph(PopBrain* __restrict__ brains, uint32_t count, 
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) pctl->tick0 = tick0;
   if (i < count) {            // tick 0 of the graph appends into slot 0
-    brains[i].ctl->eval_count[0] = 0;
-    brains[i].ctl->eval_count[1] = 0;
+    brains[i].ctl->eval_act[0][0] = 0;
+    brains[i].ctl->eval_act[1][0] = 0;
   }
 }
 

@@ -184,6 +184,19 @@ __device__ __forceinline__ bool lsum_tick(const ShardCtl* ctl, uint32_t k) {
   return c > 0 && p * 8ull <= c && ctl->dense[k & 1] == 0u;
 }
 
+// The sparse form can run tick k: fewer than half as many axons have a head on
+// a segment of the batch as neurons are evaluated.  The dense pass tests every
+// slot of the evaluated neurons (~4.5 ns a thousand slots at 1.5M neurons), the
+// sparse form walks the hit segments' entries of the active axons.  The two
+// words were written by the prologue.
+__device__ __forceinline__ bool sparse_tick(const ShardCtl* ctl, uint32_t k) {
+  return ctl->eval_act[k & 1][1] * 2u < ctl->eval_act[k & 1][0];
+}
+
+// The inverted index matches the rows: it was built, from a layout with the
+// same targets at the same row positions.
+__device__ __forceinline__ bool index_ok(const ShardCtl* ctl) { return ctl->idx_ok && ctl->idx_sum == ctl->lay_sum; }
+
 // Per-neuron GSOP constants (physics.cu:290-345).
 struct GsopConsts {
   int32_t bm, raw_pot, final_dep;
@@ -284,6 +297,17 @@ struct LearnDev {
   uint32_t* evbits;         // [N/32+1] evaluated neurons of the tick
 };
 
+// The form of tick k, the same for every kernel that asks after the prologue.
+// lc: the learned engine's control block (its planned sparse ticks), or null;
+// index: the tick may run sparse by the exact counts (the learned engine's
+// graphs, whose memory holds the inverted index).
+enum TickForm { kFormDense = 0, kFormLitSum = 1, kFormSparse = 2, kFormScatter = 3 };
+__device__ __forceinline__ TickForm tick_form(const ShardCtl* ctl, uint32_t k, const LearnCtl* lc, uint32_t index) {
+  if (lc && lc->mode == 1u && !lc->overflow) return index_ok(ctl) ? kFormSparse : kFormScatter;
+  if (lsum_tick(ctl, k)) return kFormLitSum;
+  return index && index_ok(ctl) && sparse_tick(ctl, k) ? kFormSparse : kFormDense;
+}
+
 // 64-bit mix of one live slot for the targets checksum (order-independent sum).
 __device__ __forceinline__ unsigned long long slot_mix(uint32_t t, uint32_t r) {
   unsigned long long x = ((unsigned long long)t << 32) ^ (unsigned long long)r;
@@ -340,6 +364,7 @@ struct RowBuilt {
   uint32_t smx;
   unsigned long long hsum;
   uint32_t pfx;
+  unsigned long long psum;  // checksum of the targets by row position
 };
 
 __device__ __forceinline__ RowBuilt build_row(uint32_t (*s_t)[33], const int16_t (*s_w)[34], uint32_t j, uint32_t n,
@@ -401,6 +426,7 @@ __device__ __forceinline__ RowBuilt build_row(uint32_t (*s_t)[33], const int16_t
     o[ch] = permute ? mv[ch] : all[ch];
     x[ch] = permute ? (all[ch] & ~mv[ch] & ~rs[ch]) : 0u;
   }
+  unsigned long long psum = 0;
   uint32_t po = 0, px = 0, pr = 0, am[4];
   const uint32_t below = (1u << lane) - 1u;
 #pragma unroll
@@ -415,6 +441,7 @@ __device__ __forceinline__ RowBuilt build_row(uint32_t (*s_t)[33], const int16_t
     px += __popc(x[ch]);
     pr += __popc(rs[ch]);
     if (q < c) {
+      if (want_sum) psum += slot_mix(s_t[q][j], n * kRowStride + pos);
       rt[(size_t)n * kRowStride + pos] = s_t[q][j];
       rw[(size_t)n * kRowStride + pos] = s_w[q][j];
       if (posmap) posmap[(size_t)n * kRowStride + q] = (uint8_t)pos;
@@ -430,7 +457,8 @@ __device__ __forceinline__ RowBuilt build_row(uint32_t (*s_t)[33], const int16_t
     lfz[n] = (uint8_t)lf;
     if (lsum) lsum[n] = make_int2((int32_t)rsum, (int32_t)pfx);
   }
-  return RowBuilt{smx, hsum, pfx};
+  if (want_sum) psum = warp_sum(psum);
+  return RowBuilt{smx, hsum, pfx, psum};
 }
 
 // Batch end, 32 neurons from n0 by a 256-thread block: weights rows -> columnar
@@ -520,10 +548,11 @@ __global__ void __launch_bounds__(256) k_rows_build(const uint32_t* __restrict__
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // the block's longest row, largest segment, tested and live slots and (when
   // asked) targets checksum, one atomic each per block
-  __shared__ uint32_t s_bc[8], s_bs[8], s_bp[8], s_bl[8];
-  __shared__ unsigned long long s_bh[8];
+  __shared__ uint32_t s_bc[8], s_bs[8], s_bp[8], s_bl[8], s_bx[8];
+  __shared__ unsigned long long s_bh[8], s_bq[8];
   uint32_t wc = 0, ws = 0, wp = 0, wl = 0;
-  unsigned long long wh = 0;
+  bool mixed = false;
+  unsigned long long wh = 0, wq = 0;
   for (uint32_t j = warp; j < 32; j += 8) {
     const uint32_t n = n0 + j;
     if (n >= N) continue;
@@ -537,25 +566,31 @@ __global__ void __launch_bounds__(256) k_rows_build(const uint32_t* __restrict__
       wh += rb.hsum + slot_mix(c, n);
       wp += rb.pfx;
       wl += c;
+      if (want_sum) wq += rb.psum + slot_mix(c, ~n);
+      mixed |= vp.signal_propagation_length != s_pmax;
     }
   }
-  if (lane == 0) { s_bc[warp] = wc; s_bs[warp] = ws; s_bh[warp] = wh; s_bp[warp] = wp; s_bl[warp] = wl; }
+  if (lane == 0) { s_bc[warp] = wc; s_bs[warp] = ws; s_bh[warp] = wh; s_bp[warp] = wp; s_bl[warp] = wl; s_bx[warp] = mixed; s_bq[warp] = wq; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t bc = 0, bs = 0, bp = 0, bl = 0;
-    unsigned long long bh = 0;
+    uint32_t bc = 0, bs = 0, bp = 0, bl = 0, bx = 0;
+    unsigned long long bh = 0, bq = 0;
     for (int q = 0; q < 8; q++) {
       bc = max(bc, s_bc[q]);
       bs = max(bs, s_bs[q]);
       bh += s_bh[q];
       bp += s_bp[q];
       bl += s_bl[q];
+      bx |= s_bx[q];
+      bq += s_bq[q];
     }
     if (bc > *(volatile uint32_t*)&ctl->row_smax) atomicMax(&ctl->row_smax, bc);
     if (bs > *(volatile uint32_t*)&ctl->seg_max) atomicMax(&ctl->seg_max, bs);
     if (want_sum) atomicAdd(&ctl->row_sum, bh);
     if (bp) atomicAdd(&ctl->pfx_total, (unsigned long long)bp);
     if (bl) atomicAdd(&ctl->slot_total, (unsigned long long)bl);
+    if (bx) ctl->mixed_len = 1u;
+    if (bq) atomicAdd(&ctl->lay_sum, bq);
   }
 }
 
@@ -587,6 +622,8 @@ __global__ void __launch_bounds__(256) k_rows_mult(const uint32_t* __restrict__ 
     ctl->pmax = lut_pmax();
     ctl->pfx_total = 0;
     ctl->slot_total = 0;
+    ctl->mixed_len = 0;
+    ctl->lay_sum = 0;   // the index holds while the layout it was built from does (checksum)
   }
   if (n >= N) return;
   const uint32_t a = s2a[n];
@@ -662,6 +699,14 @@ __device__ __forceinline__ void learn_axons(const LearnDev& L, uint32_t i, uint3
   if (sparse && act) L.alist[(size_t)j * 1024u + s_base2 + s_red[2][w] + __popc(ball & ((1u << lane) - 1u))] = i;
 }
 
+// Counts a prologue block's evaluated neurons and active axons of tick k with
+// one atomic; returns the block's first position in the evaluated list.
+__device__ __forceinline__ uint32_t append_count(ShardCtl* ctl, uint32_t k, uint32_t eval, uint32_t act) {
+  if (!(eval | act)) return 0u;
+  return (uint32_t)atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->eval_act[k & 1][0]),
+                             ((unsigned long long)act << 32) | eval);
+}
+
 // ---------------------------------------------------------------------------
 // per tick 1/4 of the learned engine (LEARN): axons (inject, network pushes,
 // propagate, split masks) and somas (refractory countdown, list of neurons to
@@ -680,9 +725,10 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
                                                        ShardCtl* __restrict__ ctl, uint32_t raise_err,
                                                        uint32_t* __restrict__ lit_bits, LearnDev L,
                                                        uint32_t* __restrict__ pend_apply,
-                                                       const uint32_t* __restrict__ xlit) {
+                                                       const uint32_t* __restrict__ xlit,
+                                                       uint32_t* __restrict__ live, uint32_t* __restrict__ evb) {
   __shared__ uint32_t s_base;
-  __shared__ uint32_t s_warp[8];
+  __shared__ uint32_t s_warp[8], s_act[8];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t xw = (xlit && i < A) ? __ldg(xlit + (i >> 5)) : 0u;   // axons the row layout took as fully lit
   // every load first, with no barrier before them: heads, owners, pending
@@ -714,7 +760,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     ctl->fix_count = 0;      // the previous tick's fix-up is done
     ctl->fix_overflow = 0;
   }
-  bool lit = false;
+  bool lit = false, on = false;
   uint32_t fan = 0, inflight = 0;   // LEARN: active synapses and heads in flight of axon i
   if (i < A) {
     uint32_t h[8] = {hx.x, hx.y, hx.z, hx.w, hy.x, hy.y, hy.z, hy.w};
@@ -739,7 +785,8 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     lit = (m.x & need) == need && !(m.y >> 31);
     if (LEARN) {
       // active: some head covers a segment that a slot of the batch uses
-      if (((m.x | (m.y & 0x7FFFFFFFu)) & act) != 0u) fan = __ldg(L.inv_off + i + 1) - __ldg(L.inv_off + i);
+      on = ((m.x | (m.y & 0x7FFFFFFFu)) & act) != 0u;
+      if (on) fan = __ldg(L.inv_off + i + 1) - __ldg(L.inv_off + i);
 #pragma unroll
       for (int j = 0; j < 8; j++) inflight += h[j] < 255u + pmax ? 1u : 0u;
     }
@@ -762,14 +809,18 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     }
   }
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t ballot = __ballot_sync(kFull, ev);
-  if (LEARN && lane == 0 && i < N) L.evbits[i >> 5] = ballot;
-  if (lane == 0) s_warp[w] = __popc(ballot);
+  const uint32_t ballot = __ballot_sync(kFull, ev), onb = __ballot_sync(kFull, on);
+  if (lane == 0) {
+    if (LEARN && i < N) L.evbits[i >> 5] = evb[i >> 5] = ballot;
+    if (LEARN && i < A) live[i >> 5] = onb;
+    s_warp[w] = __popc(ballot);
+    s_act[w] = __popc(onb);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t tot = 0;
-    for (int q = 0; q < 8; q++) { const uint32_t c = s_warp[q]; s_warp[q] = tot; tot += c; }
-    s_base = tot ? atomicAdd(&ctl->eval_count[k & 1], tot) : 0u;
+    uint32_t tot = 0, on_tot = 0;
+    for (int q = 0; q < 8; q++) { const uint32_t c = s_warp[q]; s_warp[q] = tot; tot += c; on_tot += s_act[q]; }
+    s_base = append_count(ctl, k, tot, on_tot);
   }
   __syncthreads();
   if (ev) eval[s_base + s_warp[w] + __popc(ballot & ((1u << lane) - 1u))] = i;
@@ -1050,7 +1101,7 @@ __device__ __forceinline__ GlifOut glif_step(const VariantParameters& p, int32_t
 
 // GSOP of a spiker's slots held by this lane (physics.cu:281-373): fast slots
 // from the gtab deltas, slow ones on the exact path or deferred to the fix-up
-// list.  Writes the changed weights back to the row (rt_n / rw_n: the
+// list.  same: 4-slot groups visited << 16 | those that kept their weights.  Writes the changed weights back to the row (rt_n / rw_n: the
 // neuron's row); returns the slots done.
 template <bool WT = false>
 __device__ __forceinline__ uint32_t row_gsop(uint2 (&W)[4], uint32_t hitb, uint32_t slowb,
@@ -1059,7 +1110,7 @@ __device__ __forceinline__ uint32_t row_gsop(uint2 (&W)[4], uint32_t hitb, uint3
                                              const BurstHeads8* heads, const uint2* mask2, uint32_t A,
                                              const VariantParameters& p, uint8_t flags, int32_t dopamine,
                                              ShardCtl* ctl, uint32_t* fix, uint32_t fix_cap, uint32_t n,
-                                             const ColWT& wt = ColWT{}) {
+                                             uint32_t& same, const ColWT& wt = ColWT{}) {
   uint32_t gdone = 0;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
@@ -1096,7 +1147,10 @@ __device__ __forceinline__ uint32_t row_gsop(uint2 (&W)[4], uint32_t hitb, uint3
       }
       set_half(wj, i, nw);
     }
-    if (wj.x != W[j].x || wj.y != W[j].y) {
+    same += 0x10000u;   // visited, and (low half) left as they were
+    if (wj.x == W[j].x && wj.y == W[j].y) {
+      same++;
+    } else {
       *reinterpret_cast<uint2*>(rw_n + q0) = wj;
       if (WT) {
 #pragma unroll
@@ -1157,7 +1211,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
                   const uint32_t* __restrict__ eval, uint32_t* __restrict__ pend, uint32_t* __restrict__ fix,
                   ShardCtl* __restrict__ ctl, uint32_t k, uint32_t fix_cap, const uint32_t* __restrict__ lit_bits,
                   const LearnCtl* __restrict__ lc, uint32_t* __restrict__ gs_n, uint32_t* __restrict__ gd_n,
-                  const uint8_t* __restrict__ lfz, uint32_t* __restrict__ wcnt, ColWT wt) {
+                  const uint8_t* __restrict__ lfz, uint32_t* __restrict__ wcnt, ColWT wt, uint32_t index) {
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
@@ -1165,8 +1219,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   extern __shared__ __align__(128) uint32_t s_lit[];
   chain_wait();
   chain_open();
-  if (lc && lc->mode == 1u && !lc->overflow) return;   // learned engine: this tick runs sparse
-  if (INLINE && lsum_tick(ctl, k)) return;              // k_rows_update_lsum runs this tick
+  if (tick_form(ctl, k, lc, index) != kFormDense) return;                    // k_rows_update_lsum or the learned engine's kernels run this tick
   if (LIT && threadIdx.x == 0) mbar_init(&s_bar, 1);
   lut_to_smem(lut);
   if (threadIdx.x == 0) s_pmax = lut_pmax();
@@ -1179,7 +1232,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
     __syncthreads();
   }
   const uint32_t tick = ctl->tick_base + k;
-  const uint32_t ecount = ctl->eval_count[k & 1];
+  const uint32_t ecount = ctl->eval_act[k & 1][0];
   const uint32_t smax = ctl->row_smax;   // longest row of the shard: rows are loaded up to here
   const RowShape sh = row_shape(smax);
   const uint32_t seg_hi = min(ctl->seg_max, 30u);   // lit bits cover segments 1..seg_hi
@@ -1191,6 +1244,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   const uint32_t beg = min(wid * per_warp, ecount), end = min(beg + per_warp, ecount);
   uint32_t ev_slots = 0, hits = 0, nspk = 0, gdone = 0, nev = 0, err = 0;
   uint32_t wc = 0, wd = 0;   // spikers this warp listed for the GSOP passes
+  uint32_t same = 0;         // row_gsop
   bool lit_on = true;
   if (LIT) {
     lit_on = mbar_wait_bounded(&s_bar, 0, g_first_wait_limit);
@@ -1255,7 +1309,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
         // of its row; frozen slots (GSOP leaves them as they are) are counted
         if (spike && lf > 0u)
           gdone += row_gsop<WT>(W, hitb, slowb, lf, g8, sh, gtab, var, rt_n, rw_n, P.axon_heads, mask2, A, p,
-                                flags, dopamine, ctl, fix, fix_cap, n, wt);
+                                flags, dopamine, ctl, fix, fix_cap, n, same, wt);
         if (spike && g8 == 0) gdone += c - lf;
         continue;
       }
@@ -1283,6 +1337,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   if (err_any && lane == 0) atomicOr(&ctl->err, err_any);
   block_count(ev_slots, hits, nspk, &ctl->ctr[1]);
   block_count(gdone, nev, 0, &ctl->ctr[4]);
+  if (INLINE) block_count(same & 0xFFFFu, same >> 16, 0, ctl->gsop_same);
 }
 
 // Sums six per-thread counters over a 256-thread block into ctr[1..5] and
@@ -1330,6 +1385,340 @@ __device__ __forceinline__ bool slot_hit(uint32_t t, bool exact, bool gfast, uin
   return hit;
 }
 
+// GSOP (physics.cu:281-373) of row position q of spiker n, weight w16, target
+// *t: the rank's delta where the hit decides (fast), else the exact path or the
+// fix-up list.  Returns the slots done (0: an invalid target).
+template <bool WT>
+__device__ __forceinline__ uint32_t gsop_slot(int16_t w16, const uint32_t* t, int16_t* w, bool hit, bool fast,
+                                              const int2* gtab_v, const BurstHeads8* heads, const uint2* mask2,
+                                              uint32_t A, const VariantParameters& p, uint8_t flags, int32_t dopamine,
+                                              ShardCtl* ctl, uint32_t* fix, uint32_t fix_cap, uint32_t n, uint32_t q,
+                                              const ColWT& wt) {
+  int16_t nw = w16;
+  if (fast) {
+    const int32_t aw = w16 < 0 ? -(int32_t)w16 : (int32_t)w16;
+    const int2 e = gtab_v[min((uint32_t)aw >> 11, 15u)];
+    int32_t na = aw + (hit ? e.x : -e.y);
+    na = min(max(na, 0), 32767);
+    nw = (int16_t)(w16 < 0 ? -na : na);
+  } else {
+    const uint32_t tt = *t;
+    const int r = gsop_general(heads, mask2, A, (tt & AXC_TARGET_AXON_MASK) - 1u, tt >> AXC_TARGET_SEG_SHIFT, p, flags,
+                               dopamine, &nw);
+    if (r == 2) return 0u;
+    if (r == 1) {
+      const uint32_t slot = atomicAdd(&ctl->fix_count, 1u);
+      if (slot < fix_cap) fix[slot] = (uint32_t)((size_t)n * kRowStride + q);
+      else ctl->fix_overflow = 1u;
+      return 1u;
+    }
+  }
+  if (nw != w16) {
+    *w = nw;
+    if (WT) col_write(wt, n, q, nw);
+  }
+  return 1u;
+}
+
+// ---------------------------------------------------------------------------
+// Sparse form of a tick (tick_form: few axons carry a head on the segments the
+// batch's slots use).  The dendrite sum is a wrapping i32 sum, so it may be
+// taken from the axons' side in any order:
+//   k_sparse_hits    a warp per 64 axons: for every
+//                    run of hit segments of an active axon, the entries of the
+//                    inverted index (RowIndex: one segment's together) are
+//                    spread over the lanes; each adds its slot's weight into
+//                    the neuron's acc with an integer atomic
+//   k_sparse_neurons GLIF from acc, GSOP of the spikers' movable slots
+// At 1.5M quiet neurons (12 % of the axons active, 1 % of the slots hit) the
+// dense pass spends its 719 us a tick on 150M mask gathers; the sparse form
+// touches the 1.5M hits.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kSegUnsorted = 0xFFFFu;
+constexpr int kHitUnroll = 4;
+
+// The lane that owns item `it` of a warp whose lanes hold consecutive ranges of
+// items: the first whose inclusive prefix sum incl exceeds it (31 past the end).
+__device__ __forceinline__ uint32_t lane_of_item(uint32_t incl, uint32_t it) {
+  uint32_t owner = 0;
+#pragma unroll
+  for (int stp = 16; stp > 0; stp >>= 1) {
+    const uint32_t v = __shfl_sync(kFull, incl, owner + stp - 1);
+    if (v <= it) owner += stp;
+  }
+  return min(owner, 31u);
+}
+
+__device__ __forceinline__ uint32_t warp_incl(uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  return x;
+}
+
+__global__ void __launch_bounds__(256, 6)
+    k_sparse_hits(ShardVramPtrs P, uint32_t A, const uint32_t* __restrict__ rt, const int16_t* __restrict__ rw,
+                  const uint2* __restrict__ mask2, const uint32_t* __restrict__ live, const uint32_t* __restrict__ evb,
+                  int32_t* __restrict__ acc, ShardCtl* __restrict__ ctl, uint32_t k, const LearnCtl* __restrict__ lc) {
+  if (tick_form(ctl, k, lc, 1u) != kFormSparse) return;
+  const uint32_t* __restrict__ off = ctl->ix_off;
+  const uint16_t* __restrict__ seg = ctl->ix_seg;
+  const uint32_t* __restrict__ ent = ctl->ix_ent;
+  const bool mixed = ctl->mixed_len != 0u;
+  const uint32_t pmax = ctl->pmax, seg_max = ctl->seg_max;
+  const uint32_t act = seg_max >= 31u ? 0xFFFFFFFFu : ((2u << seg_max) - 1u);
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t groups = (A + 63) / 64;
+  uint32_t hits = 0;
+  for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < groups; g += nwarps) {
+    const uint32_t a0 = 64u * g + 2u * lane;   // this lane's two axons
+    const uint32_t lw = live[2u * g + (lane >> 4)] >> (2u * (lane & 15u));
+    const bool on0 = (lw & 1u) && a0 < A, on1 = (lw & 2u) && a0 + 1u < A;
+    uint32_t h0 = 0, h1 = 0;   // hit segments not taken yet (bit 31: "may hit", segments >= 31)
+    if (on0) { const uint2 m = __ldg(mask2 + a0); h0 = (m.x | (m.y & 0x7FFFFFFFu)) & act; }
+    if (on1) { const uint2 m = __ldg(mask2 + a0 + 1u); h1 = (m.x | (m.y & 0x7FFFFFFFu)) & act; }
+    uint32_t o0 = 0, o1 = 0, d0 = 0, d1 = 0;   // first entry and entries of the axon
+    if (on0) { o0 = __ldg(off + a0); d0 = __ldg(off + a0 + 1u) - o0; }
+    if (on1) { o1 = __ldg(off + a0 + 1u); d1 = __ldg(off + a0 + 2u) - o1; }
+    while (__any_sync(kFull, h0 | h1)) {
+      // each lane's lowest run of hit segments [s0, s1]
+      uint32_t first = 0, count = 0, ax = a0;
+      bool test = false;   // the entries' segments are not known to be hit
+      if (h0 | h1) {
+        const bool second = h0 == 0u;
+        uint32_t h = second ? h1 : h0;
+        ax = a0 + (second ? 1u : 0u);
+        const uint32_t o = second ? o1 : o0, d = second ? d1 : d0;
+        const uint16_t* sg = seg + (size_t)ax * 32u;
+        if (__ldg(sg) == kSegUnsorted) {
+          first = o;
+          count = d;
+          test = true;
+          h = 0;
+        } else {
+          const uint32_t s0 = (uint32_t)__ffs(h) - 1u;
+          const uint32_t run = h >> s0;
+          // segment 31's bucket ("may hit") is taken alone: its entries are tested
+          const uint32_t len = s0 == 31u ? 1u : min((uint32_t)__ffs(~run) - 1u, 31u - s0);
+          const uint32_t s1 = s0 + len;   // one past the run
+          const uint32_t e0 = __ldg(sg + s0), e1 = s1 < 32u ? (uint32_t)__ldg(sg + s1) : d;
+          first = o + e0;
+          count = e1 - e0;
+          test = s0 == 31u;
+          h &= s1 < 32u ? (0xFFFFFFFFu << s1) : 0u;
+        }
+        if (second) h1 = h; else h0 = h;
+      }
+      const uint32_t incl = warp_incl(count);
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      const uint32_t base = first - (incl - count);
+      const bool any_test = mixed || __any_sync(kFull, test);
+      // 32 x kHitUnroll entries a step: every load of a step is issued before
+      // anything waits (entry -> weight is a chain of two cache misses)
+      for (uint32_t it0 = 0; it0 < total; it0 += 32u * kHitUnroll) {
+        uint32_t r[kHitUnroll], own[kHitUnroll];
+#pragma unroll
+        for (int u = 0; u < kHitUnroll; u++) {
+          const uint32_t it = it0 + 32u * u + lane;
+          own[u] = lane_of_item(incl, it);
+          const uint32_t b = __shfl_sync(kFull, base, own[u]);
+          r[u] = it < total ? __ldg(ent + b + it) : 0xFFFFFFFFu;
+        }
+        int32_t w[kHitUnroll];
+        bool on[kHitUnroll];
+#pragma unroll
+        for (int u = 0; u < kHitUnroll; u++) {
+          w[u] = 0;
+          on[u] = false;
+          if (r[u] != 0xFFFFFFFFu) {
+            const uint32_t n = r[u] / kRowStride;
+            w[u] = rw[r[u]];
+            on[u] = (__ldg(evb + (n >> 5)) >> (n & 31u)) & 1u;   // else refractory
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kHitUnroll; u++) {
+          if (any_test) {   // warp-uniform
+            const uint32_t a = __shfl_sync(kFull, ax, own[u]);
+            const bool tst = __shfl_sync(kFull, test ? 1u : 0u, own[u]) != 0u;
+            if (on[u] && (tst || mixed)) {
+              const uint32_t prop = VARIANT_LUT[P.soma_flags[r[u] / kRowStride] >> 4].signal_propagation_length;
+              if (tst || prop != pmax)
+                on[u] = hit_exact(P.axon_heads, A, a, rt[r[u]] >> AXC_TARGET_SEG_SHIFT, prop);
+            }
+          }
+          if (on[u]) {
+            atomicAdd(acc + r[u] / kRowStride, w[u]);
+            hits++;
+          }
+        }
+      }
+    }
+  }
+  block_count(0, hits, 0, &ctl->ctr[1]);
+}
+
+// ---------------------------------------------------------------------------
+// The sparse form's neurons: a warp per 128 consecutive ones, a lane for four
+// (16-byte loads of voltage, threshold and acc; which are evaluated comes from
+// the prologue's bits, so no list is read: nearly all are).  GLIF from acc
+// (physics.cu:209-275), then GSOP of the spikers' movable slots
+// (physics.cu:281-373) from the gtab deltas, on the exact path or deferred to
+// the fix-up stage, spread over the warp's lanes.  14 us at 393k neurons in a
+// quiet brain.
+// ---------------------------------------------------------------------------
+constexpr int kNeuronBlocks = 5;   // resident 256-thread blocks per SM (48 registers a thread)
+
+// Item `it` of the warp's rows: its neuron (of the warp's 128), row position q
+// and the neuron's flags; incl: the lanes' inclusive item counts, per: a lane's
+// four counts, a byte each.
+__device__ __forceinline__ uint32_t row_item(uint32_t incl, uint32_t per, uint32_t fl4, uint32_t it, uint32_t* q,
+                                             uint8_t* flags) {
+  const uint32_t own = lane_of_item(incl, it);
+  const uint32_t c = __shfl_sync(kFull, per, own), f = __shfl_sync(kFull, fl4, own);
+  const uint32_t lane_end = __shfl_sync(kFull, incl, own);
+  const uint32_t c0 = c & 0xFFu, c1 = c0 + ((c >> 8) & 0xFFu), c2 = c1 + ((c >> 16) & 0xFFu), c3 = c2 + (c >> 24);
+  const uint32_t x = it - (lane_end - c3);
+  const uint32_t j = (x >= c0 ? 1u : 0u) + (x >= c1 ? 1u : 0u) + (x >= c2 ? 1u : 0u);
+  *q = x - (j == 0u ? 0u : j == 1u ? c0 : j == 2u ? c1 : c2);
+  *flags = (uint8_t)(f >> (8u * j));
+  return 4u * own + j;
+}
+
+__global__ void __launch_bounds__(256, kNeuronBlocks)
+    k_sparse_neurons(ShardVramPtrs P, uint32_t N, uint32_t A, const uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
+                     const uint16_t* __restrict__ cnt, const uint8_t* __restrict__ lfz,
+                     const uint2* __restrict__ mask2, const uint32_t* __restrict__ evb, uint32_t* __restrict__ pend,
+                     uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl, uint32_t k, uint32_t fix_cap,
+                     const uint32_t* __restrict__ lit_bits, const LearnCtl* __restrict__ lc,
+                     int32_t* __restrict__ acc) {
+  if (tick_form(ctl, k, lc, 1u) != kFormSparse) return;
+  const uint32_t tiles = (N + 127u) / 128u;
+  if (blockIdx.x * 8u >= tiles) return;   // no neuron for this block: no table to build
+  __shared__ VariantParameters lut[16];
+  __shared__ int2 gtab[16][16];
+  lut_to_smem(lut);
+  const uint32_t pmax = ctl->pmax;
+  __syncthreads();
+  const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
+  build_gtab(gtab, lut, dopamine);
+  __syncthreads();
+  const uint32_t tick = ctl->tick_base + k;
+  const uint32_t seg_hi = min(ctl->seg_max, 30u);
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // 16-byte loads where the shard's arrays allow (padded_n a multiple of 16 puts
+  // them on 16-byte boundaries of an aligned blob); else a load a neuron
+  const bool vec = ((reinterpret_cast<uintptr_t>(P.soma_voltage) | reinterpret_cast<uintptr_t>(P.threshold_offset)) &
+                    15u) == 0u &&
+                   (reinterpret_cast<uintptr_t>(P.soma_flags) & 3u) == 0u;
+  uint32_t ev_slots = 0, nspk = 0, gdone = 0, nev = 0, err = 0;
+  for (uint32_t tile = blockIdx.x * 8u + wid; tile < tiles; tile += gridDim.x * 8u) {
+    const uint32_t n0 = tile * 128u, nb = n0 + 4u * lane;
+    const uint32_t ev = nb < N ? (evb[nb >> 5] >> (nb & 31u)) & 15u : 0u;
+    const bool full = vec && nb + 4u <= N;
+    int32_t v[4] = {0, 0, 0, 0}, thr[4] = {0, 0, 0, 0}, cur[4] = {0, 0, 0, 0};
+    uint32_t cw[4] = {0, 0, 0, 0}, fl4 = 0;
+    uint32_t moves = 0;   // movable slots of the spikers, a byte each
+    if (ev) {
+      if (full) {
+        const int4 a = *reinterpret_cast<const int4*>(P.soma_voltage + nb);
+        const int4 b = *reinterpret_cast<const int4*>(P.threshold_offset + nb);
+        const int4 c = *reinterpret_cast<const int4*>(acc + nb);
+        const uint2 d = __ldg(reinterpret_cast<const uint2*>(cnt + nb));
+        fl4 = *reinterpret_cast<const uint32_t*>(P.soma_flags + nb);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        thr[0] = b.x; thr[1] = b.y; thr[2] = b.z; thr[3] = b.w;
+        cur[0] = c.x; cur[1] = c.y; cur[2] = c.z; cur[3] = c.w;
+        cw[0] = d.x & 0xFFFFu; cw[1] = d.x >> 16; cw[2] = d.y & 0xFFFFu; cw[3] = d.y >> 16;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const uint32_t n = nb + j;
+          if (n >= N) continue;
+          v[j] = P.soma_voltage[n];
+          thr[j] = P.threshold_offset[n];
+          fl4 |= (uint32_t)P.soma_flags[n] << (8 * j);
+          cw[j] = cnt[n];
+          cur[j] = acc[n];
+        }
+      }
+      uint32_t nf = fl4;
+      bool vch = false, tch = false;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (!((ev >> j) & 1u)) continue;
+        const uint32_t n = nb + j, flags = (fl4 >> (8 * j)) & 0xFFu, c = cw[j] & 0xFFu;
+        const VariantParameters& p = lut[flags >> 4];
+        const GlifOut o = glif_step(p, v[j], thr[j], cur[j], tick, n);
+        vch |= o.v != v[j];
+        tch |= o.thr != thr[j];
+        v[j] = o.v;
+        thr[j] = o.thr;
+        nf = (nf & ~(0xFFu << (8 * j))) | (((flags & 0xF0u) | (o.spike ? 0x05u : 0u)) << (8 * j));
+        if (o.glif) P.timers[n] = p.refractory_period;   // an evaluated neuron's timer is 0
+        ev_slots += c;
+        nev++;
+        if (cw[j] & kRowBad) err |= AXC_ERR_TARGET_RANGE;
+        if (o.spike) {
+          const uint32_t lf = lfz[n], a = P.soma_to_axon[n];
+          nspk++;
+          gdone += c - lf;   // frozen slots: GSOP leaves them as they are
+          moves |= lf << (8 * j);
+          if (a < A) atomicAdd(&pend[a], 1u);
+          else if (a != AXC_NO_AXON) err |= AXC_ERR_SOMA_AXON;
+        }
+      }
+      if (full) {
+        if (vch) *reinterpret_cast<int4*>(P.soma_voltage + nb) = make_int4(v[0], v[1], v[2], v[3]);
+        if (tch) *reinterpret_cast<int4*>(P.threshold_offset + nb) = make_int4(thr[0], thr[1], thr[2], thr[3]);
+        if (nf != fl4) *reinterpret_cast<uint32_t*>(P.soma_flags + nb) = nf;
+        if (cur[0] | cur[1] | cur[2] | cur[3]) *reinterpret_cast<int4*>(acc + nb) = make_int4(0, 0, 0, 0);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (!((ev >> j) & 1u)) continue;
+          P.soma_voltage[nb + j] = v[j];
+          P.threshold_offset[nb + j] = thr[j];
+          P.soma_flags[nb + j] = (uint8_t)(nf >> (8 * j));
+          acc[nb + j] = 0;
+        }
+      }
+    }
+    // GSOP of the spikers' movable slots
+    const uint32_t msum = (moves & 0xFFu) + ((moves >> 8) & 0xFFu) + ((moves >> 16) & 0xFFu) + (moves >> 24);
+    if (__any_sync(kFull, msum)) {
+      const uint32_t incl = warp_incl(msum);
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      for (uint32_t it0 = 0; it0 < total; it0 += 32) {
+        const uint32_t it = it0 + lane;
+        uint32_t q;
+        uint8_t f;
+        const uint32_t i = row_item(incl, moves, fl4, it, &q, &f);
+        if (it >= total) continue;
+        const uint32_t n = n0 + i;
+        const uint32_t* t = rt + (size_t)n * kRowStride + q;
+        int16_t* w = rw + (size_t)n * kRowStride + q;
+        const int16_t w16 = *w;
+        const VariantParameters& p = lut[f >> 4];
+        const uint32_t prop = p.signal_propagation_length;
+        const bool exact = prop == pmax;
+        bool fast;
+        const bool hit = slot_hit(__ldg(t), exact, exact && prop <= 16u, prop, seg_hi, lit_bits, mask2, P.axon_heads, A,
+                                  &fast);
+        gdone += gsop_slot<false>(w16, t, w, hit, fast, gtab[f >> 4], P.axon_heads, mask2, A, p, f, dopamine, ctl, fix,
+                                  fix_cap, n, q, ColWT{});
+      }
+    }
+  }
+  const uint32_t err_any = __reduce_or_sync(kFull, err);
+  if (err_any && lane == 0) atomicOr(&ctl->err, err_any);
+  block_count256(ev_slots, 0, nspk, gdone, nev, 0, ctl->ctr);
+}
+
 // ---------------------------------------------------------------------------
 // per tick 2/4, lit-sum form (lsum_tick: short tested prefixes, and every axon
 // the row layout took as fully lit is fully lit): a thread per evaluated
@@ -1356,10 +1745,9 @@ __global__ void __launch_bounds__(256, kLsumBlocks) k_rows_update_lsum(ShardVram
                                                           const LearnCtl* __restrict__ lc) {
   chain_wait();
   chain_open();
-  if (lc && lc->mode == 1u && !lc->overflow) return;   // learned engine: this tick runs sparse
-  if (!lsum_tick(ctl, k)) return;
+  if (tick_form(ctl, k, lc, 0u) != kFormLitSum) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ctr[6] += 1;   // ticks on the lit-sum form
-  const uint32_t ecount = ctl->eval_count[k & 1];
+  const uint32_t ecount = ctl->eval_act[k & 1][0];
   if (blockIdx.x * blockDim.x >= ecount) return;   // no neuron for this block: no table to build
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
@@ -1439,31 +1827,8 @@ __global__ void __launch_bounds__(256, kLsumBlocks) k_rows_update_lsum(ShardVram
       } else {
         hit = slot_hit(rt_n[q], exact, gfast, prop, seg_hi, lit_bits, mask2, P.axon_heads, A, &fast);
       }
-      int16_t nw = w16;
-      if (fast) {
-        const int32_t aw = w16 < 0 ? -(int32_t)w16 : (int32_t)w16;
-        const int2 e = gtab[var][min((uint32_t)aw >> 11, 15u)];
-        int32_t na = aw + (hit ? e.x : -e.y);
-        na = min(max(na, 0), 32767);
-        nw = (int16_t)(w16 < 0 ? -na : na);
-        gdone++;
-      } else {
-        const uint32_t t = rt_n[q];
-        const int r = gsop_general(P.axon_heads, mask2, A, (t & AXC_TARGET_AXON_MASK) - 1u, t >> AXC_TARGET_SEG_SHIFT,
-                                   p, flags, dopamine, &nw);
-        if (r == 2) continue;
-        gdone++;
-        if (r == 1) {
-          const uint32_t slot = atomicAdd(&ctl->fix_count, 1u);
-          if (slot < fix_cap) fix[slot] = (uint32_t)((size_t)n * kRowStride + q);
-          else ctl->fix_overflow = 1u;
-          continue;
-        }
-      }
-      if (nw != w16) {
-        rw_n[q] = nw;
-        if (WT) col_write(wt, n, q, nw);
-      }
+      gdone += gsop_slot<WT>(w16, rt_n + q, rw_n + q, hit, fast, gtab[var], P.axon_heads, mask2, A, p, flags, dopamine,
+                             ctl, fix, fix_cap, n, q, wt);
     }
   }
   const uint32_t err_any = __reduce_or_sync(kFull, err);
@@ -1491,7 +1856,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop(ShardVramPtrs P, uint32_t A, 
                                                    uint32_t fix_cap, const LearnCtl* __restrict__ lc) {
   // the learned engine lists the spikers of its sparse ticks here; on its dense
   // ticks the update pass applied GSOP itself
-  if (lc && !(lc->mode == 1u && !lc->overflow)) return;
+  if (lc && tick_form(ctl, k, lc, 1u) != kFormScatter) return;
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
@@ -1501,7 +1866,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop(ShardVramPtrs P, uint32_t A, 
   const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
   build_gtab(gtab, lut, dopamine);
   __syncthreads();
-  const uint32_t ecount = ctl->eval_count[k & 1];
+  const uint32_t ecount = ctl->eval_act[k & 1][0];
   const uint32_t per_warp = (((ecount + nwu - 1) / nwu) + 3) & ~3u;
   const uint32_t seg_hi = min(ctl->seg_max, 30u);
   const uint32_t lane = threadIdx.x & 31;
@@ -1605,7 +1970,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop_rows(ShardVramPtrs P, uint32_
                                                         const uint32_t* __restrict__ wcnt, uint32_t nwu,
                                                         uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl,
                                                         uint32_t k, uint32_t fix_cap, const LearnCtl* __restrict__ lc) {
-  if (lc && !(lc->mode == 1u && !lc->overflow)) return;   // as k_rows_gsop
+  if (lc && tick_form(ctl, k, lc, 1u) != kFormScatter) return;   // as k_rows_gsop
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
@@ -1615,7 +1980,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop_rows(ShardVramPtrs P, uint32_
   const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
   build_gtab(gtab, lut, dopamine);
   __syncthreads();
-  const uint32_t ecount = ctl->eval_count[k & 1];
+  const uint32_t ecount = ctl->eval_act[k & 1][0];
   const uint32_t per_warp = (((ecount + nwu - 1) / nwu) + 3) & ~3u;
   const uint32_t smax = ctl->row_smax;
   const RowShape sh = row_shape(smax);
@@ -1623,6 +1988,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop_rows(ShardVramPtrs P, uint32_
   const uint32_t lane = threadIdx.x & 31, g8 = lane & 7, grp = lane >> 3;
   const uint32_t ngw = (gridDim.x * blockDim.x) >> 5;
   unsigned long long gdone = 0;
+  uint32_t same = 0;
   for (uint32_t uw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; uw < nwu; uw += ngw) {
     const uint32_t cntw = wcnt[uw];
     const uint32_t beg = min(uw * per_warp, ecount);
@@ -1646,7 +2012,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop_rows(ShardVramPtrs P, uint32_
                            slowb);
       if (valid)
         gdone += row_gsop(W, hitb, slowb, c, g8, sh, gtab, var, rt_n, rw_n, P.axon_heads, mask2, A, p, flags,
-                          dopamine, ctl, fix, fix_cap, n);
+                          dopamine, ctl, fix, fix_cap, n, same);
     }
   }
   block_count(gdone, 0, 0, &ctl->ctr[4]);
@@ -1678,6 +2044,10 @@ __device__ __forceinline__ void fixup_slot(const ShardVramPtrs& P, const Variant
   }
 }
 
+// Sparse-form ticks in a row before the index is asked for: building it costs
+// what the dense pass loses to the sparse form in ~20 ticks (1.5M neurons).
+constexpr uint32_t kIndexStreak = 16;
+
 __global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N, uint32_t A,
                                                     const uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
                                                     const uint16_t* __restrict__ cnt,
@@ -1685,7 +2055,8 @@ __global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N,
                                                     const uint32_t* __restrict__ eval,
                                                     const uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl,
                                                     uint32_t k, const uint32_t* __restrict__ ids,
-                                                    uint8_t* __restrict__ out, uint32_t num_outputs, ColWT wt) {
+                                                    uint8_t* __restrict__ out, uint32_t num_outputs, ColWT wt,
+                                                    volatile uint32_t* wish) {
   chain_wait();
   chain_open();
   const uint32_t nfix = ctl->fix_count;
@@ -1694,8 +2065,14 @@ __global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N,
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid == 0) {
-      ctl->eval_count[(k + 1) & 1] = 0;   // the next tick's list (last used two ticks ago)
+      ctl->eval_act[(k + 1) & 1][0] = ctl->eval_act[(k + 1) & 1][1] = 0;   // the next tick's (last used two ticks ago)
       ctl->dense[(k + 1) & 1] = 0;
+      // ticks in a row that the sparse form would take: ask for its index
+      if (wish) {
+        const uint32_t streak = !lsum_tick(ctl, k) && sparse_tick(ctl, k) ? ctl->streak + 1u : 0u;
+        ctl->streak = streak;
+        if (!index_ok(ctl) && streak >= kIndexStreak) *wish = 1u;
+      }
     }
     // readout of the tick (physics.cu:378-395): flags are final once the update pass is done
     uint32_t err = 0;
@@ -1724,7 +2101,7 @@ __global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N,
     return;
   }
   // the list overflowed: rescan every spiker's slots with the update pass's rule
-  const uint32_t ecount = ctl->eval_count[k & 1];
+  const uint32_t ecount = ctl->eval_act[k & 1][0];
   for (uint32_t w = tid; w < ecount * kRowStride; w += stride) {
     const uint32_t n = eval[w / kRowStride], q = w % kRowStride;
     if (!(P.soma_flags[n] & 1) || q >= (cnt[n] & 0xFFu)) continue;
@@ -1758,11 +2135,11 @@ __global__ void __launch_bounds__(256) k_rows_push(BurstHeads8* __restrict__ hea
                                                    ShardCtl* __restrict__ ctl, uint32_t k) {
   chain_wait();
   chain_open();
-  const uint32_t ecount = ctl->eval_count[k & 1];
+  const uint32_t ecount = ctl->eval_act[k & 1][0];
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid == 0) {
-    ctl->eval_count[(k + 1) & 1] = 0;
+    ctl->eval_act[(k + 1) & 1][0] = ctl->eval_act[(k + 1) & 1][1] = 0;
     ctl->dense[(k + 1) & 1] = 0;
     ctl->fix_count = 0;
     ctl->fix_overflow = 0;
@@ -1795,8 +2172,8 @@ __global__ void __launch_bounds__(256) k_rows_push(BurstHeads8* __restrict__ hea
 }
 
 __global__ void k_rows_reset_lists(ShardCtl* ctl) {
-  ctl->eval_count[0] = 0;
-  ctl->eval_count[1] = 0;
+  ctl->eval_act[0][0] = ctl->eval_act[0][1] = 0;
+  ctl->eval_act[1][0] = ctl->eval_act[1][1] = 0;
   ctl->fix_count = 0;
   ctl->fix_overflow = 0;
   ctl->dense[0] = 0;
@@ -1823,7 +2200,9 @@ __device__ __forceinline__ void push_few(uint32_t h[8], uint32_t c) {
   }
 }
 
-template <int ITEMS>
+// INDEX: also the live axons' and evaluated neurons' bits and the active axons'
+// count, for the sparse form (the learned engine's plain graph).
+template <int ITEMS, bool INDEX>
 __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __restrict__ heads, uint32_t A,
                                                              uint32_t v_seg, const uint32_t* __restrict__ bitmask,
                                                              uint32_t voff, uint32_t nv,
@@ -1837,9 +2216,12 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
                                                              uint32_t raise_err, uint32_t* __restrict__ lit_bits,
                                                              uint32_t* __restrict__ pend_apply, uint32_t inc_direct,
                                                              uint32_t set_tick, uint32_t tick_base, int32_t dopamine,
-                                                             const uint32_t* __restrict__ xlit) {
+                                                             const uint32_t* __restrict__ xlit,
+                                                             uint32_t* __restrict__ live,
+                                                             uint32_t* __restrict__ evb) {
   __shared__ uint32_t s_base;
-  __shared__ uint32_t s_warp[ITEMS][8];
+  __shared__ uint32_t s_warp[ITEMS][8];   // evaluated neurons | active axons << 16
+
   chain_wait();
   chain_open();
   const uint32_t i0 = blockIdx.x * (256u * ITEMS) + threadIdx.x;
@@ -1887,12 +2269,14 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
   }
   const uint32_t hi = min(seg_max, 30u);   // segments 1..hi are the ones the batch's slots use
   const uint32_t need = hi ? (((2u << hi) - 1u) & ~1u) : 0xFFFFFFFFu;
+  // segments the batch's slots use: 0..seg_max (bit 31: any segment >= 31)
+  const uint32_t act = seg_max >= 31u ? 0xFFFFFFFFu : ((2u << seg_max) - 1u);
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t evb[ITEMS];
+  uint32_t ebal[ITEMS];
 #pragma unroll
   for (int r = 0; r < ITEMS; r++) {
     const uint32_t i = i0 + 256u * r;
-    bool lit = false;
+    bool lit = false, on = false;
     if (i < A) {
       uint32_t c = npush[r];
       if (pend_apply && c) pend_apply[i] = 0;
@@ -1914,10 +2298,12 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
       // most one soma owns the axon (for those segments the hit is 1 and one
       // push cannot change it)
       lit = (m.x & need) == need && !(m.y >> 31);
+      if (INDEX) on = ((m.x | (m.y & 0x7FFFFFFFu)) & act) != 0u;
     }
-    const uint32_t lb = __ballot_sync(kFull, lit);
+    const uint32_t lb = __ballot_sync(kFull, lit), onb = INDEX ? __ballot_sync(kFull, on) : 0u;
     if (lane == 0 && i < A) {
       lit_bits[i >> 5] = lb;
+      if (INDEX) live[i >> 5] = onb;
       // an axon the row layout summed as fully lit is not: this tick takes the full pass
       if (xw[r] & ~lb) atomicOr(&ctl->dense[k & 1], 1u);
     }
@@ -1930,24 +2316,30 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
         ev = true;
       }
     }
-    evb[r] = __ballot_sync(kFull, ev);
-    if (lane == 0) s_warp[r][w] = __popc(evb[r]);
+    ebal[r] = __ballot_sync(kFull, ev);
+    if (lane == 0) {
+      if (INDEX && i < N) evb[i >> 5] = ebal[r];
+      s_warp[r][w] = __popc(ebal[r]) | (INDEX ? __popc(onb) << 16 : 0);
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t tot = 0;
     for (int q = 0; q < ITEMS * 8; q++) {
       const uint32_t c = (&s_warp[0][0])[q];
-      (&s_warp[0][0])[q] = tot;
+      (&s_warp[0][0])[q] = INDEX ? tot & 0xFFFFu : tot;
       tot += c;
     }
-    s_base = tot ? atomicAdd(&ctl->eval_count[k & 1], tot) : 0u;
+    if (INDEX)
+      s_base = append_count(ctl, k, tot & 0xFFFFu, tot >> 16);
+    else
+      s_base = tot ? atomicAdd(&ctl->eval_act[k & 1][0], tot) : 0u;
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < ITEMS; r++)
-    if ((evb[r] >> lane) & 1u)
-      eval[s_base + s_warp[r][w] + __popc(evb[r] & ((1u << lane) - 1u))] = i0 + 256u * r;
+    if ((ebal[r] >> lane) & 1u)
+      eval[s_base + s_warp[r][w] + __popc(ebal[r] & ((1u << lane) - 1u))] = i0 + 256u * r;
 }
 // Items (an axon and a neuron each) per thread of k_rows_prologue_plain: two
 // halve the blocks, and with them the list-append atomics on one counter and
@@ -1967,6 +2359,13 @@ uint32_t set_first_wait_limit(uint32_t tries) {
   return prev;
 }
 
+cudaError_t rows_wish_alloc(ShardScratch& s) {
+  if (s.h_counts_pinned) return cudaSuccess;
+  const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&s.h_counts_pinned), 64, cudaHostAllocDefault);
+  if (e == cudaSuccess) *s.h_counts_pinned = 0u;
+  return e;
+}
+
 cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, cudaStream_t stream) {
   if (s.rows && s.rows->N >= N && s.rows->A >= A && (s.rows->fix || !with_fix)) return cudaSuccess;
   graph_cache_drop(&s);   // captured graphs hold the old buffers' addresses
@@ -1982,6 +2381,9 @@ cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, c
   const size_t o_eval = off; off = al(off + (size_t)N * 4 + 4);
   const size_t o_fix = off; off = al(off + (with_fix ? (size_t)kFixCap * 4 : 0));
   const size_t o_lit = off; off = al(off + ((size_t)std::max(A, N) / 32 + 2) * 4 + 16);
+  const size_t o_live = off; off = al(off + ((size_t)A / 64 + 1) * 8);
+  const size_t o_evb = off; off = al(off + ((size_t)N / 32 + 1) * 4);
+  const size_t o_acc = off; off = al(off + (size_t)N * 4 + 4);
   const size_t o_gsn = off; off = al(off + (size_t)N * 4 + 4);
   const size_t o_gdn = off; off = al(off + (size_t)N * 4 + 4);
   const size_t o_am = off; off = al(off + (size_t)N * 16 + 16);
@@ -1999,6 +2401,7 @@ cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, c
   // into this shard's first batch)
   e = cudaMemsetAsync(base, 0, off, stream);
   if (e == cudaSuccess && stream == nullptr) e = cudaStreamSynchronize(nullptr);
+  if (e == cudaSuccess) e = cudaMemsetAsync(&s.ctl->idx_ok, 0, 4, stream);   // an index went with the old rows
   if (e != cudaSuccess) { cudaFree(base); return e; }
   RowCache* r = new RowCache();
   char* b = static_cast<char*>(base);
@@ -2013,6 +2416,9 @@ cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, c
   r->eval = reinterpret_cast<uint32_t*>(b + o_eval);
   r->fix = with_fix ? reinterpret_cast<uint32_t*>(b + o_fix) : nullptr;
   r->lit = reinterpret_cast<uint32_t*>(b + o_lit);
+  r->live = reinterpret_cast<uint32_t*>(b + o_live);
+  r->evb = reinterpret_cast<uint32_t*>(b + o_evb);
+  r->acc = reinterpret_cast<int32_t*>(b + o_acc);
   r->gs_n = reinterpret_cast<uint32_t*>(b + o_gsn);
   r->gd_n = reinterpret_cast<uint32_t*>(b + o_gdn);
   r->amask = reinterpret_cast<uint4*>(b + o_am);
@@ -2038,9 +2444,22 @@ cudaError_t rows_posmap(ShardScratch& s, cudaStream_t stream) {
 void rows_free(ShardScratch& s) {
   if (!s.rows) return;
   if (s.rows->posmap) cudaFree(s.rows->posmap);
+  if (s.rows->ix.base) cudaFree(s.rows->ix.base);
   cudaFree(s.rows->base);
   delete s.rows;
   s.rows = nullptr;
+}
+
+namespace {
+__global__ void __launch_bounds__(512) k_rows_decide(ShardCtl* ctl, uint32_t force, uint32_t ticks,
+                                                    const uint32_t* lit, uint32_t A) {
+  layout_decide(ctl, force, ticks, lit, A);
+}
+}  // namespace
+
+cudaError_t launch_rows_decide(ShardScratch& s, uint32_t A, bool force, uint32_t ticks, cudaStream_t stream) {
+  k_rows_decide<<<1, 512, 0, stream>>>(s.ctl, force ? 1u : 0u, ticks, s.rows->lit, A);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_rows_begin(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, cudaStream_t stream,
@@ -2094,7 +2513,7 @@ static bool rows_lit(uint32_t A) { return (size_t)lit_smem_bytes(A) <= lit_smem_
 template <bool INLINE>
 static void launch_rows_update(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, uint32_t k,
                                uint32_t fix_cap, const LearnCtl* lc, cudaStream_t stream, ColWT wt = ColWT{},
-                               bool pdl = false) {
+                               bool pdl = false, bool index = false) {
   RowCache& r = *s.rows;
   const int sms = sm_count();
   const bool lit = rows_lit(A);
@@ -2102,7 +2521,7 @@ static void launch_rows_update(const ShardVramPtrs& v, ShardScratch& s, uint32_t
   const size_t smem = lit ? lit_smem_bytes(A) : 0;
   auto go = [&](auto kern) {
     launch_chain(kern, grid, block, smem, stream, pdl, v, N, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix,
-                 s.ctl, k, fix_cap, r.lit, lc, r.gs_n, r.gd_n, r.lfz, r.wcnt, wt);
+                 s.ctl, k, fix_cap, r.lit, lc, r.gs_n, r.gd_n, r.lfz, r.wcnt, wt, index ? 1u : 0u);
   };
   if constexpr (INLINE) {
     if (wt.w) {   // the per-tick entry point: weight changes written through
@@ -2117,6 +2536,25 @@ static void launch_rows_update(const ShardVramPtrs& v, ShardScratch& s, uint32_t
     go(k_rows_update<true, INLINE>);
   else
     go(k_rows_update<false, INLINE>);
+}
+
+// The lit-sum form's pass.
+static void launch_rows_lsum(const ShardVramPtrs& v, ShardScratch& s, uint32_t A, uint32_t k, uint32_t fix_cap,
+                             const LearnCtl* lc, cudaStream_t stream, ColWT wt = ColWT{}, bool pdl = false) {
+  RowCache& r = *s.rows;
+  launch_chain(wt.w ? k_rows_update_lsum<true> : k_rows_update_lsum<false>, dim3(kLsumBlocks * sm_count()), dim3(256),
+               0, stream, pdl, v, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix, s.ctl, k, fix_cap, r.lit, r.lfz,
+               r.lsum, wt, lc);
+}
+
+// The sparse form (the learned engine's graphs): hits, then neurons, persistent warps.
+static void launch_rows_sparse(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, uint32_t k,
+                               uint32_t fix_cap, const LearnCtl* lc, cudaStream_t stream) {
+  RowCache& r = *s.rows;
+  k_sparse_hits<<<6 * sm_count(), 256, 0, stream>>>(v, A, r.rt, r.rw, r.mask2, r.live, r.evb, r.acc, s.ctl, k, lc);
+  const uint32_t blocks = max(1u, min((N + 1023) / 1024, (uint32_t)(kNeuronBlocks * sm_count())));
+  k_sparse_neurons<<<blocks, 256, 0, stream>>>(v, N, A, r.rt, r.rw, r.cnt, r.lfz, r.mask2, r.evb, s.pend, r.fix, s.ctl,
+                                               k, fix_cap, r.lit, lc, r.acc);
 }
 
 // The GSOP passes over the spikers the tick's update pass listed (32 warps per
@@ -2165,13 +2603,14 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
   const bool pdl = per_tick && ev == nullptr;
   if (G) {
     const bool wide = (G + 255) / 256 >= kProWide;
-    launch_chain(wide ? k_rows_prologue_plain<2> : k_rows_prologue_plain<1>,
+    launch_chain(wide ? (a.index ? k_rows_prologue_plain<2, true> : k_rows_prologue_plain<2, false>)
+                      : (a.index ? k_rows_prologue_plain<1, true> : k_rows_prologue_plain<1, false>),
                  dim3(wide ? (G + 511) / 512 : (G + 255) / 256), dim3(256), 0, stream, false, v.axon_heads, A,
                  a.v_seg, bitmask, a.virtual_offset, a.num_virtual, s.incoming,
                  (have_incoming && !per_tick) ? s.batch_counts : nullptr, a.k, r.mask2, r.mult, v.soma_flags,
                  v.timers, N, r.eval, s.ctl, raise, r.lit, (a.k > 0 && !per_tick) ? s.pend : nullptr,
                  (have_incoming && per_tick) ? 1u : 0u, per_tick ? 1u : 0u, a.tick - a.k, (int32_t)a.dopamine,
-                 r.xlit);
+                 r.xlit, r.live, r.evb);
   }
   if (ev) cudaEventRecord(ev[2], stream);
   ColWT wt{};
@@ -2185,20 +2624,193 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
   // with GSOP; both are launched and each returns at once on the other's
   // ticks), ev[4]..ev[5] fix-up and push.
   const uint32_t fix_cap = min(a.fix_cap, kFixCap);
-  launch_rows_update<true>(v, s, N, A, a.k, fix_cap, nullptr, stream, wt, pdl && G);
+  launch_rows_update<true>(v, s, N, A, a.k, fix_cap, nullptr, stream, wt, pdl && G, a.index);
   if (ev) cudaEventRecord(ev[3], stream);
-  launch_chain(per_tick ? k_rows_update_lsum<true> : k_rows_update_lsum<false>, dim3(kLsumBlocks * sms), dim3(256),
-               0, stream, pdl, v, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix, s.ctl, a.k, fix_cap, r.lit,
-               r.lfz, r.lsum, wt, (const LearnCtl*)nullptr);
+  launch_rows_lsum(v, s, A, a.k, fix_cap, nullptr, stream, wt, pdl);
+  if (a.index) launch_rows_sparse(v, s, N, A, a.k, fix_cap, nullptr, stream);
   if (ev) cudaEventRecord(ev[4], stream);
   const bool readout = a.num_outputs > 0 && a.mapped_soma_ids && a.output_history;
   launch_chain(k_rows_fixup, dim3(2 * sms), dim3(256), 0, stream, pdl, v, N, A, r.rt, r.rw, r.cnt, r.mask2, s.pend,
-               r.eval, r.fix, s.ctl, a.k, a.mapped_soma_ids, a.output_history, readout ? a.num_outputs : 0, wt);
+               r.eval, r.fix, s.ctl, a.k, a.mapped_soma_ids, a.output_history, readout ? a.num_outputs : 0, wt,
+               (volatile uint32_t*)(a.index ? s.h_counts_pinned : nullptr));
   // the soma pushes: by the next tick's prologue within a batch, here on its last tick
   if (!a.defer_push)
     launch_chain(k_rows_push, dim3(8 * sms), dim3(256), 0, stream, pdl, v.axon_heads, v.soma_to_axon, A, s.pend,
                  r.eval, v.soma_flags, N, (const uint32_t*)nullptr, (uint8_t*)nullptr, 0u, s.ctl, a.k);
   if (ev) cudaEventRecord(ev[5], stream);
+  return cudaGetLastError();
+}
+
+// Index of the current rows.  Entries are counted per axon, placed through a
+// cursor (any order), then sorted by segment within the axon, a warp per axon.
+namespace {
+__global__ void __launch_bounds__(256) k_ix_count(const uint32_t* __restrict__ rt, const uint16_t* __restrict__ cnt,
+                                                  uint32_t N, uint32_t A, uint32_t* __restrict__ deg) {
+  const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= (size_t)N * kRowStride) return;
+  const uint32_t n = (uint32_t)(r / kRowStride), q = (uint32_t)(r % kRowStride);
+  if (q >= (cnt[n] & 0xFFu)) return;
+  const uint32_t a = (rt[r] & AXC_TARGET_AXON_MASK) - 1u;
+  if (a < A) atomicAdd(deg + a, 1u);   // invalid targets (redirected to A) never hit
+}
+
+__global__ void __launch_bounds__(256) k_ix_fill(const uint32_t* __restrict__ rt, const uint16_t* __restrict__ cnt,
+                                                 uint32_t N, uint32_t A, uint32_t* __restrict__ cursor,
+                                                 uint32_t* __restrict__ ent) {
+  const size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= (size_t)N * kRowStride) return;
+  const uint32_t n = (uint32_t)(r / kRowStride), q = (uint32_t)(r % kRowStride);
+  if (q >= (cnt[n] & 0xFFu)) return;
+  const uint32_t a = (rt[r] & AXC_TARGET_AXON_MASK) - 1u;
+  if (a < A) ent[atomicAdd(cursor + a, 1u)] = (uint32_t)r;
+}
+
+// Entries of an axon sorted in registers: up to kIxPer a lane.
+constexpr uint32_t kIxPer = 16;
+
+__global__ void __launch_bounds__(256) k_ix_sort(const uint32_t* __restrict__ rt, const uint32_t* __restrict__ off,
+                                                 uint32_t A, uint32_t* __restrict__ ent, uint16_t* __restrict__ seg) {
+  __shared__ uint32_t s_cnt[8][32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t a = blockIdx.x * 8u + w;
+  if (a >= A) return;
+  const uint32_t o = off[a], d = off[a + 1] - o;
+  if (d > 32u * kIxPer) {
+    if (lane == 0) seg[(size_t)a * 32u] = (uint16_t)kSegUnsorted;
+    return;
+  }
+  s_cnt[w][lane] = 0;
+  __syncwarp();
+  uint32_t e[kIxPer], b[kIxPer];   // entry, bucket | rank within the bucket << 8
+#pragma unroll
+  for (uint32_t i = 0; i < kIxPer; i++) {
+    const uint32_t x = lane + 32u * i;
+    b[i] = 0;
+    e[i] = 0;
+    if (x < d) {
+      e[i] = ent[o + x];
+      const uint32_t s = min(__ldg(rt + e[i]) >> AXC_TARGET_SEG_SHIFT, 31u);
+      b[i] = s | (atomicAdd(&s_cnt[w][s], 1u) << 8);
+    }
+  }
+  __syncwarp();
+  const uint32_t mine = s_cnt[w][lane];
+  uint32_t incl = mine;
+#pragma unroll
+  for (int st = 1; st < 32; st <<= 1) {
+    const uint32_t x = __shfl_up_sync(kFull, incl, st);
+    if (lane >= (uint32_t)st) incl += x;
+  }
+  __syncwarp();
+  s_cnt[w][lane] = incl - mine;
+  seg[(size_t)a * 32u + lane] = (uint16_t)(incl - mine);
+  __syncwarp();
+#pragma unroll
+  for (uint32_t i = 0; i < kIxPer; i++)
+    if (lane + 32u * i < d) ent[o + s_cnt[w][b[i] & 0xFFu] + (b[i] >> 8)] = e[i];
+}
+
+// Exclusive scan of in[0..n) (also kept in cur) into out[0..n]: blocks of 4096
+// values, then one block over the block sums, then their addition.
+__global__ void __launch_bounds__(1024) k_ix_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                  uint32_t n, uint32_t* __restrict__ bsum) {
+  __shared__ uint32_t s[32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t base = blockIdx.x * 4096u + threadIdx.x * 4u;
+  uint32_t v[4], t = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[i] = base + i < n ? in[base + i] : 0u;
+    t += v[i];
+  }
+  uint32_t incl = t;
+#pragma unroll
+  for (int st = 1; st < 32; st <<= 1) {
+    const uint32_t x = __shfl_up_sync(kFull, incl, st);
+    if (lane >= (uint32_t)st) incl += x;
+  }
+  if (lane == 31) s[w] = incl;
+  __syncthreads();
+  if (w == 0) {
+    uint32_t x = s[lane];
+#pragma unroll
+    for (int st = 1; st < 32; st <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, x, st);
+      if (lane >= (uint32_t)st) x += y;
+    }
+    s[lane] = x;
+  }
+  __syncthreads();
+  uint32_t run = incl - t + (w ? s[w - 1] : 0u);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    if (base + i < n) out[base + i] = run;
+    run += v[i];
+  }
+  if (threadIdx.x == 1023 && bsum) bsum[blockIdx.x] = run;
+}
+
+__global__ void __launch_bounds__(256) k_ix_add(uint32_t* __restrict__ off, uint32_t* __restrict__ cur, uint32_t n,
+                                                const uint32_t* __restrict__ bsum) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t x = off[i] + bsum[i / 4096u];
+  if (i + 1u == n) off[n] = x + cur[i];
+  off[i] = x;
+  cur[i] = x;
+}
+
+__global__ void k_ix_done(ShardCtl* ctl, RowIndex ix) {
+  ctl->ix_off = ix.off;
+  ctl->ix_seg = ix.seg;
+  ctl->ix_ent = ix.ent;
+  ctl->idx_ok = 1u;
+  ctl->idx_sum = ctl->lay_sum;
+  ctl->lay_now = 0u;   // laid out above: the batch's own layout kernels return at once
+}
+}  // namespace
+
+cudaError_t rows_index_wish(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, cudaStream_t stream,
+                            bool row_sum, bool with_posmap) {
+  volatile uint32_t* wish = s.h_counts_pinned;
+  if (!wish || !*wish || !s.rows || N == 0 || A == 0) return cudaSuccess;
+  *wish = 0u;
+  RowCache& r = *s.rows;
+  // 4096 blocks of 4096 axons in the scan, 32-bit entries
+  if (r.ix_failed || A > (1u << 24) || (size_t)r.N * kRowStride > 0xFFFFFFFFull) return cudaSuccess;
+  RowIndex& ix = r.ix;
+  if (!ix.base) {
+    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    size_t off = 0;
+    const size_t o_off = off; off = al(off + ((size_t)r.A + 2) * 4);
+    const size_t o_cur = off; off = al(off + (size_t)r.A * 4);
+    const size_t o_bsum = off; off = al(off + 4097 * 4);
+    const size_t o_seg = off; off = al(off + (size_t)r.A * 64);
+    const size_t o_ent = off; off = al(off + (size_t)r.N * kRowStride * 4);
+    if (cudaMalloc(&ix.base, off) != cudaSuccess) {
+      cudaGetLastError();   // no room: the dense pass goes on
+      ix.base = nullptr;
+      r.ix_failed = true;
+      return cudaSuccess;
+    }
+    char* b = static_cast<char*>(ix.base);
+    ix.off = reinterpret_cast<uint32_t*>(b + o_off);
+    ix.cur = reinterpret_cast<uint32_t*>(b + o_cur);
+    ix.bsum = reinterpret_cast<uint32_t*>(b + o_bsum);
+    ix.seg = reinterpret_cast<uint16_t*>(b + o_seg);
+    ix.ent = reinterpret_cast<uint32_t*>(b + o_ent);
+  }
+  cudaError_t e = launch_rows_begin(v, s, N, A, stream, row_sum, true, with_posmap, true);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ix.cur, 0, (size_t)A * 4, stream);
+  if (e != cudaSuccess) return e;
+  const uint32_t gb = (uint32_t)(((size_t)N * kRowStride + 255) / 256), nb = (A + 4095) / 4096;
+  k_ix_count<<<gb, 256, 0, stream>>>(r.rt, r.cnt, N, A, ix.cur);
+  k_ix_scan<<<nb, 1024, 0, stream>>>(ix.cur, ix.off, A, ix.bsum);
+  k_ix_scan<<<1, 1024, 0, stream>>>(ix.bsum, ix.bsum, nb, nullptr);
+  k_ix_add<<<(A + 255) / 256, 256, 0, stream>>>(ix.off, ix.cur, A, ix.bsum);
+  k_ix_fill<<<gb, 256, 0, stream>>>(r.rt, r.cnt, N, A, ix.cur, ix.ent);
+  k_ix_sort<<<(A + 7) / 8, 256, 0, stream>>>(r.rt, ix.off, A, ix.ent, ix.seg);
+  k_ix_done<<<1, 1, 0, stream>>>(s.ctl, ix);
   return cudaGetLastError();
 }
 
