@@ -153,7 +153,7 @@ cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* ou
     e = cudaMemsetAsync(s->batch_counts, 0, (size_t)b.ticks * 4, stream);
   if (e != cudaSuccess) return e;
   k_set_batch_ctl<<<1, 512, 0, stream>>>(s->ctl, b.tick_base, (int32_t)b.dopamine, rows, force ? 1u : 0u, b.ticks,
-                                         rows ? s->rows->lit : nullptr, b.total_axons);
+                                         rows ? s->rows->alit : nullptr, b.total_axons);
   // burst-counter reset before the batch (shard.rs:71)
   e = launch_reset_burst(*b.vram, b.padded_n, stream);
   if (e != cudaSuccess) return e;
@@ -189,6 +189,7 @@ cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, ui
     a.batch = true;
     a.k = k;
     a.rows = rows != 0;
+    a.lit_new = k == (b.ticks > kLitWindow ? b.ticks - kLitWindow : 0u);
     a.defer_push = rows != 0 && k + 1 < b.ticks;
     a.fix_cap = fix_cap;
     le = launch_tick(*b.vram, s, a, cap);
@@ -306,6 +307,7 @@ extern "C" int32_t axc_profile_ticks(const ShardVramPtrs* vram, uint32_t padded_
     a.batch = rows;
     a.k = k;
     a.rows = rows;
+    a.lit_new = k == (ticks > kLitWindow ? ticks - kLitWindow : 0u);
     a.defer_push = rows && k + 1 < ticks;
     a.fix_cap = g_fix_cap.load();
     e = launch_tick(*vram, *s, a, st, ev);

@@ -46,15 +46,19 @@ struct ShardCtl {
   uint32_t pad2;
   unsigned long long ctr[8];  // statistics, see axc_shard_counters
   uint32_t dense[2];      // row engine: tick k (slot k & 1) has an axon off the lit set the row layout assumed
-  unsigned long long pfx_total;   // row engine: slots outside the frozen lit-sum part of the rows (batch start)
+  unsigned long long pfx_total;   // row engine: slots of the rows tested on every tick (batch start)
   unsigned long long slot_total;  // row engine: live slots of the rows (batch start)
   uint32_t lay_now;       // row engine: this batch lays the row copy out anew (layout_decide)
   uint32_t lay_since;     // row engine: ticks since the last layout
   uint32_t lay_every;     // row engine: ticks between layouts while the lit-sum criterion holds
   uint32_t lay_wait;      // row engine: ticks a layout must last while it does not hold
   uint32_t lay_lit;       // row engine: fully-lit axons when the layout was made
-  uint32_t pad4;
-  unsigned long long lay_pfx;     // row engine: pfx_total of the layout before the current one
+  uint32_t dec_ticks;     // row engine: ticks of the last decision
+  uint32_t lay_forced;    // row engine: the layout was forced
+  uint32_t pad5;
+  unsigned long long mov_total;   // row engine: movable slots of the rows (batch start)
+  unsigned long long lit_seen;    // row engine: ctr[6] at the last decision
+  unsigned long long lay_work;    // row engine: tested and movable slots of the layout before the current one
   unsigned long long gsop_same[2];  // row engine: 4-slot groups the 8-lane pass's GSOP visited and left as they
                                     // were, and all it visited, since the last decision
   uint32_t mixed_len;     // row engine: a neuron with slots has another signal_propagation_length than pmax
@@ -91,7 +95,7 @@ struct RowCache {
   int16_t* rw = nullptr;    // [N][128] weights, neuron-major
   uint16_t* cnt = nullptr;  // [N] slots before the first empty target; bit 15: an invalid target
   uint2* mask2 = nullptr;   // [A+1] split segment-hit masks (heads 0..6 | head 7); [A] dummy
-  uint32_t* mult = nullptr; // [A] number of somas that own the axon
+  uint32_t* axw = nullptr;  // [A] owners and used segments of the axon (kAxOwned); population: somas that own it
   uint32_t* eval = nullptr; // [N] non-refractory neurons of the tick
   uint32_t* fix = nullptr;  // [kFixCap] deferred GSOP slots (n*128 + slot)
   uint32_t* lit = nullptr;  // [A/32+1] fully-lit axons of the tick, one bit each
@@ -104,8 +108,10 @@ struct RowCache {
   uint8_t* lfz = nullptr;   // [N] number of those slots (set at batch start)
   uint4* omask = nullptr;   // [N] columnar slots placed first in the row (the movable ones; all when unpermuted)
   uint32_t* wcnt = nullptr; // [2][kMaxUpdateWarps] spikers each warp of the update pass listed (gs_n, gd_n)
-  int2* lsum = nullptr;     // [N] x: wrapping sum of the row's lit-sum weights, y: row positions before them
-  uint32_t* xlit = nullptr; // [A/32+1] axons taken as fully lit when the row layout was made
+  int2* rec = nullptr;      // [N] x: wrapping sum of the row's lit-sum weights, y: its groups' bounds (build_row)
+  uint4* lmask = nullptr;   // [N] the columnar slots of omask placed before the others (movable, lit)
+  uint32_t* alit = nullptr; // [A/32+1] axons fully lit in every one of the last ticks (kLitWindow)
+  uint32_t* xlit = nullptr; // [A/32+1] axons (of alit) taken as fully lit when the row layout was made
   RowIndex ix;
   bool ix_failed = false;   // no room for the index: not tried again
   uint8_t* posmap = nullptr;  // [N][128] row position of each columnar slot (learned engine only; own allocation)
@@ -146,6 +152,7 @@ struct ShardScratch {
   uint64_t batch_rows_lut = 0;           // LUT generation of the batch layout
 };
 
+constexpr uint32_t kLitWindow = 32;   // last ticks before a layout in which an axon must have been fully lit
 constexpr uint32_t kBatchRelayoutMin = 100, kBatchRelayoutMax = 1600;   // ticks between batch layouts
 
 uint64_t lut_generation();
@@ -163,22 +170,26 @@ inline bool batch_rows_force(ShardScratch& s) {
 
 #ifdef __CUDACC__
 // The device's layout decision for the next `ticks` ticks of a batch (one
-// block, before the batch; lit: the last tick's fully-lit bitmap of A axons).
+// block, before the batch; lit: the always-lit axons of the last ticks, of A).
 // A new layout when forced; every lay_every ticks, doubling from
 // kBatchRelayoutMin to kBatchRelayoutMax, while the current one meets the
-// lit-sum criterion (at most an eighth of the live slots outside the lit-sum
-// groups); while it does not, when it could do better: a tenth more axons are
-// fully lit than when it was made, or an eighth of the 4-slot groups that GSOP
-// visited since the last decision no longer moved (the weights froze), but at
-// most every lay_wait ticks, doubling from 16 while the new layouts gain less
-// than a tenth, and at least every kBatchRelayoutMax.  A brain whose weights
-// never freeze, or that is quiet, so keeps its layout instead of paying for
-// one each batch (1.5 ms at 1.5M neurons).  The layout kernels of the batch
+// lit-sum criterion (at most an eighth of the live slots tested); while it does
+// not, when a tenth more axons are fully lit than when it was made; while it
+// does, when axons it took as lit were dark on half of the ticks; and in both
+// cases when an eighth of the groups of movable slots that GSOP visited since the
+// last decision no longer moved; but for these at most every lay_wait ticks,
+// doubling from 16 while the new layouts gain less than a tenth, and at least
+// every kBatchRelayoutMax.  A brain whose weights never freeze, or that is
+// quiet, so keeps its layout instead of paying for one each batch (1.5 ms at
+// 1.5M neurons).  The layout kernels of the batch
 // return at once when lay_now is 0.
 __device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint32_t ticks, const uint32_t* lit,
                                               uint32_t A) {
   __shared__ uint32_t s_lit;
+  // the layout meets the criterion, and its lit axons stayed lit on most ticks since the last decision
   const bool met = c->slot_total > 0 && c->pfx_total * 8ull <= c->slot_total;
+  const unsigned long long lit6 = c->ctr[6] < c->lit_seen ? c->ctr[6] : c->ctr[6] - c->lit_seen;
+  const bool missed = met && lit6 * 2ull < c->dec_ticks;   // dark axons: the rows were checked slot by slot
   uint32_t n = 0;
   if (threadIdx.x == 0) s_lit = 0;
   __syncthreads();
@@ -190,28 +201,31 @@ __device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint3
   __syncthreads();
   if (threadIdx.x) return;
   bool build = force;
+  const bool froze = c->gsop_same[0] > 0 && c->gsop_same[0] * 8ull >= c->gsop_same[1];
   if (!force && met) {
-    build = c->lay_since >= c->lay_every;
+    build = c->lay_since >= c->lay_every || ((froze || missed) && c->lay_since >= c->lay_wait);
   } else if (!force) {
-    const bool froze = c->gsop_same[0] > 0 && c->gsop_same[0] * 8ull >= c->gsop_same[1];
     const bool grew = (unsigned long long)s_lit * 10ull > (unsigned long long)c->lay_lit * 11ull;
     // (the sparse form reads no more than the movable slots of a few spikers: its rows stay)
     build = (c->lay_since >= kBatchRelayoutMax && c->streak == 0u) ||
             (c->lay_since >= c->lay_wait && (froze || grew) && c->slot_total > 0);
   }
-  if (build && (force || !met)) c->lay_lit = s_lit;
-  // the last layout left a tenth fewer slots outside the groups than the one before
-  const bool paid = c->pfx_total * 10ull < c->lay_pfx * 9ull;
+  if (build && (force || !met)) c->lay_lit = force ? 0u : s_lit;   // a forced layout leaves movable slots out
+  // the last layout left a tenth fewer tested and movable slots than the one before
+  const bool paid = (c->pfx_total + c->mov_total) * 10ull < c->lay_work * 9ull;
   if (build) {
     const uint32_t twice = 2u * c->lay_every;
     c->lay_every = (force || !met || c->lay_every < kBatchRelayoutMin) ? kBatchRelayoutMin
                    : twice < kBatchRelayoutMax                          ? twice
                                                                         : kBatchRelayoutMax;
-    c->lay_wait = (force || met) ? 0u : (paid || c->lay_wait < 16u) ? 16u : min(2u * c->lay_wait, kBatchRelayoutMax);
-    c->lay_pfx = c->pfx_total;
+    c->lay_wait = force ? 0u : (paid || c->lay_wait < 16u) ? 16u : min(2u * c->lay_wait, kBatchRelayoutMax);
+    c->lay_work = c->pfx_total + c->mov_total;
     c->lay_since = 0;
   }
+  if (build) c->lay_forced = force;
   c->gsop_same[0] = c->gsop_same[1] = 0;
+  c->lit_seen = c->ctr[6];
+  c->dec_ticks = ticks;
   c->lay_since += ticks;
   c->lay_now = build ? 1u : 0u;
 }
@@ -288,6 +302,7 @@ struct TickArgs {
   uint32_t k;                 // tick index inside the batch
   bool rows;                  // use the neuron-major row engine (batch mode only)
   uint32_t fix_cap;           // row engine: deferred-GSOP list capacity (<= kFixCap)
+  bool lit_new;               // row engine: the window of always-lit axons (RowCache::alit) starts at this tick
   bool index;                 // row engine: the tick may run its sparse form (the learned engine's plain graph)
   bool defer_push;            // row engine: leave this tick's soma pushes to the next tick's prologue
                               // (never on the last tick of a batch)

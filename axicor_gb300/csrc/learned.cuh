@@ -1232,7 +1232,7 @@ static void learned_update_forms(Learned& L, ShardScratch& s, uint32_t k, cudaSt
 
 // One tick: schedule, prologue, both update forms (the one not picked returns
 // at once), fix-up, push, features + prediction.
-static cudaError_t learned_tick(Learned& L, ShardScratch& s, uint32_t k, bool last, bool features_on,
+static cudaError_t learned_tick(Learned& L, ShardScratch& s, uint32_t k, bool last, bool lit_new, bool features_on,
                                 cudaStream_t st) {
   RowCache& r = *s.rows;
   const uint32_t N = L.N, A = L.A;
@@ -1245,9 +1245,9 @@ static cudaError_t learned_tick(Learned& L, ShardScratch& s, uint32_t k, bool la
   if (G)
     k_rows_prologue<true><<<(G + 255) / 256, 256, 0, st>>>(L.v.axon_heads, A, L.v_seg, bits_k, L.voff,
                                                            bits_k ? L.nv : 0u, s.incoming, nullptr, k, r.mask2,
-                                                           r.mult, L.v.soma_flags, L.v.timers, N, r.eval, s.ctl,
+                                                           r.axw, L.v.soma_flags, L.v.timers, N, r.eval, s.ctl,
                                                            raise, r.lit, D, k > 0 ? s.pend : nullptr, r.xlit,
-                                                           r.live, r.evb);
+                                                           r.live, r.evb, r.alit, lit_new ? 1u : 0u);
   learned_update_forms(L, s, k, st);
   k_rows_fixup<<<2 * sms, 256, 0, st>>>(L.v, N, A, r.rt, r.rw, r.cnt, r.mask2, s.pend, r.eval, r.fix, s.ctl, k,
                                         nullptr, nullptr, 0, ColWT{}, (volatile uint32_t*)s.h_counts_pinned);
@@ -1479,9 +1479,11 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
         a.defer_push = k + 1 < tpg;
         a.fix_cap = kFixCap;
         a.index = true;
+        a.lit_new = k == (tpg > kLitWindow ? tpg - kLitWindow : 0u);
         le = launch_tick(L->v, *s, a, L->capture);
       } else {
-        le = learned_tick(*L, *s, k, k + 1 == tpg, kind == 1, L->capture);
+        le = learned_tick(*L, *s, k, k + 1 == tpg, k == (tpg > kLitWindow ? tpg - kLitWindow : 0u), kind == 1,
+                          L->capture);
       }
     }
     if (le == cudaSuccess) le = launch_rows_end(L->v, *s, L->N, L->capture);
@@ -1528,7 +1530,7 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
       if (e != cudaSuccess) break;
     }
     k_learn_set_ctl<<<1, 512, 0, st>>>(s->ctl, L->tick_base + t0, (int32_t)L->dopamine, force ? 1u : 0u, tpg,
-                                       s->rows->lit, L->A);
+                                       s->rows->alit, L->A);
     e = rows_index_wish(L->v, *s, L->N, L->A, st, true, true);
     if (e == cudaSuccess) e = launch_reset_burst(L->v, L->N, st);
     unsigned long long picked0 = 0, picked1 = 0;

@@ -105,43 +105,32 @@ __global__ void __launch_bounds__(256) k_pop_mult(const PopBrain* __restrict__ b
 __global__ void __launch_bounds__(256) k_pop_build(const PopBrain* __restrict__ brains,
                                                    const uint32_t* __restrict__ map,
                                                    const uint32_t* __restrict__ first) {
-  __shared__ uint32_t s_t[AXC_MAX_DENDRITES][33];
-  __shared__ int16_t s_w[AXC_MAX_DENDRITES][34];
-  __shared__ uint32_t s_cnt[32];
+  __shared__ SlotStage st;
   uint32_t lb;
   const PopBrain& b = brains[block_brain(map, first, &lb)];
-  const uint32_t N = b.N, A = b.A;
+  const uint32_t N = b.N;
   const uint32_t n0 = lb * 32;
-  const uint32_t col = threadIdx.x & 31, r0 = threadIdx.x >> 5;
   if (threadIdx.x < 32) {
-    s_cnt[threadIdx.x] = AXC_MAX_DENDRITES;
-    if (n0 + threadIdx.x < N) b.P.soma_flags[n0 + threadIdx.x] &= 0xF1;
+    const uint32_t n = n0 + threadIdx.x;
+    uint8_t f = 0;
+    if (n < N) {
+      f = b.P.soma_flags[n] & 0xF1;
+      b.P.soma_flags[n] = f;
+    }
+    st.cnt[threadIdx.x] = AXC_MAX_DENDRITES;
+    st.fz[threadIdx.x] = frozen_from(b.lut[f >> 4]);
+    st.lit[threadIdx.x] = 0u;
   }
   __syncthreads();
-  for (uint32_t ch = 0; ch < AXC_MAX_DENDRITES / 8; ch++) {
-    const uint32_t r = ch * 8 + r0, n = n0 + col;
-    uint32_t t = 0;
-    int16_t w = 0;
-    if (n < N) {
-      t = __ldcs(b.P.dendrite_targets + (size_t)r * N + n);
-      w = __ldcs(b.P.dendrite_weights + (size_t)r * N + n);
-    }
-    s_t[r][col] = t;
-    s_w[r][col] = w;
-    if (t == 0) atomicMin(&s_cnt[col], r);
-    __syncthreads();
-    const int mine = threadIdx.x < 32 ? (s_cnt[threadIdx.x] < (ch + 1) * 8) : 1;
-    if (__syncthreads_and(mine)) break;
-  }
+  stage_columns(st, b.P.dendrite_targets, b.P.dendrite_weights, N, n0, b.A, nullptr, false, nullptr);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ uint32_t s_bc[8], s_bs[8];
   uint32_t wc = 0, ws = 0;
   for (uint32_t j = warp; j < 32; j += 8) {
     const uint32_t n = n0 + j;
     if (n >= N) continue;
-    const uint32_t c = s_cnt[j];
-    const RowBuilt rb = build_row(s_t, s_w, j, n, c, frozen_from(b.lut[b.P.soma_flags[n] >> 4]), A, false, true,
-                                  b.rt, b.rw, b.cnt, b.amask, b.omask, b.lfz);
+    const uint32_t c = st.cnt[j];
+    const RowBuilt rb = build_row(st, j, n, c, false, true, b.rt, b.rw, b.cnt, b.amask, b.omask, b.lfz);
     if (lane == 0 && c) {
       wc = max(wc, c);
       ws = max(ws, rb.smx);
@@ -715,7 +704,7 @@ int32_t axc_population_create(const AxcPopBrainDesc* brains, uint32_t count, voi
     h.rw = s->rows->rw;
     h.cnt = s->rows->cnt;
     h.mask2 = s->rows->mask2;
-    h.mult = s->rows->mult;
+    h.mult = s->rows->axw;
     h.eval = s->rows->eval;
     h.pend = s->pend;
     h.ctl = s->ctl;

@@ -8,7 +8,7 @@
 // the spikers' slots with one sector per slot.  For the length of one batch the
 // engine keeps a neuron-major copy ([neuron][128]) of targets and weights:
 //
-//   batch start  k_rows_mult       somas per axon (soma_to_axon multiplicity)
+//   batch start  k_rows_mult       owners of each axon (none, one, several)
 //                k_rows_build      columnar -> rows (the slots whose weights may
 //                                  still move first), per-neuron counts and masks
 //   per tick     k_rows_prologue   the previous tick's soma pushes, axon pushes +
@@ -76,6 +76,13 @@ static void launch_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
   // launch sequences return
   cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
+// Axon word axw[a], set by the layout: a soma owns the axon; two or more do; bits
+// 1..30: a used slot of the shard targets that segment of it.  The axon is fully
+// lit when heads 0..6 cover those segments (not every segment that some axon
+// uses: after two pushes close together the eight heads reach less far, but few
+// axons have slots on their last segments).
+constexpr uint32_t kAxOwned = 1u, kAxShared = 0x80000000u, kAxSegs = 0x7FFFFFFEu;
+__device__ __forceinline__ uint32_t ax_owners(uint32_t axw) { return (axw & kAxOwned) + (axw >> 31); }
 constexpr uint32_t kRowBad = 0x8000u;    // cnt flag: the row holds an invalid target
 
 // Bytes of the fully-lit bitmap of A axons as staged in shared memory (one
@@ -138,8 +145,8 @@ __device__ __forceinline__ void md_pair(const BurstHeads8* heads, uint32_t a, ui
 // every weight back at batch end).
 struct ColWT {
   int16_t* w = nullptr;         // columnar weights of the shard
-  const uint4* om = nullptr;    // per neuron: the columnar slots placed first in its row
-  const uint16_t* cnt = nullptr;
+  const uint4* om = nullptr;    // per neuron: the columnar slots placed first in its row,
+  const uint4* lm = nullptr;    // and those of them placed before the others
   uint32_t N = 0;
 };
 
@@ -156,32 +163,35 @@ __device__ __forceinline__ uint32_t nth_bit128(uint4 m, uint32_t r) {
   return 96u + __fns(m.w, 0, r - c2 + 1);
 }
 
-// Columnar slot of row position pos in a row of c used slots whose slots of om
-// come first (in slot order) and the other used slots after them (in slot order).
-__device__ __forceinline__ uint32_t col_of_pos(uint4 om, uint32_t pos, uint32_t c) {
-  const uint32_t olf = __popc(om.x) + __popc(om.y) + __popc(om.z) + __popc(om.w);
-  if (pos < olf) return nth_bit128(om, pos);
-  const auto used = [c](uint32_t lo) { return c >= lo + 32u ? 0xFFFFFFFFu : (c > lo ? (1u << (c - lo)) - 1u : 0u); };
-  const uint4 rest = make_uint4(used(0) & ~om.x, used(32) & ~om.y, used(64) & ~om.z, used(96) & ~om.w);
-  return nth_bit128(rest, pos - olf);
+// Columnar slot of row position pos < lf, in a row whose movable slots are om,
+// those of lm first and then the others, each in slot order.
+__device__ __forceinline__ uint32_t col_of_pos(uint4 om, uint4 lm, uint32_t pos) {
+  const uint32_t nl = __popc(lm.x) + __popc(lm.y) + __popc(lm.z) + __popc(lm.w);
+  return pos < nl ? nth_bit128(lm, pos)
+                  : nth_bit128(make_uint4(om.x & ~lm.x, om.y & ~lm.y, om.z & ~lm.z, om.w & ~lm.w), pos - nl);
 }
 
 __device__ __forceinline__ void col_write(const ColWT& wt, uint32_t n, uint32_t pos, int16_t w) {
-  const uint32_t q = col_of_pos(wt.om[n], pos, wt.cnt[n] & 0xFFu);
+  const uint32_t q = col_of_pos(wt.om[n], wt.lm[n], pos);
   wt.w[(size_t)q * wt.N + n] = w;
 }
 
-// The lit-sum form runs tick k when the rows' tested prefixes are short (at most
+// The lit-sum form runs tick k when the rows' tested slots are few (at most
 // an eighth of the live slots: otherwise the 8-lane pass is faster) and every
-// axon the row layout took as fully lit is fully lit this tick.  Every thread
+// axon the row layout took as fully lit is fully lit this tick; with a few of
+// them dark (a network spike on an axon that its soma keeps lit moves its
+// oldest heads on) the rows are checked slot by slot (kFormVerify).  Every thread
 // of both update kernels asks at its start; the three words were written by
 // earlier kernels and no kernel that asks writes them, so plain loads (cached
 // in L1 after the first warp of an SM) serve it: uncached loads sent every
 // warp's request to the one L2 slice that holds the control block, a few
 // microseconds per launch.
-__device__ __forceinline__ bool lsum_tick(const ShardCtl* ctl, uint32_t k) {
+__device__ __forceinline__ bool lit_layout(const ShardCtl* ctl) {
   const unsigned long long p = ctl->pfx_total, c = ctl->slot_total;
-  return c > 0 && p * 8ull <= c && ctl->dense[k & 1] == 0u;
+  return c > 0 && p * 8ull <= c;
+}
+__device__ __forceinline__ bool lsum_tick(const ShardCtl* ctl, uint32_t k) {
+  return lit_layout(ctl) && ctl->dense[k & 1] == 0u;
 }
 
 // The sparse form can run tick k: fewer than half as many axons have a head on
@@ -301,10 +311,36 @@ struct LearnDev {
 // lc: the learned engine's control block (its planned sparse ticks), or null;
 // index: the tick may run sparse by the exact counts (the learned engine's
 // graphs, whose memory holds the inverted index).
-enum TickForm { kFormDense = 0, kFormLitSum = 1, kFormSparse = 2, kFormScatter = 3 };
+enum TickForm {
+  kFormDense = 0,     // k_rows_update: every slot tested
+  kFormLitSum = 1,    // k_rows_update_lsum: a thread per neuron
+  kFormSparse = 2,    // k_sparse_hits, k_sparse_neurons
+  kFormScatter = 3,   // the learned engine's kernels without the rows' index
+  kFormLitRows = 4,   // k_rows_update: lit_row_step
+  kFormVerify = 5     // the same, with dark axons: each lit slot is looked up
+};
+
+// The control words are read at once (volatile, so that no load waits behind the
+// branch on another) through L1, as lsum_tick's comment says.
+__device__ __forceinline__ unsigned long long ctl_ld64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ctl_ld32(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+// kFormLitRows where more than a sixteenth of the live slots are movable or
+// tested: a settled brain has 0.5 % of them so, one that learns all its life
+// nearly all.
 __device__ __forceinline__ TickForm tick_form(const ShardCtl* ctl, uint32_t k, const LearnCtl* lc, uint32_t index) {
+  const unsigned long long p = ctl_ld64(&ctl->pfx_total), c = ctl_ld64(&ctl->slot_total), m = ctl_ld64(&ctl->mov_total);
+  const uint32_t dark = ctl_ld32(&ctl->dense[k & 1]);
   if (lc && lc->mode == 1u && !lc->overflow) return index_ok(ctl) ? kFormSparse : kFormScatter;
-  if (lsum_tick(ctl, k)) return kFormLitSum;
+  if (c > 0 && p * 8ull <= c) return dark ? kFormVerify : (m + p) * 16ull > c ? kFormLitRows : kFormLitSum;
   return index && index_ok(ctl) && sparse_tick(ctl, k) ? kFormSparse : kFormDense;
 }
 
@@ -346,104 +382,180 @@ __device__ __forceinline__ uint32_t row_pos(uint32_t word, uint32_t lane, uint32
   return ((word >> lane) & 1u) ? below : lf + q - below;
 }
 
-// One neuron's row of the row copy, by one warp, from the columns staged in
-// shared memory (column j, c used slots): invalid targets redirected, movable
-// marks, placement, and the neuron's cnt / amask / omask / lfz.
-// Placement with permute: the movable slots first, then (with xlit) the other
-// slots the update pass must test each tick, then the lit-sum slots, each
-// group in slot order; without permute every slot keeps its position.
-// A lit-sum slot (xlit given, permute) is frozen (GSOP cannot move its weight),
-// has a segment in 1..30, belongs to a neuron whose variant length is the LUT
-// maximum, and targets an axon that xlit marks as fully lit: while that axon
-// stays fully lit (the prologue checks it every tick) the slot is a hit, so the
-// update pass adds the row's lit-sum weights as one precomputed wrapping sum
-// (lsum[n].x) and tests only the first lsum[n].y positions.
+// One neuron's row of the row copy, by one warp, from the staged columns (column
+// j, c used slots): placement, and the neuron's cnt / amask / omask / lfz.
+// A slot is movable when GSOP may still move its weight, and lit (stage_columns)
+// when it has a segment in 1..30, belongs to a neuron whose variant
+// length is the LUT maximum, and targets an axon that xlit marks as fully lit:
+// while that axon stays fully lit (the prologue checks it every tick) the slot
+// is a hit, and GSOP takes its delta from the rank table (movable slots only
+// with mov_lit).  With permute the row
+// holds, each group in slot order,
+//   [0, lm)    movable, lit: hits, their weights read each tick
+//   [lm, lf)   movable, not lit: tested each tick
+//   [lf, end)  frozen, not lit: tested each tick
+//   [end, c)   frozen, lit: hits whose weights are summed once (rec[n].x)
+// and rec[n].y = lm | lf << 8 | end << 16; lmask marks the columnar slots of the
+// first group.  Without permute every slot keeps its position.
 // Returns, in every lane, the row's largest segment, (want_sum) its targets
-// checksum and its tested-prefix length.
+// checksums by columnar slot and by row position, and its tested slots.
 struct RowBuilt {
   uint32_t smx;
   unsigned long long hsum;
   uint32_t pfx;
-  unsigned long long psum;  // checksum of the targets by row position
+  uint32_t lf;
+  unsigned long long psum;
 };
 
-__device__ __forceinline__ RowBuilt build_row(uint32_t (*s_t)[33], const int16_t (*s_w)[34], uint32_t j, uint32_t n,
-                                              uint32_t c, int32_t fz, uint32_t A, bool want_sum, bool permute,
-                                              uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
+__device__ __forceinline__ uint32_t popc4(const uint32_t (&m)[4]) {
+  return __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
+}
+
+// 32 neurons' columns staged in shared memory, with a class byte a slot.
+struct SlotStage {
+  uint32_t t[AXC_MAX_DENDRITES][33];
+  int16_t w[AXC_MAX_DENDRITES][34];
+  uint8_t k[AXC_MAX_DENDRITES][36];   // kSlotMov | kSlotLit | kSlotBad
+  uint32_t cnt[32];                   // used slots of the neurons
+  int32_t fz[32];                     // frozen_from of their variants
+  uint32_t lit[32];                   // their lit slots may be taken as such
+};
+constexpr uint32_t kSlotMov = 1u, kSlotLit = 2u, kSlotBad = 4u;
+
+// Columns -> stage, by a 256-thread block that has set cnt (AXC_MAX_DENDRITES),
+// fz and lit: 32 slots of the 32 neurons a round, until every neuron has met its
+// first empty target.  A thread has four targets and weights of the next round in
+// flight while it looks up the four of this one (xlit: the lit axons; axw: marks
+// the axon's segment as used), so a round costs the latency of one gather.
+__device__ __forceinline__ void stage_columns(SlotStage& st, const uint32_t* __restrict__ targets,
+                                              const int16_t* __restrict__ weights, uint32_t N, uint32_t n0, uint32_t A,
+                                              const uint32_t* __restrict__ xlit, bool mov_lit, uint32_t* axw) {
+  const uint32_t col = threadIdx.x & 31, r0 = threadIdx.x >> 5, n = n0 + col;
+  const int32_t fz = st.fz[col];
+  const bool lit_on = xlit && st.lit[col];
+  uint32_t t[4];
+  int16_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const size_t at = (size_t)(8 * i + r0) * N + n;
+    t[i] = n < N ? __ldcs(targets + at) : 0u;
+    w[i] = n < N ? __ldcs(weights + at) : (int16_t)0;
+  }
+#pragma unroll 1
+  for (uint32_t ch = 0; ch < AXC_MAX_DENDRITES / 32; ch++) {
+    uint32_t tn[4] = {0, 0, 0, 0};
+    int16_t wn[4] = {0, 0, 0, 0};
+    if (ch + 1 < AXC_MAX_DENDRITES / 32 && n < N) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const size_t at = (size_t)((ch + 1) * 32 + 8 * i + r0) * N + n;
+        tn[i] = __ldcs(targets + at);
+        wn[i] = __ldcs(weights + at);
+      }
+    }
+    uint32_t lw[4], aw[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t a = (t[i] & AXC_TARGET_AXON_MASK) - 1u, seg = t[i] >> AXC_TARGET_SEG_SHIFT;
+      const bool in = a < A && seg - 1u < 30u;
+      lw[i] = in && lit_on ? __ldg(xlit + (a >> 5)) : 0u;
+      aw[i] = in && axw ? axw[a] : 0xFFFFFFFFu;   // (a stale word only costs an atomic that changes nothing)
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t r = ch * 32 + 8 * i + r0;
+      const uint32_t a = (t[i] & AXC_TARGET_AXON_MASK) - 1u, seg = t[i] >> AXC_TARGET_SEG_SHIFT;
+      if (!((aw[i] >> (seg & 31u)) & 1u)) atomicOr(axw + a, 1u << seg);
+      const bool mov = !frozen_weight(w[i], fz);
+      const bool lit = ((lw[i] >> (a & 31u)) & 1u) && (mov_lit || !mov);
+      // an invalid axon id (field 0 or >= A) points at the dummy mask entry A,
+      // which sends the slot down the exact path (hit_exact / gsop_general skip it)
+      const bool bad = a >= A;
+      st.t[r][col] = bad && t[i] ? (t[i] & ~AXC_TARGET_AXON_MASK) | (A + 1u) : t[i];
+      st.w[r][col] = w[i];
+      st.k[r][col] = (uint8_t)((mov ? kSlotMov : 0u) | (lit ? kSlotLit : 0u) | (bad ? kSlotBad : 0u));
+      if (t[i] == 0) atomicMin(&st.cnt[col], r);
+      t[i] = tn[i];
+      w[i] = wn[i];
+    }
+    __syncthreads();
+    const int mine = threadIdx.x < 32 ? (st.cnt[threadIdx.x] < (ch + 1) * 32) : 1;
+    if (__syncthreads_and(mine)) break;
+  }
+}
+
+__device__ __forceinline__ RowBuilt build_row(const SlotStage& st, uint32_t j, uint32_t n, uint32_t c, bool want_sum,
+                                              bool permute, uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
                                               uint16_t* __restrict__ cnt, uint4* __restrict__ amask,
                                               uint4* __restrict__ omask, uint8_t* __restrict__ lfz,
-                                              const uint32_t* __restrict__ xlit = nullptr, bool exact_var = false,
-                                              int2* __restrict__ lsum = nullptr, uint8_t* __restrict__ posmap = nullptr) {
+                                              int2* __restrict__ rec = nullptr, uint4* __restrict__ lmask = nullptr,
+                                              uint8_t* __restrict__ posmap = nullptr) {
   const uint32_t lane = threadIdx.x & 31;
-  const bool lsum_on = permute && xlit != nullptr && exact_var;
   bool bad = false;
   uint32_t smx = 0, rsum = 0;
-  unsigned long long hsum = 0;
-  uint32_t mv[4], rs[4], all[4];   // movable / lit-sum / used slots, by columnar position
+  unsigned long long hsum = 0, psum = 0;
+  uint32_t t[4], mv[4], lt[4], all[4];   // movable / lit / used slots, by columnar position
+  int16_t w[4];
 #pragma unroll
   for (int ch = 0; ch < 4; ch++) {
     const uint32_t q = 32u * ch + lane;
-    bool mov = false, rest = false;
+    all[ch] = c >= 32u * ch + 32u ? kFull : c > 32u * ch ? (1u << (c - 32u * ch)) - 1u : 0u;
+    uint32_t k = 0;
+    t[ch] = 0;
+    w[ch] = 0;
     if (q < c) {
-      uint32_t t = s_t[q][j];
-      // an invalid axon id (field 0 or >= A) points at the dummy mask entry A,
-      // which sends the slot down the exact path (hit_exact / gsop_general skip it)
-      if ((t & AXC_TARGET_AXON_MASK) - 1u >= A) {
-        t = (t & ~AXC_TARGET_AXON_MASK) | (A + 1u);
-        s_t[q][j] = t;
-        bad = true;
-      }
-      const uint32_t seg = t >> AXC_TARGET_SEG_SHIFT;
-      smx = max(smx, seg);
-      if (want_sum) hsum += slot_mix(t, n * kRowStride + q);
-      mov = !frozen_weight(s_w[q][j], fz);
-      if (lsum_on && !mov && seg - 1u < 30u) {
-        const uint32_t a = (t & AXC_TARGET_AXON_MASK) - 1u;
-        rest = a < A && ((__ldg(xlit + (a >> 5)) >> (a & 31u)) & 1u);
-      }
-      if (rest) rsum += (uint32_t)(int32_t)s_w[q][j];
+      t[ch] = st.t[q][j];
+      w[ch] = st.w[q][j];
+      k = st.k[q][j];
+      bad |= (k & kSlotBad) != 0u;
+      smx = max(smx, t[ch] >> AXC_TARGET_SEG_SHIFT);
+      if (want_sum) hsum += slot_mix(t[ch], n * kRowStride + q);
+      if ((k & (kSlotLit | kSlotMov)) == kSlotLit) rsum += (uint32_t)(int32_t)w[ch];
     }
-    mv[ch] = __ballot_sync(kFull, mov);
-    rs[ch] = __ballot_sync(kFull, rest);
-    all[ch] = __ballot_sync(kFull, q < c);
+    mv[ch] = __ballot_sync(kFull, (k & kSlotMov) != 0u);
+    lt[ch] = permute ? __ballot_sync(kFull, (k & kSlotLit) != 0u) : 0u;
   }
   bad = __any_sync(kFull, bad);
   smx = __reduce_max_sync(kFull, smx);
+  rsum = __reduce_add_sync(kFull, rsum);
   if (want_sum) hsum = warp_sum(hsum);
-  rsum = warp_sum(rsum);
   if (bad) {
 #pragma unroll
-    for (int ch = 0; ch < 4; ch++) { mv[ch] = all[ch]; rs[ch] = 0u; }
+    for (int ch = 0; ch < 4; ch++) { mv[ch] = all[ch]; lt[ch] = 0u; }
     rsum = 0;
   }
-  const uint32_t lf = __popc(mv[0]) + __popc(mv[1]) + __popc(mv[2]) + __popc(mv[3]);
-  const uint32_t nrs = __popc(rs[0]) + __popc(rs[1]) + __popc(rs[2]) + __popc(rs[3]);
-  const uint32_t pfx = c - nrs;   // row positions the update pass tests: movable, then the others
-  // placement: movable (o), then tested (x), then lit-sum (rs) with permute; else the identity
-  uint32_t o[4], x[4];
+  uint32_t g0[4], g1[4], g2[4];   // the first three groups
 #pragma unroll
   for (int ch = 0; ch < 4; ch++) {
-    o[ch] = permute ? mv[ch] : all[ch];
-    x[ch] = permute ? (all[ch] & ~mv[ch] & ~rs[ch]) : 0u;
+    g0[ch] = mv[ch] & lt[ch];
+    g1[ch] = mv[ch] & ~lt[ch];
+    g2[ch] = all[ch] & ~mv[ch] & ~lt[ch];
   }
-  unsigned long long psum = 0;
-  uint32_t po = 0, px = 0, pr = 0, am[4];
-  const uint32_t below = (1u << lane) - 1u;
+  const uint32_t lm = popc4(g0), lf = lm + popc4(g1), end = lf + popc4(g2);
+  const uint32_t below = (1u << lane) - 1u, bit = 1u << lane;
+  // one group holds the whole row (a plastic brain, a quiet one, a settled one):
+  // every slot keeps its place
+  const bool moved = permute && lm != c && !(lm == 0u && lf == c) && !(lf == 0u && (end == c || end == 0u));
+  uint32_t p0 = 0, p1 = lm, p2 = lf, p3 = end, am[4];
 #pragma unroll
   for (int ch = 0; ch < 4; ch++) {
     const uint32_t q = 32u * ch + lane;
-    const uint32_t bit = 1u << lane;
-    uint32_t pos;
-    if (o[ch] & bit) pos = po + __popc(o[ch] & below);
-    else if (x[ch] & bit) pos = lf + px + __popc(x[ch] & below);
-    else pos = pfx + pr + __popc(rs[ch] & below);
-    po += __popc(o[ch]);
-    px += __popc(x[ch]);
-    pr += __popc(rs[ch]);
+    uint32_t pos = q;
+    if (moved) {
+      const uint32_t g3 = all[ch] & ~(g0[ch] | g1[ch] | g2[ch]);
+      if (g0[ch] & bit) pos = p0 + __popc(g0[ch] & below);
+      else if (g1[ch] & bit) pos = p1 + __popc(g1[ch] & below);
+      else if (g2[ch] & bit) pos = p2 + __popc(g2[ch] & below);
+      else pos = p3 + __popc(g3 & below);
+      p0 += __popc(g0[ch]);
+      p1 += __popc(g1[ch]);
+      p2 += __popc(g2[ch]);
+      p3 += __popc(g3);
+    }
     if (q < c) {
-      if (want_sum) psum += slot_mix(s_t[q][j], n * kRowStride + pos);
-      rt[(size_t)n * kRowStride + pos] = s_t[q][j];
-      rw[(size_t)n * kRowStride + pos] = s_w[q][j];
+      if (want_sum) psum += slot_mix(t[ch], n * kRowStride + pos);
+      rt[(size_t)n * kRowStride + pos] = t[ch];
+      rw[(size_t)n * kRowStride + pos] = w[ch];
       if (posmap) posmap[(size_t)n * kRowStride + q] = (uint8_t)pos;
     }
     // the movable slots by row position: the first lf positions, or mv itself
@@ -453,12 +565,13 @@ __device__ __forceinline__ RowBuilt build_row(uint32_t (*s_t)[33], const int16_t
   if (lane == 0) {
     cnt[n] = (uint16_t)(c | (bad ? kRowBad : 0u));
     amask[n] = make_uint4(am[0], am[1], am[2], am[3]);
-    omask[n] = make_uint4(o[0], o[1], o[2], o[3]);
+    omask[n] = permute ? make_uint4(mv[0], mv[1], mv[2], mv[3]) : make_uint4(all[0], all[1], all[2], all[3]);
+    if (lmask) lmask[n] = permute ? make_uint4(g0[0], g0[1], g0[2], g0[3]) : make_uint4(all[0], all[1], all[2], all[3]);
     lfz[n] = (uint8_t)lf;
-    if (lsum) lsum[n] = make_int2((int32_t)rsum, (int32_t)pfx);
+    if (rec) rec[n] = make_int2((int32_t)rsum, (int32_t)(lm | (lf << 8) | (end << 16)));
   }
   if (want_sum) psum = warp_sum(psum);
-  return RowBuilt{smx, hsum, pfx, psum};
+  return RowBuilt{smx, hsum, end - lm, lf, psum};
 }
 
 // Batch end, 32 neurons from n0 by a 256-thread block: weights rows -> columnar
@@ -499,18 +612,15 @@ __device__ __forceinline__ void writeback_tile(int16_t* __restrict__ weights, ui
     if (r < c_mine && ((o[r >> 5] >> (r & 31u)) & 1u)) weights[(size_t)r * N + n0 + lane] = s_w[r][lane];
 }
 
-// Batch start: columnar -> rows.  32 neurons per 256-thread block; the
-// columns are read 8 slots at a time until every neuron of the tile has met
-// its first empty target.  A slot whose weight GSOP may still move (not
-// frozen_weight, or any slot of a row with an invalid target) is movable;
-// weights only freeze, so the marks hold for the whole batch.  With permute
-// the movable slots go first in the row, then the others (each group in slot
-// order), so that GSOP reads a short prefix of the row; the dendrite sum (a
-// wrapping i32 sum) and GSOP (per slot) do not depend on the order.
+// Batch start: columnar -> rows, 32 neurons per 256-thread block (stage_columns,
+// build_row).  A slot whose weight GSOP may still move (not frozen_weight, or any
+// slot of a row with an invalid target) is movable; weights only freeze, so the
+// marks hold for the whole batch.  The dendrite sum (a wrapping i32 sum) and GSOP
+// (per slot) do not depend on the order of a row.
 // Per neuron: cnt = used slots (| kRowBad), lfz = movable slots, amask = their
 // row positions, omask = the columnar slots placed first (read by the
 // write-back; every used slot when the row keeps the columnar order).
-__global__ void __launch_bounds__(256) k_rows_build(const uint32_t* __restrict__ targets,
+__global__ void __launch_bounds__(256, 4) k_rows_build(const uint32_t* __restrict__ targets,
                                                     const int16_t* __restrict__ weights,
                                                     const uint8_t* __restrict__ flags, uint32_t N,
                                                     uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
@@ -518,62 +628,64 @@ __global__ void __launch_bounds__(256) k_rows_build(const uint32_t* __restrict__
                                                     uint4* __restrict__ omask, uint8_t* __restrict__ lfz,
                                                     ShardCtl* __restrict__ ctl, uint32_t A, uint32_t want_sum,
                                                     uint32_t permute, const uint32_t* __restrict__ xlit,
-                                                    int2* __restrict__ lsum, uint8_t* __restrict__ posmap,
-                                                    uint32_t cond) {
+                                                    int2* __restrict__ rec, uint4* __restrict__ lmask,
+                                                    uint8_t* __restrict__ posmap, uint32_t* axw, uint32_t cond) {
   if (cond && !ctl->lay_now) return;   // the batch keeps the last layout
-  __shared__ uint32_t s_t[AXC_MAX_DENDRITES][33];
-  __shared__ int16_t s_w[AXC_MAX_DENDRITES][34];
-  __shared__ uint32_t s_cnt[32];
+  __shared__ SlotStage st;
   __shared__ uint32_t s_pmax;
   const uint32_t n0 = blockIdx.x * 32;
-  const uint32_t col = threadIdx.x & 31, r0 = threadIdx.x >> 5;
-  if (threadIdx.x < 32) s_cnt[threadIdx.x] = AXC_MAX_DENDRITES;
-  if (threadIdx.x == 0) s_pmax = lut_pmax();
-  __syncthreads();
-  for (uint32_t ch = 0; ch < AXC_MAX_DENDRITES / 8; ch++) {
-    const uint32_t r = ch * 8 + r0, n = n0 + col;
-    uint32_t t = 0;
-    int16_t w = 0;
-    if (n < N) {
-      t = __ldcs(targets + (size_t)r * N + n);
-      w = __ldcs(weights + (size_t)r * N + n);
-    }
-    s_t[r][col] = t;
-    s_w[r][col] = w;
-    if (t == 0) atomicMin(&s_cnt[col], r);
-    __syncthreads();
-    const int mine = threadIdx.x < 32 ? (s_cnt[threadIdx.x] < (ch + 1) * 8) : 1;
-    if (__syncthreads_and(mine)) break;
+  if (threadIdx.x < 32) {
+    const uint32_t n = n0 + threadIdx.x, pmax = lut_pmax();
+    const VariantParameters& vp = VARIANT_LUT[n < N ? flags[n] >> 4 : 0];
+    st.cnt[threadIdx.x] = AXC_MAX_DENDRITES;
+    st.fz[threadIdx.x] = frozen_from(vp);
+    st.lit[threadIdx.x] = vp.signal_propagation_length == pmax ? 1u : 0u;
+    if (threadIdx.x == 0) s_pmax = pmax;
   }
+  __syncthreads();
+  // movable slots join the lit groups (no cooling step up to length 16), except in
+  // a layout that was forced: the window of always-lit axons is from before what
+  // forced it (a LUT, new targets)
+  const bool mov_lit = s_pmax <= 16u && cond && !ctl->lay_forced;
+  stage_columns(st, targets, weights, N, n0, A, xlit, mov_lit, axw);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // the block's longest row, largest segment, tested and live slots and (when
   // asked) targets checksum, one atomic each per block
-  __shared__ uint32_t s_bc[8], s_bs[8], s_bp[8], s_bl[8], s_bx[8];
+  __shared__ uint32_t s_bc[8], s_bs[8], s_bp[8], s_bl[8], s_bx[8], s_bm[8];
   __shared__ unsigned long long s_bh[8], s_bq[8];
-  uint32_t wc = 0, ws = 0, wp = 0, wl = 0;
+  uint32_t wc = 0, ws = 0, wp = 0, wl = 0, wm = 0;
   bool mixed = false;
   unsigned long long wh = 0, wq = 0;
   for (uint32_t j = warp; j < 32; j += 8) {
     const uint32_t n = n0 + j;
     if (n >= N) continue;
-    const uint32_t c = s_cnt[j];
-    const VariantParameters& vp = VARIANT_LUT[flags[n] >> 4];
-    const RowBuilt rb = build_row(s_t, s_w, j, n, c, frozen_from(vp), A, want_sum != 0u, permute != 0u, rt, rw, cnt,
-                                  amask, omask, lfz, xlit, vp.signal_propagation_length == s_pmax, lsum, posmap);
+    const uint32_t c = st.cnt[j];
+    const RowBuilt rb = build_row(st, j, n, c, want_sum != 0u, permute != 0u, rt, rw, cnt, amask, omask, lfz, rec, lmask,
+                                  posmap);
     if (lane == 0 && c) {
       wc = max(wc, c);
       ws = max(ws, rb.smx);
       wh += rb.hsum + slot_mix(c, n);
       wp += rb.pfx;
       wl += c;
+      wm += rb.lf;
       if (want_sum) wq += rb.psum + slot_mix(c, ~n);
-      mixed |= vp.signal_propagation_length != s_pmax;
+      mixed |= st.lit[j] == 0u;
     }
   }
-  if (lane == 0) { s_bc[warp] = wc; s_bs[warp] = ws; s_bh[warp] = wh; s_bp[warp] = wp; s_bl[warp] = wl; s_bx[warp] = mixed; s_bq[warp] = wq; }
+  if (lane == 0) {
+    s_bc[warp] = wc;
+    s_bs[warp] = ws;
+    s_bh[warp] = wh;
+    s_bp[warp] = wp;
+    s_bl[warp] = wl;
+    s_bx[warp] = mixed;
+    s_bm[warp] = wm;
+    s_bq[warp] = wq;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t bc = 0, bs = 0, bp = 0, bl = 0, bx = 0;
+    uint32_t bc = 0, bs = 0, bp = 0, bl = 0, bx = 0, bm = 0;
     unsigned long long bh = 0, bq = 0;
     for (int q = 0; q < 8; q++) {
       bc = max(bc, s_bc[q]);
@@ -582,6 +694,7 @@ __global__ void __launch_bounds__(256) k_rows_build(const uint32_t* __restrict__
       bp += s_bp[q];
       bl += s_bl[q];
       bx |= s_bx[q];
+      bm += s_bm[q];
       bq += s_bq[q];
     }
     if (bc > *(volatile uint32_t*)&ctl->row_smax) atomicMax(&ctl->row_smax, bc);
@@ -590,27 +703,29 @@ __global__ void __launch_bounds__(256) k_rows_build(const uint32_t* __restrict__
     if (bp) atomicAdd(&ctl->pfx_total, (unsigned long long)bp);
     if (bl) atomicAdd(&ctl->slot_total, (unsigned long long)bl);
     if (bx) ctl->mixed_len = 1u;
+    if (bm) atomicAdd(&ctl->mov_total, (unsigned long long)bm);
     if (bq) atomicAdd(&ctl->lay_sum, bq);
   }
 }
 
-// Layout start: the owner counts cleared and, for permuted rows, the axons
-// fully lit in the last tick the rows saw (the lit bitmap it left) taken as
-// the lit set of the layout (the prologue checks every tick that they still
-// are).
-__global__ void __launch_bounds__(256) k_rows_prep(const ShardCtl* __restrict__ ctl, uint32_t* __restrict__ mult,
-                                                   uint32_t A, const uint32_t* __restrict__ lit,
+// Layout start: the axon words cleared and, for permuted rows, the axons
+// that were fully lit in every one of the last ticks the rows saw (up to
+// kLitWindow of them: one that flickers would send every tick it is dark to the
+// dense pass) taken as the lit set of the layout (the prologue checks every tick
+// that they still are).
+__global__ void __launch_bounds__(256) k_rows_prep(const ShardCtl* __restrict__ ctl, uint32_t* __restrict__ axw,
+                                                   uint32_t A, const uint32_t* __restrict__ alit,
                                                    uint32_t* __restrict__ xlit, uint32_t cond) {
   if (cond && !ctl->lay_now) return;
   const uint32_t words = A / 32 + 1;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < A; i += gridDim.x * blockDim.x) {
-    mult[i] = 0u;
-    if (xlit && i < words) xlit[i] = lit[i];
+    axw[i] = 0u;
+    if (xlit && i < words) xlit[i] = alit[i];
   }
 }
 
 __global__ void __launch_bounds__(256) k_rows_mult(const uint32_t* __restrict__ s2a, uint32_t N, uint32_t A,
-                                                   uint32_t* __restrict__ mult, uint2* __restrict__ mask2,
+                                                   uint32_t* __restrict__ axw, uint2* __restrict__ mask2,
                                                    ShardCtl* __restrict__ ctl, uint32_t cond) {
   if (cond && !ctl->lay_now) return;
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -623,36 +738,87 @@ __global__ void __launch_bounds__(256) k_rows_mult(const uint32_t* __restrict__ 
     ctl->pfx_total = 0;
     ctl->slot_total = 0;
     ctl->mixed_len = 0;
+    ctl->mov_total = 0;
     ctl->lay_sum = 0;   // the index holds while the layout it was built from does (checksum)
   }
   if (n >= N) return;
   const uint32_t a = s2a[n];
-  if (a < A) atomicAdd(&mult[a], 1u);
+  if (a < A && (atomicOr(&axw[a], kAxOwned) & kAxOwned)) atomicOr(&axw[a], kAxShared);
 }
 
-// Batch end: weights rows -> columnar, a thread per neuron.  The k-th set bit
-// of omask[n] (a columnar slot q) is row position k: the row's first group,
-// the only slots whose weights GSOP can have changed.  A neuron without such
-// slots (every neuron of a frozen row) costs one 16-byte load, so in a brain
-// whose weights have mostly frozen the write-back reads 16 bytes a neuron
-// instead of a tile's rows.  Where every slot is movable, neighbouring threads
-// write the same slot of neighbouring neurons: 64 contiguous bytes a warp.
+// Batch end: weights rows -> columnar.  The slots of lmask[n] (in slot order) and
+// then the others of omask[n] are the row's first positions, the only slots
+// whose weights GSOP can have changed.  A thread per neuron where few are (a
+// neuron without any, every one of a frozen row, costs one 16-byte load: 19 us at
+// 1.5M settled neurons); a block with a neuron that has more than 8 goes
+// through shared memory, 32 neurons at a time: rows read whole, columns written
+// 64 bytes a warp.
 __global__ void __launch_bounds__(256) k_rows_writeback(int16_t* __restrict__ weights, uint32_t N,
                                                         const int16_t* __restrict__ rw,
-                                                        const uint4* __restrict__ omask) {
-  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const uint4 om = omask[n];
-  const uint32_t o[4] = {om.x, om.y, om.z, om.w};
-  const int16_t* row = rw + (size_t)n * kRowStride;
-  uint32_t k = 0;
+                                                        const uint4* __restrict__ omask,
+                                                        const uint4* __restrict__ lmask) {
+  __shared__ int16_t s_w[AXC_MAX_DENDRITES][34];
+  __shared__ uint32_t s_m[32][4];
+  const uint32_t nb = blockIdx.x * 256u, n = nb + threadIdx.x;
+  const uint4 om = n < N ? omask[n] : make_uint4(0, 0, 0, 0);
+  const uint32_t mine = __popc(om.x) + __popc(om.y) + __popc(om.z) + __popc(om.w);
+  if (!__syncthreads_or(mine > 8u)) {
+    if (!mine) return;
+    const uint4 lm = lmask[n];
+    const uint32_t o[4] = {om.x, om.y, om.z, om.w}, x[4] = {lm.x, lm.y, lm.z, lm.w};
+    const int16_t* row = rw + (size_t)n * kRowStride;
+    uint32_t k = 0;
 #pragma unroll
-  for (int ch = 0; ch < 4; ch++) {
-    uint32_t b = o[ch];
-    while (b) {
-      const uint32_t q = 32u * ch + (uint32_t)(__ffs(b) - 1);
-      b &= b - 1u;
-      weights[(size_t)q * N + n] = row[k++];
+    for (int pass = 0; pass < 2; pass++) {
+#pragma unroll
+      for (int ch = 0; ch < 4; ch++) {
+        uint32_t b = pass ? o[ch] & ~x[ch] : x[ch];
+        while (b) {
+          const uint32_t q = 32u * ch + (uint32_t)(__ffs(b) - 1);
+          b &= b - 1u;
+          weights[(size_t)q * N + n] = row[k++];
+        }
+      }
+    }
+    return;
+  }
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t t0 = 0; t0 < 256u && nb + t0 < N; t0 += 32u) {
+    int16_t v[4][4];   // four neurons a warp, every load first
+    uint32_t m[4][4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const uint32_t nn = nb + t0 + warp * 4u + e;
+      const uint4 a = nn < N ? omask[nn] : make_uint4(0, 0, 0, 0), b = nn < N ? lmask[nn] : make_uint4(0, 0, 0, 0);
+      const uint32_t o[4] = {a.x, a.y, a.z, a.w}, x[4] = {b.x, b.y, b.z, b.w};
+      uint32_t px = 0, po = popc4(x);
+#pragma unroll
+      for (int ch = 0; ch < 4; ch++) {
+        m[e][ch] = o[ch];
+        const uint32_t rest = o[ch] & ~x[ch], below = (1u << lane) - 1u;
+        const uint32_t pos = ((x[ch] >> lane) & 1u) ? px + __popc(x[ch] & below) : po + __popc(rest & below);
+        v[e][ch] = ((o[ch] >> lane) & 1u) ? rw[(size_t)nn * kRowStride + pos] : (int16_t)0;
+        px += __popc(x[ch]);
+        po += __popc(rest);
+      }
+    }
+    __syncthreads();   // the previous 32 are written
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+#pragma unroll
+      for (int ch = 0; ch < 4; ch++) {
+        s_w[32u * ch + lane][warp * 4u + e] = v[e][ch];
+        if (lane == 0) s_m[warp * 4u + e][ch] = m[e][ch];
+      }
+    }
+    __syncthreads();
+    uint32_t c[4];
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) c[ch] = s_m[lane][ch];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const uint32_t r = warp + 8u * i;
+      if ((c[i >> 2] >> (r & 31u)) & 1u) weights[(size_t)r * N + nb + t0 + lane] = s_w[r][lane];
     }
   }
 }
@@ -699,6 +865,12 @@ __device__ __forceinline__ void learn_axons(const LearnDev& L, uint32_t i, uint3
   if (sparse && act) L.alist[(size_t)j * 1024u + s_base2 + s_red[2][w] + __popc(ball & ((1u << lane) - 1u))] = i;
 }
 
+// 32 axons' bits of the window of always-lit axons (RowCache::alit).
+__device__ __forceinline__ void always_lit(uint32_t* word, uint32_t lit, uint32_t first) {
+  if (first) *word = lit;
+  else if (lit != 0xFFFFFFFFu) atomicAnd(word, lit);
+}
+
 // Counts a prologue block's evaluated neurons and active axons of tick k with
 // one atomic; returns the block's first position in the evaluated list.
 __device__ __forceinline__ uint32_t append_count(ShardCtl* ctl, uint32_t k, uint32_t eval, uint32_t act) {
@@ -719,14 +891,15 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
                                                        const uint32_t* __restrict__ bitmask, uint32_t voff,
                                                        uint32_t nv, uint32_t* __restrict__ incoming,
                                                        const uint32_t* __restrict__ batch_counts, uint32_t k,
-                                                       uint2* __restrict__ mask2, const uint32_t* __restrict__ mult,
+                                                       uint2* __restrict__ mask2, const uint32_t* __restrict__ axw,
                                                        uint8_t* __restrict__ flags, uint8_t* __restrict__ timers,
                                                        uint32_t N, uint32_t* __restrict__ eval,
                                                        ShardCtl* __restrict__ ctl, uint32_t raise_err,
                                                        uint32_t* __restrict__ lit_bits, LearnDev L,
                                                        uint32_t* __restrict__ pend_apply,
                                                        const uint32_t* __restrict__ xlit,
-                                                       uint32_t* __restrict__ live, uint32_t* __restrict__ evb) {
+                                                       uint32_t* __restrict__ live, uint32_t* __restrict__ evb,
+                                                       uint32_t* __restrict__ alit, uint32_t alit_new) {
   __shared__ uint32_t s_base;
   __shared__ uint32_t s_warp[8], s_act[8];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -741,7 +914,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     const uint4* p = reinterpret_cast<const uint4*>(heads + i);
     hx = p[0];
     hy = p[1];
-    own = __ldg(mult + i);
+    own = __ldg(axw + i);
     if (pend_apply) pc = pend_apply[i];   // the previous tick's soma pushes (pushes commute)
     if (bitmask) {
       const uint32_t v = i - voff;
@@ -749,8 +922,6 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     }
   }
   const uint32_t pmax = ctl->pmax, seg_max = ctl->seg_max;
-  const uint32_t hi = min(seg_max, 30u);   // segments 1..hi are the ones the batch's slots use
-  const uint32_t need = hi ? (((2u << hi) - 1u) & ~1u) : 0xFFFFFFFFu;
   // segments the batch's slots use: 0..seg_max (bit 31: any segment >= 31)
   const uint32_t act = seg_max >= 31u ? 0xFFFFFFFFu : ((2u << seg_max) - 1u);
   const bool inc = batch_counts && batch_counts[k] > 0;
@@ -777,12 +948,12 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     uint4* p = reinterpret_cast<uint4*>(heads + i);
     p[0] = make_uint4(h[0], h[1], h[2], h[3]);
     p[1] = make_uint4(h[4], h[5], h[6], h[7]);
-    const uint2 m = split_masks(h, pmax, own);
+    const uint2 m = split_masks(h, pmax, ax_owners(own));
     mask2[i] = m;
-    // fully lit: heads 0..6 hit every segment 1..seg_max the batch uses and at
+    // fully lit: heads 0..6 hit every segment 1..30 the axon's slots use and at
     // most one soma owns the axon, so for those segments the hit is 1 and one
     // push cannot change it
-    lit = (m.x & need) == need && !(m.y >> 31);
+    lit = (m.x & own & kAxSegs) == (own & kAxSegs) && !(m.y >> 31);
     if (LEARN) {
       // active: some head covers a segment that a slot of the batch uses
       on = ((m.x | (m.y & 0x7FFFFFFFu)) & act) != 0u;
@@ -796,6 +967,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     const uint32_t lb = __ballot_sync(kFull, lit);
     if ((threadIdx.x & 31) == 0 && i < A) {
       lit_bits[i >> 5] = lb;
+      always_lit(alit + (i >> 5), lb, alit_new);
       if (xw & ~lb) atomicOr(&ctl->dense[k & 1], 1u);   // the lit-sum form cannot run this tick
     }
   }
@@ -1197,6 +1369,293 @@ __device__ __forceinline__ uint32_t row_gsop(uint2 (&W)[4], uint32_t hitb, uint3
   return gdone;
 }
 
+// The hit test of one slot as the 8-lane pass makes it (row_slots): the
+// fully-lit shortcut for segments 1..seg_hi of variants whose length is the LUT
+// maximum (<= 16), else the tick's split masks and, where they do not decide,
+// the eight heads.  *fast: GSOP may take the slot's delta from the gtab table
+// (the hit decides and one same-tick push cannot change it).
+__device__ __forceinline__ bool slot_hit(uint32_t t, bool exact, bool gfast, uint32_t prop, uint32_t seg_hi,
+                                         const uint32_t* __restrict__ lit_bits, const uint2* __restrict__ mask2,
+                                         const BurstHeads8* heads, uint32_t A, bool* fast) {
+  const uint32_t s = t >> AXC_TARGET_SEG_SHIFT;
+  const uint32_t ax = (t & AXC_TARGET_AXON_MASK) - 1u;   // invalid ids were redirected to A (dummy mask entry)
+  if (gfast && (s - 1u) < seg_hi && ((__ldg(lit_bits + (ax >> 5)) >> (ax & 31u)) & 1u)) {
+    *fast = true;
+    return true;
+  }
+  const uint2 m = __ldg(mask2 + ax);
+  const uint32_t sh = min(s, 31u);
+  const uint32_t bx = (m.x >> sh) & 1u, by = (m.y >> sh) & 1u;
+  bool hit = (bx | by) != 0u;
+  if (hit && (s >= 31u || !exact)) hit = hit_exact(heads, A, ax, s, prop);
+  *fast = gfast && s < 31u && !(m.y >> 31) && (bx || by == (s == 0u));
+  return hit;
+}
+
+// GSOP (physics.cu:281-373) of row position q of spiker n, weight w16, target
+// *t: the rank's delta where the hit decides (fast), else the exact path or the
+// fix-up list.  Returns the slots done (0: an invalid target).
+template <bool WT>
+__device__ __forceinline__ uint32_t gsop_slot(int16_t w16, const uint32_t* t, int16_t* w, bool hit, bool fast,
+                                              const int2* gtab_v, const BurstHeads8* heads, const uint2* mask2,
+                                              uint32_t A, const VariantParameters& p, uint8_t flags, int32_t dopamine,
+                                              ShardCtl* ctl, uint32_t* fix, uint32_t fix_cap, uint32_t n, uint32_t q,
+                                              const ColWT& wt) {
+  int16_t nw = w16;
+  if (fast) {
+    const int32_t aw = w16 < 0 ? -(int32_t)w16 : (int32_t)w16;
+    const int2 e = gtab_v[min((uint32_t)aw >> 11, 15u)];
+    int32_t na = aw + (hit ? e.x : -e.y);
+    na = min(max(na, 0), 32767);
+    nw = (int16_t)(w16 < 0 ? -na : na);
+  } else {
+    const uint32_t tt = *t;
+    const int r = gsop_general(heads, mask2, A, (tt & AXC_TARGET_AXON_MASK) - 1u, tt >> AXC_TARGET_SEG_SHIFT, p, flags,
+                               dopamine, &nw);
+    if (r == 2) return 0u;
+    if (r == 1) {
+      const uint32_t slot = atomicAdd(&ctl->fix_count, 1u);
+      if (slot < fix_cap) fix[slot] = (uint32_t)((size_t)n * kRowStride + q);
+      else ctl->fix_overflow = 1u;
+      return 1u;
+    }
+  }
+  if (nw != w16) {
+    *w = nw;
+    if (WT) col_write(wt, n, q, nw);
+  }
+  return 1u;
+}
+
+struct LsumCount {
+  uint32_t ev_slots, hits, nspk, gdone, nev, err, tested, same;
+};
+
+// The state of a neuron after GLIF and its spike's push.
+__device__ __forceinline__ void neuron_store(const ShardVramPtrs& P, uint32_t n, const GlifOut& o, uint8_t flags,
+                                             const VariantParameters& p, uint32_t my_axon, uint32_t A, uint32_t* pend,
+                                             LsumCount& k) {
+  P.soma_voltage[n] = o.v;
+  P.soma_flags[n] = (uint8_t)((flags & 0xF0) | (o.spike ? 0x05 : 0x00));
+  P.threshold_offset[n] = o.thr;
+  P.timers[n] = o.glif ? p.refractory_period : 0;
+  if (!o.spike) return;
+  k.nspk++;
+  if (my_axon != AXC_NO_AXON) {
+    if (my_axon < A) atomicAdd(&pend[my_axon], 1u);
+    else k.err |= AXC_ERR_SOMA_AXON;
+  }
+}
+
+// GSOP of a movable lit slot: a hit within the first 16 segments' cooling step,
+// so the weight takes its rank's potentiation.
+__device__ __forceinline__ int16_t gsop_lit(int16_t w16, const int2* gtab_v) {
+  const int32_t aw = w16 < 0 ? -(int32_t)w16 : (int32_t)w16;
+  int32_t na = aw + gtab_v[min((uint32_t)aw >> 11, 15u)].x;
+  na = min(max(na, 0), 32767);
+  return (int16_t)(w16 < 0 ? -na : na);
+}
+
+// GSOP of two movable lit slots in one register (gsop_lit for each half), for
+// potentiations 0..16383 (tab: per rank 0..16, in the low half): |w| is w xor its
+// sign mask plus one where negative, the sums stay below 2^16, and a weight that
+// was negative stays at least 1 in size, so no half carries into the other.
+__device__ __forceinline__ uint32_t gsop_lit2(uint32_t w, const uint32_t* tab) {
+  uint32_t s;   // 0xFFFF in a negative half (prmt with the sign-replicating selectors 8 + byte)
+  asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(s) : "r"(w));
+  const uint32_t aw = (w ^ s) + (s & 0x00010001u);
+  const uint32_t d = __byte_perm(tab[(aw >> 11) & 31u], tab[aw >> 27], 0x5410);
+  const uint32_t na = __vminu2(aw + d, 0x7FFF7FFFu);
+  return (na ^ s) + (s & 0x00010001u);
+}
+
+// One step of the lit rows, 8 lanes per neuron: lane g8 holds row positions
+// 64 r + 8 g8 .. + 7 (r = 0, 1), the movable slots' weights in two 16-byte
+// registers.  VERIFY: the row's lit slots are looked up in the tick's fully-lit
+// bitmap (s_lit; lit_on false: not there); a row with a dark one is tested slot
+// by slot.  tab (null: some potentiation does not fit) serves GSOP two slots at a
+// time.  All 32 lanes take part.
+// Bound by instructions: 12.3M movable lit slots a tick (512k neurons, 96 slots,
+// a quarter evaluated) cost ~15 each with the look-up, where the slot-by-slot
+// pass spent ~85.
+template <bool VERIFY, bool WT>
+__device__ __forceinline__ void lit_row_step(const ShardVramPtrs& P, uint32_t A, const uint32_t* __restrict__ rt,
+                                             int16_t* __restrict__ rw, const uint16_t* __restrict__ cnt,
+                                             const uint2* __restrict__ mask2, uint32_t* __restrict__ pend,
+                                             uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl, uint32_t fix_cap,
+                                             const int2* __restrict__ rec, const ColWT& wt,
+                                             const VariantParameters* lut, const int2 (*gtab)[16],
+                                             const uint32_t (*tab)[17], uint32_t pmax, uint32_t smax, uint32_t tick,
+                                             int32_t dopamine, uint32_t n, bool valid, const uint32_t* s_lit,
+                                             bool lit_on, LsumCount& kc) {
+  const uint32_t g8 = threadIdx.x & 7u;
+  // every load of the neuron at once; the movable slots are most of the row
+  const uint8_t flags = P.soma_flags[n];
+  const uint32_t cw = cnt[n];
+  const int2 ls = __ldg(rec + n);
+  const int32_t thr0 = P.threshold_offset[n];
+  const int32_t v0 = P.soma_voltage[n];
+  const uint32_t my_axon = __ldg(P.soma_to_axon + n);
+  const uint32_t* rt_n = rt + (size_t)n * kRowStride;
+  int16_t* rw_n = rw + (size_t)n * kRowStride;
+  uint4 W[2], T[VERIFY ? 4 : 1];
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const bool in = 64u * r + 8u * g8 < smax;
+    W[r] = in ? *reinterpret_cast<const uint4*>(rw_n + 64 * r + 8 * g8) : make_uint4(0, 0, 0, 0);
+    if (VERIFY) {
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+        T[2 * r + x] = in ? __ldg(reinterpret_cast<const uint4*>(rt_n + 64 * r + 8 * g8) + x) : make_uint4(0, 0, 0, 0);
+    }
+  }
+  const uint32_t c = cw & 0xFFu, y = (uint32_t)ls.y;
+  const uint32_t lm = y & 0xFFu, lf = (y >> 8) & 0xFFu, end = (y >> 16) & 0xFFu;
+  const uint32_t var = flags >> 4;
+  const VariantParameters& p = lut[var];
+  const uint32_t prop = p.signal_propagation_length;
+  const bool exact = prop == pmax;
+  const bool gfast = exact && prop <= 16u;
+  int32_t i_in = g8 == 0 ? ls.x : 0;
+  uint32_t all_lit = 1u;   // bit 0: every lit slot looked up so far is on a fully-lit axon
+  // movable lit slots: positions 0 .. lm - 1
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const uint32_t q0 = 64u * r + 8u * g8;
+    if (q0 + 8u <= lm) {
+#pragma unroll
+      for (int h = 0; h < 4; h++) i_in = __dp2a_lo((int)word_of(W[r], h), 0x0101, i_in);
+      if (VERIFY && lit_on) {
+#pragma unroll
+        for (int h = 0; h < 8; h++) {
+          const uint32_t u = word_of(T[2 * r + (h >> 2)], h & 3) - 1u;   // axon in the low 24 bits
+          all_lit &= s_lit[(u & AXC_TARGET_AXON_MASK) >> 5] >> (u & 31u);
+        }
+      }
+    } else if (q0 < lm) {
+#pragma unroll 1
+      for (uint32_t q = q0; q < lm; q++) {
+        i_in = wadd(i_in, (int32_t)rw_n[q]);
+        if (VERIFY && lit_on) {
+          const uint32_t u = __ldg(rt_n + q) - 1u;
+          all_lit &= s_lit[(u & AXC_TARGET_AXON_MASK) >> 5] >> (u & 31u);
+        }
+      }
+    }
+  }
+  bool dark = false;   // the row is tested slot by slot
+  if (VERIFY) {
+    // the frozen lit slots end .. c - 1 (few or none where most slots move)
+    if (lit_on)
+      for (uint32_t q = end + g8; q < c; q += 8u) {
+        const uint32_t u = __ldg(rt_n + q) - 1u;
+        all_lit &= s_lit[(u & AXC_TARGET_AXON_MASK) >> 5] >> (u & 31u);
+      }
+    const uint32_t b = __ballot_sync(kFull, !lit_on || !(all_lit & 1u));
+    dark = (b >> (threadIdx.x & 24u)) & 0xFFu;
+  }
+  // tested slots: positions lm .. end - 1, one a lane; of a dark row every slot
+  const uint32_t q0 = dark ? 0u : lm, nt = dark ? c : end - lm;
+  if (dark) i_in = 0;
+  uint32_t hb = 0, fb = 0;   // bit r: this lane's r-th tested slot is a hit / in GSOP's fast class
+  // four a lane at a time, each load of the four before any is waited for (slot
+  // -> mask is a chain of two cache misses, and one such row in a warp's slice
+  // would hold up its block)
+  for (uint32_t x0 = 0; x0 < nt; x0 += 32u) {
+    uint32_t t[4];
+    int32_t w[4];
+    uint2 m[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const uint32_t x = x0 + 8u * u + g8;
+      t[u] = x < nt ? __ldg(rt_n + q0 + x) : 0u;
+      w[u] = x < nt ? (int32_t)rw_n[q0 + x] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)   // invalid ids were redirected to A (dummy mask entry)
+      m[u] = x0 + 8u * u + g8 < nt ? __ldg(mask2 + (t[u] & AXC_TARGET_AXON_MASK) - 1u) : make_uint2(0, 0);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (x0 + 8u * u + g8 >= nt) continue;
+      const uint32_t s = t[u] >> AXC_TARGET_SEG_SHIFT, sh = min(s, 31u);
+      const uint32_t bx = (m[u].x >> sh) & 1u, by = (m[u].y >> sh) & 1u;
+      bool hit = (bx | by) != 0u;              // bit 31 (s >= 31): "may hit", tested below
+      if (hit && (s >= 31u || !exact)) hit = hit_exact(P.axon_heads, A, (t[u] & AXC_TARGET_AXON_MASK) - 1u, s, prop);
+      const uint32_t bit = 1u << (x0 / 8u + u);
+      if (hit) {
+        i_in = wadd(i_in, w[u]);
+        hb |= bit;
+      }
+      fb |= gfast && s < 31u && !(m[u].y >> 31) && (bx || by == (s == 0u)) ? bit : 0u;
+    }
+  }
+  i_in = wadd(i_in, __shfl_xor_sync(kFull, i_in, 1));
+  i_in = wadd(i_in, __shfl_xor_sync(kFull, i_in, 2));
+  i_in = wadd(i_in, __shfl_xor_sync(kFull, i_in, 4));
+  if (!valid) return;
+  kc.hits += __popc(hb);
+  const GlifOut o = glif_step(p, v0, thr0, i_in, tick, n);
+  if (g8 == 0) {
+    if (cw & kRowBad) kc.err |= AXC_ERR_TARGET_RANGE;
+    kc.ev_slots += c;
+    if (!dark) kc.hits += (c - end) + lm;
+    kc.tested += nt;
+    kc.nev++;
+    neuron_store(P, n, o, flags, p, my_axon, A, pend, kc);
+    if (o.spike) kc.gdone += (c - lf) + (dark ? 0u : lm);   // the frozen slots are left as they are
+  }
+  if (!o.spike) return;
+  if (!dark) {
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const uint32_t qr = 64u * r + 8u * g8;
+      if (qr + 8u <= lm && tab) {
+        const uint4 nw = make_uint4(gsop_lit2(W[r].x, tab[var]), gsop_lit2(W[r].y, tab[var]),
+                                    gsop_lit2(W[r].z, tab[var]), gsop_lit2(W[r].w, tab[var]));
+        kc.same += 0x10000u;   // groups visited << 16 | left as they were
+        if (nw.x == W[r].x && nw.y == W[r].y && nw.z == W[r].z && nw.w == W[r].w) {
+          kc.same++;
+          continue;
+        }
+        *reinterpret_cast<uint4*>(rw_n + qr) = nw;
+        if (WT) {
+#pragma unroll 1
+          for (uint32_t h = 0; h < 8; h++) {
+            const int16_t a = (int16_t)(word_of(nw, h >> 1) >> (16u * (h & 1u)));
+            if (a != (int16_t)(word_of(W[r], h >> 1) >> (16u * (h & 1u)))) col_write(wt, n, qr + h, a);
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (uint32_t q = qr; q < min(qr + 8u, lm); q++) {
+          const int16_t w16 = rw_n[q];
+          const int16_t nw = gsop_lit(w16, gtab[var]);
+          if (nw == w16) continue;
+          rw_n[q] = nw;
+          if (WT) col_write(wt, n, q, nw);
+        }
+      }
+    }
+  }
+  // the movable ones among the tested slots
+  const uint32_t mt = dark ? lf : lf - lm;
+  for (uint32_t x = g8, r = 0; x < mt; x += 8u, r++)
+    kc.gdone += gsop_slot<WT>(rw_n[q0 + x], rt_n + q0 + x, rw_n + q0 + x, (hb >> r) & 1u, (fb >> r) & 1u, gtab[var],
+                              P.axon_heads, mask2, A, p, flags, dopamine, ctl, fix, fix_cap, n, q0 + x, wt);
+}
+
+// The potentiations of gtab for gsop_lit2; false (in every thread) when one does
+// not fit.  Called by all threads of the block.
+__device__ __forceinline__ bool build_ptab(uint32_t (*tab)[17], const int2 (*gtab)[16]) {
+  bool ok = true;
+  for (uint32_t i = threadIdx.x; i < 16u * 17u; i += blockDim.x) {
+    const int32_t x = gtab[i / 17u][min(i % 17u, 15u)].x;
+    ok = ok && x >= 0 && x <= 16383;
+    tab[i / 17u][i % 17u] = (uint32_t)x;
+  }
+  return __syncthreads_and(ok);
+}
+
 // LIT: 1024-thread blocks (one per SM) that first copy the prologue's
 // fully-lit bitmap (one bit per axon) into shared memory; slots whose axon is
 // fully lit need no mask gather from L2.
@@ -1211,7 +1670,8 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
                   const uint32_t* __restrict__ eval, uint32_t* __restrict__ pend, uint32_t* __restrict__ fix,
                   ShardCtl* __restrict__ ctl, uint32_t k, uint32_t fix_cap, const uint32_t* __restrict__ lit_bits,
                   const LearnCtl* __restrict__ lc, uint32_t* __restrict__ gs_n, uint32_t* __restrict__ gd_n,
-                  const uint8_t* __restrict__ lfz, uint32_t* __restrict__ wcnt, ColWT wt, uint32_t index) {
+                  const uint8_t* __restrict__ lfz, uint32_t* __restrict__ wcnt, ColWT wt, uint32_t index,
+                  const int2* __restrict__ rec) {
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
@@ -1219,7 +1679,8 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   extern __shared__ __align__(128) uint32_t s_lit[];
   chain_wait();
   chain_open();
-  if (tick_form(ctl, k, lc, index) != kFormDense) return;                    // k_rows_update_lsum or the learned engine's kernels run this tick
+  const TickForm form = tick_form(ctl, k, lc, index);
+  if (form != kFormDense && form != kFormLitRows && form != kFormVerify) return;                    // k_rows_update_lsum or the learned engine's kernels run this tick
   if (LIT && threadIdx.x == 0) mbar_init(&s_bar, 1);
   lut_to_smem(lut);
   if (threadIdx.x == 0) s_pmax = lut_pmax();
@@ -1245,12 +1706,40 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   uint32_t ev_slots = 0, hits = 0, nspk = 0, gdone = 0, nev = 0, err = 0;
   uint32_t wc = 0, wd = 0;   // spikers this warp listed for the GSOP passes
   uint32_t same = 0;         // row_gsop
+  uint32_t beg_dense = beg, lit_tested = 0;
   bool lit_on = true;
   if (LIT) {
     lit_on = mbar_wait_bounded(&s_bar, 0, g_first_wait_limit);
     if (!lit_on) err |= AXC_ERR_WAIT_LIMIT;   // then without the shortcut (results exact)
   }
-  for (uint32_t base = beg; base < end; base += 32) {
+  if (form != kFormDense) {
+    __shared__ uint32_t ptab[16][17];
+    const bool packed = build_ptab(ptab, gtab);
+    LsumCount kc = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (form == kFormVerify) {
+      for (uint32_t i0 = beg; i0 < end; i0 += 4)
+        lit_row_step<true, WT>(P, A, rt, rw, cnt, mask2, pend, fix, ctl, fix_cap, rec, wt, lut, gtab,
+                               packed ? ptab : nullptr, s_pmax, smax, tick, dopamine,
+                               __ldg(eval + min(i0 + grp, end - 1u)), i0 + grp < end, LIT ? s_lit : lit_bits, lit_on,
+                               kc);
+    } else {
+      if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ctr[6] += 1;   // ticks on the lit-sum form
+      for (uint32_t i0 = beg; i0 < end; i0 += 4)
+        lit_row_step<false, WT>(P, A, rt, rw, cnt, mask2, pend, fix, ctl, fix_cap, rec, wt, lut, gtab,
+                                packed ? ptab : nullptr, s_pmax, smax, tick, dopamine,
+                                __ldg(eval + min(i0 + grp, end - 1u)), i0 + grp < end, nullptr, false, kc);
+      lit_tested = kc.tested;
+    }
+    ev_slots = kc.ev_slots;
+    hits = kc.hits;
+    nspk = kc.nspk;
+    gdone = kc.gdone;
+    nev = kc.nev;
+    err |= kc.err;
+    same = kc.same;
+    beg_dense = end;
+  }
+  for (uint32_t base = beg_dense; base < end; base += 32) {
     const uint32_t mine = (base + lane < end) ? __ldg(eval + base + lane) : 0u;
     for (uint32_t sub = 0; sub < 32 && base + sub < end; sub += 4) {
       const bool valid = base + sub + grp < end;
@@ -1338,6 +1827,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   block_count(ev_slots, hits, nspk, &ctl->ctr[1]);
   block_count(gdone, nev, 0, &ctl->ctr[4]);
   if (INLINE) block_count(same & 0xFFFFu, same >> 16, 0, ctl->gsop_same);
+  if (form == kFormLitRows) block_count(lit_tested, 0, 0, &ctl->ctr[7]);
 }
 
 // Sums six per-thread counters over a 256-thread block into ctr[1..5] and
@@ -1360,64 +1850,6 @@ __device__ __forceinline__ void block_count256(uint32_t a1, uint32_t a2, uint32_
     for (int q = 0; q < 8; q++) sum += red[threadIdx.x][q];
     if (sum) atomicAdd(ctr + (threadIdx.x == 5 ? 7 : threadIdx.x + 1), sum);
   }
-}
-
-// The hit test of one slot as the 8-lane pass makes it (row_slots): the
-// fully-lit shortcut for segments 1..seg_hi of variants whose length is the LUT
-// maximum (<= 16), else the tick's split masks and, where they do not decide,
-// the eight heads.  *fast: GSOP may take the slot's delta from the gtab table
-// (the hit decides and one same-tick push cannot change it).
-__device__ __forceinline__ bool slot_hit(uint32_t t, bool exact, bool gfast, uint32_t prop, uint32_t seg_hi,
-                                         const uint32_t* __restrict__ lit_bits, const uint2* __restrict__ mask2,
-                                         const BurstHeads8* heads, uint32_t A, bool* fast) {
-  const uint32_t s = t >> AXC_TARGET_SEG_SHIFT;
-  const uint32_t ax = (t & AXC_TARGET_AXON_MASK) - 1u;   // invalid ids were redirected to A (dummy mask entry)
-  if (gfast && (s - 1u) < seg_hi && ((__ldg(lit_bits + (ax >> 5)) >> (ax & 31u)) & 1u)) {
-    *fast = true;
-    return true;
-  }
-  const uint2 m = __ldg(mask2 + ax);
-  const uint32_t sh = min(s, 31u);
-  const uint32_t bx = (m.x >> sh) & 1u, by = (m.y >> sh) & 1u;
-  bool hit = (bx | by) != 0u;
-  if (hit && (s >= 31u || !exact)) hit = hit_exact(heads, A, ax, s, prop);
-  *fast = gfast && s < 31u && !(m.y >> 31) && (bx || by == (s == 0u));
-  return hit;
-}
-
-// GSOP (physics.cu:281-373) of row position q of spiker n, weight w16, target
-// *t: the rank's delta where the hit decides (fast), else the exact path or the
-// fix-up list.  Returns the slots done (0: an invalid target).
-template <bool WT>
-__device__ __forceinline__ uint32_t gsop_slot(int16_t w16, const uint32_t* t, int16_t* w, bool hit, bool fast,
-                                              const int2* gtab_v, const BurstHeads8* heads, const uint2* mask2,
-                                              uint32_t A, const VariantParameters& p, uint8_t flags, int32_t dopamine,
-                                              ShardCtl* ctl, uint32_t* fix, uint32_t fix_cap, uint32_t n, uint32_t q,
-                                              const ColWT& wt) {
-  int16_t nw = w16;
-  if (fast) {
-    const int32_t aw = w16 < 0 ? -(int32_t)w16 : (int32_t)w16;
-    const int2 e = gtab_v[min((uint32_t)aw >> 11, 15u)];
-    int32_t na = aw + (hit ? e.x : -e.y);
-    na = min(max(na, 0), 32767);
-    nw = (int16_t)(w16 < 0 ? -na : na);
-  } else {
-    const uint32_t tt = *t;
-    const int r = gsop_general(heads, mask2, A, (tt & AXC_TARGET_AXON_MASK) - 1u, tt >> AXC_TARGET_SEG_SHIFT, p, flags,
-                               dopamine, &nw);
-    if (r == 2) return 0u;
-    if (r == 1) {
-      const uint32_t slot = atomicAdd(&ctl->fix_count, 1u);
-      if (slot < fix_cap) fix[slot] = (uint32_t)((size_t)n * kRowStride + q);
-      else ctl->fix_overflow = 1u;
-      return 1u;
-    }
-  }
-  if (nw != w16) {
-    *w = nw;
-    if (WT) col_write(wt, n, q, nw);
-  }
-  return 1u;
 }
 
 // ---------------------------------------------------------------------------
@@ -1720,29 +2152,29 @@ __global__ void __launch_bounds__(256, kNeuronBlocks)
 }
 
 // ---------------------------------------------------------------------------
-// per tick 2/4, lit-sum form (lsum_tick: short tested prefixes, and every axon
-// the row layout took as fully lit is fully lit): a thread per evaluated
-// neuron.  Its input current is the row's lit-sum (frozen slots on fully-lit
-// axons with segments 1..30: hits whatever the tick, their weights summed once
-// per batch; the dendrite sum is a wrapping i32 sum, so the order cannot change
-// a bit) plus the hits among the first lsum[n].y row positions, tested as the
-// 8-lane pass tests them (physics.cu:182-206); GLIF (physics.cu:209-275); then
-// GSOP of a spiker's movable slots, the first lf positions (physics.cu:281-373),
-// from the gtab deltas, on the exact path or deferred to the fix-up stage.
+// per tick 2/4, lit-sum form (lsum_tick: few tested slots, and every axon the row
+// layout took as fully lit is fully lit).  An evaluated neuron's input current is
+// the row's lit-sum (frozen slots on fully-lit axons with segments 1..30: hits
+// whatever the tick, their weights summed once per layout; the dendrite sum is a
+// wrapping i32 sum, so the order cannot change a bit), plus the weights of its
+// movable lit slots (hits too), plus the hits among its tested slots, tested as
+// the 8-lane pass tests them (physics.cu:182-206); GLIF (physics.cu:209-275);
+// then GSOP of a spiker's movable slots (physics.cu:281-373): the lit ones take
+// their rank's potentiation, the tested ones the gtab deltas, the exact path or
+// the fix-up stage.  No target of a lit slot is read.
+// A thread per neuron, where few slots need work (a settled brain: 0.5 a
+// neuron); where many do (lit_rows) k_rows_update takes 8 lanes a neuron.
 // WT: weight changes written through to the columnar blob (per-tick entry point).
 // ---------------------------------------------------------------------------
 constexpr int kLsumBlocks = 5;   // resident 256-thread blocks per SM (48 registers a thread)
+
 template <bool WT>
-__global__ void __launch_bounds__(256, kLsumBlocks) k_rows_update_lsum(ShardVramPtrs P, uint32_t A, const uint32_t* __restrict__ rt,
-                                                          int16_t* __restrict__ rw, const uint16_t* __restrict__ cnt,
-                                                          const uint2* __restrict__ mask2,
-                                                          const uint32_t* __restrict__ eval, uint32_t* __restrict__ pend,
-                                                          uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl,
-                                                          uint32_t k, uint32_t fix_cap,
-                                                          const uint32_t* __restrict__ lit_bits,
-                                                          const uint8_t* __restrict__ lfz,
-                                                          const int2* __restrict__ lsum, ColWT wt,
-                                                          const LearnCtl* __restrict__ lc) {
+__global__ void __launch_bounds__(256, kLsumBlocks)
+    k_rows_update_lsum(ShardVramPtrs P, uint32_t A, const uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
+                       const uint16_t* __restrict__ cnt, const uint2* __restrict__ mask2,
+                       const uint32_t* __restrict__ eval, uint32_t* __restrict__ pend, uint32_t* __restrict__ fix,
+                       ShardCtl* __restrict__ ctl, uint32_t k, uint32_t fix_cap, const uint32_t* __restrict__ lit_bits,
+                       const int2* __restrict__ rec, ColWT wt, const LearnCtl* __restrict__ lc) {
   chain_wait();
   chain_open();
   if (tick_form(ctl, k, lc, 0u) != kFormLitSum) return;
@@ -1760,38 +2192,39 @@ __global__ void __launch_bounds__(256, kLsumBlocks) k_rows_update_lsum(ShardVram
   __syncthreads();
   const uint32_t tick = ctl->tick_base + k;
   const uint32_t seg_hi = min(ctl->seg_max, 30u);
-  uint32_t ev_slots = 0, hits = 0, nspk = 0, gdone = 0, nev = 0, err = 0, tested = 0;
+  LsumCount kc = {0, 0, 0, 0, 0, 0, 0, 0};
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ecount; i += gridDim.x * blockDim.x) {
     const uint32_t n = eval[i];
     // every load of the neuron at once
     const uint8_t flags = P.soma_flags[n];
     const uint32_t cw = cnt[n];
-    const uint32_t lf = lfz[n];
-    const int2 ls = lsum[n];
+    const int2 ls = rec[n];
     const int32_t thr0 = P.threshold_offset[n];
     const int32_t v0 = P.soma_voltage[n];
     const uint32_t my_axon = P.soma_to_axon[n];
-    const uint32_t c = cw & 0xFFu, pfx = (uint32_t)ls.y;
+    const uint32_t c = cw & 0xFFu, y = (uint32_t)ls.y;
+    const uint32_t lm = y & 0xFFu, lf = (y >> 8) & 0xFFu, end = (y >> 16) & 0xFFu;
     const uint32_t var = flags >> 4;
     const VariantParameters& p = lut[var];
     const uint32_t prop = p.signal_propagation_length;
     const bool exact = prop == s_pmax;
     const bool gfast = exact && prop <= 16u;
-    if (cw & kRowBad) err |= AXC_ERR_TARGET_RANGE;
+    if (cw & kRowBad) kc.err |= AXC_ERR_TARGET_RANGE;
     const uint32_t* rt_n = rt + (size_t)n * kRowStride;
     int16_t* rw_n = rw + (size_t)n * kRowStride;
     int32_t i_in = ls.x;
-    uint32_t h = c - pfx;   // the lit-sum slots are hits
+    uint32_t h = c - end;   // the lit-sum slots are hits
     // the tests of row positions 0..31 (the movable slots come first), kept for GSOP
     uint32_t hit_bits = 0, fast_bits = 0;
-    for (uint32_t q = 0; q < pfx; q += 4) {
+    for (uint32_t q = 0; q < end; q += 4) {
       const uint4 T4 = *reinterpret_cast<const uint4*>(rt_n + q);
       const uint2 W4 = *reinterpret_cast<const uint2*>(rw_n + q);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        if (q + j >= pfx) break;
-        bool fast;
-        const bool hit = slot_hit(word_of(T4, j), exact, gfast, prop, seg_hi, lit_bits, mask2, P.axon_heads, A, &fast);
+        if (q + j >= end) break;
+        bool fast = true, hit = true;   // movable and lit
+        if (q + j >= lm)
+          hit = slot_hit(word_of(T4, j), exact, gfast, prop, seg_hi, lit_bits, mask2, P.axon_heads, A, &fast);
         if (hit) {
           i_in = wadd(i_in, (int32_t)half_of(W4, j));
           h++;
@@ -1801,39 +2234,31 @@ __global__ void __launch_bounds__(256, kLsumBlocks) k_rows_update_lsum(ShardVram
         fast_bits |= fast ? bit : 0u;
       }
     }
-    ev_slots += c;
-    hits += h;
-    tested += pfx;
-    nev++;
+    kc.ev_slots += c;
+    kc.hits += h;
+    kc.tested += end - lm;
+    kc.nev++;
     const GlifOut o = glif_step(p, v0, thr0, i_in, tick, n);
-    P.soma_voltage[n] = o.v;
-    P.soma_flags[n] = (uint8_t)((flags & 0xF0) | (o.spike ? 0x05 : 0x00));
-    P.threshold_offset[n] = o.thr;
-    P.timers[n] = o.glif ? p.refractory_period : 0;
+    neuron_store(P, n, o, flags, p, my_axon, A, pend, kc);
     if (!o.spike) continue;
-    nspk++;
-    if (my_axon != AXC_NO_AXON) {
-      if (my_axon < A) atomicAdd(&pend[my_axon], 1u);
-      else err |= AXC_ERR_SOMA_AXON;
-    }
     // GSOP (physics.cu:281-373) of the movable slots; the frozen ones are left as they are
-    gdone += c - lf;
+    kc.gdone += c - lf;
     for (uint32_t q = 0; q < lf; q++) {
       const int16_t w16 = rw_n[q];
-      bool fast, hit;
-      if (q < 32u) {   // tested in the prefix loop (lf <= pfx)
+      bool fast = true, hit = true;
+      if (q < 32u) {   // tested in the loop above (lf <= end)
         hit = (hit_bits >> q) & 1u;
         fast = (fast_bits >> q) & 1u;
-      } else {
+      } else if (q >= lm) {
         hit = slot_hit(rt_n[q], exact, gfast, prop, seg_hi, lit_bits, mask2, P.axon_heads, A, &fast);
       }
-      gdone += gsop_slot<WT>(w16, rt_n + q, rw_n + q, hit, fast, gtab[var], P.axon_heads, mask2, A, p, flags, dopamine,
-                             ctl, fix, fix_cap, n, q, wt);
+      kc.gdone += gsop_slot<WT>(w16, rt_n + q, rw_n + q, hit, fast, gtab[var], P.axon_heads, mask2, A, p, flags,
+                                dopamine, ctl, fix, fix_cap, n, q, wt);
     }
   }
-  const uint32_t err_any = __reduce_or_sync(kFull, err);
+  const uint32_t err_any = __reduce_or_sync(kFull, kc.err);
   if (err_any && (threadIdx.x & 31) == 0) atomicOr(&ctl->err, err_any);
-  block_count256(ev_slots, hits, nspk, gdone, nev, tested, ctl->ctr);
+  block_count256(kc.ev_slots, kc.hits, kc.nspk, kc.gdone, kc.nev, kc.tested, ctl->ctr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2209,7 +2634,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
                                                              uint32_t* __restrict__ incoming,
                                                              const uint32_t* __restrict__ batch_counts, uint32_t k,
                                                              uint2* __restrict__ mask2,
-                                                             const uint32_t* __restrict__ mult,
+                                                             const uint32_t* __restrict__ axw,
                                                              uint8_t* __restrict__ flags,
                                                              uint8_t* __restrict__ timers, uint32_t N,
                                                              uint32_t* __restrict__ eval, ShardCtl* __restrict__ ctl,
@@ -2218,7 +2643,8 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
                                                              uint32_t set_tick, uint32_t tick_base, int32_t dopamine,
                                                              const uint32_t* __restrict__ xlit,
                                                              uint32_t* __restrict__ live,
-                                                             uint32_t* __restrict__ evb) {
+                                                             uint32_t* __restrict__ evb, uint32_t* __restrict__ alit,
+                                                             uint32_t alit_new) {
   __shared__ uint32_t s_base;
   __shared__ uint32_t s_warp[ITEMS][8];   // evaluated neurons | active axons << 16
 
@@ -2242,7 +2668,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
       const uint4* p = reinterpret_cast<const uint4*>(heads + i);
       hx[r] = p[0];
       hy[r] = p[1];
-      own[r] = __ldg(mult + i);
+      own[r] = __ldg(axw + i);
       if (pend_apply) npush[r] = pend_apply[i];   // the previous tick's soma pushes
       if (bitmask) {
         const uint32_t v = i - voff;
@@ -2267,8 +2693,6 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
       ctl->dopamine = dopamine;
     }
   }
-  const uint32_t hi = min(seg_max, 30u);   // segments 1..hi are the ones the batch's slots use
-  const uint32_t need = hi ? (((2u << hi) - 1u) & ~1u) : 0xFFFFFFFFu;
   // segments the batch's slots use: 0..seg_max (bit 31: any segment >= 31)
   const uint32_t act = seg_max >= 31u ? 0xFFFFFFFFu : ((2u << seg_max) - 1u);
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -2292,17 +2716,18 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
       uint4* p = reinterpret_cast<uint4*>(heads + i);
       p[0] = make_uint4(h[0], h[1], h[2], h[3]);
       p[1] = make_uint4(h[4], h[5], h[6], h[7]);
-      const uint2 m = split_masks(h, pmax, own[r]);
+      const uint2 m = split_masks(h, pmax, ax_owners(own[r]));
       mask2[i] = m;
-      // fully lit: heads 0..6 hit every segment 1..seg_max the batch uses and at
+      // fully lit: heads 0..6 hit every segment 1..30 the axon's slots use and at
       // most one soma owns the axon (for those segments the hit is 1 and one
       // push cannot change it)
-      lit = (m.x & need) == need && !(m.y >> 31);
+      lit = (m.x & own[r] & kAxSegs) == (own[r] & kAxSegs) && !(m.y >> 31);
       if (INDEX) on = ((m.x | (m.y & 0x7FFFFFFFu)) & act) != 0u;
     }
     const uint32_t lb = __ballot_sync(kFull, lit), onb = INDEX ? __ballot_sync(kFull, on) : 0u;
     if (lane == 0 && i < A) {
       lit_bits[i >> 5] = lb;
+      always_lit(alit + (i >> 5), lb, alit_new);
       if (INDEX) live[i >> 5] = onb;
       // an axon the row layout summed as fully lit is not: this tick takes the full pass
       if (xw[r] & ~lb) atomicOr(&ctl->dense[k & 1], 1u);
@@ -2377,7 +2802,7 @@ cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, c
   const size_t o_rw = off; off = al(off + (size_t)N * kRowStride * 2);
   const size_t o_cnt = off; off = al(off + (size_t)N * 2);
   const size_t o_m2 = off; off = al(off + ((size_t)A + 1) * 8);
-  const size_t o_mult = off; off = al(off + (size_t)A * 4);
+  const size_t o_axw = off; off = al(off + (size_t)A * 4);
   const size_t o_eval = off; off = al(off + (size_t)N * 4 + 4);
   const size_t o_fix = off; off = al(off + (with_fix ? (size_t)kFixCap * 4 : 0));
   const size_t o_lit = off; off = al(off + ((size_t)std::max(A, N) / 32 + 2) * 4 + 16);
@@ -2391,6 +2816,8 @@ cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, c
   const size_t o_om = off; off = al(off + (size_t)N * 16 + 16);
   const size_t o_wcnt = off; off = al(off + (size_t)kMaxUpdateWarps * 8);
   const size_t o_lsum = off; off = al(off + (size_t)N * 8 + 8);
+  const size_t o_lm = off; off = al(off + (size_t)N * 16 + 16);
+  const size_t o_alit = off; off = al(off + ((size_t)std::max(A, N) / 32 + 2) * 4 + 16);
   const size_t o_xlit = off; off = al(off + ((size_t)A / 32 + 2) * 4 + 16);
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, off);
@@ -2412,7 +2839,7 @@ cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, c
   r->rw = reinterpret_cast<int16_t*>(b + o_rw);
   r->cnt = reinterpret_cast<uint16_t*>(b + o_cnt);
   r->mask2 = reinterpret_cast<uint2*>(b + o_m2);
-  r->mult = reinterpret_cast<uint32_t*>(b + o_mult);
+  r->axw = reinterpret_cast<uint32_t*>(b + o_axw);
   r->eval = reinterpret_cast<uint32_t*>(b + o_eval);
   r->fix = with_fix ? reinterpret_cast<uint32_t*>(b + o_fix) : nullptr;
   r->lit = reinterpret_cast<uint32_t*>(b + o_lit);
@@ -2425,7 +2852,9 @@ cudaError_t rows_alloc(ShardScratch& s, uint32_t N, uint32_t A, bool with_fix, c
   r->lfz = reinterpret_cast<uint8_t*>(b + o_lfz);
   r->omask = reinterpret_cast<uint4*>(b + o_om);
   r->wcnt = reinterpret_cast<uint32_t*>(b + o_wcnt);
-  r->lsum = reinterpret_cast<int2*>(b + o_lsum);
+  r->rec = reinterpret_cast<int2*>(b + o_lsum);
+  r->lmask = reinterpret_cast<uint4*>(b + o_lm);
+  r->alit = reinterpret_cast<uint32_t*>(b + o_alit);
   r->xlit = reinterpret_cast<uint32_t*>(b + o_xlit);
   s.rows = r;
   return cudaSuccess;
@@ -2458,7 +2887,7 @@ __global__ void __launch_bounds__(512) k_rows_decide(ShardCtl* ctl, uint32_t for
 }  // namespace
 
 cudaError_t launch_rows_decide(ShardScratch& s, uint32_t A, bool force, uint32_t ticks, cudaStream_t stream) {
-  k_rows_decide<<<1, 512, 0, stream>>>(s.ctl, force ? 1u : 0u, ticks, s.rows->lit, A);
+  k_rows_decide<<<1, 512, 0, stream>>>(s.ctl, force ? 1u : 0u, ticks, s.rows->alit, A);
   return cudaGetLastError();
 }
 
@@ -2468,14 +2897,14 @@ cudaError_t launch_rows_begin(const ShardVramPtrs& v, ShardScratch& s, uint32_t 
   const uint32_t cond = conditional ? 1u : 0u;
   k_rows_reset_lists<<<1, 1, 0, stream>>>(s.ctl);
   if (A) k_rows_prep<<<std::min((A + 255) / 256, 4u * (uint32_t)sm_count()), 256, 0, stream>>>(
-             s.ctl, r.mult, A, r.lit, permute ? r.xlit : nullptr, cond);
+             s.ctl, r.axw, A, r.alit, permute ? r.xlit : nullptr, cond);
   if (N) {
-    k_rows_mult<<<(N + 255) / 256, 256, 0, stream>>>(v.soma_to_axon, N, A, r.mult, r.mask2, s.ctl, cond);
+    k_rows_mult<<<(N + 255) / 256, 256, 0, stream>>>(v.soma_to_axon, N, A, r.axw, r.mask2, s.ctl, cond);
     k_rows_build<<<(N + 31) / 32, 256, 0, stream>>>(v.dendrite_targets, v.dendrite_weights, v.soma_flags, N, r.rt,
                                                     r.rw, r.cnt, r.amask, r.omask, r.lfz, s.ctl, A,
                                                     row_sum ? 1u : 0u, permute ? 1u : 0u,
-                                                    permute ? r.xlit : nullptr, permute ? r.lsum : nullptr,
-                                                    with_posmap ? r.posmap : nullptr, cond);
+                                                    permute ? r.xlit : nullptr, permute ? r.rec : nullptr, r.lmask,
+                                                    with_posmap ? r.posmap : nullptr, r.axw, cond);
   }
   return cudaGetLastError();
 }
@@ -2521,7 +2950,7 @@ static void launch_rows_update(const ShardVramPtrs& v, ShardScratch& s, uint32_t
   const size_t smem = lit ? lit_smem_bytes(A) : 0;
   auto go = [&](auto kern) {
     launch_chain(kern, grid, block, smem, stream, pdl, v, N, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix,
-                 s.ctl, k, fix_cap, r.lit, lc, r.gs_n, r.gd_n, r.lfz, r.wcnt, wt, index ? 1u : 0u);
+                 s.ctl, k, fix_cap, r.lit, lc, r.gs_n, r.gd_n, r.lfz, r.wcnt, wt, index ? 1u : 0u, r.rec);
   };
   if constexpr (INLINE) {
     if (wt.w) {   // the per-tick entry point: weight changes written through
@@ -2543,8 +2972,8 @@ static void launch_rows_lsum(const ShardVramPtrs& v, ShardScratch& s, uint32_t A
                              const LearnCtl* lc, cudaStream_t stream, ColWT wt = ColWT{}, bool pdl = false) {
   RowCache& r = *s.rows;
   launch_chain(wt.w ? k_rows_update_lsum<true> : k_rows_update_lsum<false>, dim3(kLsumBlocks * sm_count()), dim3(256),
-               0, stream, pdl, v, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix, s.ctl, k, fix_cap, r.lit, r.lfz,
-               r.lsum, wt, lc);
+               0, stream, pdl, v, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix, s.ctl, k, fix_cap, r.lit,
+               r.rec, wt, lc);
 }
 
 // The sparse form (the learned engine's graphs): hits, then neurons, persistent warps.
@@ -2607,17 +3036,17 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
                       : (a.index ? k_rows_prologue_plain<1, true> : k_rows_prologue_plain<1, false>),
                  dim3(wide ? (G + 511) / 512 : (G + 255) / 256), dim3(256), 0, stream, false, v.axon_heads, A,
                  a.v_seg, bitmask, a.virtual_offset, a.num_virtual, s.incoming,
-                 (have_incoming && !per_tick) ? s.batch_counts : nullptr, a.k, r.mask2, r.mult, v.soma_flags,
+                 (have_incoming && !per_tick) ? s.batch_counts : nullptr, a.k, r.mask2, r.axw, v.soma_flags,
                  v.timers, N, r.eval, s.ctl, raise, r.lit, (a.k > 0 && !per_tick) ? s.pend : nullptr,
                  (have_incoming && per_tick) ? 1u : 0u, per_tick ? 1u : 0u, a.tick - a.k, (int32_t)a.dopamine,
-                 r.xlit, r.live, r.evb);
+                 r.xlit, r.live, r.evb, r.alit, a.lit_new ? 1u : 0u);
   }
   if (ev) cudaEventRecord(ev[2], stream);
   ColWT wt{};
   if (per_tick) {
     wt.w = v.dendrite_weights;
     wt.om = r.omask;
-    wt.cnt = r.cnt;
+    wt.lm = r.lmask;
     wt.N = N;
   }
   // stages: ev[2]..ev[3] the 8-lane pass, ev[3]..ev[4] the lit-sum pass (both
@@ -2816,7 +3245,7 @@ cudaError_t rows_index_wish(const ShardVramPtrs& v, ShardScratch& s, uint32_t N,
 
 cudaError_t launch_rows_end(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, cudaStream_t stream) {
   RowCache& r = *s.rows;
-  if (N) k_rows_writeback<<<(N + 255) / 256, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.omask);
+  if (N) k_rows_writeback<<<(N + 255) / 256, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.omask, r.lmask);
   return cudaGetLastError();
 }
 

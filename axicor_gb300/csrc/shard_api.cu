@@ -317,6 +317,7 @@ int32_t cu_step_day_phase(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t
     a.rows = true;
     a.k = s->tick_parity;
     a.defer_push = false;
+    a.lit_new = s->tick_since_build == 1 || s->tick_since_build == kTickRelayout - kLitWindow + 1;
     a.fix_cap = s->rows->fix ? fix_capacity() : 0u;   // no list (population rows): the fix-up rescans
     s->tick_parity ^= 1u;
   }

@@ -248,9 +248,10 @@ int32_t axc_last_spikes(const ShardVramPtrs* vram, uint32_t* out_count, uint32_t
  * neuron-major row copy the ticks run on is kept from one batch to the next
  * (its weights are written back to the .state blob at the end of every
  * batch).  The device decides before each batch whether to lay it out anew:
- * at every batch while the layout leaves more than an eighth of the live
- * slots outside its lit-sum groups (the weights are still freezing), then
- * after 100, 200, 400, ... up to every 1,600 ticks; and for sure after the
+ * while the layout leaves more than an eighth of the live slots to be tested
+ * one by one, when more axons have become fully lit or weights have frozen
+ * since (and at least every 1,600 ticks); else after 100, 200, 400, ... up to
+ * every 1,600 ticks; and for sure after the
  * shard's memory or the LUT may have changed: after any entry point of this
  * library that writes them, per-tick calls, and axc_shard_invalidate.
  * h_output_history, when not NULL, receives num_outputs x batch bytes
