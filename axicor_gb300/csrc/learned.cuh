@@ -1218,7 +1218,7 @@ static void learned_update_forms(Learned& L, ShardScratch& s, uint32_t k, cudaSt
   const uint32_t fix_cap = kFixCap;
   // dense: the plain engine's passes on the movable-first rows, GSOP inside them
   // (the 8-lane pass, or the lit-sum form when its lit set held)
-  launch_rows_update<true>(L.v, s, N, A, k, fix_cap, L.ctl, st, ColWT{}, false, true);
+  launch_rows_update(L.v, s, N, A, k, fix_cap, L.ctl, st, ColWT{}, false, true);
   launch_rows_lsum(L.v, s, A, k, fix_cap, L.ctl, st);
   launch_rows_sparse(L.v, s, N, A, k, fix_cap, L.ctl, st);
   // sparse: the axon-driven gather, GLIF, and GSOP of the spikers it listed

@@ -150,17 +150,30 @@ struct ColWT {
   uint32_t N = 0;
 };
 
+// The r-th set bit (0-based, r < popc) of a word: a binary search over the counts
+// (__fns walks the bits: 15 of the 37 us of a plastic per-tick call at 6,000 neurons).
+__device__ __forceinline__ uint32_t nth_bit32(uint32_t m, uint32_t r) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (uint32_t st = 16; st > 0; st >>= 1) {
+    const uint32_t c = __popc(m & ((1u << st) - 1u));
+    if (r >= c) {
+      r -= c;
+      pos += st;
+      m >>= st;
+    }
+  }
+  return pos;
+}
+
 // The r-th set bit (0-based) of a 128-bit mask.
 __device__ __forceinline__ uint32_t nth_bit128(uint4 m, uint32_t r) {
-  const uint32_t c0 = __popc(m.x);
-  if (r < c0) return __fns(m.x, 0, r + 1);
-  r -= c0;
-  const uint32_t c1 = __popc(m.y);
-  if (r < c1) return 32u + __fns(m.y, 0, r + 1);
-  r -= c1;
-  const uint32_t c2 = __popc(m.z);
-  if (r < c2) return 64u + __fns(m.z, 0, r + 1);
-  return 96u + __fns(m.w, 0, r - c2 + 1);
+  uint32_t w = m.x, base = 0;
+  uint32_t c = __popc(w);
+  if (r >= c) { r -= c; w = m.y; base = 32; c = __popc(w); }
+  if (base == 32u && r >= c) { r -= c; w = m.z; base = 64; c = __popc(w); }
+  if (base == 64u && r >= c) { r -= c; w = m.w; base = 96; }
+  return base + nth_bit32(w, r);
 }
 
 // Columnar slot of row position pos < lf, in a row whose movable slots are om,
@@ -175,6 +188,52 @@ __device__ __forceinline__ void col_write(const ColWT& wt, uint32_t n, uint32_t 
   const uint32_t q = col_of_pos(wt.om[n], wt.lm[n], pos);
   wt.w[(size_t)q * wt.N + n] = w;
 }
+
+// The columnar slots of consecutive row positions: the first by search, each further
+// one the mask's next bit.
+struct ColRun {
+  uint4 m;
+  uint32_t cur, base, left;   // the word's bits not yet passed, its first slot, positions before the other mask
+
+  __device__ __forceinline__ uint32_t word() const {
+    return base == 0u ? m.x : base == 32u ? m.y : base == 64u ? m.z : m.w;
+  }
+  __device__ __forceinline__ void others(const ColWT& wt, uint32_t n) {
+    const uint4 om = wt.om[n], lm = wt.lm[n];
+    m = make_uint4(om.x & ~lm.x, om.y & ~lm.y, om.z & ~lm.z, om.w & ~lm.w);
+    left = kRowStride;
+  }
+  __device__ __forceinline__ ColRun(const ColWT& wt, uint32_t n, uint32_t pos) {
+    m = wt.lm[n];
+    const uint32_t nl = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+    uint32_t r = pos;
+    if (pos < nl) {
+      left = nl - pos;
+    } else {
+      r = pos - nl;
+      others(wt, n);
+    }
+    base = nth_bit128(m, r);
+    const uint32_t bit = base & 31u;
+    base -= bit;
+    cur = word() & (~0u << bit);
+  }
+  __device__ __forceinline__ uint32_t next(const ColWT& wt, uint32_t n) {
+    if (left-- == 0u) {
+      others(wt, n);
+      left--;
+      base = 0;
+      cur = m.x;
+    }
+    while (cur == 0u && base < 96u) {
+      base += 32u;
+      cur = word();
+    }
+    const uint32_t q = base + __ffs(cur) - 1u;
+    cur &= cur - 1u;
+    return q;
+  }
+};
 
 // The lit-sum form runs tick k when the rows' tested slots are few (at most
 // an eighth of the live slots: otherwise the 8-lane pass is faster) and every
@@ -1029,7 +1088,7 @@ __device__ __noinline__ int gsop_general(const BurstHeads8* heads, const uint2* 
                                          uint32_t s, const VariantParameters& p, uint8_t flags, int32_t dopamine,
                                          int16_t* w16) {
   if (a >= A) return 2;
-  const uint2 m = __ldg(mask2 + a);
+  const uint2 m = mask2[a];
   uint32_t md, md1;
   md_pair(heads, a, s, p.signal_propagation_length, &md, &md1);
   if ((m.y >> 31) || md != md1) return 1;
@@ -1041,6 +1100,14 @@ __device__ __noinline__ int gsop_general(const BurstHeads8* heads, const uint2* 
 // GSOP deltas per variant and inertia rank for a spiker (flags type | 0b101:
 // burst multiplier 2, physics.cu:255, 271-273, 290-291; physics.cu:336-349).
 // Called by the first 256 threads of the block.
+// The LUT's largest signal_propagation_length; seen by all after the next barrier.
+__device__ __forceinline__ void pmax_of(uint32_t* dst, const VariantParameters* lut) {
+  if (threadIdx.x < 32) {
+    const uint32_t m = __reduce_max_sync(kFull, lut[threadIdx.x & 15].signal_propagation_length);
+    if (threadIdx.x == 0) *dst = m;
+  }
+}
+
 __device__ __forceinline__ void build_gtab(int2 (*gtab)[16], const VariantParameters* lut, int32_t dopamine) {
   if (threadIdx.x < 256) {
     const uint32_t v = threadIdx.x >> 4, r = threadIdx.x & 15;
@@ -1136,7 +1203,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // slowb = GSOP needs the exact path (physics.cu:186-207 for the hit test).
 template <bool LIT>
 __device__ __forceinline__ int32_t row_slots(const uint4 (&T)[4], const uint2 (&W)[4], uint32_t c, uint32_t g8,
-                                             RowShape sh, const uint2* __restrict__ mask2, const uint32_t* s_lit,
+                                             RowShape sh, const uint2* mask2, const uint32_t* s_lit,
                                              uint32_t seg_hi, bool exact, bool gfast, uint32_t prop,
                                              const BurstHeads8* heads, uint32_t A, uint32_t& hitb_out,
                                              uint32_t& slowb_out, bool lit_on = true) {
@@ -1154,7 +1221,7 @@ __device__ __forceinline__ int32_t row_slots(const uint4 (&T)[4], const uint2 (&
       const uint32_t t = word_of(T[j], i);
       const uint32_t ax = (t & AXC_TARGET_AXON_MASK) - 1u;   // invalid ids were redirected to A
       lit[i] = glit && ((t >> AXC_TARGET_SEG_SHIFT) - 1u) < seg_hi && ((s_lit[ax >> 5] >> (ax & 31u)) & 1u);
-      m[i] = (q0 + i < c && !lit[i]) ? __ldg(mask2 + ax) : make_uint2(0, 0);
+      m[i] = (q0 + i < c && !lit[i]) ? mask2[ax] : make_uint2(0, 0);
     }
     uint32_t need = 0;   // live slots off the fully-lit path
 #pragma unroll
@@ -1204,7 +1271,7 @@ __device__ __forceinline__ int32_t row_slots(const uint4 (&T)[4], const uint2 (&
         i_in = wadd(i_in, (int32_t)half_of(W[3], t));
         hitb |= 1u << (12 + t);
       } else {
-        m[t] = __ldg(mask2 + ax);
+        m[t] = mask2[ax];
         need |= 1u << t;
       }
     }
@@ -1325,9 +1392,13 @@ __device__ __forceinline__ uint32_t row_gsop(uint2 (&W)[4], uint32_t hitb, uint3
     } else {
       *reinterpret_cast<uint2*>(rw_n + q0) = wj;
       if (WT) {
+        ColRun cols(wt, n, q0);
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-          if (half_of(wj, i) != half_of(W[j], i)) col_write(wt, n, q0 + i, half_of(wj, i));
+        for (int i = 0; i < 4; i++) {
+          if (q0 + i >= c) break;
+          const uint32_t q = cols.next(wt, n);
+          if (half_of(wj, i) != half_of(W[j], i)) wt.w[(size_t)q * wt.N + n] = half_of(wj, i);
+        }
       }
     }
   }
@@ -1375,15 +1446,15 @@ __device__ __forceinline__ uint32_t row_gsop(uint2 (&W)[4], uint32_t hitb, uint3
 // the eight heads.  *fast: GSOP may take the slot's delta from the gtab table
 // (the hit decides and one same-tick push cannot change it).
 __device__ __forceinline__ bool slot_hit(uint32_t t, bool exact, bool gfast, uint32_t prop, uint32_t seg_hi,
-                                         const uint32_t* __restrict__ lit_bits, const uint2* __restrict__ mask2,
+                                         const uint32_t* lit_bits, const uint2* mask2,
                                          const BurstHeads8* heads, uint32_t A, bool* fast) {
   const uint32_t s = t >> AXC_TARGET_SEG_SHIFT;
   const uint32_t ax = (t & AXC_TARGET_AXON_MASK) - 1u;   // invalid ids were redirected to A (dummy mask entry)
-  if (gfast && (s - 1u) < seg_hi && ((__ldg(lit_bits + (ax >> 5)) >> (ax & 31u)) & 1u)) {
+  if (gfast && (s - 1u) < seg_hi && ((lit_bits[ax >> 5] >> (ax & 31u)) & 1u)) {
     *fast = true;
     return true;
   }
-  const uint2 m = __ldg(mask2 + ax);
+  const uint2 m = mask2[ax];
   const uint32_t sh = min(s, 31u);
   const uint32_t bx = (m.x >> sh) & 1u, by = (m.y >> sh) & 1u;
   bool hit = (bx | by) != 0u;
@@ -1480,9 +1551,9 @@ __device__ __forceinline__ uint32_t gsop_lit2(uint32_t w, const uint32_t* tab) {
 // pass spent ~85.
 template <bool VERIFY, bool WT>
 __device__ __forceinline__ void lit_row_step(const ShardVramPtrs& P, uint32_t A, const uint32_t* __restrict__ rt,
-                                             int16_t* __restrict__ rw, const uint16_t* __restrict__ cnt,
-                                             const uint2* __restrict__ mask2, uint32_t* __restrict__ pend,
-                                             uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl, uint32_t fix_cap,
+                                             int16_t* rw, const uint16_t* __restrict__ cnt,
+                                             const uint2* mask2, uint32_t* pend,
+                                             uint32_t* fix, ShardCtl* ctl, uint32_t fix_cap,
                                              const int2* __restrict__ rec, const ColWT& wt,
                                              const VariantParameters* lut, const int2 (*gtab)[16],
                                              const uint32_t (*tab)[17], uint32_t pmax, uint32_t smax, uint32_t tick,
@@ -1573,7 +1644,7 @@ __device__ __forceinline__ void lit_row_step(const ShardVramPtrs& P, uint32_t A,
     }
 #pragma unroll
     for (int u = 0; u < 4; u++)   // invalid ids were redirected to A (dummy mask entry)
-      m[u] = x0 + 8u * u + g8 < nt ? __ldg(mask2 + (t[u] & AXC_TARGET_AXON_MASK) - 1u) : make_uint2(0, 0);
+      m[u] = x0 + 8u * u + g8 < nt ? mask2[(t[u] & AXC_TARGET_AXON_MASK) - 1u] : make_uint2(0, 0);
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       if (x0 + 8u * u + g8 >= nt) continue;
@@ -1619,10 +1690,12 @@ __device__ __forceinline__ void lit_row_step(const ShardVramPtrs& P, uint32_t A,
         }
         *reinterpret_cast<uint4*>(rw_n + qr) = nw;
         if (WT) {
+          ColRun cols(wt, n, qr);
 #pragma unroll 1
           for (uint32_t h = 0; h < 8; h++) {
+            const uint32_t q = cols.next(wt, n);
             const int16_t a = (int16_t)(word_of(nw, h >> 1) >> (16u * (h & 1u)));
-            if (a != (int16_t)(word_of(W[r], h >> 1) >> (16u * (h & 1u)))) col_write(wt, n, qr + h, a);
+            if (a != (int16_t)(word_of(W[r], h >> 1) >> (16u * (h & 1u)))) wt.w[(size_t)q * wt.N + n] = a;
           }
         }
       } else {
@@ -1656,78 +1729,78 @@ __device__ __forceinline__ bool build_ptab(uint32_t (*tab)[17], const int2 (*gta
   return __syncthreads_and(ok);
 }
 
-// LIT: 1024-thread blocks (one per SM) that first copy the prologue's
-// fully-lit bitmap (one bit per axon) into shared memory; slots whose axon is
-// fully lit need no mask gather from L2.
-// INLINE (rows with their movable slots first): GSOP of each spiker's movable
-// slots on the weights still in registers; else the spikers with movable
-// slots are listed for k_rows_gsop / k_rows_gsop_rows.
-// WT: write GSOP's changes through to the columnar blob (the per-tick entry point).
-template <bool LIT, bool INLINE, bool WT = false>
-__global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
-    k_rows_update(ShardVramPtrs P, uint32_t N, uint32_t A, const uint32_t* __restrict__ rt,
-                  int16_t* __restrict__ rw, const uint16_t* __restrict__ cnt, const uint2* __restrict__ mask2,
-                  const uint32_t* __restrict__ eval, uint32_t* __restrict__ pend, uint32_t* __restrict__ fix,
-                  ShardCtl* __restrict__ ctl, uint32_t k, uint32_t fix_cap, const uint32_t* __restrict__ lit_bits,
-                  const LearnCtl* __restrict__ lc, uint32_t* __restrict__ gs_n, uint32_t* __restrict__ gd_n,
-                  const uint8_t* __restrict__ lfz, uint32_t* __restrict__ wcnt, ColWT wt, uint32_t index,
-                  const int2* __restrict__ rec) {
-  __shared__ VariantParameters lut[16];
-  __shared__ int2 gtab[16][16];
-  __shared__ uint32_t s_pmax;
-  __shared__ uint64_t s_bar;
-  extern __shared__ __align__(128) uint32_t s_lit[];
-  chain_wait();
-  chain_open();
-  const TickForm form = tick_form(ctl, k, lc, index);
-  if (form != kFormDense && form != kFormLitRows && form != kFormVerify) return;                    // k_rows_update_lsum or the learned engine's kernels run this tick
-  if (LIT && threadIdx.x == 0) mbar_init(&s_bar, 1);
-  lut_to_smem(lut);
-  if (threadIdx.x == 0) s_pmax = lut_pmax();
+// Sums per-thread counters over a block: v[0..5] into ctr[1..5] and ctr[7] (evaluated
+// slots, hits, spikes, GSOP slots, evaluated neurons, tested slots), v[6..7] into
+// gsop_same.  Two warp reductions, one barrier and one atomic per counter: 64-bit
+// shuffles and a serial sum over 32 warps were 8,000 cycles of the 8-lane pass.
+template <int NC>
+__device__ __forceinline__ void block_counts(const uint32_t (&v)[NC], ShardCtl* ctl) {
+  __shared__ uint32_t red[NC][32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    const uint32_t x = __reduce_add_sync(kFull, v[c]);
+    if (lane == 0) red[c][w] = x;
+  }
   __syncthreads();
-  // the fully-lit bitmap: one bulk copy into shared memory
-  if (LIT && threadIdx.x == 0) bulk_to_smem(s_lit, lit_bits, lit_smem_bytes(A), &s_bar);
-  const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
-  if (INLINE) {
-    build_gtab(gtab, lut, dopamine);
-    __syncthreads();
+  if (w < (uint32_t)NC) {
+    const uint32_t sum = __reduce_add_sync(kFull, lane < nw ? red[w][lane] : 0u);
+    unsigned long long* dst = w < 5u ? ctl->ctr + 1 + w : w == 5u ? ctl->ctr + 7 : ctl->gsop_same + (w - 6u);
+    if (lane == 0 && sum) atomicAdd(dst, (unsigned long long)sum);
   }
-  const uint32_t tick = ctl->tick_base + k;
-  const uint32_t ecount = ctl->eval_act[k & 1][0];
-  const uint32_t smax = ctl->row_smax;   // longest row of the shard: rows are loaded up to here
+}
+
+// What a pass reads of the control block, asked for in one go.
+struct PassCtl {
+  uint32_t tick, smax, seg_max;
+};
+__device__ __forceinline__ PassCtl pass_ctl(const ShardCtl* ctl, uint32_t k) {
+  return {ctl_ld32(&ctl->tick_base) + k, ctl_ld32(&ctl->row_smax), ctl_ld32(&ctl->seg_max)};
+}
+
+// The 8-lane pass over the tick's evaluated neurons, one form of three (dense,
+// lit rows, checked lit rows).  s_lit: the tick's fully-lit bitmap (one bit per
+// axon), in shared memory where it fits, else in global memory; lit_on false: it
+// did not arrive, the pass does without it (results exact).  Slots whose axon is
+// fully lit need no mask gather from L2.
+// WT: write GSOP's changes through to the columnar blob (the per-tick entry point).
+// Warp wid of the nwarps that share the list; counts: this thread's (block_counts).
+template <bool WT>
+__device__ __forceinline__ void rows_update(TickForm form, uint32_t wid, uint32_t nwarps, const PassCtl& pc,
+                                            const ShardVramPtrs& P, uint32_t A, const uint32_t* rt, int16_t* rw,
+                                            const uint16_t* cnt, const uint2* mask2, const uint32_t* eval,
+                                            uint32_t ecount, uint32_t* pend, uint32_t* fix, ShardCtl* ctl,
+                                            uint32_t fix_cap, const uint8_t* lfz, const ColWT& wt, const int2* rec,
+                                            const VariantParameters* lut, const int2 (*gtab)[16],
+                                            const uint32_t (*ptab)[17], uint32_t pmax, int32_t dopamine,
+                                            const uint32_t* s_lit, bool lit_on, uint32_t (&counts)[8]) {
+  const uint32_t tick = pc.tick;
+  const uint32_t smax = pc.smax;   // longest row of the shard: rows are loaded up to here
   const RowShape sh = row_shape(smax);
-  const uint32_t seg_hi = min(ctl->seg_max, 30u);   // lit bits cover segments 1..seg_hi
+  const uint32_t seg_hi = min(pc.seg_max, 30u);   // lit bits cover segments 1..seg_hi
   const uint32_t lane = threadIdx.x & 31, g8 = lane & 7, grp = lane >> 3;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  // each warp owns a contiguous slice of the list, 4 neurons per step
-  const uint32_t per_warp = (((ecount + nwarps - 1) / nwarps) + 3) & ~3u;
-  const uint32_t beg = min(wid * per_warp, ecount), end = min(beg + per_warp, ecount);
+  // Four neurons a step.  The warps take the steps in turn, which evens out a short
+  // list; of a long one each has a slice of its own.
+  const uint32_t per_warp = ecount < 64u * nwarps ? 0u : (((ecount + nwarps - 1) / nwarps) + 3u) & ~3u;
+  const uint32_t step = per_warp ? 4u : 4u * nwarps;
+  const uint32_t beg = per_warp ? wid * per_warp : 4u * wid;
+  const uint32_t end = per_warp ? min(beg + per_warp, ecount) : ecount;
   uint32_t ev_slots = 0, hits = 0, nspk = 0, gdone = 0, nev = 0, err = 0;
-  uint32_t wc = 0, wd = 0;   // spikers this warp listed for the GSOP passes
   uint32_t same = 0;         // row_gsop
-  uint32_t beg_dense = beg, lit_tested = 0;
-  bool lit_on = true;
-  if (LIT) {
-    lit_on = mbar_wait_bounded(&s_bar, 0, g_first_wait_limit);
-    if (!lit_on) err |= AXC_ERR_WAIT_LIMIT;   // then without the shortcut (results exact)
-  }
+  uint32_t lit_tested = 0;
   if (form != kFormDense) {
-    __shared__ uint32_t ptab[16][17];
-    const bool packed = build_ptab(ptab, gtab);
     LsumCount kc = {0, 0, 0, 0, 0, 0, 0, 0};
     if (form == kFormVerify) {
-      for (uint32_t i0 = beg; i0 < end; i0 += 4)
+      for (uint32_t i0 = beg; i0 < end; i0 += step)
         lit_row_step<true, WT>(P, A, rt, rw, cnt, mask2, pend, fix, ctl, fix_cap, rec, wt, lut, gtab,
-                               packed ? ptab : nullptr, s_pmax, smax, tick, dopamine,
-                               __ldg(eval + min(i0 + grp, end - 1u)), i0 + grp < end, LIT ? s_lit : lit_bits, lit_on,
-                               kc);
+                               ptab, pmax, smax, tick, dopamine,
+                               eval[min(i0 + grp, end - 1u)], i0 + grp < end, s_lit, lit_on, kc);
     } else {
       if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ctr[6] += 1;   // ticks on the lit-sum form
-      for (uint32_t i0 = beg; i0 < end; i0 += 4)
+      for (uint32_t i0 = beg; i0 < end; i0 += step)
         lit_row_step<false, WT>(P, A, rt, rw, cnt, mask2, pend, fix, ctl, fix_cap, rec, wt, lut, gtab,
-                                packed ? ptab : nullptr, s_pmax, smax, tick, dopamine,
-                                __ldg(eval + min(i0 + grp, end - 1u)), i0 + grp < end, nullptr, false, kc);
+                                ptab, pmax, smax, tick, dopamine,
+                                eval[min(i0 + grp, end - 1u)], i0 + grp < end, nullptr, false, kc);
       lit_tested = kc.tested;
     }
     ev_slots = kc.ev_slots;
@@ -1737,13 +1810,13 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
     nev = kc.nev;
     err |= kc.err;
     same = kc.same;
-    beg_dense = end;
   }
-  for (uint32_t base = beg_dense; base < end; base += 32) {
-    const uint32_t mine = (base + lane < end) ? __ldg(eval + base + lane) : 0u;
-    for (uint32_t sub = 0; sub < 32 && base + sub < end; sub += 4) {
-      const bool valid = base + sub + grp < end;
-      const uint32_t n = __shfl_sync(kFull, mine, sub + grp);
+  for (uint32_t base = beg; form == kFormDense && base < end; base += 8u * step) {
+    const uint32_t at = base + (lane >> 2) * step + (lane & 3u);   // eight steps' neurons, one a lane
+    const uint32_t mine = at < end ? eval[at] : 0u;
+    for (uint32_t sub = 0; sub < 8 && base + sub * step < end; sub++) {
+      const bool valid = base + sub * step + grp < end;
+      const uint32_t n = __shfl_sync(kFull, mine, 4u * sub + grp);
       // every load of the neuron at once: state, count, and its row up to smax
       const uint8_t flags = P.soma_flags[n];
       const uint32_t cw = valid ? cnt[n] : 0u;
@@ -1759,14 +1832,14 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
       const uint32_t var = flags >> 4;
       const VariantParameters& p = lut[var];
       const uint32_t prop = p.signal_propagation_length;
-      const bool exact = prop == s_pmax;
+      const bool exact = prop == pmax;
       const bool gfast = exact && prop <= 16u;
       if (cw & kRowBad) err |= AXC_ERR_TARGET_RANGE;
       uint32_t hitb, slowb;
       // the fully-lit test reads the bitmap from shared memory (LIT) or, when it
       // did not fit there, from global memory (1 bit per axon: far fewer bytes
       // to keep in L1/L2 than the 8-byte masks)
-      int32_t i_in = row_slots<true>(T, W, c, g8, sh, mask2, LIT ? s_lit : lit_bits, seg_hi, exact, gfast, prop,
+      int32_t i_in = row_slots<true>(T, W, c, g8, sh, mask2, s_lit, seg_hi, exact, gfast, prop,
                                      P.axon_heads, A, hitb, slowb, lit_on);
       i_in = wadd(i_in, __shfl_xor_sync(kFull, i_in, 1));
       i_in = wadd(i_in, __shfl_xor_sync(kFull, i_in, 2));
@@ -1793,63 +1866,76 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
           }
         }
       }
-      if (INLINE) {
-        // GSOP (physics.cu:281-373) of the spiker's movable slots, the first lf
-        // of its row; frozen slots (GSOP leaves them as they are) are counted
-        if (spike && lf > 0u)
-          gdone += row_gsop<WT>(W, hitb, slowb, lf, g8, sh, gtab, var, rt_n, rw_n, P.axon_heads, mask2, A, p,
-                                flags, dopamine, ctl, fix, fix_cap, n, same, wt);
-        if (spike && g8 == 0) gdone += c - lf;
-        continue;
-      }
-      // GSOP (physics.cu:281-373) runs in k_rows_gsop / k_rows_gsop_rows over
-      // the spikers listed here (those with slots that may move: a few, or
-      // many), in this warp's segments of the lists; frozen slots (GSOP leaves
-      // them as they are) of a row with a few movable ones or none are only
-      // counted here
-      const bool few = spike && lf > 0u && lf <= 8u, many = spike && lf > 8u;
-      if (spike && lf <= 8u && g8 == 0) gdone += c - lf;
-      const uint32_t ab = __ballot_sync(kFull, few && g8 == 0), db = __ballot_sync(kFull, many && g8 == 0);
-      if (few && g8 == 0) gs_n[beg + wc + __popc(ab & ((1u << lane) - 1u))] = n;
-      if (many && g8 == 0) gd_n[beg + wd + __popc(db & ((1u << lane) - 1u))] = n;
-      wc += __popc(ab);
-      wd += __popc(db);
+      // GSOP (physics.cu:281-373) of the spiker's movable slots, the first lf
+      // of its row; frozen slots (GSOP leaves them as they are) are counted
+      if (spike && lf > 0u)
+        gdone += row_gsop<WT>(W, hitb, slowb, lf, g8, sh, gtab, var, rt_n, rw_n, P.axon_heads, mask2, A, p, flags,
+                              dopamine, ctl, fix, fix_cap, n, same, wt);
+      if (spike && g8 == 0) gdone += c - lf;
     }
   }
-  if (!INLINE && lane == 0) {
-    wcnt[wid] = wc;
-    wcnt[kMaxUpdateWarps + wid] = wd;
-  }
-  // a warp that gave up: the copy must land before the block exits
-  if (LIT && !lit_on && !mbar_wait_bounded(&s_bar, 0)) err |= AXC_ERR_WAIT_LIMIT;
+  if (!lit_on) err |= AXC_ERR_WAIT_LIMIT;
   const uint32_t err_any = __reduce_or_sync(kFull, err);
   if (err_any && lane == 0) atomicOr(&ctl->err, err_any);
-  block_count(ev_slots, hits, nspk, &ctl->ctr[1]);
-  block_count(gdone, nev, 0, &ctl->ctr[4]);
-  if (INLINE) block_count(same & 0xFFFFu, same >> 16, 0, ctl->gsop_same);
-  if (form == kFormLitRows) block_count(lit_tested, 0, 0, &ctl->ctr[7]);
+  counts[0] = ev_slots;
+  counts[1] = hits;
+  counts[2] = nspk;
+  counts[3] = gdone;
+  counts[4] = nev;
+  counts[5] = lit_tested;
+  counts[6] = same & 0xFFFFu;
+  counts[7] = same >> 16;
 }
 
-// Sums six per-thread counters over a 256-thread block into ctr[1..5] and
-// ctr[7] (evaluated slots, hits, spikes, GSOP slots, evaluated neurons, tested
-// slots): one barrier, one atomic per counter.
-__device__ __forceinline__ void block_count256(uint32_t a1, uint32_t a2, uint32_t a3, uint32_t a4, uint32_t a5,
-                                               uint32_t a7, unsigned long long* ctr) {
-  __shared__ uint32_t red[6][8];
-  const uint32_t v[6] = {__reduce_add_sync(kFull, a1), __reduce_add_sync(kFull, a2), __reduce_add_sync(kFull, a3),
-                         __reduce_add_sync(kFull, a4), __reduce_add_sync(kFull, a5), __reduce_add_sync(kFull, a7)};
-  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) {
-#pragma unroll
-    for (int c = 0; c < 6; c++) red[c][w] = v[c];
-  }
+// LIT: 1024-thread blocks (one per SM) that first copy the prologue's
+// fully-lit bitmap into shared memory.
+template <bool LIT, bool WT>
+__global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
+    k_rows_update(ShardVramPtrs P, uint32_t A, const uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
+                  const uint16_t* __restrict__ cnt, const uint2* __restrict__ mask2, const uint32_t* __restrict__ eval,
+                  uint32_t* __restrict__ pend, uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl, uint32_t k,
+                  uint32_t fix_cap, const uint32_t* __restrict__ lit_bits, const LearnCtl* __restrict__ lc,
+                  const uint8_t* __restrict__ lfz, ColWT wt, uint32_t index, const int2* __restrict__ rec,
+                  uint32_t unit) {
+  __shared__ VariantParameters lut[16];
+  __shared__ int2 gtab[16][16];
+  __shared__ uint32_t ptab[16][17];
+  __shared__ uint32_t s_pmax;
+  __shared__ uint64_t s_bar;
+  extern __shared__ __align__(128) uint32_t s_lit[];
+  chain_wait();
+  chain_open();
+  const PassCtl pc = pass_ctl(ctl, k);
+  const uint32_t ecount = ctl_ld32(&ctl->eval_act[k & 1][0]);
+  const TickForm form = tick_form(ctl, k, lc, index);
+  // else k_rows_update_lsum or the learned engine's kernels run this tick
+  if (form != kFormDense && form != kFormLitRows && form != kFormVerify) return;
+  if (LIT && threadIdx.x == 0) mbar_init(&s_bar, 1);
+  lut_to_smem(lut);
   __syncthreads();
-  if (threadIdx.x < 6) {
-    unsigned long long sum = 0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) sum += red[threadIdx.x][q];
-    if (sum) atomicAdd(ctr + (threadIdx.x == 5 ? 7 : threadIdx.x + 1), sum);
-  }
+  // the fully-lit bitmap: one bulk copy into shared memory
+  if (LIT && threadIdx.x == 0) bulk_to_smem(s_lit, lit_bits, lit_smem_bytes(A), &s_bar);
+  const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
+  pmax_of(&s_pmax, lut);
+  build_gtab(gtab, lut, dopamine);
+  __syncthreads();
+  const bool packed = form != kFormDense && build_ptab(ptab, gtab);
+  const bool lit_on = !LIT || mbar_wait_bounded(&s_bar, 0, g_first_wait_limit);
+  uint32_t counts[8];
+  // An equal, contiguous part of the list per block, a multiple of `unit` neurons: 4
+  // where the shard has the GPU to itself (6,000 plastic neurons, 1,500 of them
+  // evaluated, sat on 12 SMs), else whole steps of the block, so that fewer blocks
+  // stand in the way of the other shards' (four zone shards of 100,000: 2,160 us per
+  // 20 ticks against 2,450).  The neighbours in a part, whose targets are near each
+  // other, share an L1.
+  const uint32_t part = ((ecount + gridDim.x - 1) / gridDim.x + unit - 1u) / unit * unit;
+  const uint32_t first = min(blockIdx.x * part, ecount);
+  rows_update<WT>(form, threadIdx.x >> 5, blockDim.x >> 5, pc, P, A, rt, rw, cnt, mask2, eval + first,
+                  min(part, ecount - first), pend, fix, ctl, fix_cap, lfz, wt, rec, lut, gtab, packed ? ptab : nullptr,
+                  s_pmax, dopamine, LIT ? s_lit : lit_bits, lit_on, counts);
+  block_counts(counts, ctl);
+  // a wait that gave up: the copy must land before the block exits
+  if (LIT && !lit_on && !mbar_wait_bounded(&s_bar, 0)) atomicOr(&ctl->err, AXC_ERR_WAIT_LIMIT);
 }
 
 // ---------------------------------------------------------------------------
@@ -2148,7 +2234,8 @@ __global__ void __launch_bounds__(256, kNeuronBlocks)
   }
   const uint32_t err_any = __reduce_or_sync(kFull, err);
   if (err_any && lane == 0) atomicOr(&ctl->err, err_any);
-  block_count256(ev_slots, 0, nspk, gdone, nev, 0, ctl->ctr);
+  const uint32_t counts[6] = {ev_slots, 0, nspk, gdone, nev, 0};
+  block_counts(counts, ctl);
 }
 
 // ---------------------------------------------------------------------------
@@ -2174,26 +2261,28 @@ __global__ void __launch_bounds__(256, kLsumBlocks)
                        const uint16_t* __restrict__ cnt, const uint2* __restrict__ mask2,
                        const uint32_t* __restrict__ eval, uint32_t* __restrict__ pend, uint32_t* __restrict__ fix,
                        ShardCtl* __restrict__ ctl, uint32_t k, uint32_t fix_cap, const uint32_t* __restrict__ lit_bits,
-                       const int2* __restrict__ rec, ColWT wt, const LearnCtl* __restrict__ lc) {
+                       const int2* __restrict__ rec, ColWT wt, const LearnCtl* __restrict__ lc, uint32_t unit) {
   chain_wait();
   chain_open();
+  const PassCtl pc = pass_ctl(ctl, k);
+  const uint32_t ecount = ctl_ld32(&ctl->eval_act[k & 1][0]);
   if (tick_form(ctl, k, lc, 0u) != kFormLitSum) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ctr[6] += 1;   // ticks on the lit-sum form
-  const uint32_t ecount = ctl->eval_act[k & 1][0];
-  if (blockIdx.x * blockDim.x >= ecount) return;   // no neuron for this block: no table to build
+  // neurons per block and pass: fewer than its threads where that spreads a short list over all blocks
+  const uint32_t span = min(256u, ((ecount + gridDim.x - 1) / gridDim.x + unit - 1u) / unit * unit);
+  if (blockIdx.x * span >= ecount) return;   // no neuron for this block: no table to build
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
   lut_to_smem(lut);
-  if (threadIdx.x == 0) s_pmax = lut_pmax();
   __syncthreads();
   const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
+  pmax_of(&s_pmax, lut);
   build_gtab(gtab, lut, dopamine);
   __syncthreads();
-  const uint32_t tick = ctl->tick_base + k;
-  const uint32_t seg_hi = min(ctl->seg_max, 30u);
+  const uint32_t tick = pc.tick, seg_hi = min(pc.seg_max, 30u), pmax = s_pmax;
   LsumCount kc = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ecount; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = threadIdx.x < span ? blockIdx.x * span + threadIdx.x : ecount; i < ecount; i += gridDim.x * span) {
     const uint32_t n = eval[i];
     // every load of the neuron at once
     const uint8_t flags = P.soma_flags[n];
@@ -2207,7 +2296,7 @@ __global__ void __launch_bounds__(256, kLsumBlocks)
     const uint32_t var = flags >> 4;
     const VariantParameters& p = lut[var];
     const uint32_t prop = p.signal_propagation_length;
-    const bool exact = prop == s_pmax;
+    const bool exact = prop == pmax;
     const bool gfast = exact && prop <= 16u;
     if (cw & kRowBad) kc.err |= AXC_ERR_TARGET_RANGE;
     const uint32_t* rt_n = rt + (size_t)n * kRowStride;
@@ -2258,7 +2347,8 @@ __global__ void __launch_bounds__(256, kLsumBlocks)
   }
   const uint32_t err_any = __reduce_or_sync(kFull, kc.err);
   if (err_any && (threadIdx.x & 31) == 0) atomicOr(&ctl->err, err_any);
-  block_count256(kc.ev_slots, kc.hits, kc.nspk, kc.gdone, kc.nev, kc.tested, ctl->ctr);
+  const uint32_t counts[6] = {kc.ev_slots, kc.hits, kc.nspk, kc.gdone, kc.nev, kc.tested};
+  block_counts(counts, ctl);
 }
 
 // ---------------------------------------------------------------------------
@@ -2286,9 +2376,9 @@ __global__ void __launch_bounds__(256) k_rows_gsop(ShardVramPtrs P, uint32_t A, 
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
   lut_to_smem(lut);
-  if (threadIdx.x == 0) s_pmax = lut_pmax();
   __syncthreads();
   const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
+  pmax_of(&s_pmax, lut);
   build_gtab(gtab, lut, dopamine);
   __syncthreads();
   const uint32_t ecount = ctl->eval_act[k & 1][0];
@@ -2328,12 +2418,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop(ShardVramPtrs P, uint32_t A, 
         const uint32_t am0 = __shfl_sync(kFull, my_am.x, owner), am1 = __shfl_sync(kFull, my_am.y, owner);
         const uint32_t am2 = __shfl_sync(kFull, my_am.z, owner), am3 = __shfl_sync(kFull, my_am.w, owner);
         if (it >= total) continue;
-        uint32_t rank = it - prev, q;   // the rank-th set bit of the owner's mask
-        const uint32_t c0 = __popc(am0), c1 = __popc(am1), c2 = __popc(am2);
-        if (rank < c0) q = __fns(am0, 0, rank + 1);
-        else if ((rank -= c0) < c1) q = 32u + __fns(am1, 0, rank + 1);
-        else if ((rank -= c1) < c2) q = 64u + __fns(am2, 0, rank + 1);
-        else q = 96u + __fns(am3, 0, rank - c2 + 1);
+        const uint32_t q = nth_bit128(make_uint4(am0, am1, am2, am3), it - prev);
         const uint8_t flags = P.soma_flags[n];
         const uint32_t var = flags >> 4;
         const VariantParameters& p = lut[var];
@@ -2400,9 +2485,9 @@ __global__ void __launch_bounds__(256) k_rows_gsop_rows(ShardVramPtrs P, uint32_
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
   lut_to_smem(lut);
-  if (threadIdx.x == 0) s_pmax = lut_pmax();
   __syncthreads();
   const int32_t dopamine = (int32_t)(int16_t)ctl->dopamine;
+  pmax_of(&s_pmax, lut);
   build_gtab(gtab, lut, dopamine);
   __syncthreads();
   const uint32_t ecount = ctl->eval_act[k & 1][0];
@@ -2473,25 +2558,23 @@ __device__ __forceinline__ void fixup_slot(const ShardVramPtrs& P, const Variant
 // what the dense pass loses to the sparse form in ~20 ticks (1.5M neurons).
 constexpr uint32_t kIndexStreak = 16;
 
-__global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N, uint32_t A,
-                                                    const uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
-                                                    const uint16_t* __restrict__ cnt,
-                                                    const uint2* __restrict__ mask2, const uint32_t* __restrict__ pend,
-                                                    const uint32_t* __restrict__ eval,
-                                                    const uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl,
-                                                    uint32_t k, const uint32_t* __restrict__ ids,
-                                                    uint8_t* __restrict__ out, uint32_t num_outputs, ColWT wt,
-                                                    volatile uint32_t* wish) {
-  chain_wait();
-  chain_open();
+// The next tick's lists (last used two ticks ago).
+__device__ __forceinline__ void rows_next_lists(ShardCtl* ctl, uint32_t k) {
+  ctl->eval_act[(k + 1) & 1][0] = ctl->eval_act[(k + 1) & 1][1] = 0;
+  ctl->dense[(k + 1) & 1] = 0;
+}
+
+__device__ __forceinline__ void rows_fixup(const ShardVramPtrs& P, uint32_t N, uint32_t A, const uint32_t* rt,
+                                           int16_t* rw, const uint16_t* cnt, const uint2* mask2, const uint32_t* pend,
+                                           const uint32_t* eval, const uint32_t* fix, ShardCtl* ctl, uint32_t k,
+                                           const uint32_t* ids, uint8_t* out, uint32_t num_outputs, const ColWT& wt,
+                                           volatile uint32_t* wish) {
   const uint32_t nfix = ctl->fix_count;
   const uint32_t overflow = ctl->fix_overflow;
   {
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid == 0) {
-      ctl->eval_act[(k + 1) & 1][0] = ctl->eval_act[(k + 1) & 1][1] = 0;   // the next tick's (last used two ticks ago)
-      ctl->dense[(k + 1) & 1] = 0;
       // ticks in a row that the sparse form would take: ask for its index
       if (wish) {
         const uint32_t streak = !lsum_tick(ctl, k) && sparse_tick(ctl, k) ? ctl->streak + 1u : 0u;
@@ -2549,23 +2632,32 @@ __global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N,
   }
 }
 
+__global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N, uint32_t A,
+                                                    const uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
+                                                    const uint16_t* __restrict__ cnt,
+                                                    const uint2* __restrict__ mask2, const uint32_t* __restrict__ pend,
+                                                    const uint32_t* __restrict__ eval,
+                                                    const uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl,
+                                                    uint32_t k, const uint32_t* __restrict__ ids,
+                                                    uint8_t* __restrict__ out, uint32_t num_outputs, ColWT wt,
+                                                    volatile uint32_t* wish) {
+  chain_wait();
+  chain_open();
+  if (blockIdx.x == 0 && threadIdx.x == 0) rows_next_lists(ctl, k);
+  rows_fixup(P, N, A, rt, rw, cnt, mask2, pend, eval, fix, ctl, k, ids, out, num_outputs, wt, wish);
+}
+
 // per tick 4/4, on a batch's (or learned graph's) last tick: the spikers'
 // own-axon pushes (physics.cu:257-261), found in the evaluated list; on the
 // other ticks the next prologue applies them.
-__global__ void __launch_bounds__(256) k_rows_push(BurstHeads8* __restrict__ heads, const uint32_t* __restrict__ s2a,
-                                                   uint32_t A, uint32_t* __restrict__ pend,
-                                                   const uint32_t* __restrict__ eval, const uint8_t* __restrict__ flags,
-                                                   uint32_t N, const uint32_t* __restrict__ ids,
-                                                   uint8_t* __restrict__ out, uint32_t num_outputs,
-                                                   ShardCtl* __restrict__ ctl, uint32_t k) {
-  chain_wait();
-  chain_open();
+__device__ __forceinline__ void rows_push(BurstHeads8* heads, const uint32_t* s2a, uint32_t A, uint32_t* pend,
+                                          const uint32_t* eval, const uint8_t* flags, uint32_t N, const uint32_t* ids,
+                                          uint8_t* out, uint32_t num_outputs, ShardCtl* ctl, uint32_t k) {
   const uint32_t ecount = ctl->eval_act[k & 1][0];
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid == 0) {
-    ctl->eval_act[(k + 1) & 1][0] = ctl->eval_act[(k + 1) & 1][1] = 0;
-    ctl->dense[(k + 1) & 1] = 0;
+    rows_next_lists(ctl, k);
     ctl->fix_count = 0;
     ctl->fix_overflow = 0;
   }
@@ -2594,6 +2686,17 @@ __global__ void __launch_bounds__(256) k_rows_push(BurstHeads8* __restrict__ hea
     out[j] = v;
   }
   if (err) atomicOr(&ctl->err, err);
+}
+
+__global__ void __launch_bounds__(256) k_rows_push(BurstHeads8* __restrict__ heads, const uint32_t* __restrict__ s2a,
+                                                   uint32_t A, uint32_t* __restrict__ pend,
+                                                   const uint32_t* __restrict__ eval, const uint8_t* __restrict__ flags,
+                                                   uint32_t N, const uint32_t* __restrict__ ids,
+                                                   uint8_t* __restrict__ out, uint32_t num_outputs,
+                                                   ShardCtl* __restrict__ ctl, uint32_t k) {
+  chain_wait();
+  chain_open();
+  rows_push(heads, s2a, A, pend, eval, flags, N, ids, out, num_outputs, ctl, k);
 }
 
 __global__ void k_rows_reset_lists(ShardCtl* ctl) {
@@ -2627,30 +2730,22 @@ __device__ __forceinline__ void push_few(uint32_t h[8], uint32_t c) {
 
 // INDEX: also the live axons' and evaluated neurons' bits and the active axons'
 // count, for the sparse form (the learned engine's plain graph).
-template <int ITEMS, bool INDEX>
-__global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __restrict__ heads, uint32_t A,
-                                                             uint32_t v_seg, const uint32_t* __restrict__ bitmask,
-                                                             uint32_t voff, uint32_t nv,
-                                                             uint32_t* __restrict__ incoming,
-                                                             const uint32_t* __restrict__ batch_counts, uint32_t k,
-                                                             uint2* __restrict__ mask2,
-                                                             const uint32_t* __restrict__ axw,
-                                                             uint8_t* __restrict__ flags,
-                                                             uint8_t* __restrict__ timers, uint32_t N,
-                                                             uint32_t* __restrict__ eval, ShardCtl* __restrict__ ctl,
-                                                             uint32_t raise_err, uint32_t* __restrict__ lit_bits,
-                                                             uint32_t* __restrict__ pend_apply, uint32_t inc_direct,
-                                                             uint32_t set_tick, uint32_t tick_base, int32_t dopamine,
-                                                             const uint32_t* __restrict__ xlit,
-                                                             uint32_t* __restrict__ live,
-                                                             uint32_t* __restrict__ evb, uint32_t* __restrict__ alit,
-                                                             uint32_t alit_new) {
+// The flags that a refractory neuron's tick clears (physics.cu:168-174): stored here,
+// or with SMALL (one item) returned with bit 8 set for the caller to store; the listed
+// neurons stay in s_list, their count and place in the tick's list in s_place.
+template <int ITEMS, bool INDEX, int THREADS, bool SMALL>
+__device__ __forceinline__ uint32_t rows_prologue(uint32_t i0, BurstHeads8* heads, uint32_t A, uint32_t v_seg,
+                                                  const uint32_t* bitmask, uint32_t voff, uint32_t nv,
+                                                  uint32_t* incoming, const uint32_t* batch_counts, uint32_t k,
+                                                  uint2* mask2, const uint32_t* axw, uint8_t* flags, uint8_t* timers,
+                                                  uint32_t N, uint32_t* eval, ShardCtl* ctl, uint32_t raise_err,
+                                                  uint32_t* lit_bits, uint32_t* pend_apply, uint32_t inc_direct,
+                                                  uint32_t set_tick, uint32_t tick_base, int32_t dopamine,
+                                                  const uint32_t* xlit, uint32_t* live, uint32_t* evb, uint32_t* alit,
+                                                  uint32_t alit_new, uint32_t* s_list, uint32_t* s_place) {
   __shared__ uint32_t s_base;
-  __shared__ uint32_t s_warp[ITEMS][8];   // evaluated neurons | active axons << 16
+  __shared__ uint32_t s_warp[ITEMS][THREADS / 32];   // evaluated neurons | active axons << 16
 
-  chain_wait();
-  chain_open();
-  const uint32_t i0 = blockIdx.x * (256u * ITEMS) + threadIdx.x;
   // all loads first: heads, owners, pending pushes, input bits, timers, constants,
   // and the axons the row layout took as fully lit (xlit, 32 per warp)
   uint4 hx[ITEMS], hy[ITEMS];
@@ -2658,7 +2753,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
   uint8_t tm[ITEMS], fl[ITEMS];
 #pragma unroll
   for (int r = 0; r < ITEMS; r++) {
-    const uint32_t i = i0 + 256u * r;
+    const uint32_t i = i0 + (uint32_t)THREADS * r;
     npush[r] = 0;
     own[r] = 0;
     tm[r] = 0;
@@ -2696,10 +2791,10 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
   // segments the batch's slots use: 0..seg_max (bit 31: any segment >= 31)
   const uint32_t act = seg_max >= 31u ? 0xFFFFFFFFu : ((2u << seg_max) - 1u);
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t ebal[ITEMS];
+  uint32_t ebal[ITEMS], clear = 0;
 #pragma unroll
   for (int r = 0; r < ITEMS; r++) {
-    const uint32_t i = i0 + 256u * r;
+    const uint32_t i = i0 + (uint32_t)THREADS * r;
     bool lit = false, on = false;
     if (i < A) {
       uint32_t c = npush[r];
@@ -2736,7 +2831,12 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
     if (i < N) {
       if (tm[r] > 0) {                              // physics.cu:168-174 after the burst reset
         timers[i] = (uint8_t)(tm[r] - 1);
-        if (fl[r] & 0x0Fu) flags[i] = fl[r] & 0xF0u;
+        if (fl[r] & 0x0Fu) {
+          if (SMALL)
+            clear = 0x100u | (fl[r] & 0xF0u);
+          else
+            flags[i] = fl[r] & 0xF0u;
+        }
       } else {
         ev = true;
       }
@@ -2748,23 +2848,66 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t tot = 0;
-    for (int q = 0; q < ITEMS * 8; q++) {
-      const uint32_t c = (&s_warp[0][0])[q];
-      (&s_warp[0][0])[q] = INDEX ? tot & 0xFFFFu : tot;
-      tot += c;
+  if (w == 0) {   // exclusive scan of the warps' counts, then the block's place in the list
+    constexpr uint32_t E = ITEMS * (THREADS / 32), PER = (E + 31) / 32;
+    uint32_t c[PER], sum = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+      c[q] = lane * PER + q < E ? (&s_warp[0][0])[lane * PER + q] : 0u;
+      sum += c[q];
     }
-    if (INDEX)
-      s_base = append_count(ctl, k, tot & 0xFFFFu, tot >> 16);
-    else
-      s_base = tot ? atomicAdd(&ctl->eval_act[k & 1][0], tot) : 0u;
+    const uint32_t incl = warp_incl(sum);
+    uint32_t run = incl - sum;
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+      if (lane * PER + q < E) (&s_warp[0][0])[lane * PER + q] = INDEX ? run & 0xFFFFu : run;
+      run += c[q];
+    }
+    if (lane == 31) {
+      if (INDEX)
+        s_base = append_count(ctl, k, incl & 0xFFFFu, incl >> 16);
+      else if (SMALL)
+        s_place[0] = incl;
+      else
+        s_base = incl ? atomicAdd(&ctl->eval_act[k & 1][0], incl) : 0u;
+    }
   }
   __syncthreads();
+  if (SMALL) {   // the block's own list; its place in the tick's list (for the fix-up and the push) arrives later
+    if (w == 1 && lane == 0) s_place[1] = s_place[0] ? atomicAdd(&ctl->eval_act[k & 1][0], s_place[0]) : 0u;
+    if ((ebal[0] >> lane) & 1u) s_list[s_warp[0][w] + __popc(ebal[0] & ((1u << lane) - 1u))] = i0;
+    return clear;
+  }
 #pragma unroll
   for (int r = 0; r < ITEMS; r++)
     if ((ebal[r] >> lane) & 1u)
-      eval[s_base + s_warp[r][w] + __popc(ebal[r] & ((1u << lane) - 1u))] = i0 + 256u * r;
+      eval[s_base + s_warp[r][w] + __popc(ebal[r] & ((1u << lane) - 1u))] = i0 + (uint32_t)THREADS * r;
+  return clear;
+}
+
+template <int ITEMS, bool INDEX>
+__global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __restrict__ heads, uint32_t A,
+                                                             uint32_t v_seg, const uint32_t* __restrict__ bitmask,
+                                                             uint32_t voff, uint32_t nv,
+                                                             uint32_t* __restrict__ incoming,
+                                                             const uint32_t* __restrict__ batch_counts, uint32_t k,
+                                                             uint2* __restrict__ mask2,
+                                                             const uint32_t* __restrict__ axw,
+                                                             uint8_t* __restrict__ flags,
+                                                             uint8_t* __restrict__ timers, uint32_t N,
+                                                             uint32_t* __restrict__ eval, ShardCtl* __restrict__ ctl,
+                                                             uint32_t raise_err, uint32_t* __restrict__ lit_bits,
+                                                             uint32_t* __restrict__ pend_apply, uint32_t inc_direct,
+                                                             uint32_t set_tick, uint32_t tick_base, int32_t dopamine,
+                                                             const uint32_t* __restrict__ xlit,
+                                                             uint32_t* __restrict__ live,
+                                                             uint32_t* __restrict__ evb, uint32_t* __restrict__ alit,
+                                                             uint32_t alit_new) {
+  chain_wait();
+  chain_open();
+  rows_prologue<ITEMS, INDEX, 256, false>(blockIdx.x * (256u * ITEMS) + threadIdx.x, heads, A, v_seg, bitmask, voff,
+      nv, incoming, batch_counts, k, mask2, axw, flags, timers, N, eval, ctl, raise_err, lit_bits, pend_apply,
+      inc_direct, set_tick, tick_base, dopamine, xlit, live, evb, alit, alit_new, nullptr, nullptr);
 }
 // Items (an axon and a neuron each) per thread of k_rows_prologue_plain: two
 // halve the blocks, and with them the list-append atomics on one counter and
@@ -2774,6 +2917,180 @@ __global__ void __launch_bounds__(256) k_rows_prologue_plain(BurstHeads8* __rest
 // item per thread and twice the blocks (16k neurons: 66,644 ticks/s with one
 // item and 64 blocks, 60,629 with two and 32).
 constexpr uint32_t kProWide = 4864;
+
+// ---------------------------------------------------------------------------
+// small brains: a batch's ticks (or a per-tick call) in one launch
+// ---------------------------------------------------------------------------
+// A tick of a small brain is launches and latency: four kernels of 2 to 8 us, most
+// of it their start, their tables and one chain of dependent loads each.  Here the
+// stages of all ticks run in one grid of resident blocks with two barriers a tick
+// (a third where a GSOP slot was deferred or network spikes follow), the tables are
+// built once, a block keeps the neurons it lists, and a graph has one node for its
+// ticks.  16,384 neurons: 14.8 -> 9.6 us per tick of a batch; 2,048: 20.4 -> 18.8 us
+// per call of the per-tick entry point.
+struct SmallArgs {
+  ShardVramPtrs P;
+  uint32_t N, A, v_seg;
+  const uint32_t* bitmask;   // words per tick; null without input
+  uint32_t words, voff, nv, raise;
+  const uint32_t* spikes;    // network spikes, spike_cap per tick; null without
+  uint32_t spike_cap, spike_count;   // spike_count: without counts
+  const uint32_t* counts;
+  uint32_t* incoming;
+  uint32_t *rt, *eval, *pend, *fix, *lit, *alit, *xlit;
+  int16_t* rw;
+  const uint16_t* cnt;
+  const uint8_t* lfz;
+  const int2* rec;
+  const uint32_t* axw;
+  uint2* mask2;
+  ShardCtl* ctl;
+  const uint32_t* ids;       // readout; outputs 0 without
+  uint8_t* out;
+  uint32_t outputs, fix_cap;
+  uint32_t ticks, k0, lit_tick;   // lit_tick: the tick that starts alit anew, or ticks
+  uint32_t set_tick, tick_base;   // set_tick: a per-tick call (tick_base, dopamine from here)
+  int32_t dopamine;
+  ColWT wt;
+};
+
+constexpr uint32_t kGridWaitLimit = 1u << 22;   // tries: about 3 s
+
+// All threads of the grid.  CLUSTER: the cluster's hardware barrier.  Else a counter
+// that every block adds to (zeroed before each launch), with a bounded wait: false
+// once a block gave up, on which the grid's blocks all return.
+template <bool CLUSTER>
+__device__ __forceinline__ bool small_barrier(ShardCtl* ctl, uint32_t& target, uint32_t* s_ok) {
+  if (CLUSTER) {
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+    return true;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    target += gridDim.x;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->barrier) : "memory");
+    bool ok = false;
+    for (uint32_t it = 0; it < kGridWaitLimit && !ok; it++) {
+      uint32_t seen;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&ctl->barrier) : "memory");
+      ok = (int32_t)(seen - target) >= 0;
+    }
+    if (!ok) atomicOr(&ctl->err, AXC_ERR_WAIT_LIMIT);
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+__device__ __forceinline__ uint32_t small_spikes(const SmallArgs& b, uint32_t t) {
+  if (!b.spikes) return 0u;
+  return b.counts ? min(b.counts[t], b.spike_cap) : b.spike_count;
+}
+
+__device__ __forceinline__ void small_incoming(const SmallArgs& b, uint32_t t) {
+  const uint32_t n = small_spikes(b, t);
+  const uint32_t* ids = b.spikes + (size_t)t * b.spike_cap;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    if (ids[i] < b.A) atomicAdd(&b.incoming[ids[i]], 1u);
+}
+
+template <bool CLUSTER, bool WT>
+__global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ SmallArgs b) {
+  __shared__ VariantParameters lut[16];
+  __shared__ int2 gtab[16][16];
+  __shared__ uint32_t ptab[16][17];
+  __shared__ uint32_t s_pmax, s_ok, s_place[2];
+  __shared__ uint32_t s_list[1024];     // the block's evaluated neurons of the tick
+  __shared__ uint32_t s_cnt[8][32];     // each warp's counts
+  __shared__ uint64_t s_bar;
+  extern __shared__ __align__(128) uint32_t s_lit[];
+  ShardCtl* ctl = b.ctl;
+  if (threadIdx.x == 0) mbar_init(&s_bar, 1);
+  if (threadIdx.x < 256) (&s_cnt[0][0])[threadIdx.x] = 0;
+  lut_to_smem(lut);
+  __syncthreads();
+  pmax_of(&s_pmax, lut);
+  const int32_t dopamine = (int32_t)(int16_t)(b.set_tick ? b.dopamine : ctl->dopamine);
+  build_gtab(gtab, lut, dopamine);
+  __syncthreads();
+  const bool packed = build_ptab(ptab, gtab);
+  // axons and list entries go to the blocks warp by warp: few of them use every SM
+  const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  uint32_t target = 0, parity = 0;
+  bool staging = true;
+  const uint32_t smax = ctl->row_smax, seg_max = ctl->seg_max;
+  const uint32_t tick0 = (b.set_tick ? b.tick_base : ctl->tick_base) + b.k0;
+  if (small_spikes(b, 0)) {
+    small_incoming(b, 0);
+    if (!small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+  }
+  for (uint32_t t = 0; t < b.ticks; t++) {
+    const uint32_t k = b.k0 + t;
+    const uint32_t item = wid * 32u + (threadIdx.x & 31u);
+    const uint32_t clear = rows_prologue<1, false, 1024, true>(item, b.P.axon_heads, b.A, b.v_seg,
+                                  b.bitmask ? b.bitmask + (size_t)t * b.words : nullptr, b.voff, b.nv, b.incoming,
+                                  nullptr, k, b.mask2, b.axw, b.P.soma_flags, b.P.timers, b.N, b.eval, ctl, b.raise,
+                                  b.lit, t ? b.pend : nullptr, small_spikes(b, t) != 0u, b.set_tick, b.tick_base,
+                                  b.dopamine, b.xlit, nullptr, nullptr, b.alit, t == b.lit_tick ? 1u : 0u, s_list,
+                                  s_place);
+    if (!small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+    const TickForm form = tick_form(ctl, k, nullptr, 0u);
+    const uint32_t ecount = s_place[0];
+    if (threadIdx.x < ecount) b.eval[s_place[1] + threadIdx.x] = s_list[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 0) rows_next_lists(ctl, k);
+    if (clear) b.P.soma_flags[item] = (uint8_t)clear;   // after the readout of the tick before
+    // The lit-sum form's ticks take the 8-lane pass over the same rows: with a thread
+    // per neuron each neuron's slots are a serial chain, and there are few neurons.
+    const bool lit_rows = form == kFormLitSum || form == kFormLitRows;
+    // Else the fully-lit bitmap: other blocks' plain stores, then a bulk copy, over
+    // what this block's threads read in an earlier tick.
+    const bool stage = staging && !lit_rows;
+    bool lit_on = staging;
+    if (stage) {
+      if (threadIdx.x == 0) {
+        asm volatile("fence.proxy.async;" ::: "memory");
+        bulk_to_smem(s_lit, b.lit, lit_smem_bytes(b.A), &s_bar);
+      }
+      lit_on = __syncthreads_and(mbar_wait_bounded(&s_bar, parity, g_first_wait_limit));
+    }
+    uint32_t counts[8];
+    rows_update<WT>(lit_rows ? kFormLitRows : form, threadIdx.x >> 5, 32u, PassCtl{tick0 + t, smax, seg_max}, b.P, b.A,
+                    b.rt, b.rw, b.cnt, b.mask2, s_list, ecount, b.pend, b.fix, ctl, b.fix_cap, b.lfz, b.wt, b.rec, lut,
+                    gtab, form != kFormDense && packed ? ptab : nullptr, s_pmax, dopamine, s_lit, lit_on, counts);
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      const uint32_t x = __reduce_add_sync(kFull, counts[c]);
+      if ((threadIdx.x & 31u) == 0) s_cnt[c][threadIdx.x >> 5] += x;
+    }
+    if ((t & 255u) == 255u || t + 1 == b.ticks) {   // before 32 bits could overflow
+      __syncwarp();
+      uint32_t mine[8];
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        mine[c] = (threadIdx.x & 31u) == 0 ? s_cnt[c][threadIdx.x >> 5] : 0u;
+        if ((threadIdx.x & 31u) == 0) s_cnt[c][threadIdx.x >> 5] = 0;
+      }
+      block_counts(mine, ctl);
+    }
+    if (stage) {
+      // a wait that gave up: the copy must land before the next one
+      if (!lit_on) staging = __syncthreads_and(mbar_wait_bounded(&s_bar, parity));
+      parity ^= 1u;
+    }
+    if (!small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+    const uint32_t nfix = ctl->fix_count | ctl->fix_overflow;
+    rows_fixup(b.P, b.N, b.A, b.rt, b.rw, b.cnt, b.mask2, b.pend, b.eval, b.fix, ctl, k, b.ids,
+               b.out + (size_t)t * b.outputs, b.outputs, b.wt, nullptr);
+    const bool spikes = t + 1 < b.ticks && small_spikes(b, t + 1) != 0u;
+    if (spikes) small_incoming(b, t + 1);
+    // What comes next writes what the fix-up reads (heads, pending pushes) and reads
+    // the network spikes' counts, but leaves the readout's flags: no barrier without them.
+    if ((nfix || spikes) && !small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+  }
+  // the last tick's soma pushes
+  rows_push(b.P.axon_heads, b.P.soma_to_axon, b.A, b.pend, b.eval, b.P.soma_flags, b.N, nullptr, nullptr, 0u, ctl,
+            b.k0 + b.ticks - 1u);
+}
 
 }  // namespace
 
@@ -2920,9 +3237,7 @@ static size_t lit_smem_limit() {
     if (cudaFuncSetAttribute(k_rows_update<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_rows_update<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_rows_update<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)lim) != cudaSuccess) {
+            cudaSuccess) {
       cudaGetLastError();
       lim = 0;
     }
@@ -2936,44 +3251,39 @@ static size_t lit_smem_limit() {
 // sparse ticks), or null.
 static bool rows_lit(uint32_t A) { return (size_t)lit_smem_bytes(A) <= lit_smem_limit(); }
 
-// inline: GSOP inside the pass (rows with their movable slots first), else
-// the spikers are listed for launch_rows_gsop.
 // pdl: launched into the tick's kernel chain (launch_chain).
-template <bool INLINE>
 static void launch_rows_update(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, uint32_t k,
                                uint32_t fix_cap, const LearnCtl* lc, cudaStream_t stream, ColWT wt = ColWT{},
-                               bool pdl = false, bool index = false) {
+                               bool pdl = false, bool index = false, bool shared_gpu = false) {
   RowCache& r = *s.rows;
   const int sms = sm_count();
   const bool lit = rows_lit(A);
   const dim3 grid(lit ? sms : 4 * sms), block(lit ? 1024 : 256);
   const size_t smem = lit ? lit_smem_bytes(A) : 0;
   auto go = [&](auto kern) {
-    launch_chain(kern, grid, block, smem, stream, pdl, v, N, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix,
-                 s.ctl, k, fix_cap, r.lit, lc, r.gs_n, r.gd_n, r.lfz, r.wcnt, wt, index ? 1u : 0u, r.rec);
+    launch_chain(kern, grid, block, smem, stream, pdl, v, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix, s.ctl,
+                 k, fix_cap, r.lit, lc, r.lfz, wt, index ? 1u : 0u, r.rec, shared_gpu ? block.x / 8u : 4u);
   };
-  if constexpr (INLINE) {
-    if (wt.w) {   // the per-tick entry point: weight changes written through
-      if (lit)
-        go(k_rows_update<true, true, true>);
-      else
-        go(k_rows_update<false, true, true>);
-      return;
-    }
+  if (wt.w) {   // the per-tick entry point: weight changes written through
+    if (lit)
+      go(k_rows_update<true, true>);
+    else
+      go(k_rows_update<false, true>);
+  } else if (lit) {
+    go(k_rows_update<true, false>);
+  } else {
+    go(k_rows_update<false, false>);
   }
-  if (lit)
-    go(k_rows_update<true, INLINE>);
-  else
-    go(k_rows_update<false, INLINE>);
 }
 
 // The lit-sum form's pass.
 static void launch_rows_lsum(const ShardVramPtrs& v, ShardScratch& s, uint32_t A, uint32_t k, uint32_t fix_cap,
-                             const LearnCtl* lc, cudaStream_t stream, ColWT wt = ColWT{}, bool pdl = false) {
+                             const LearnCtl* lc, cudaStream_t stream, ColWT wt = ColWT{}, bool pdl = false,
+                             bool shared_gpu = false) {
   RowCache& r = *s.rows;
   launch_chain(wt.w ? k_rows_update_lsum<true> : k_rows_update_lsum<false>, dim3(kLsumBlocks * sm_count()), dim3(256),
                0, stream, pdl, v, A, r.rt, r.rw, r.cnt, r.mask2, r.eval, s.pend, r.fix, s.ctl, k, fix_cap, r.lit,
-               r.rec, wt, lc);
+               r.rec, wt, lc, shared_gpu ? 256u : 32u);
 }
 
 // The sparse form (the learned engine's graphs): hits, then neurons, persistent warps.
@@ -3053,9 +3363,9 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
   // with GSOP; both are launched and each returns at once on the other's
   // ticks), ev[4]..ev[5] fix-up and push.
   const uint32_t fix_cap = min(a.fix_cap, kFixCap);
-  launch_rows_update<true>(v, s, N, A, a.k, fix_cap, nullptr, stream, wt, pdl && G, a.index);
+  launch_rows_update(v, s, N, A, a.k, fix_cap, nullptr, stream, wt, pdl && G, a.index, a.shared_gpu);
   if (ev) cudaEventRecord(ev[3], stream);
-  launch_rows_lsum(v, s, A, a.k, fix_cap, nullptr, stream, wt, pdl);
+  launch_rows_lsum(v, s, A, a.k, fix_cap, nullptr, stream, wt, pdl, a.shared_gpu);
   if (a.index) launch_rows_sparse(v, s, N, A, a.k, fix_cap, nullptr, stream);
   if (ev) cudaEventRecord(ev[4], stream);
   const bool readout = a.num_outputs > 0 && a.mapped_soma_ids && a.output_history;
@@ -3068,6 +3378,135 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
                  r.eval, v.soma_flags, N, (const uint32_t*)nullptr, (uint8_t*)nullptr, 0u, s.ctl, a.k);
   if (ev) cudaEventRecord(ev[5], stream);
   return cudaGetLastError();
+}
+
+// Rows that run in one cluster / in one resident grid (k_rows_small), by the larger
+// of neurons and axons.  A cluster's barrier takes 0.7 us and the grid's 1.2, but its
+// 16 SMs take longer over 4,000 plastic rows (45 us a per-tick call) than the
+// kernel chain (39); the grid is even with the chain at 100,000 axons (saturated
+// rows: 370 us per 20 ticks on both) and behind it at 150,000 (432 against 400).
+constexpr uint32_t kSmallCluster = 4096, kSmallTick = 3072;   // the latter: per-tick calls
+constexpr uint32_t kSmallBlocks = 640;   // a resident grid: neurons or axons per SM
+
+// Blocks of k_rows_small's cluster here, 0 where none fits.
+static uint32_t small_cluster() {
+  static uint32_t size = [] {
+    for (const uint32_t c : {16u, 8u}) {
+      int n = 0, m = 0;
+      auto fits = [&](auto kern, int* out) {
+        if (c > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+          return false;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(1024);
+        cfg.dynamicSmemBytes = lit_smem_bytes(kSmallCluster);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = c;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaOccupancyMaxActiveClusters(out, kern, &cfg) == cudaSuccess && *out > 0;
+      };
+      if (fits(k_rows_small<true, false>, &n) && fits(k_rows_small<true, true>, &m)) return c;
+      cudaGetLastError();
+    }
+    return 0u;
+  }();
+  return size;
+}
+
+// Blocks of k_rows_small's resident grid here, 0 where it does not fit.
+static uint32_t small_grid() {
+  static uint32_t size = [] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_rows_small<false, false>, 1024,
+                                                      lit_smem_bytes(kSmallBlocks * sm_count())) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    return n > 0 ? (uint32_t)sm_count() : 0u;
+  }();
+  return size;
+}
+
+bool rows_small(uint32_t N, uint32_t A, bool whole_gpu, bool batch) {
+  const uint32_t G = max(N, A);
+  if (G <= (batch ? kSmallCluster : kSmallTick) && small_cluster()) return true;
+  return whole_gpu && G <= kSmallBlocks * (uint32_t)sm_count() && small_grid();
+}
+
+cudaError_t launch_rows_small(const ShardVramPtrs& v, ShardScratch& s, const TickArgs& a, uint32_t ticks,
+                              uint32_t words, cudaStream_t stream) {
+  RowCache& r = *s.rows;
+  SmallArgs b{};
+  b.P = v;
+  b.N = a.padded_n;
+  b.A = a.total_axons;
+  b.v_seg = a.v_seg;
+  b.bitmask = a.num_virtual > 0 ? a.input_bitmask : nullptr;
+  b.words = words;
+  b.voff = a.virtual_offset;
+  b.nv = a.num_virtual;
+  b.raise = b.bitmask && (uint64_t)a.virtual_offset + a.num_virtual > b.A ? AXC_ERR_VIRTUAL_RANGE : 0u;
+  b.spikes = a.batch || a.num_incoming > 0 ? a.incoming_spikes : nullptr;
+  b.spike_cap = a.max_incoming;
+  b.spike_count = a.num_incoming;
+  b.counts = a.batch ? s.batch_counts : nullptr;
+  b.incoming = s.incoming;
+  b.rt = r.rt;
+  b.eval = r.eval;
+  b.pend = s.pend;
+  b.fix = r.fix;
+  b.lit = r.lit;
+  b.alit = r.alit;
+  b.xlit = r.xlit;
+  b.rw = r.rw;
+  b.cnt = r.cnt;
+  b.lfz = r.lfz;
+  b.rec = r.rec;
+  b.axw = r.axw;
+  b.mask2 = r.mask2;
+  b.ctl = s.ctl;
+  if (a.num_outputs > 0 && a.mapped_soma_ids && a.output_history) {
+    b.ids = a.mapped_soma_ids;
+    b.out = a.output_history;
+    b.outputs = a.num_outputs;
+  }
+  b.fix_cap = min(a.fix_cap, kFixCap);
+  b.ticks = ticks;
+  b.k0 = a.k;
+  b.lit_tick = a.batch ? (ticks > kLitWindow ? ticks - kLitWindow : 0u) : a.lit_new ? 0u : ticks;
+  b.set_tick = a.batch ? 0u : 1u;
+  b.tick_base = a.tick - a.k;
+  b.dopamine = a.dopamine;
+  if (!a.batch) {
+    b.wt.w = v.dendrite_weights;
+    b.wt.om = r.omask;
+    b.wt.lm = r.lmask;
+    b.wt.N = b.N;
+  }
+  const bool cluster = max(b.N, b.A) <= kSmallCluster && small_cluster();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster ? small_cluster() : small_grid());
+  cfg.blockDim = dim3(1024);
+  cfg.dynamicSmemBytes = lit_smem_bytes(b.A);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  if (cluster) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cfg.gridDim.x;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg,
+                            !cluster ? k_rows_small<false, false> : a.batch ? k_rows_small<true, false>
+                                                                            : k_rows_small<true, true>,
+                            b);
 }
 
 // Index of the current rows.  Entries are counted per axon, placed through a

@@ -139,7 +139,7 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
     // fork: every shard's tick loop on its own branch
     for (uint32_t i = 0; i < nshards && le == cudaSuccess; i++) {
       le = cudaStreamWaitEvent(c.branch[i], c.events[0], 0);
-      if (le == cudaSuccess) le = batch_capture(args[i], *scr[i], rows[i], fix_cap, c.branch[i]);
+      if (le == cudaSuccess) le = batch_capture(args[i], *scr[i], rows[i], fix_cap, c.branch[i], nshards == 1);
       if (le == cudaSuccess) le = cudaEventRecord(c.events[1 + i], c.branch[i]);
       if (le == cudaSuccess) le = cudaStreamWaitEvent(c.root, c.events[1 + i], 0);
     }
