@@ -807,47 +807,56 @@ __global__ void __launch_bounds__(256) k_rows_mult(const uint32_t* __restrict__ 
 
 // Batch end: weights rows -> columnar.  The slots of lmask[n] (in slot order) and
 // then the others of omask[n] are the row's first positions, the only slots
-// whose weights GSOP can have changed.  A thread per neuron where few are (a
-// neuron without any, every one of a frozen row, costs one 16-byte load: 19 us at
-// 1.5M settled neurons); a block with a neuron that has more than 8 goes
-// through shared memory, 32 neurons at a time: rows read whole, columns written
-// 64 bytes a warp.
+// whose weights GSOP can have changed.  Two kernels, one of which returns at once: a
+// thread per neuron where the rows have few such slots (a neuron without any, every
+// one of a frozen row, costs one 16-byte load; 8M settled neurons: 66 us, 176 through
+// the tiles' registers and shared memory), else tiles of 32 neurons: rows read whole,
+// columns written 64 bytes a warp (512k plastic neurons: 100 us against 228).
+__device__ __forceinline__ bool writeback_tiled(const ShardCtl* ctl, uint32_t N) {
+  return ctl->mov_total + ctl->pfx_total > 24ull * N;
+}
+
 __global__ void __launch_bounds__(256) k_rows_writeback(int16_t* __restrict__ weights, uint32_t N,
                                                         const int16_t* __restrict__ rw,
                                                         const uint4* __restrict__ omask,
-                                                        const uint4* __restrict__ lmask) {
-  __shared__ int16_t s_w[AXC_MAX_DENDRITES][34];
-  __shared__ uint32_t s_m[32][4];
-  const uint32_t nb = blockIdx.x * 256u, n = nb + threadIdx.x;
-  const uint4 om = n < N ? omask[n] : make_uint4(0, 0, 0, 0);
-  const uint32_t mine = __popc(om.x) + __popc(om.y) + __popc(om.z) + __popc(om.w);
-  if (!__syncthreads_or(mine > 8u)) {
-    if (!mine) return;
-    const uint4 lm = lmask[n];
-    const uint32_t o[4] = {om.x, om.y, om.z, om.w}, x[4] = {lm.x, lm.y, lm.z, lm.w};
-    const int16_t* row = rw + (size_t)n * kRowStride;
-    uint32_t k = 0;
+                                                        const uint4* __restrict__ lmask,
+                                                        const ShardCtl* __restrict__ ctl) {
+  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint4 om = n < N ? omask[n] : make_uint4(0, 0, 0, 0);   // asked for beside the control block
+  if (writeback_tiled(ctl, N) || !(om.x | om.y | om.z | om.w)) return;
+  const uint4 lm = lmask[n];
+  const uint32_t o[4] = {om.x, om.y, om.z, om.w}, x[4] = {lm.x, lm.y, lm.z, lm.w};
+  const int16_t* row = rw + (size_t)n * kRowStride;
+  uint32_t k = 0;
 #pragma unroll
-    for (int pass = 0; pass < 2; pass++) {
+  for (int pass = 0; pass < 2; pass++) {
 #pragma unroll
-      for (int ch = 0; ch < 4; ch++) {
-        uint32_t b = pass ? o[ch] & ~x[ch] : x[ch];
-        while (b) {
-          const uint32_t q = 32u * ch + (uint32_t)(__ffs(b) - 1);
-          b &= b - 1u;
-          weights[(size_t)q * N + n] = row[k++];
-        }
+    for (int ch = 0; ch < 4; ch++) {
+      uint32_t b = pass ? o[ch] & ~x[ch] : x[ch];
+      while (b) {
+        const uint32_t q = 32u * ch + (uint32_t)(__ffs(b) - 1);
+        b &= b - 1u;
+        weights[(size_t)q * N + n] = row[k++];
       }
     }
-    return;
   }
+}
+
+__global__ void __launch_bounds__(256) k_rows_writeback_tiles(int16_t* __restrict__ weights, uint32_t N,
+                                                              const int16_t* __restrict__ rw,
+                                                              const uint4* __restrict__ omask,
+                                                              const uint4* __restrict__ lmask,
+                                                              const ShardCtl* __restrict__ ctl) {
+  __shared__ int16_t s_w[AXC_MAX_DENDRITES][34];
+  __shared__ uint32_t s_m[32][4];
+  if (!writeback_tiled(ctl, N)) return;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t t0 = 0; t0 < 256u && nb + t0 < N; t0 += 32u) {
+  for (uint32_t t0 = blockIdx.x * 32u; t0 < N; t0 += gridDim.x * 32u) {
     int16_t v[4][4];   // four neurons a warp, every load first
     uint32_t m[4][4];
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-      const uint32_t nn = nb + t0 + warp * 4u + e;
+      const uint32_t nn = t0 + warp * 4u + e;
       const uint4 a = nn < N ? omask[nn] : make_uint4(0, 0, 0, 0), b = nn < N ? lmask[nn] : make_uint4(0, 0, 0, 0);
       const uint32_t o[4] = {a.x, a.y, a.z, a.w}, x[4] = {b.x, b.y, b.z, b.w};
       uint32_t px = 0, po = popc4(x);
@@ -877,7 +886,7 @@ __global__ void __launch_bounds__(256) k_rows_writeback(int16_t* __restrict__ we
 #pragma unroll
     for (int i = 0; i < 16; i++) {
       const uint32_t r = warp + 8u * i;
-      if ((c[i >> 2] >> (r & 31u)) & 1u) weights[(size_t)r * N + nb + t0 + lane] = s_w[r][lane];
+      if ((c[i >> 2] >> (r & 31u)) & 1u) weights[(size_t)r * N + t0 + lane] = s_w[r][lane];
     }
   }
 }
@@ -1734,7 +1743,8 @@ __device__ __forceinline__ bool build_ptab(uint32_t (*tab)[17], const int2 (*gta
 // gsop_same.  Two warp reductions, one barrier and one atomic per counter: 64-bit
 // shuffles and a serial sum over 32 warps were 8,000 cycles of the 8-lane pass.
 template <int NC>
-__device__ __forceinline__ void block_counts(const uint32_t (&v)[NC], ShardCtl* ctl) {
+__device__ __forceinline__ void block_counts(const uint32_t (&v)[NC], unsigned long long* ctr,
+                                             unsigned long long* gsop_same = nullptr) {
   __shared__ uint32_t red[NC][32];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
@@ -1745,7 +1755,7 @@ __device__ __forceinline__ void block_counts(const uint32_t (&v)[NC], ShardCtl* 
   __syncthreads();
   if (w < (uint32_t)NC) {
     const uint32_t sum = __reduce_add_sync(kFull, lane < nw ? red[w][lane] : 0u);
-    unsigned long long* dst = w < 5u ? ctl->ctr + 1 + w : w == 5u ? ctl->ctr + 7 : ctl->gsop_same + (w - 6u);
+    unsigned long long* dst = w < 5u ? ctr + 1 + w : w == 5u ? ctr + 7 : gsop_same + (w - 6u);
     if (lane == 0 && sum) atomicAdd(dst, (unsigned long long)sum);
   }
 }
@@ -1933,7 +1943,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   rows_update<WT>(form, threadIdx.x >> 5, blockDim.x >> 5, pc, P, A, rt, rw, cnt, mask2, eval + first,
                   min(part, ecount - first), pend, fix, ctl, fix_cap, lfz, wt, rec, lut, gtab, packed ? ptab : nullptr,
                   s_pmax, dopamine, LIT ? s_lit : lit_bits, lit_on, counts);
-  block_counts(counts, ctl);
+  block_counts(counts, ctl->ctr, ctl->gsop_same);
   // a wait that gave up: the copy must land before the block exits
   if (LIT && !lit_on && !mbar_wait_bounded(&s_bar, 0)) atomicOr(&ctl->err, AXC_ERR_WAIT_LIMIT);
 }
@@ -2077,7 +2087,8 @@ __global__ void __launch_bounds__(256, 6)
       }
     }
   }
-  block_count(0, hits, 0, &ctl->ctr[1]);
+  const uint32_t counts[6] = {0, hits, 0, 0, 0, 0};
+  block_counts(counts, ctl->ctr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2235,7 +2246,7 @@ __global__ void __launch_bounds__(256, kNeuronBlocks)
   const uint32_t err_any = __reduce_or_sync(kFull, err);
   if (err_any && lane == 0) atomicOr(&ctl->err, err_any);
   const uint32_t counts[6] = {ev_slots, 0, nspk, gdone, nev, 0};
-  block_counts(counts, ctl);
+  block_counts(counts, ctl->ctr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2348,7 +2359,7 @@ __global__ void __launch_bounds__(256, kLsumBlocks)
   const uint32_t err_any = __reduce_or_sync(kFull, kc.err);
   if (err_any && (threadIdx.x & 31) == 0) atomicOr(&ctl->err, err_any);
   const uint32_t counts[6] = {kc.ev_slots, kc.hits, kc.nspk, kc.gdone, kc.nev, kc.tested};
-  block_counts(counts, ctl);
+  block_counts(counts, ctl->ctr);
 }
 
 // ---------------------------------------------------------------------------
@@ -3070,7 +3081,7 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
         mine[c] = (threadIdx.x & 31u) == 0 ? s_cnt[c][threadIdx.x >> 5] : 0u;
         if ((threadIdx.x & 31u) == 0) s_cnt[c][threadIdx.x >> 5] = 0;
       }
-      block_counts(mine, ctl);
+      block_counts(mine, ctl->ctr, ctl->gsop_same);
     }
     if (stage) {
       // a wait that gave up: the copy must land before the next one
@@ -3684,7 +3695,12 @@ cudaError_t rows_index_wish(const ShardVramPtrs& v, ShardScratch& s, uint32_t N,
 
 cudaError_t launch_rows_end(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, cudaStream_t stream) {
   RowCache& r = *s.rows;
-  if (N) k_rows_writeback<<<(N + 255) / 256, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.omask, r.lmask);
+  if (N) {
+    const uint32_t blocks = (N + 255) / 256;
+    k_rows_writeback<<<blocks, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.omask, r.lmask, s.ctl);
+    k_rows_writeback_tiles<<<std::min((N + 31) / 32, 4u * (uint32_t)sm_count()), 256, 0, stream>>>(
+        v.dendrite_weights, N, r.rw, r.omask, r.lmask, s.ctl);
+  }
   return cudaGetLastError();
 }
 
