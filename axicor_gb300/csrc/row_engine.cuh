@@ -8,20 +8,24 @@
 // the spikers' slots with one sector per slot.  For the length of one batch the
 // engine keeps a neuron-major copy ([neuron][128]) of targets and weights:
 //
-//   batch start  k_rows_mult       owners of each axon (none, one, several)
-//                k_rows_build      columnar -> rows (the slots whose weights may
-//                                  still move first), per-neuron counts and masks
-//   per tick     k_rows_prologue   the previous tick's soma pushes, axon pushes +
-//                                  propagation + split masks, fully-lit bitmap,
-//                                  refractory countdown, list of evaluated neurons
-//                k_rows_update     8 lanes per evaluated neuron: gather/sum, GLIF;
-//                                  lists the spikers with movable slots
-//                k_rows_gsop       GSOP of spikers with 1..8 movable slots
-//                k_rows_gsop_rows  GSOP of spikers with more, 8 lanes per row
+//   layout       k_rows_mult       owners of each axon (none, one, several)
+//                k_rows_build      columnar -> rows in groups by what a tick has to
+//                                  test and GSOP may move (build_row)
+//   per tick     k_rows_prologue_plain  the previous tick's soma pushes, axon
+//                                  pushes + propagation + split masks, fully-lit
+//                                  bitmap, refractory countdown, list of
+//                                  evaluated neurons
+//                k_rows_update     8 lanes per evaluated neuron: gather/sum, GLIF,
+//                                  GSOP of the movable slots
+//                k_rows_update_lsum  the same, a thread per neuron, on ticks that
+//                                  test few slots (tick_form)
+//                k_sparse_*        the same from an inverted index, on the learned
+//                                  engine's quiet ticks
 //                k_rows_fixup      readout, the GSOP slots whose result depends on
 //                                  same-tick pushes
 //                k_rows_push       the spikers' pushes (a batch's last tick only;
 //                                  otherwise the next prologue applies them)
+//   small brains k_rows_small      all of that for a batch's ticks in one launch
 //   batch end    k_rows_writeback  weights rows -> columnar
 //
 // GSOP against same-tick pushes.  GSOP must see the heads after this tick's
@@ -1349,8 +1353,9 @@ __device__ __forceinline__ GlifOut glif_step(const VariantParameters& p, int32_t
 
 // GSOP of a spiker's slots held by this lane (physics.cu:281-373): fast slots
 // from the gtab deltas, slow ones on the exact path or deferred to the fix-up
-// list.  same: 4-slot groups visited << 16 | those that kept their weights.  Writes the changed weights back to the row (rt_n / rw_n: the
-// neuron's row); returns the slots done.
+// list.  same: 4-slot groups visited << 16 | those that kept their weights.
+// Writes the changed weights back to the row (rt_n / rw_n: the neuron's row);
+// returns the slots done.
 template <bool WT = false>
 __device__ __forceinline__ uint32_t row_gsop(uint2 (&W)[4], uint32_t hitb, uint32_t slowb,
                                              uint32_t c, uint32_t g8, RowShape sh, const int2 (*gtab)[16],

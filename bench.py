@@ -322,6 +322,8 @@ def run_gb300(args, dist: Dist) -> dict | None:
     top = int(np.argmax(stage_ms))
     ev, hits, spk, gs, nev, lit_ticks, tested = (int(x) for x in out_cnt)
     A_ = lay.total_axons
+    # brains whose ticks run in one launch (k_rows_small): 640 neurons or axons an SM
+    small = max(lay.padded_n, A_) <= 640 * torch.cuda.get_device_properties(0).multi_processor_count
     if engine == 1 and names[top] in ("update", "update_lsum"):
         # the bytes of the ticks that pass ran (the other returns at once)
         f = lit_ticks / prof_ticks
@@ -360,10 +362,10 @@ def run_gb300(args, dist: Dist) -> dict | None:
         "h2d": B * words * 4,
         "d2h": B * n_out,
         # per batch of B ticks: rows: prologue, 8-lane pass, lit-sum pass, fix-up per tick (one of the two
-        # passes returns at once); push on the last tick; batch control, burst reset, list reset, layout
-        # start, owner counts, row layout (the three layout kernels return at once on batches that keep
-        # the copy), write-back
-        "launches": K * ((4 * B + 8) if engine == 1 else (4 * B + 2)),
+        # passes returns at once), push on the last tick (all of these one launch for a small brain); batch
+        # control, burst reset, list reset, layout start, owner counts, row layout (the three layout kernels
+        # return at once on batches that keep the copy), the two write-backs (one returns at once)
+        "launches": K * ((8 + (1 if small else 4 * B + 1)) if engine == 1 else (4 * B + 2)),
         "roofline": {"bound": "hbm", "kernel": kernels.get(names[top], names[top]),
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": TRAFFIC.get((args.workload, kernels.get(names[top], names[top]))),
