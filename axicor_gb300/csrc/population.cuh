@@ -319,9 +319,10 @@ __global__ void __launch_bounds__(256, 3) k_pop_update(const PopBrain* __restric
   const uint32_t nch = pctl->nchunks[k & 1];
   const uint32_t lane = threadIdx.x & 31, gl = lane % LANES, grp = lane / LANES, warp = threadIdx.x >> 5;
   uint32_t ev_slots = 0, hits = 0, nspk = 0, gdone = 0, nev = 0, err = 0;
-  // a run of the chunk list per block: few blocks stage a second brain
-  const uint32_t c1 = (uint32_t)((unsigned long long)nch * (blockIdx.x + 1u) / gridDim.x);
-  for (uint32_t ci = (uint32_t)((unsigned long long)nch * blockIdx.x / gridDim.x); ci < c1; ci++) {
+  // The blocks take the chunks in turn, so that the GPU works on few brains at a time:
+  // a run of the list per block stages fewer brains, but 512 brains' masks and rows
+  // then pass through L2 at once (1.44 ms a tick against 1.19).
+  for (uint32_t ci = blockIdx.x; ci < nch; ci += gridDim.x) {
     const uint2 cd = chunks[ci];
     stage_brain(st, brains, cd.x, s_lit, lit_cap);
     const PopBrain& b = st.b;
