@@ -125,6 +125,7 @@ cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* ou
   e = ensure_counts(*s, b.ticks, &realloc, stream);
   if (e != cudaSuccess) return e;
   const uint32_t rows = g_batch_mode.load() == 1 ? 1u : 0u;
+  if (!rows) rows_touched(*s);   // the columnar kernels move the blob's weights
   if (rows) {
     const void* before = s->rows ? s->rows->base : nullptr;
     e = rows_alloc(*s, b.padded_n, b.total_axons, true, stream);

@@ -295,6 +295,8 @@ int32_t cu_step_day_phase(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t
       s->tick_since_build = 0;
     }
     s->tick_since_build++;
+  } else {
+    rows_touched(*s);   // the columnar kernels move the blob's weights
   }
   TickArgs a{};
   a.padded_n = padded_n;
