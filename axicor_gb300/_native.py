@@ -201,6 +201,7 @@ SIGNATURES: dict[str, tuple] = {
     "axc_shard_invalidate": (I32, [PV]),
     "axc_row_engine_fix_capacity": (U32, [U32]),
     "axc_row_engine_wait_limit": (U32, [U32]),
+    "axc_row_engine_barrier_limit": (U32, [U32]),
     "axc_extract_outgoing_spikes_noalloc": (I32, [P, P, P, U32, U32, U32, P, P, P]),
     "axc_population_create": (I32, [P, U32, C.POINTER(P)]),
     "axc_step_zone_batch": (I32, [C.POINTER(AxcZoneShard), U32, C.POINTER(AxcGhostRoute), U32, U32, U32, P]),

@@ -108,6 +108,8 @@ extern "C" uint32_t axc_row_engine_fix_capacity(uint32_t cap) {
 
 extern "C" uint32_t axc_row_engine_wait_limit(uint32_t tries) { return set_first_wait_limit(tries); }
 
+extern "C" uint32_t axc_row_engine_barrier_limit(uint32_t tries) { return set_barrier_limit(tries); }
+
 namespace axc {
 
 // Prepares one shard for a batch (shard.rs:40-71): scratch and row cache, then

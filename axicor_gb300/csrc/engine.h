@@ -55,7 +55,7 @@ struct ShardCtl {
   uint32_t lay_lit;       // row engine: fully-lit axons when the layout was made
   uint32_t dec_ticks;     // row engine: ticks of the last decision
   uint32_t lay_forced;    // row engine: the layout was forced
-  uint32_t pad5;
+  uint32_t gave_up;       // row engine: a barrier of k_rows_small's resident grid ran out of tries
   unsigned long long mov_total;   // row engine: movable slots of the rows (batch start)
   unsigned long long lit_seen;    // row engine: ctr[6] at the last decision
   unsigned long long lay_work;    // row engine: tested and movable slots of the layout before the current one
@@ -264,6 +264,8 @@ cudaError_t rows_wish_alloc(ShardScratch& s);
 
 // Tries of the update pass's first wait for its staged bitmap; returns the previous value.
 uint32_t set_first_wait_limit(uint32_t tries);
+// Tries of the barriers of k_rows_small's resident grid; returns the previous value.
+uint32_t set_barrier_limit(uint32_t tries);
 
 // Registry keyed by the axon_heads pointer.  Created by cu_allocate_shard;
 // created lazily (and sized) for shards whose memory the caller allocated.

@@ -827,8 +827,11 @@ __global__ void __launch_bounds__(256) k_rows_writeback(int16_t* __restrict__ we
                                                         const int16_t* __restrict__ rw,
                                                         const uint4* __restrict__ omask,
                                                         const uint4* __restrict__ lmask,
-                                                        const ShardCtl* __restrict__ ctl) {
+                                                        const ShardCtl* __restrict__ ctl, uint32_t* __restrict__ pend,
+                                                        uint32_t* __restrict__ incoming, uint32_t A) {
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ctl->gave_up)   // pushes of ticks that never ended
+    for (uint32_t a = n; a < A; a += gridDim.x * blockDim.x) pend[a] = incoming[a] = 0u;
   const uint4 om = n < N ? omask[n] : make_uint4(0, 0, 0, 0);   // asked for beside the control block
   if (writeback_tiled(ctl, N) || !(om.x | om.y | om.z | om.w)) return;
   const uint4 lm = lmask[n];
@@ -853,9 +856,10 @@ __global__ void __launch_bounds__(256) k_rows_writeback_tiles(int16_t* __restric
                                                               const int16_t* __restrict__ rw,
                                                               const uint4* __restrict__ omask,
                                                               const uint4* __restrict__ lmask,
-                                                              const ShardCtl* __restrict__ ctl) {
+                                                              ShardCtl* __restrict__ ctl) {
   __shared__ int16_t s_w[AXC_MAX_DENDRITES][34];
   __shared__ uint32_t s_m[32][4];
+  if (blockIdx.x == 0 && threadIdx.x == 0 && ctl->gave_up) ctl->gave_up = 0u;   // cleared by the kernel before
   if (!writeback_tiled(ctl, N)) return;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (uint32_t t0 = blockIdx.x * 32u; t0 < N; t0 += gridDim.x * 32u) {
@@ -2973,13 +2977,17 @@ struct SmallArgs {
   ColWT wt;
 };
 
-constexpr uint32_t kGridWaitLimit = 1u << 22;   // tries: about 3 s
+// Tries of a barrier of the resident grid: about 3 s (axc_row_engine_barrier_limit;
+// tests set 0 to take the give-up path).
+constexpr uint32_t kGridWaitLimit = 1u << 22;
+__device__ uint32_t g_barrier_limit = kGridWaitLimit;
 
 // All threads of the grid.  CLUSTER: the cluster's hardware barrier.  Else a counter
-// that every block adds to (zeroed before each launch), with a bounded wait: false
-// once a block gave up, on which the grid's blocks all return.
+// that every block adds to (zeroed before each launch), with a bounded wait (tries):
+// false once a block gave up, on which the grid's blocks all return.  The pushes that
+// are then left in pend and incoming are dropped by the write-back behind (gave_up).
 template <bool CLUSTER>
-__device__ __forceinline__ bool small_barrier(ShardCtl* ctl, uint32_t& target, uint32_t* s_ok) {
+__device__ __forceinline__ bool small_barrier(ShardCtl* ctl, uint32_t& target, uint32_t tries, uint32_t* s_ok) {
   if (CLUSTER) {
     asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
     return true;
@@ -2989,12 +2997,15 @@ __device__ __forceinline__ bool small_barrier(ShardCtl* ctl, uint32_t& target, u
     target += gridDim.x;
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->barrier) : "memory");
     bool ok = false;
-    for (uint32_t it = 0; it < kGridWaitLimit && !ok; it++) {
+    for (uint32_t it = 0; it < tries && !ok; it++) {
       uint32_t seen;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&ctl->barrier) : "memory");
       ok = (int32_t)(seen - target) >= 0;
     }
-    if (!ok) atomicOr(&ctl->err, AXC_ERR_WAIT_LIMIT);
+    if (!ok) {
+      atomicOr(&ctl->err, AXC_ERR_WAIT_LIMIT);
+      ctl->gave_up = 1u;
+    }
     *s_ok = ok;
   }
   __syncthreads();
@@ -3035,13 +3046,14 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
   const bool packed = build_ptab(ptab, gtab);
   // axons and list entries go to the blocks warp by warp: few of them use every SM
   const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const uint32_t tries = CLUSTER ? 0u : g_barrier_limit;
   uint32_t target = 0, parity = 0;
   bool staging = true;
   const uint32_t smax = ctl->row_smax, seg_max = ctl->seg_max;
   const uint32_t tick0 = (b.set_tick ? b.tick_base : ctl->tick_base) + b.k0;
   if (small_spikes(b, 0)) {
     small_incoming(b, 0);
-    if (!small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+    if (!small_barrier<CLUSTER>(ctl, target, tries, &s_ok)) return;
   }
   for (uint32_t t = 0; t < b.ticks; t++) {
     const uint32_t k = b.k0 + t;
@@ -3052,7 +3064,7 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
                                   b.lit, t ? b.pend : nullptr, small_spikes(b, t) != 0u, b.set_tick, b.tick_base,
                                   b.dopamine, b.xlit, nullptr, nullptr, b.alit, t == b.lit_tick ? 1u : 0u, s_list,
                                   s_place);
-    if (!small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+    if (!small_barrier<CLUSTER>(ctl, target, tries, &s_ok)) return;
     const TickForm form = tick_form(ctl, k, nullptr, 0u);
     const uint32_t ecount = s_place[0];
     if (threadIdx.x < ecount) b.eval[s_place[1] + threadIdx.x] = s_list[threadIdx.x];
@@ -3096,7 +3108,7 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
       if (!lit_on) staging = __syncthreads_and(mbar_wait_bounded(&s_bar, parity));
       parity ^= 1u;
     }
-    if (!small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+    if (!small_barrier<CLUSTER>(ctl, target, tries, &s_ok)) return;
     const uint32_t nfix = ctl->fix_count | ctl->fix_overflow;
     rows_fixup(b.P, b.N, b.A, b.rt, b.rw, b.cnt, b.mask2, b.pend, b.eval, b.fix, ctl, k, b.ids,
                b.out + (size_t)t * b.outputs, b.outputs, b.wt, nullptr);
@@ -3104,7 +3116,7 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
     if (spikes) small_incoming(b, t + 1);
     // What comes next writes what the fix-up reads (heads, pending pushes) and reads
     // the network spikes' counts, but leaves the readout's flags: no barrier without them.
-    if ((nfix || spikes) && !small_barrier<CLUSTER>(ctl, target, &s_ok)) return;
+    if ((nfix || spikes) && !small_barrier<CLUSTER>(ctl, target, tries, &s_ok)) return;
   }
   // the last tick's soma pushes
   rows_push(b.P.axon_heads, b.P.soma_to_axon, b.A, b.pend, b.eval, b.P.soma_flags, b.N, nullptr, nullptr, 0u, ctl,
@@ -3117,6 +3129,13 @@ uint32_t set_first_wait_limit(uint32_t tries) {
   static uint32_t current = kWaitLimit;
   const uint32_t prev = current;
   if (cudaMemcpyToSymbol(g_first_wait_limit, &tries, sizeof(tries)) == cudaSuccess) current = tries;
+  return prev;
+}
+
+uint32_t set_barrier_limit(uint32_t tries) {
+  static uint32_t current = kGridWaitLimit;
+  const uint32_t prev = current;
+  if (cudaMemcpyToSymbol(g_barrier_limit, &tries, sizeof(tries)) == cudaSuccess) current = tries;
   return prev;
 }
 
@@ -3703,12 +3722,11 @@ cudaError_t rows_index_wish(const ShardVramPtrs& v, ShardScratch& s, uint32_t N,
 
 cudaError_t launch_rows_end(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, cudaStream_t stream) {
   RowCache& r = *s.rows;
-  if (N) {
-    const uint32_t blocks = (N + 255) / 256;
-    k_rows_writeback<<<blocks, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.omask, r.lmask, s.ctl);
-    k_rows_writeback_tiles<<<std::min((N + 31) / 32, 4u * (uint32_t)sm_count()), 256, 0, stream>>>(
-        v.dendrite_weights, N, r.rw, r.omask, r.lmask, s.ctl);
-  }
+  const uint32_t blocks = std::max(1u, (N + 255) / 256), tiles = std::max(1u, (N + 31) / 32);
+  k_rows_writeback<<<blocks, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.omask, r.lmask, s.ctl, s.pend, s.incoming,
+                                               s.total_axons);
+  k_rows_writeback_tiles<<<std::min(tiles, 4u * (uint32_t)sm_count()), 256, 0, stream>>>(v.dendrite_weights, N, r.rw,
+                                                                                         r.omask, r.lmask, s.ctl);
   return cudaGetLastError();
 }
 

@@ -394,6 +394,12 @@ uint32_t axc_row_engine_fix_capacity(uint32_t cap);
  * limit, so that no copy is left in flight.  0 makes every first wait give up
  * at once: for tests of that path.  Returns the previous value. */
 uint32_t axc_row_engine_wait_limit(uint32_t tries);
+/* Tries of each barrier of the one launch that runs all ticks of a small
+ * brain's batch (default 2^22, about 3 s); returns the previous value.  A
+ * batch whose barrier gives up raises AXC_ERR_WAIT_LIMIT and ends without its
+ * remaining ticks: the shard's state and heads are then those of no tick and
+ * have to be uploaded again; its pending pushes are dropped.  Tests set 0. */
+uint32_t axc_row_engine_barrier_limit(uint32_t tries);
 
 /* Per-tick counters accumulated by the device since the last reset:
  *  [0] ticks, [1] evaluated slots (non-refractory neurons, up to first empty),
