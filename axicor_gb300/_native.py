@@ -194,6 +194,7 @@ SIGNATURES: dict[str, tuple] = {
     "axc_step_day_phase_batch": (I32, [PV, U32, U32, U32, C.POINTER(AxcIoBuffers), P, P, P, U32, U32, P, U32,
                                        I16, U32, P, P]),
     "axc_shard_counters": (I32, [PV, U32, C.POINTER(C.c_uint64)]),
+    "axc_shard_forms": (I32, [PV, U32, C.POINTER(C.c_uint64)]),
     "axc_profile_ticks": (I32, [PV, U32, U32, U32, U32, U32, P, U32, U32, U32, I16, I32, P, C.POINTER(C.c_float),
                                 C.POINTER(C.c_uint64)]),
     "axc_batch_engine_mode": (I32, [I32]),

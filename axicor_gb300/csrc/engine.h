@@ -69,6 +69,7 @@ struct ShardCtl {
   const uint32_t* ix_off; // inverted index of the rows (RowIndex)
   const uint16_t* ix_seg;
   const uint32_t* ix_ent;
+  unsigned long long forms[8];   // row engine: ticks per form, one-launch ticks, layouts (axc_shard_forms)
 };
 
 // Inverted index of the row copy: per axon the row slots that target it

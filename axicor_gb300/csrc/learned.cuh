@@ -410,6 +410,7 @@ __global__ void __launch_bounds__(256) k_learn_update(ShardVramPtrs P, LearnDev 
                                                       uint32_t k) {
   LearnCtl& c = *L.ctl;
   if (c.mode != 1u || c.overflow || index_ok(ctl)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) count_form(ctl, kFormScatter);
   __shared__ VariantParameters lut[16];
   lut_to_smem(lut);
   __syncthreads();

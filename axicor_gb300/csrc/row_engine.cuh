@@ -376,6 +376,7 @@ struct LearnDev {
 // lc: the learned engine's control block (its planned sparse ticks), or null;
 // index: the tick may run sparse by the exact counts (the learned engine's
 // graphs, whose memory holds the inverted index).
+// The kernels that run a tick count it by its form (ShardCtl::forms).
 enum TickForm {
   kFormDense = 0,     // k_rows_update: every slot tested
   kFormLitSum = 1,    // k_rows_update_lsum: a thread per neuron
@@ -384,6 +385,10 @@ enum TickForm {
   kFormLitRows = 4,   // k_rows_update: lit_row_step
   kFormVerify = 5     // the same, with dark axons: each lit slot is looked up
 };
+constexpr int kCountSmall = 6, kCountLayout = 7;   // forms[]: ticks inside k_rows_small; layouts of the rows
+
+// One thread of a tick's kernel.
+__device__ __forceinline__ void count_form(ShardCtl* ctl, int form) { atomicAdd(&ctl->forms[form], 1ull); }
 
 // The control words are read at once (volatile, so that no load waits behind the
 // branch on another) through L1, as lsum_tick's comment says.
@@ -797,6 +802,7 @@ __global__ void __launch_bounds__(256) k_rows_mult(const uint32_t* __restrict__ 
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n == 0) {
     mask2[A] = make_uint2(0u, 0x80000000u);   // dummy entry of invalid targets: no hit, exact path
+    count_form(ctl, kCountLayout);
     ctl->row_smax = 0;
     ctl->seg_max = 0;
     ctl->row_sum = 0;
@@ -1932,6 +1938,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   const TickForm form = tick_form(ctl, k, lc, index);
   // else k_rows_update_lsum or the learned engine's kernels run this tick
   if (form != kFormDense && form != kFormLitRows && form != kFormVerify) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) count_form(ctl, form);
   if (LIT && threadIdx.x == 0) mbar_init(&s_bar, 1);
   lut_to_smem(lut);
   __syncthreads();
@@ -2140,6 +2147,7 @@ __global__ void __launch_bounds__(256, kNeuronBlocks)
   if (tick_form(ctl, k, lc, 1u) != kFormSparse) return;
   const uint32_t tiles = (N + 127u) / 128u;
   if (blockIdx.x * 8u >= tiles) return;   // no neuron for this block: no table to build
+  if (blockIdx.x == 0 && threadIdx.x == 0) count_form(ctl, kFormSparse);
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   lut_to_smem(lut);
@@ -2290,7 +2298,10 @@ __global__ void __launch_bounds__(256, kLsumBlocks)
   const PassCtl pc = pass_ctl(ctl, k);
   const uint32_t ecount = ctl_ld32(&ctl->eval_act[k & 1][0]);
   if (tick_form(ctl, k, lc, 0u) != kFormLitSum) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ctr[6] += 1;   // ticks on the lit-sum form
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->ctr[6] += 1;   // ticks on the lit-sum form
+    count_form(ctl, kFormLitSum);
+  }
   // neurons per block and pass: fewer than its threads where that spreads a short list over all blocks
   const uint32_t span = min(256u, ((ecount + gridDim.x - 1) / gridDim.x + unit - 1u) / unit * unit);
   if (blockIdx.x * span >= ecount) return;   // no neuron for this block: no table to build
@@ -3073,6 +3084,10 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
     // The lit-sum form's ticks take the 8-lane pass over the same rows: with a thread
     // per neuron each neuron's slots are a serial chain, and there are few neurons.
     const bool lit_rows = form == kFormLitSum || form == kFormLitRows;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      count_form(ctl, lit_rows ? kFormLitRows : form);
+      count_form(ctl, kCountSmall);
+    }
     // Else the fully-lit bitmap: other blocks' plain stores, then a bulk copy, over
     // what this block's threads read in an earlier tick.
     const bool stage = staging && !lit_rows;

@@ -468,6 +468,18 @@ int32_t axc_shard_counters(const ShardVramPtrs* vram, uint32_t reset, uint64_t o
   return (int32_t)e;
 }
 
+int32_t axc_shard_forms(const ShardVramPtrs* vram, uint32_t reset, uint64_t out[8]) {
+  if (!vram || !out) return (int32_t)cudaErrorInvalidValue;
+  ShardScratch* s = scratch_lookup(vram);
+  if (!s) { for (int i = 0; i < 8; i++) out[i] = 0; return 0; }
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) return (int32_t)e;
+  e = cudaMemcpy(out, s->ctl->forms, 8 * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && reset) e = cudaMemset(s->ctl->forms, 0, 8 * sizeof(uint64_t));
+  if (e == cudaSuccess && reset) e = cudaDeviceSynchronize();
+  return (int32_t)e;
+}
+
 int32_t axc_last_spikes(const ShardVramPtrs* vram, uint32_t* out_count, uint32_t* out_ids, uint32_t capacity,
                         void* stream) {
   if (!vram || !out_count) return (int32_t)cudaErrorInvalidValue;

@@ -133,6 +133,13 @@ class VramState:
                                            out.ctypes.data_as(C.POINTER(C.c_uint64))), "axc_shard_counters")
         return out
 
+    def forms(self, reset: bool = False) -> np.ndarray:
+        """Ticks per form of the row engine, one-launch ticks and layouts (axc_shard_forms)."""
+        out = np.zeros(8, dtype=np.uint64)
+        N.check(N.lib().axc_shard_forms(C.byref(self.ptrs), 1 if reset else 0,
+                                        out.ctypes.data_as(C.POINTER(C.c_uint64))), "axc_shard_forms")
+        return out
+
     def last_spikes(self, stream: int | None = None) -> np.ndarray:
         cnt = C.c_uint32(0)
         ids = np.empty(self.padded_n, dtype=np.uint32)

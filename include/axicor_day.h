@@ -410,6 +410,15 @@ uint32_t axc_row_engine_barrier_limit(uint32_t tries);
  *  one by one. */
 int32_t axc_shard_counters(const ShardVramPtrs* vram, uint32_t reset, uint64_t out[8]);
 
+/* Ticks the row engine ran in each of its forms since the last reset (the
+ * results are the same in all; tests ask which ran): [0] dense, every slot
+ * tested, [1] lit-sum, [2] sparse from the inverted index, [3] the learned
+ * engine's scatter, [4] lit rows (in one launch, lit-sum ticks too), [5] lit
+ * rows checked slot by slot; [6] those of them that ran inside one launch of
+ * all a batch's ticks or of a whole call; [7] layouts of the row copy.  The
+ * columnar kernels count none. */
+int32_t axc_shard_forms(const ShardVramPtrs* vram, uint32_t reset, uint64_t out[8]);
+
 /* Allocation-free outgoing-spike extraction.  No counterpart in the
  * reference: it is launch_extract_outgoing_spikes (same arguments, same
  * events in the same order) for callers that may not allocate device memory
