@@ -170,12 +170,12 @@ cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* ou
 // captured: the row copy, `ticks` ticks with global tick = tick_base + k read
 // from the control block, the weight write-back.
 cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, uint32_t fix_cap, cudaStream_t cap,
-                          bool whole_gpu) {
+                          bool whole_gpu, bool one_launch) {
   const AxcIoBuffers* io = b.io;
   const uint32_t words = io->input_words_per_tick;
   cudaError_t le = cudaSuccess;
   if (rows) le = launch_rows_begin(*b.vram, s, b.padded_n, b.total_axons, cap, false, true, true, true);
-  const bool small = rows && rows_small(b.padded_n, b.total_axons, whole_gpu, true);
+  const bool small = rows && one_launch && rows_small(b.padded_n, b.total_axons, whole_gpu, true);
   for (uint32_t k = 0; k < b.ticks && le == cudaSuccess; k++) {
     TickArgs a{};
     a.padded_n = b.padded_n;
@@ -247,14 +247,18 @@ extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t 
         e = cudaStreamCreateWithFlags(&gc->capture, cudaStreamNonBlocking);
         if (e != cudaSuccess) return (int32_t)e;
       }
-      e = cudaStreamBeginCapture(gc->capture, cudaStreamCaptureModeThreadLocal);
-      if (e != cudaSuccess) return (int32_t)e;
-      const cudaError_t le = batch_capture(b, *s, rows, key.fix_cap, gc->capture, true);
-      cudaGraph_t graph = nullptr;
-      e = cudaStreamEndCapture(gc->capture, &graph);
-      if (le != cudaSuccess) e = le;
-      if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-      if (graph) cudaGraphDestroy(graph);
+      for (const bool one_launch : {true, false}) {
+        e = cudaStreamBeginCapture(gc->capture, cudaStreamCaptureModeThreadLocal);
+        if (e != cudaSuccess) return (int32_t)e;
+        const cudaError_t le = batch_capture(b, *s, rows, key.fix_cap, gc->capture, true, one_launch);
+        cudaGraph_t graph = nullptr;
+        e = cudaStreamEndCapture(gc->capture, &graph);
+        if (le != cudaSuccess) e = le;
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+        if (!launch_refused(e)) break;
+        cudaGetLastError();   // not the second capture's
+      }
       if (e != cudaSuccess) return (int32_t)e;
       gc->execs[key] = exec;
     }

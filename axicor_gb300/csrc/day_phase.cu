@@ -527,15 +527,20 @@ __global__ void __launch_bounds__(kListBlock) k_list_write(const uint8_t* __rest
 
 namespace axc {
 
+int current_device() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return dev;
+}
+
 int sm_count() {
-  static int cached = 0;
-  if (!cached) {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
+  static PerDevice<int> count;
+  const int dev = current_device();
+  return count.get(dev, [dev] {
+    int v = 0;
     cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    cached = v > 0 ? v : 1;
-  }
-  return cached;
+    return v > 0 ? v : 1;
+  });
 }
 
 static std::atomic<uint64_t> g_lut_gen{1};

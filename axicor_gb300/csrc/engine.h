@@ -10,6 +10,7 @@
 #include <utility>
 
 #include "../../include/axicor_day.h"
+#include "per_device.h"
 
 namespace axc {
 
@@ -320,6 +321,12 @@ cudaError_t launch_tick(const ShardVramPtrs& v, ShardScratch& s, const TickArgs&
 // Small brains: `ticks` ticks from a (its arrays those of the first; words of the
 // input per tick) in one launch, where rows_small says so.
 bool rows_small(uint32_t N, uint32_t A, bool whole_gpu, bool batch);
+// Its cluster or resident grid does not fit after all (a context that may not use
+// every SM): the kernel chain runs the ticks.
+inline bool launch_refused(cudaError_t e) {
+  return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorInvalidClusterSize ||
+         e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidConfiguration || e == cudaErrorNotSupported;
+}
 cudaError_t launch_rows_small(const ShardVramPtrs& v, ShardScratch& s, const TickArgs& a, uint32_t ticks,
                               uint32_t words, cudaStream_t stream);
 cudaError_t launch_reset_burst(const ShardVramPtrs& v, uint32_t padded_n, cudaStream_t stream);
@@ -338,8 +345,10 @@ struct BatchArgs {
 };
 cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* out_rows, cudaStream_t stream);
 // whole_gpu: the batch may hold every SM (no other shard's branch runs beside it).
+// one_launch: a small brain's ticks may run in one launch; a capture that is refused
+// with it (launch_refused) is made again without.
 cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, uint32_t fix_cap, cudaStream_t cap,
-                          bool whole_gpu);
+                          bool whole_gpu, bool one_launch);
 // dst[dst_indices[i]] = src[src_indices[i]] for src_indices[i] < 2^31 (side_kernels.cu, bindings.cu:341-368).
 cudaError_t ghost_sync(const BurstHeads8* src_heads, BurstHeads8* dst_heads, const uint32_t* src_indices,
                        const uint32_t* dst_indices, uint32_t count, cudaStream_t stream);
@@ -360,6 +369,7 @@ cudaError_t launch_gsop_stage(const ShardVramPtrs& v, ShardScratch& s, uint32_t 
 cudaError_t lut_upload(const VariantParameters* lut, cudaStream_t stream, bool async);
 uint64_t lut_generation();
 
-int sm_count();
+int current_device();
+int sm_count();   // of the current device
 
 }  // namespace axc

@@ -3282,9 +3282,10 @@ cudaError_t launch_rows_begin(const ShardVramPtrs& v, ShardScratch& s, uint32_t 
 // Largest fully-lit bitmap the update kernel stages in shared memory (the
 // 1024-thread variant also uses ~3.4 KB of static shared memory).
 static size_t lit_smem_limit() {
-  static size_t limit = [] {
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
+  static PerDevice<size_t> limit;
+  const int dev = current_device();
+  return limit.get(dev, [dev] {
+    int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     size_t lim = optin > 8192 ? (size_t)optin - 8192 : 0;
     if (cudaFuncSetAttribute(k_rows_update<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) !=
@@ -3295,8 +3296,7 @@ static size_t lit_smem_limit() {
       lim = 0;
     }
     return lim;
-  }();
-  return limit;
+  });
 }
 
 // The update pass (with the fully-lit bitmap in shared memory when it fits).
@@ -3443,7 +3443,8 @@ constexpr uint32_t kSmallBlocks = 640;   // a resident grid: neurons or axons pe
 
 // Blocks of k_rows_small's cluster here, 0 where none fits.
 static uint32_t small_cluster() {
-  static uint32_t size = [] {
+  static PerDevice<uint32_t> size;
+  return size.get(current_device(), [] {
     for (const uint32_t c : {16u, 8u}) {
       int n = 0, m = 0;
       auto fits = [&](auto kern, int* out) {
@@ -3465,13 +3466,13 @@ static uint32_t small_cluster() {
       cudaGetLastError();
     }
     return 0u;
-  }();
-  return size;
+  });
 }
 
 // Blocks of k_rows_small's resident grid here, 0 where it does not fit.
 static uint32_t small_grid() {
-  static uint32_t size = [] {
+  static PerDevice<uint32_t> size;
+  return size.get(current_device(), [] {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_rows_small<false, false>, 1024,
                                                       lit_smem_bytes(kSmallBlocks * sm_count())) != cudaSuccess) {
@@ -3479,8 +3480,7 @@ static uint32_t small_grid() {
       n = 0;
     }
     return n > 0 ? (uint32_t)sm_count() : 0u;
-  }();
-  return size;
+  });
 }
 
 bool rows_small(uint32_t N, uint32_t A, bool whole_gpu, bool batch) {

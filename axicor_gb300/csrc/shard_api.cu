@@ -322,7 +322,11 @@ int32_t cu_step_day_phase(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t
     a.lit_new = s->tick_since_build == 1 || s->tick_since_build == kTickRelayout - kLitWindow + 1;
     a.fix_cap = s->rows->fix ? fix_capacity() : 0u;   // no list (population rows): the fix-up rescans
     s->tick_parity ^= 1u;
-    if (rows_small(padded_n, total_axons, false, false)) return (int32_t)launch_rows_small(*vram, *s, a, 1u, 0u, st);
+    if (rows_small(padded_n, total_axons, false, false)) {
+      err = launch_rows_small(*vram, *s, a, 1u, 0u, st);
+      if (!launch_refused(err)) return (int32_t)err;
+      cudaGetLastError();   // nothing ran: the chain takes the tick
+    }
   }
   return (int32_t)launch_tick(*vram, *s, a, st);
 }

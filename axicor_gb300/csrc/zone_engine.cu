@@ -133,27 +133,32 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
     }
     e = ensure_streams(c, nshards);
     if (e != cudaSuccess) return (int32_t)e;
-    e = cudaStreamBeginCapture(c.root, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return (int32_t)e;
-    cudaError_t le = cudaEventRecord(c.events[0], c.root);
-    // fork: every shard's tick loop on its own branch
-    for (uint32_t i = 0; i < nshards && le == cudaSuccess; i++) {
-      le = cudaStreamWaitEvent(c.branch[i], c.events[0], 0);
-      if (le == cudaSuccess) le = batch_capture(args[i], *scr[i], rows[i], fix_cap, c.branch[i], nshards == 1);
-      if (le == cudaSuccess) le = cudaEventRecord(c.events[1 + i], c.branch[i]);
-      if (le == cudaSuccess) le = cudaStreamWaitEvent(c.root, c.events[1 + i], 0);
+    for (const bool one_launch : {true, false}) {
+      e = cudaStreamBeginCapture(c.root, cudaStreamCaptureModeThreadLocal);
+      if (e != cudaSuccess) return (int32_t)e;
+      cudaError_t le = cudaEventRecord(c.events[0], c.root);
+      // fork: every shard's tick loop on its own branch
+      for (uint32_t i = 0; i < nshards && le == cudaSuccess; i++) {
+        le = cudaStreamWaitEvent(c.branch[i], c.events[0], 0);
+        if (le == cudaSuccess)
+          le = batch_capture(args[i], *scr[i], rows[i], fix_cap, c.branch[i], nshards == 1, one_launch);
+        if (le == cudaSuccess) le = cudaEventRecord(c.events[1 + i], c.branch[i]);
+        if (le == cudaSuccess) le = cudaStreamWaitEvent(c.root, c.events[1 + i], 0);
+      }
+      // join, then the ghost sync of every route (mod.rs:409-411)
+      for (uint32_t r = 0; r < nroutes && le == cudaSuccess; r++) {
+        const AxcGhostRoute& g = routes[r];
+        le = ghost_sync(shards[g.src_shard].vram.axon_heads, shards[g.dst_shard].vram.axon_heads, g.d_src_indices,
+                        g.d_dst_indices, g.count, c.root);
+      }
+      cudaGraph_t graph = nullptr;
+      e = cudaStreamEndCapture(c.root, &graph);
+      if (le != cudaSuccess) e = le;
+      if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+      if (graph) cudaGraphDestroy(graph);
+      if (!launch_refused(e)) break;
+      cudaGetLastError();   // not the second capture's
     }
-    // join, then the ghost sync of every route (mod.rs:409-411)
-    for (uint32_t r = 0; r < nroutes && le == cudaSuccess; r++) {
-      const AxcGhostRoute& g = routes[r];
-      le = ghost_sync(shards[g.src_shard].vram.axon_heads, shards[g.dst_shard].vram.axon_heads, g.d_src_indices,
-                      g.d_dst_indices, g.count, c.root);
-    }
-    cudaGraph_t graph = nullptr;
-    e = cudaStreamEndCapture(c.root, &graph);
-    if (le != cudaSuccess) e = le;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-    if (graph) cudaGraphDestroy(graph);
     if (e != cudaSuccess) return (int32_t)e;
     c.execs[key] = exec;
   }
