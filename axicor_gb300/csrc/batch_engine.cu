@@ -18,6 +18,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <vector>
 
 #include "engine.h"
 
@@ -26,13 +27,13 @@ namespace axc {
 namespace {
 
 struct GraphKey {
-  uint32_t N, A, batch, voff, nv, v_seg, max_spikes, words, num_outputs, rows, fix_cap;
+  uint32_t N, A, batch, voff, nv, v_seg, max_spikes, words, num_outputs, rows, fix_cap, whole;
   const void *bitmask, *incoming, *out, *ids;
   bool operator<(const GraphKey& o) const {
-    return std::tie(N, A, batch, voff, nv, v_seg, max_spikes, words, num_outputs, rows, fix_cap, bitmask, incoming,
-                    out, ids) <
+    return std::tie(N, A, batch, voff, nv, v_seg, max_spikes, words, num_outputs, rows, fix_cap, whole, bitmask,
+                    incoming, out, ids) <
            std::tie(o.N, o.A, o.batch, o.voff, o.nv, o.v_seg, o.max_spikes, o.words, o.num_outputs, o.rows, o.fix_cap,
-                    o.bitmask, o.incoming, o.out, o.ids);
+                    o.whole, o.bitmask, o.incoming, o.out, o.ids);
   }
 };
 
@@ -92,6 +93,84 @@ void graph_cache_drop(ShardScratch* s) {
 }
 
 uint32_t fix_capacity() { return g_fix_cap.load(); }
+
+namespace {
+std::mutex g_work_mu;
+std::vector<ShardScratch*>& work_list() {
+  static auto* l = new std::vector<ShardScratch*>();
+  return *l;
+}
+std::atomic<uint64_t> g_ticks{0};   // per-tick calls of all shards
+
+// Event calls beside another thread's global-mode capture would end it.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+}  // namespace
+
+void work_started(ShardScratch& s, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
+  const RelaxedCapture relaxed;
+  std::lock_guard<std::mutex> lk(g_work_mu);
+  if (!s.work_done && cudaEventCreateWithFlags(&s.work_done, cudaEventDisableTiming) != cudaSuccess) {
+    s.work_done = nullptr;
+    return;
+  }
+  if (cudaEventRecord(s.work_done, st) != cudaSuccess) return;
+  s.work_stream = st;
+  if (!s.work_listed) work_list().push_back(&s);
+  s.work_listed = true;
+}
+
+void tick_started(ShardScratch& s) {
+  s.own_ticks++;
+  g_ticks.fetch_add(1, std::memory_order_relaxed);
+}
+
+void work_created(ShardScratch& s) { s.other_ticks = g_ticks.load(std::memory_order_relaxed); }
+
+bool others_running(ShardScratch& s, cudaStream_t st) {
+  const uint64_t ticks = g_ticks.load(std::memory_order_relaxed) - s.own_ticks;
+  bool running = ticks != s.other_ticks;
+  s.other_ticks = ticks;
+  if (cudaPeekAtLastError() != cudaSuccess) return running;   // an earlier call's error stays pending
+  const RelaxedCapture relaxed;
+  std::lock_guard<std::mutex> lk(g_work_mu);
+  auto& l = work_list();
+  for (size_t i = 0; i < l.size();) {
+    ShardScratch& o = *l[i];
+    if (&o == &s || o.work_stream == st) {   // in order with this batch
+      i++;
+      continue;
+    }
+    if (cudaEventQuery(o.work_done) == cudaErrorNotReady) {
+      running = true;
+      i++;
+      continue;
+    }
+    o.work_listed = false;
+    l[i] = l.back();
+    l.pop_back();
+  }
+  cudaGetLastError();   // cudaErrorNotReady counts as one
+  return running;
+}
+
+void work_forget(ShardScratch& s) {
+  std::lock_guard<std::mutex> lk(g_work_mu);
+  auto& l = work_list();
+  for (size_t i = 0; s.work_listed && i < l.size(); i++)
+    if (l[i] == &s) {
+      l[i] = l.back();
+      l.pop_back();
+      s.work_listed = false;
+    }
+  if (s.work_done) cudaEventDestroy(s.work_done);
+  s.work_done = nullptr;
+}
 
 }  // namespace axc
 
@@ -231,8 +310,10 @@ extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t 
 
   // the tick loop, as one graph (shard.rs:75-120), captured once per shape
   const uint32_t words = io->input_words_per_tick;
+  // a cluster leaves the other SMs free: one shape of those sizes
+  const uint32_t whole = !rows || rows_small(padded_n, total_axons, false, true) || !others_running(*s, stream);
   GraphKey key{padded_n, total_axons, sync_batch_ticks, virtual_offset, num_virtual_axons, v_seg,
-               io->max_spikes_per_tick, words, io->num_outputs, rows, g_fix_cap.load(), io->d_input_bitmask,
+               io->max_spikes_per_tick, words, io->num_outputs, rows, g_fix_cap.load(), whole, io->d_input_bitmask,
                io->d_incoming_spikes, io->d_output_history, mapped_soma_ids_device};
   if (!s->graph_cache) s->graph_cache = new GraphCache();
   GraphCache* gc = static_cast<GraphCache*>(s->graph_cache);
@@ -250,7 +331,7 @@ extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t 
       for (const bool one_launch : {true, false}) {
         e = cudaStreamBeginCapture(gc->capture, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return (int32_t)e;
-        const cudaError_t le = batch_capture(b, *s, rows, key.fix_cap, gc->capture, true, one_launch);
+        const cudaError_t le = batch_capture(b, *s, rows, key.fix_cap, gc->capture, whole != 0u, one_launch);
         cudaGraph_t graph = nullptr;
         e = cudaStreamEndCapture(gc->capture, &graph);
         if (le != cudaSuccess) e = le;
@@ -265,6 +346,7 @@ extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t 
   }
   e = cudaGraphLaunch(exec, stream);
   if (e != cudaSuccess) return (int32_t)e;
+  work_started(*s, stream);
 
   // outputs (shard_thread.rs:208-227)
   if (h_output_history && io->d_output_history && io->num_outputs) {

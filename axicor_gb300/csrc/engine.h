@@ -152,7 +152,26 @@ struct ShardScratch {
   // entry point; the next batch then lays the rows out for sure.
   std::atomic<bool> batch_rows_valid{false};
   uint64_t batch_rows_lut = 0;           // LUT generation of the batch layout
+  // What others_running looks at (batch_engine.cu, under its lock).
+  cudaEvent_t work_done = nullptr;      // behind the shard's last batch or run
+  cudaStream_t work_stream = nullptr;
+  bool work_listed = false;             // not known to be done
+  uint64_t own_ticks = 0;               // per-tick calls of this shard, of all others at its last batch
+  uint64_t other_ticks = 0;
 };
+
+// The shards of a process share the GPU: a batch that takes every SM for all of its
+// ticks (k_rows_small's resident grid) would make the others' wait, kernel by kernel
+// they run beside each other (four shards of 16,384 saturated neurons on streams of
+// their own: 39.0 us a tick of all four in resident grids, 18.4 in chains).
+// Behind a batch's, run's or zone's launches on st, and for each per-tick call:
+void work_started(ShardScratch& s, cudaStream_t st);
+void tick_started(ShardScratch& s);
+// Another shard's batch or run is under way on another stream, or another shard was
+// stepped tick by tick since this one's last batch.
+bool others_running(ShardScratch& s, cudaStream_t st);
+void work_created(ShardScratch& s);   // a new shard: the ticks before it are none of its batches'
+void work_forget(ShardScratch& s);
 
 constexpr uint32_t kLitWindow = 32;   // last ticks before a layout in which an axon must have been fully lit
 constexpr uint32_t kBatchRelayoutMin = 100, kBatchRelayoutMax = 1600;   // ticks between batch layouts

@@ -1543,6 +1543,7 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
       e = cudaMemcpyAsync(L->h_gate[slot].before, snap_src, kGateSnapBytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaGraphLaunch(exec, st);
     if (e != cudaSuccess) break;
+    work_started(*s, st);
     if (gated) {
       e = cudaMemcpyAsync(L->h_gate[slot].after, snap_src, kGateSnapBytes, cudaMemcpyDeviceToHost, st);
       if (e == cudaSuccess) e = cudaEventRecord(L->gate_ev[slot], st);

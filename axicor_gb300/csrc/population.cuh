@@ -801,6 +801,7 @@ int32_t axc_population_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_
   for (uint32_t c = 0; c < ticks / tpg && e == cudaSuccess; c++) {
     k_pop_next_graph<<<(P->count + 255) / 256, 256, 0, st>>>(P->d_brains, P->count, P->d_ctl, tick0 + c * tpg);
     e = cudaGraphLaunch(exec, st);
+    if (e == cudaSuccess && !P->scr.empty()) work_started(*P->scr[0], st);
   }
   if (e == cudaSuccess) e = pop_end(*P, st);
   return (int32_t)e;

@@ -56,6 +56,7 @@ cudaError_t scratch_alloc(ShardScratch* s, uint32_t N, uint32_t A) {
 
 void scratch_free(ShardScratch* s) {
   if (!s) return;
+  work_forget(*s);
   graph_cache_free(s);
   if (s->base) cudaFree(s->base);
   if (s->batch_counts) cudaFree(s->batch_counts);
@@ -103,6 +104,7 @@ ShardScratch* scratch_for(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t
   if (*err != cudaSuccess) { delete s; return nullptr; }
   s->state_base = vram->soma_voltage;
   s->state_bytes = state_blob_bytes(padded_n);
+  work_created(*s);
   m[key] = s;
   return s;
 }
@@ -269,6 +271,7 @@ int32_t cu_step_day_phase(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t
   ShardScratch* s = scratch_for(vram, padded_n, total_axons, &err);
   if (!s) return (int32_t)err;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  tick_started(*s);
   // The row engine keeps its neuron-major copy of the dendrites across calls
   // (rebuilt when another entry point wrote the shard or the LUT changed) and
   // writes GSOP's weight changes through to the columnar blob, so the shard's

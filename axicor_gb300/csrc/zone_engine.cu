@@ -99,7 +99,8 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
   // the graph of this zone shape: every pointer a captured node holds is in the key
   const uint32_t fix_cap = fix_capacity();
   ZoneKey key;
-  key.v = {nshards, nroutes, sync_batch_ticks, fix_cap};
+  const bool whole = nshards == 1 && !others_running(*scr[0], stream);
+  key.v = {nshards, nroutes, sync_batch_ticks, fix_cap, whole};
   for (uint32_t i = 0; i < nshards; i++) {
     const AxcZoneShard& z = shards[i];
     const ShardScratch& s = *scr[i];
@@ -141,7 +142,7 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
       for (uint32_t i = 0; i < nshards && le == cudaSuccess; i++) {
         le = cudaStreamWaitEvent(c.branch[i], c.events[0], 0);
         if (le == cudaSuccess)
-          le = batch_capture(args[i], *scr[i], rows[i], fix_cap, c.branch[i], nshards == 1, one_launch);
+          le = batch_capture(args[i], *scr[i], rows[i], fix_cap, c.branch[i], whole, one_launch);
         if (le == cudaSuccess) le = cudaEventRecord(c.events[1 + i], c.branch[i]);
         if (le == cudaSuccess) le = cudaStreamWaitEvent(c.root, c.events[1 + i], 0);
       }
@@ -164,6 +165,7 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
   }
   e = cudaGraphLaunch(exec, stream);
   if (e != cudaSuccess) return (int32_t)e;
+  work_started(*scr[0], stream);
 
   // outputs (shard_thread.rs:208-227)
   bool wait = false;
