@@ -46,7 +46,7 @@ struct ShardCtl {
   uint32_t pmax;          // row engine: largest signal_propagation_length of the LUT (batch start)
   uint32_t barrier;       // row engine: arrivals at the barriers of k_rows_small's resident grid
   unsigned long long ctr[8];  // statistics, see axc_shard_counters
-  uint32_t dense[2];      // row engine: tick k (slot k & 1) has an axon off the lit set the row layout assumed
+  uint32_t dense[2];      // row engine: axons of tick k (slot k & 1) off the lit set the row layout assumed
   unsigned long long pfx_total;   // row engine: slots of the rows tested on every tick (batch start)
   unsigned long long slot_total;  // row engine: live slots of the rows (batch start)
   uint32_t lay_now;       // row engine: this batch lays the row copy out anew (layout_decide)

@@ -243,9 +243,9 @@ struct ColRun {
 // an eighth of the live slots: otherwise the 8-lane pass is faster) and every
 // axon the row layout took as fully lit is fully lit this tick; with a few of
 // them dark (a network spike on an axon that its soma keeps lit moves its
-// oldest heads on) the rows are checked slot by slot (kFormVerify), short ones by the
-// dense pass (504,000 plastic neurons, 32 slots: 31.7 us a tick against 36.8 checked;
-// from 48 slots on the checked form wins).  Every thread
+// oldest heads on) the rows are checked slot by slot (kFormVerify), with many, or in
+// rows of up to 32 slots, by the dense pass (504,000 plastic neurons, 32 slots: 31.7 us
+// a tick against 36.8 checked; tick_form has the other sizes).  Every thread
 // of both update kernels asks at its start; the three words were written by
 // earlier kernels and no kernel that asks writes them, so plain loads (cached
 // in L1 after the first warp of an SM) serve it: uncached loads sent every
@@ -405,13 +405,22 @@ __device__ __forceinline__ uint32_t ctl_ld32(const uint32_t* p) {
 
 // kFormLitRows where more than a sixteenth of the live slots are movable or
 // tested: a settled brain has 0.5 % of them so, one that learns all its life
-// nearly all.
-__device__ __forceinline__ TickForm tick_form(const ShardCtl* ctl, uint32_t k, const LearnCtl* lc, uint32_t index) {
+// nearly all.  kFormVerify while so few axons are dark that less than one row in
+// kDarkRows has a slot on one: such a row is tested a second time and holds up its
+// warp's other three.  A tick of 504,000 plastic neurons with 64 network spikes: 32.6
+// us checked and 37.8 dense at 33 slots a row, 39.0 and 42.2 at 64, 53.6 and 53.4 at
+// 96, 64.5 and 62.0 at 128; of 61,000 at 100 slots, with the same spikes, 26.4 and 21.1;
+// with a hundredth of the axons dark 1.5M settled neurons took 240 checked, 163 dense.
+constexpr uint32_t kDarkRows = 128;
+__device__ __forceinline__ TickForm tick_form(const ShardCtl* ctl, uint32_t k, uint32_t A, const LearnCtl* lc,
+                                              uint32_t index) {
   const unsigned long long p = ctl_ld64(&ctl->pfx_total), c = ctl_ld64(&ctl->slot_total), m = ctl_ld64(&ctl->mov_total);
   const uint32_t dark = ctl_ld32(&ctl->dense[k & 1]), smax = ctl_ld32(&ctl->row_smax);
   if (lc && lc->mode == 1u && !lc->overflow) return index_ok(ctl) ? kFormSparse : kFormScatter;
-  if (c > 0 && p * 8ull <= c)
-    return !dark ? ((m + p) * 16ull > c ? kFormLitRows : kFormLitSum) : smax > 32u ? kFormVerify : kFormDense;
+  if (c > 0 && p * 8ull <= c) {
+    if (!dark) return (m + p) * 16ull > c ? kFormLitRows : kFormLitSum;
+    return smax > 32u && (unsigned long long)dark * smax * kDarkRows <= A ? kFormVerify : kFormDense;
+  }
   return index && index_ok(ctl) && sparse_tick(ctl, k) ? kFormSparse : kFormDense;
 }
 
@@ -1053,7 +1062,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     if ((threadIdx.x & 31) == 0 && i < A) {
       lit_bits[i >> 5] = lb;
       always_lit(alit + (i >> 5), lb, alit_new);
-      if (xw & ~lb) atomicOr(&ctl->dense[k & 1], 1u);   // the lit-sum form cannot run this tick
+      if (xw & ~lb) atomicAdd(&ctl->dense[k & 1], (uint32_t)__popc(xw & ~lb));   // the lit-sum form cannot run this tick
     }
   }
   bool ev = false;
@@ -1935,7 +1944,7 @@ __global__ void __launch_bounds__(LIT ? 1024 : 256, LIT ? 1 : 4)
   chain_open();
   const PassCtl pc = pass_ctl(ctl, k);
   const uint32_t ecount = ctl_ld32(&ctl->eval_act[k & 1][0]);
-  const TickForm form = tick_form(ctl, k, lc, index);
+  const TickForm form = tick_form(ctl, k, A, lc, index);
   // else k_rows_update_lsum or the learned engine's kernels run this tick
   if (form != kFormDense && form != kFormLitRows && form != kFormVerify) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) count_form(ctl, form);
@@ -2010,7 +2019,7 @@ __global__ void __launch_bounds__(256, 6)
     k_sparse_hits(ShardVramPtrs P, uint32_t A, const uint32_t* __restrict__ rt, const int16_t* __restrict__ rw,
                   const uint2* __restrict__ mask2, const uint32_t* __restrict__ live, const uint32_t* __restrict__ evb,
                   int32_t* __restrict__ acc, ShardCtl* __restrict__ ctl, uint32_t k, const LearnCtl* __restrict__ lc) {
-  if (tick_form(ctl, k, lc, 1u) != kFormSparse) return;
+  if (tick_form(ctl, k, A, lc, 1u) != kFormSparse) return;
   const uint32_t* __restrict__ off = ctl->ix_off;
   const uint16_t* __restrict__ seg = ctl->ix_seg;
   const uint32_t* __restrict__ ent = ctl->ix_ent;
@@ -2144,7 +2153,7 @@ __global__ void __launch_bounds__(256, kNeuronBlocks)
                      uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl, uint32_t k, uint32_t fix_cap,
                      const uint32_t* __restrict__ lit_bits, const LearnCtl* __restrict__ lc,
                      int32_t* __restrict__ acc) {
-  if (tick_form(ctl, k, lc, 1u) != kFormSparse) return;
+  if (tick_form(ctl, k, A, lc, 1u) != kFormSparse) return;
   const uint32_t tiles = (N + 127u) / 128u;
   if (blockIdx.x * 8u >= tiles) return;   // no neuron for this block: no table to build
   if (blockIdx.x == 0 && threadIdx.x == 0) count_form(ctl, kFormSparse);
@@ -2297,7 +2306,7 @@ __global__ void __launch_bounds__(256, kLsumBlocks)
   chain_open();
   const PassCtl pc = pass_ctl(ctl, k);
   const uint32_t ecount = ctl_ld32(&ctl->eval_act[k & 1][0]);
-  if (tick_form(ctl, k, lc, 0u) != kFormLitSum) return;
+  if (tick_form(ctl, k, A, lc, 0u) != kFormLitSum) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctl->ctr[6] += 1;   // ticks on the lit-sum form
     count_form(ctl, kFormLitSum);
@@ -2405,7 +2414,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop(ShardVramPtrs P, uint32_t A, 
                                                    uint32_t fix_cap, const LearnCtl* __restrict__ lc) {
   // the learned engine lists the spikers of its sparse ticks here; on its dense
   // ticks the update pass applied GSOP itself
-  if (lc && tick_form(ctl, k, lc, 1u) != kFormScatter) return;
+  if (lc && tick_form(ctl, k, A, lc, 1u) != kFormScatter) return;
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
@@ -2514,7 +2523,7 @@ __global__ void __launch_bounds__(256) k_rows_gsop_rows(ShardVramPtrs P, uint32_
                                                         const uint32_t* __restrict__ wcnt, uint32_t nwu,
                                                         uint32_t* __restrict__ fix, ShardCtl* __restrict__ ctl,
                                                         uint32_t k, uint32_t fix_cap, const LearnCtl* __restrict__ lc) {
-  if (lc && tick_form(ctl, k, lc, 1u) != kFormScatter) return;   // as k_rows_gsop
+  if (lc && tick_form(ctl, k, A, lc, 1u) != kFormScatter) return;   // as k_rows_gsop
   __shared__ VariantParameters lut[16];
   __shared__ int2 gtab[16][16];
   __shared__ uint32_t s_pmax;
@@ -2859,7 +2868,7 @@ __device__ __forceinline__ uint32_t rows_prologue(uint32_t i0, BurstHeads8* head
       always_lit(alit + (i >> 5), lb, alit_new);
       if (INDEX) live[i >> 5] = onb;
       // an axon the row layout summed as fully lit is not: this tick takes the full pass
-      if (xw[r] & ~lb) atomicOr(&ctl->dense[k & 1], 1u);
+      if (xw[r] & ~lb) atomicAdd(&ctl->dense[k & 1], (uint32_t)__popc(xw[r] & ~lb));
     }
     bool ev = false;
     if (i < N) {
@@ -3076,7 +3085,7 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
                                   b.dopamine, b.xlit, nullptr, nullptr, b.alit, t == b.lit_tick ? 1u : 0u, s_list,
                                   s_place);
     if (!small_barrier<CLUSTER>(ctl, target, tries, &s_ok)) return;
-    const TickForm form = tick_form(ctl, k, nullptr, 0u);
+    const TickForm form = tick_form(ctl, k, b.A, nullptr, 0u);
     const uint32_t ecount = s_place[0];
     if (threadIdx.x < ecount) b.eval[s_place[1] + threadIdx.x] = s_list[threadIdx.x];
     if (blockIdx.x == 0 && threadIdx.x == 0) rows_next_lists(ctl, k);

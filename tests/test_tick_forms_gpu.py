@@ -208,6 +208,22 @@ def test_lit_rows_and_a_dark_axon(gpu, slots, chain, per_tick):
         r.close()
 
 
+@pytest.mark.parametrize("per_tick", [False, True])
+def test_many_dark_axons_take_the_dense_pass(gpu, per_tick):
+    """Checking rows slot by slot pays while few have a slot on a dark axon."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    r = Ring(600, 640 * sms + 32, 96)
+    try:
+        for _ in range(8):
+            r.run(per_tick, 64 if per_tick else 10)
+        r.darken(300)
+        forms = r.run(per_tick, 3)
+        assert forms[DENSE] > 0 and forms[CHECKED] == 0, forms
+        r.run(per_tick, 20)
+    finally:
+        r.close()
+
+
 @pytest.mark.parametrize("odd", [False, True])
 def test_learned_quiet_ticks_run_sparse(gpu, odd):
     """The learned engine's quiet ticks do run from the inverted index of the rows."""
