@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) k_pop_build(const PopBrain* __restrict__ 
     st.lit[threadIdx.x] = 0u;
   }
   __syncthreads();
-  stage_columns(st, b.P.dendrite_targets, b.P.dendrite_weights, N, n0, b.A, nullptr, false, nullptr);
+  stage_columns(st, b.P.dendrite_targets, b.P.dendrite_weights, N, n0, b.A, nullptr, false, nullptr, 0u);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ uint32_t s_bc[8], s_bs[8];
   uint32_t wc = 0, ws = 0;

@@ -86,6 +86,17 @@ static void launch_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
 // uses: after two pushes close together the eight heads reach less far, but few
 // axons have slots on their last segments).
 constexpr uint32_t kAxOwned = 1u, kAxShared = 0x80000000u, kAxSegs = 0x7FFFFFFEu;
+// Segments 1..used_segs count as used on every axon, so that a layout asks for the
+// words of the targets beyond them only (a third of the benchmark's slots are past 7,
+// one in 16 past 12; asking for all of them was 450 us of a layout of 1.5M neurons).
+// Seven heads one tick apart reach segment 7, two ticks apart 13: an axon lit on its
+// own segments at every tick is lit on those too.  A forced layout takes the larger
+// number: it is the one that a write, a LUT or a change of path makes a program wait
+// for, and the next layout, if it pays, marks the rest.
+constexpr uint32_t kUsedSegs = 7, kUsedSegsForced = 12;
+__device__ __forceinline__ uint32_t used_segs(const ShardCtl* ctl, uint32_t cond) {
+  return cond && !ctl->lay_forced ? kUsedSegs : kUsedSegsForced;
+}
 __device__ __forceinline__ uint32_t ax_owners(uint32_t axw) { return (axw & kAxOwned) + (axw >> 31); }
 constexpr uint32_t kRowBad = 0x8000u;    // cnt flag: the row holds an invalid target
 
@@ -506,10 +517,12 @@ constexpr uint32_t kSlotMov = 1u, kSlotLit = 2u, kSlotBad = 4u;
 // fz and lit: 32 slots of the 32 neurons a round, until every neuron has met its
 // first empty target.  A thread has four targets and weights of the next round in
 // flight while it looks up the four of this one (xlit: the lit axons; axw: marks
-// the axon's segment as used), so a round costs the latency of one gather.
+// the axon's segment as used, beyond the first `used`), so a round costs the latency
+// of one gather.
 __device__ __forceinline__ void stage_columns(SlotStage& st, const uint32_t* __restrict__ targets,
                                               const int16_t* __restrict__ weights, uint32_t N, uint32_t n0, uint32_t A,
-                                              const uint32_t* __restrict__ xlit, bool mov_lit, uint32_t* axw) {
+                                              const uint32_t* __restrict__ xlit, bool mov_lit, uint32_t* axw,
+                                              uint32_t used) {
   const uint32_t col = threadIdx.x & 31, r0 = threadIdx.x >> 5, n = n0 + col;
   const int32_t fz = st.fz[col];
   const bool lit_on = xlit && st.lit[col];
@@ -539,7 +552,7 @@ __device__ __forceinline__ void stage_columns(SlotStage& st, const uint32_t* __r
       const uint32_t a = (t[i] & AXC_TARGET_AXON_MASK) - 1u, seg = t[i] >> AXC_TARGET_SEG_SHIFT;
       const bool in = a < A && seg - 1u < 30u;
       lw[i] = in && lit_on ? __ldg(xlit + (a >> 5)) : 0u;
-      aw[i] = in && axw ? axw[a] : 0xFFFFFFFFu;   // (a stale word only costs an atomic that changes nothing)
+      aw[i] = in && axw && seg > used ? axw[a] : 0xFFFFFFFFu;   // (a stale word only costs an atomic that changes nothing)
     }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -692,15 +705,23 @@ __device__ __forceinline__ void writeback_tile(int16_t* __restrict__ weights, ui
     if (r < c_mine && ((o[r >> 5] >> (r & 31u)) & 1u)) weights[(size_t)r * N + n0 + lane] = s_w[r][lane];
 }
 
-// Batch start: columnar -> rows, 32 neurons per 256-thread block (stage_columns,
-// build_row).  A slot whose weight GSOP may still move (not frozen_weight, or any
-// slot of a row with an invalid target) is movable; weights only freeze, so the
-// marks hold for the whole batch.  The dendrite sum (a wrapping i32 sum) and GSOP
-// (per slot) do not depend on the order of a row.
+// Batch start: columnar -> rows, tiles of 32 neurons by 256-thread blocks (stage_columns,
+// build_row), four resident on an SM and up to four tiles a block (`per`; as many as
+// leave each SM its blocks): with a block a tile the batches that keep their layout paid
+// 27 us at 1.5M neurons and 135 at 8M for blocks that only return (8 and 35 now), and a
+// layout of 8M took 8.8 ms against 8.5.  What the rows add up to is kept in shared
+// memory (176 bytes of spills a thread with it in registers, 100 without).
+// A slot whose weight GSOP may still move (not frozen_weight, or any slot of a row with
+// an invalid target) is movable; weights only freeze, so the marks hold for the whole
+// batch.  The dendrite sum (a wrapping i32 sum) and GSOP (per slot) do not depend on the
+// order of a row.
 // Per neuron: cnt = used slots (| kRowBad), lfz = movable slots, amask = their
 // row positions, omask = the columnar slots placed first (read by the
 // write-back; every used slot when the row keeps the columnar order).
-__global__ void __launch_bounds__(256, 4) k_rows_build(const uint32_t* __restrict__ targets,
+constexpr int kBuildBlocks = 4;
+constexpr uint32_t kBuildTiles = 4;
+
+__global__ void __launch_bounds__(256, kBuildBlocks) k_rows_build(const uint32_t* __restrict__ targets,
                                                     const int16_t* __restrict__ weights,
                                                     const uint8_t* __restrict__ flags, uint32_t N,
                                                     uint32_t* __restrict__ rt, int16_t* __restrict__ rw,
@@ -709,59 +730,57 @@ __global__ void __launch_bounds__(256, 4) k_rows_build(const uint32_t* __restric
                                                     ShardCtl* __restrict__ ctl, uint32_t A, uint32_t want_sum,
                                                     uint32_t permute, const uint32_t* __restrict__ xlit,
                                                     int2* __restrict__ rec, uint4* __restrict__ lmask,
-                                                    uint8_t* __restrict__ posmap, uint32_t* axw, uint32_t cond) {
+                                                    uint8_t* __restrict__ posmap, uint32_t* axw, uint32_t cond,
+                                                    uint32_t per) {
   if (cond && !ctl->lay_now) return;   // the batch keeps the last layout
   __shared__ SlotStage st;
-  __shared__ uint32_t s_pmax;
-  const uint32_t n0 = blockIdx.x * 32;
-  if (threadIdx.x < 32) {
-    const uint32_t n = n0 + threadIdx.x, pmax = lut_pmax();
-    const VariantParameters& vp = VARIANT_LUT[n < N ? flags[n] >> 4 : 0];
-    st.cnt[threadIdx.x] = AXC_MAX_DENDRITES;
-    st.fz[threadIdx.x] = frozen_from(vp);
-    st.lit[threadIdx.x] = vp.signal_propagation_length == pmax ? 1u : 0u;
-    if (threadIdx.x == 0) s_pmax = pmax;
-  }
-  __syncthreads();
+  const uint32_t pmax = lut_pmax(), used = used_segs(ctl, cond);
   // movable slots join the lit groups (no cooling step up to length 16), except in
   // a layout that was forced: the window of always-lit axons is from before what
   // forced it (a LUT, new targets)
-  const bool mov_lit = s_pmax <= 16u && cond && !ctl->lay_forced;
-  stage_columns(st, targets, weights, N, n0, A, xlit, mov_lit, axw);
+  const bool mov_lit = pmax <= 16u && cond && !ctl->lay_forced;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // the block's longest row, largest segment, tested and live slots and (when
-  // asked) targets checksum, one atomic each per block
+  // asked) targets checksum, a warp's each; one atomic each per block
   __shared__ uint32_t s_bc[8], s_bs[8], s_bp[8], s_bl[8], s_bx[8], s_bm[8];
   __shared__ unsigned long long s_bh[8], s_bq[8];
-  uint32_t wc = 0, ws = 0, wp = 0, wl = 0, wm = 0;
-  bool mixed = false;
-  unsigned long long wh = 0, wq = 0;
-  for (uint32_t j = warp; j < 32; j += 8) {
-    const uint32_t n = n0 + j;
-    if (n >= N) continue;
-    const uint32_t c = st.cnt[j];
-    const RowBuilt rb = build_row(st, j, n, c, want_sum != 0u, permute != 0u, rt, rw, cnt, amask, omask, lfz, rec, lmask,
-                                  posmap);
-    if (lane == 0 && c) {
-      wc = max(wc, c);
-      ws = max(ws, rb.smx);
-      wh += rb.hsum + slot_mix(c, n);
-      wp += rb.pfx;
-      wl += c;
-      wm += rb.lf;
-      if (want_sum) wq += rb.psum + slot_mix(c, ~n);
-      mixed |= st.lit[j] == 0u;
-    }
+  if (threadIdx.x < 8) {
+    s_bc[threadIdx.x] = s_bs[threadIdx.x] = s_bp[threadIdx.x] = s_bl[threadIdx.x] = s_bx[threadIdx.x] = 0;
+    s_bm[threadIdx.x] = 0;
+    s_bh[threadIdx.x] = s_bq[threadIdx.x] = 0;
   }
-  if (lane == 0) {
-    s_bc[warp] = wc;
-    s_bs[warp] = ws;
-    s_bh[warp] = wh;
-    s_bp[warp] = wp;
-    s_bl[warp] = wl;
-    s_bx[warp] = mixed;
-    s_bm[warp] = wm;
-    s_bq[warp] = wq;
+  const uint32_t n_end = min(N, (blockIdx.x + 1u) * (32u * per));
+#pragma unroll 1
+  for (uint32_t n0 = blockIdx.x * (32u * per); n0 < n_end; n0 += 32u) {
+    __syncthreads();   // the previous tile's rows are built
+    if (threadIdx.x < 32) {
+      const uint32_t n = n0 + threadIdx.x;
+      const VariantParameters& vp = VARIANT_LUT[n < N ? flags[n] >> 4 : 0];
+      st.cnt[threadIdx.x] = AXC_MAX_DENDRITES;
+      st.fz[threadIdx.x] = frozen_from(vp);
+      st.lit[threadIdx.x] = vp.signal_propagation_length == pmax ? 1u : 0u;
+    }
+    __syncthreads();
+    stage_columns(st, targets, weights, N, n0, A, xlit, mov_lit, axw, used);
+    for (uint32_t j = warp; j < 32; j += 8) {
+      const uint32_t n = n0 + j;
+      if (n >= N) continue;
+      const uint32_t c = st.cnt[j];
+      const RowBuilt rb = build_row(st, j, n, c, want_sum != 0u, permute != 0u, rt, rw, cnt, amask, omask, lfz, rec,
+                                    lmask, posmap);
+      if (lane == 0 && c) {   // in shared memory: registers are short
+        s_bc[warp] = max(s_bc[warp], c);
+        s_bs[warp] = max(s_bs[warp], rb.smx);
+        s_bp[warp] += rb.pfx;
+        s_bl[warp] += c;
+        s_bm[warp] += rb.lf;
+        s_bx[warp] |= st.lit[j] == 0u;
+        if (want_sum) {
+          s_bh[warp] += rb.hsum + slot_mix(c, n);
+          s_bq[warp] += rb.psum + slot_mix(c, ~n);
+        }
+      }
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -797,9 +816,9 @@ __global__ void __launch_bounds__(256) k_rows_prep(const ShardCtl* __restrict__ 
                                                    uint32_t A, const uint32_t* __restrict__ alit,
                                                    uint32_t* __restrict__ xlit, uint32_t cond) {
   if (cond && !ctl->lay_now) return;
-  const uint32_t words = A / 32 + 1;
+  const uint32_t words = A / 32 + 1, used = (2u << used_segs(ctl, cond)) - 2u;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < A; i += gridDim.x * blockDim.x) {
-    axw[i] = 0u;
+    axw[i] = used;
     if (xlit && i < words) xlit[i] = alit[i];
   }
 }
@@ -3279,11 +3298,13 @@ cudaError_t launch_rows_begin(const ShardVramPtrs& v, ShardScratch& s, uint32_t 
              s.ctl, r.axw, A, r.alit, permute ? r.xlit : nullptr, cond);
   if (N) {
     k_rows_mult<<<(N + 255) / 256, 256, 0, stream>>>(v.soma_to_axon, N, A, r.axw, r.mask2, s.ctl, cond);
-    k_rows_build<<<(N + 31) / 32, 256, 0, stream>>>(v.dendrite_targets, v.dendrite_weights, v.soma_flags, N, r.rt,
+    const uint32_t tiles = (N + 31) / 32, wave = kBuildBlocks * (uint32_t)sm_count();
+    const uint32_t per = std::min(kBuildTiles, (tiles + wave - 1) / wave);
+    k_rows_build<<<(tiles + per - 1) / per, 256, 0, stream>>>(v.dendrite_targets, v.dendrite_weights, v.soma_flags, N, r.rt,
                                                     r.rw, r.cnt, r.amask, r.omask, r.lfz, s.ctl, A,
                                                     row_sum ? 1u : 0u, permute ? 1u : 0u,
                                                     permute ? r.xlit : nullptr, permute ? r.rec : nullptr, r.lmask,
-                                                    with_posmap ? r.posmap : nullptr, r.axw, cond);
+                                                    with_posmap ? r.posmap : nullptr, r.axw, cond, per);
   }
   return cudaGetLastError();
 }

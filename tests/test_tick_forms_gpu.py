@@ -139,7 +139,7 @@ def test_chain_bitmap_wait_gives_up(gpu):
 class Ring:
     """n neurons on the first of A axons, `slots` slots a row, in step with the oracle; every weight moves."""
 
-    def __init__(self, n, A, slots):
+    def __init__(self, n, A, slots, segs=9):
         self.n, self.A = n, A
         self.lut = W.small().lut
         for v in (0, 1):
@@ -148,7 +148,7 @@ class Ring:
         self.state = np.zeros(state_blob_size(n), np.uint8)
         sv = StateView(self.state, n)
         for s in range(slots):
-            sv.targets[s] = ((1 + s % 9) << 24) | (1 + (np.arange(n) + 3 * s + 1) % n)
+            sv.targets[s] = ((1 + s % segs) << 24) | (1 + (np.arange(n) + 3 * s + 1) % n)
         sv.weights[:slots] = rng.integers(2100, 2900, size=(slots, n)) * rng.choice([1, 1, 1, -1], size=(slots, n))
         sv.soma_to_axon[:] = np.arange(n, dtype=np.uint32)
         sv.voltage[:] = rng.integers(0, 1999, size=n)
@@ -204,6 +204,23 @@ def test_lit_rows_and_a_dark_axon(gpu, slots, chain, per_tick):
         assert forms[:6].sum() == 10 and forms[LIT_ROWS] < 10, forms
         if A > 90_000:   # one dark axon among many
             assert forms[CHECKED] > 0, forms
+    finally:
+        r.close()
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 4])
+def test_layout_tiles(gpu, tiles):
+    """Layouts whose blocks take one, two or four tiles of 32 neurons, the last of them ragged; slots on both sides of
+    the segments that every axon counts as using."""
+    wave = 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = 32 * (tiles - 1) * wave + 32 * 5 + 4
+    r = Ring(n, (n + 63) // 32 * 32, 48, segs=23)
+    try:
+        layouts = 0
+        for _ in range(7):
+            forms = r.run(False)
+            layouts += int(forms[LAYOUTS])
+        assert layouts >= 2 and forms[LIT_ROWS] > 0, (layouts, forms)
     finally:
         r.close()
 
