@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(512) k_set_batch_ctl(ShardCtl* ctl, uint32_t t
     ctl->dopamine = dopamine;
     ctl->barrier = 0;
   }
-  if (rows) layout_decide(ctl, force, ticks, lit, A);
+  if (rows) layout_decide(ctl, force, ticks, lit, A, false);
 }
 
 cudaError_t ensure_counts(ShardScratch& s, uint32_t batch, bool* realloc, cudaStream_t stream) {

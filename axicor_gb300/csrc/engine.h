@@ -190,8 +190,17 @@ inline bool batch_rows_force(ShardScratch& s) {
 }
 
 #ifdef __CUDACC__
-// The device's layout decision for the next `ticks` ticks of a batch (one
-// block, before the batch; lit: the always-lit axons of the last ticks, of A).
+#define AXC_HD __host__ __device__
+#else
+#define AXC_HD
+#endif
+
+// The current layout meets the lit-sum criterion: at most an eighth of the live
+// slots are tested one by one.
+AXC_HD inline bool layout_met(const ShardCtl* c) { return c->slot_total > 0 && c->pfx_total * 8ull <= c->slot_total; }
+
+// The layout decision for the next `ticks` ticks (lit: always-lit axons of the last
+// ticks, counted when forced or not met; index: the ticks may run the sparse form).
 // A new layout when forced; every lay_every ticks, doubling from
 // kBatchRelayoutMin to kBatchRelayoutMax, while the current one meets the
 // lit-sum criterion (at most an eighth of the live slots tested); while it does
@@ -201,37 +210,25 @@ inline bool batch_rows_force(ShardScratch& s) {
 // last decision no longer moved; but for these at most every lay_wait ticks,
 // doubling from 16 while the new layouts gain less than a tenth, and at least
 // every kBatchRelayoutMax.  A brain whose weights never freeze, or that is
-// quiet, so keeps its layout instead of paying for one each batch (1.5 ms at
-// 1.5M neurons).  The layout kernels of the batch
-// return at once when lay_now is 0.
-__device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint32_t ticks, const uint32_t* lit,
-                                              uint32_t A) {
-  __shared__ uint32_t s_lit;
+// quiet, so keeps its layout instead of paying for one each batch (1.6 ms at
+// 1.5M neurons).  The layout kernels of the batch return at once when lay_now is 0.
+AXC_HD inline void layout_decision(ShardCtl* c, uint32_t force, uint32_t ticks, uint32_t lit, bool index) {
   // the layout meets the criterion, and its lit axons stayed lit on most ticks since the last decision
-  const bool met = c->slot_total > 0 && c->pfx_total * 8ull <= c->slot_total;
+  const bool met = layout_met(c);
   const unsigned long long lit6 = c->ctr[6] < c->lit_seen ? c->ctr[6] : c->ctr[6] - c->lit_seen;
-  const bool missed = met && lit6 * 2ull < c->dec_ticks;   // dark axons: the rows were checked slot by slot
-  uint32_t n = 0;
-  if (threadIdx.x == 0) s_lit = 0;
-  __syncthreads();
-  if (force || !met) {
-    for (uint32_t i = threadIdx.x; i < (A + 31) / 32; i += blockDim.x) n += __popc(lit[i]);
-    n = __reduce_add_sync(0xFFFFFFFFu, n);
-    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&s_lit, n);
-  }
-  __syncthreads();
-  if (threadIdx.x) return;
+  const bool missed = met && lit6 * 2ull < c->dec_ticks;   // ticks with dark axons
+  if (!index) c->streak = 0;   // of the learned engine's last ticks
   bool build = force;
   const bool froze = c->gsop_same[0] > 0 && c->gsop_same[0] * 8ull >= c->gsop_same[1];
   if (!force && met) {
     build = c->lay_since >= c->lay_every || ((froze || missed) && c->lay_since >= c->lay_wait);
   } else if (!force) {
-    const bool grew = (unsigned long long)s_lit * 10ull > (unsigned long long)c->lay_lit * 11ull;
+    const bool grew = (unsigned long long)lit * 10ull > (unsigned long long)c->lay_lit * 11ull;
     // (the sparse form reads no more than the movable slots of a few spikers: its rows stay)
     build = (c->lay_since >= kBatchRelayoutMax && c->streak == 0u) ||
             (c->lay_since >= c->lay_wait && (froze || grew) && c->slot_total > 0);
   }
-  if (build && (force || !met)) c->lay_lit = force ? 0u : s_lit;   // a forced layout leaves movable slots out
+  if (build && (force || !met)) c->lay_lit = force ? 0u : lit;   // a forced layout leaves movable slots out
   // the last layout left a tenth fewer tested and movable slots than the one before
   const bool paid = (c->pfx_total + c->mov_total) * 10ull < c->lay_work * 9ull;
   if (build) {
@@ -239,7 +236,8 @@ __device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint3
     c->lay_every = (force || !met || c->lay_every < kBatchRelayoutMin) ? kBatchRelayoutMin
                    : twice < kBatchRelayoutMax                          ? twice
                                                                         : kBatchRelayoutMax;
-    c->lay_wait = force ? 0u : (paid || c->lay_wait < 16u) ? 16u : min(2u * c->lay_wait, kBatchRelayoutMax);
+    const uint32_t wait = 2u * c->lay_wait < kBatchRelayoutMax ? 2u * c->lay_wait : kBatchRelayoutMax;
+    c->lay_wait = force ? 0u : (paid || c->lay_wait < 16u) ? 16u : wait;
     c->lay_work = c->pfx_total + c->mov_total;
     c->lay_since = 0;
   }
@@ -249,6 +247,24 @@ __device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint3
   c->dec_ticks = ticks;
   c->lay_since += ticks;
   c->lay_now = build ? 1u : 0u;
+}
+
+#ifdef __CUDACC__
+// The decision on the device, by one block before the batch (lit: the always-lit
+// axons of the last ticks, a bit each, of A).
+__device__ __forceinline__ void layout_decide(ShardCtl* c, uint32_t force, uint32_t ticks, const uint32_t* lit,
+                                              uint32_t A, bool index) {
+  __shared__ uint32_t s_lit;
+  uint32_t n = 0;
+  if (threadIdx.x == 0) s_lit = 0;
+  __syncthreads();
+  if (force || !layout_met(c)) {
+    for (uint32_t i = threadIdx.x; i < (A + 31) / 32; i += blockDim.x) n += __popc(lit[i]);
+    n = __reduce_add_sync(0xFFFFFFFFu, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&s_lit, n);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) layout_decision(c, force, ticks, s_lit, index);
 }
 #endif
 

@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(512) k_learn_set_ctl(ShardCtl* ctl, uint32_t t
                                                       uint32_t A) {
   ctl->tick_base = tick_base;
   ctl->dopamine = dopamine;
-  layout_decide(ctl, force, ticks, lit, A);
+  layout_decide(ctl, force, ticks, lit, A, true);
 }
 
 // splitmix64: seeded parameter init and minibatch order, identical on every host.

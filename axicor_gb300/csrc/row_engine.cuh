@@ -3280,7 +3280,7 @@ void rows_free(ShardScratch& s) {
 namespace {
 __global__ void __launch_bounds__(512) k_rows_decide(ShardCtl* ctl, uint32_t force, uint32_t ticks,
                                                     const uint32_t* lit, uint32_t A) {
-  layout_decide(ctl, force, ticks, lit, A);
+  layout_decide(ctl, force, ticks, lit, A, false);
 }
 }  // namespace
 
