@@ -776,7 +776,7 @@ int32_t axc_population_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_
   Population* P = static_cast<Population*>(handle);
   if (!P || tpg == 0 || ticks % tpg || !pop_ticks_ok(*P, tick0, ticks)) return (int32_t)cudaErrorInvalidValue;
   cudaStream_t st = static_cast<cudaStream_t>(stream_v);
-  for (ShardScratch* s : P->scr) rows_touched(*s);   // the per-tick entry point's row copies are replaced
+  for (ShardScratch* s : P->scr) rows_touched(*s);   // the row copies of the other entry points are replaced
   auto key = std::make_tuple(tpg, P->sched.lanes_per_neuron, P->sched.update_blocks_per_sm,
                              P->sched.aux_blocks_per_sm * 1000 + std::min(g_pop_fix_cap(), kFixCap) % 1000);
   cudaGraphExec_t exec = nullptr;
@@ -817,6 +817,7 @@ int32_t axc_population_tune(void* handle, uint32_t tick0, uint32_t trial_ticks, 
     for (uint32_t ub : {2u, 3u, 4u})
       for (uint32_t ab : {1u, 2u}) cands.push_back(AxcPopSchedule{lanes, ub, ab});
   if (!pop_ticks_ok(*P, tick0, (uint64_t)trial_ticks * cands.size())) return (int32_t)cudaErrorInvalidValue;
+  for (ShardScratch* s : P->scr) rows_touched(*s);   // as in a run
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

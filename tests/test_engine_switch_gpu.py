@@ -7,10 +7,13 @@ them.
 import numpy as np
 import pytest
 
+import oracle
 from axicor_gb300 import _native as N
+from axicor_gb300 import population as Pop
 from axicor_gb300 import shard as S
 from axicor_gb300 import workloads as W
-from test_batch_rows_reuse_gpu import BatchTwin
+from axicor_gb300.formats import StateView
+from test_batch_rows_reuse_gpu import BatchTwin, mostly_frozen
 
 pytestmark = pytest.mark.gpu
 
@@ -30,7 +33,7 @@ def test_columnar_steps_between_row_steps(gpu, steps):
             lib.axc_tick_engine_mode(int(step[1]))
             before = t.h_state.copy()
             t.batch(10) if step[0] == "b" else t.per_tick(10)
-            weights = [S.StateView(x, t.N).weights for x in (before, t.h_state)]
+            weights = [StateView(x, t.N).weights for x in (before, t.h_state)]
             assert np.count_nonzero(weights[0] != weights[1]) > 100, f"{step} must move weights"
         assert t.vram.error_flags() == 0
     finally:
@@ -38,3 +41,54 @@ def test_columnar_steps_between_row_steps(gpu, steps):
         lib.axc_tick_engine_mode(modes[1])
         S.upload_lut(W.default_lut())
         t.close()
+
+
+def population(steps):
+    """Two mostly frozen brains (their batches keep a layout of lit sums) stepped alone and as a population."""
+    brains = [Pop.Brain(W.small(dims=(16, 16, 8), slots=80, inputs=64, p=0.1, seed=s), 400) for s in (1, 2)]
+    pop = None
+    try:
+        tick = 0
+        for b in brains:
+            mostly_frozen(b.w, b.state0, b.lay.padded_n)
+            sv = StateView(b.state0, b.lay.padded_n)   # the others freeze at every tick, each in its turn
+            move = (sv.targets != 0) & (np.abs(sv.weights) < 2048)
+            size = np.random.default_rng(b.w.seed).integers(50, 2048, size=int(move.sum()))
+            sv.weights[move] = np.sign(sv.weights[move]) * size
+            b.reset()
+        S.upload_lut(brains[0].w.lut)
+        engines = [S.ShardEngine(b.vram) for b in brains]
+        ios = [S.IoDeviceBuffers(b.words, 0, 0, 20) for b in brains]
+        for step in steps.split():
+            ticks = {"alone": 20, "create": 0, "tune": 12, "run": 8}[step]
+            if step == "alone":
+                for b, e, io in zip(brains, engines, ios):   # (Brain.run_alone uploads the LUT, which lays the rows out anew)
+                    e.step_day_phase_batch(ticks, io, b.bitmask[tick * b.words:], None, None, b.lay.virtual_offset,
+                                           b.w.num_inputs, None, 1, 0, tick)
+            elif step == "create":
+                pop = Pop.Population(brains)
+            elif step == "tune":
+                pop.tune(tick, 1)
+            else:
+                pop.run(tick, ticks, 4)
+            tick += ticks
+            N.lib().gpu_device_synchronize()
+        assert all(b.vram.forms()[[1, 4]].sum() > 0 for b in brains)
+        for b in brains:
+            state, heads = b.state0.copy(), b.heads0.copy()
+            oracle.run_ticks(state, heads, b.w.lut, b.lay.padded_n, b.lay.total_axons, 1, 0, tick, b.bitmask, b.words,
+                             b.lay.virtual_offset, b.w.num_inputs)
+            assert np.array_equal(b.vram.download_heads(), heads)
+            assert np.array_equal(b.vram.download_state(), state)
+    finally:
+        if pop:
+            pop.close()
+        for b in brains:
+            b.free()
+        S.upload_lut(W.default_lut())
+
+
+@pytest.mark.parametrize("batches", [3, 4, 5, 6, 7, 8])   # between two layouts of the batch path, or not
+def test_batches_around_a_population_tuning(gpu, batches):
+    """The tuner's trial ticks move weights and use the rows' buffers."""
+    population("alone create" + batches * " alone" + " tune alone run alone")
