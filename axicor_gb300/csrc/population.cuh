@@ -620,6 +620,8 @@ struct Population {
   uint32_t lit_cap = 0;   // words of the largest fully-lit bitmap the update stages (<= kPopLitWords)
   std::vector<uint32_t> bm_ticks;   // per brain: bitmask rows (UINT32_MAX without a bitmask)
   std::vector<ShardScratch*> scr;   // per brain: the shard's scratch (its rows are this engine's while it runs)
+  std::vector<const void*> rows_base;   // per brain: the row buffers that hb points into
+  bool stale = false;     // d_brains is older than hb
   std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t>, cudaGraphExec_t> graphs;
   cudaStream_t capture = nullptr;
 };
@@ -629,6 +631,46 @@ static bool pop_ticks_ok(const Population& P, uint32_t tick0, uint64_t ticks) {
   for (uint32_t b : P.bm_ticks)
     if ((uint64_t)tick0 + ticks > b) return false;
   return true;
+}
+
+// The row buffers of brain b, allocated where it has none.  A batch or per-tick call of
+// the brain's own may have replaced them since (rows_alloc): the old ones are freed.
+static cudaError_t pop_take_rows(Population& P, uint32_t b) {
+  PopBrain& h = P.hb[b];
+  ShardScratch* s = P.scr[b];
+  const cudaError_t e = rows_alloc(*s, h.N, h.A, false, nullptr);
+  if (e != cudaSuccess) return e;
+  h.rt = s->rows->rt;
+  h.rw = s->rows->rw;
+  h.cnt = s->rows->cnt;
+  h.mask2 = s->rows->mask2;
+  h.mult = s->rows->axw;
+  h.eval = s->rows->eval;
+  h.lit = s->rows->lit;
+  h.lfz = s->rows->lfz;
+  h.amask = s->rows->amask;
+  h.omask = s->rows->omask;
+  P.rows_base[b] = s->rows->base;
+  return cudaSuccess;
+}
+
+// Before a run: the brains' current row buffers (freeing the old ones waited for the
+// kernels that used them), and the other entry points' copies in them out of date.
+static cudaError_t pop_rows(Population& P) {
+  for (uint32_t b = 0; b < P.count; b++) {
+    ShardScratch* s = P.scr[b];
+    if (!s->rows || s->rows->base != P.rows_base[b]) {
+      P.stale = true;
+      const cudaError_t e = pop_take_rows(P, b);
+      if (e != cudaSuccess) return e;
+    }
+    rows_touched(*s);
+  }
+  if (!P.stale) return cudaSuccess;
+  cudaError_t e = cudaMemcpy(P.d_brains, P.hb.data(), (size_t)P.count * sizeof(PopBrain), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  if (e == cudaSuccess) P.stale = false;
+  return e;
 }
 
 static cudaError_t pop_upload_map(const std::vector<uint32_t>& v, uint32_t** out) {
@@ -694,6 +736,7 @@ int32_t axc_population_create(const AxcPopBrainDesc* brains, uint32_t count, voi
   P->count = count;
   P->hb.resize(count);
   P->bm_ticks.resize(count);
+  P->rows_base.resize(count);
   cudaError_t e = cudaMalloc(&P->d_gtab, (size_t)count * 256 * sizeof(int2));
   std::vector<uint32_t> map_pro, first_pro(count), map_tile, first_tile(count), map_n, first_n(count);
   size_t max_chunks = count;
@@ -701,8 +744,6 @@ int32_t axc_population_create(const AxcPopBrainDesc* brains, uint32_t count, voi
     const AxcPopBrainDesc& d = brains[b];
     ShardScratch* s = scratch_for(&d.vram, d.padded_n, d.total_axons, &e);
     if (!s) break;
-    e = rows_alloc(*s, d.padded_n, d.total_axons, false, nullptr);
-    if (e != cudaSuccess) break;
     rows_touched(*s);
     P->scr.push_back(s);
     PopBrain& h = P->hb[b];
@@ -711,21 +752,13 @@ int32_t axc_population_create(const AxcPopBrainDesc* brains, uint32_t count, voi
     h.bitmask = d.d_input_bitmask;
     h.lut = d.d_lut;
     h.gtab = P->d_gtab + (size_t)b * 256;
-    h.rt = s->rows->rt;
-    h.rw = s->rows->rw;
-    h.cnt = s->rows->cnt;
-    h.mask2 = s->rows->mask2;
-    h.mult = s->rows->axw;
-    h.eval = s->rows->eval;
     h.pend = s->pend;
     h.ctl = s->ctl;
-    h.lit = s->rows->lit;
-    h.lfz = s->rows->lfz;
-    h.amask = s->rows->amask;
-    h.omask = s->rows->omask;
     P->lit_cap = std::max(P->lit_cap, std::min((d.total_axons >> 5) + 1, kPopLitWords));
     h.N = d.padded_n;
     h.A = d.total_axons;
+    e = pop_take_rows(*P, b);
+    if (e != cudaSuccess) break;
     h.voff = d.virtual_offset;
     h.nv = d.d_input_bitmask ? d.num_virtual : 0;
     h.words = d.words_per_tick;
@@ -776,12 +809,12 @@ int32_t axc_population_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_
   Population* P = static_cast<Population*>(handle);
   if (!P || tpg == 0 || ticks % tpg || !pop_ticks_ok(*P, tick0, ticks)) return (int32_t)cudaErrorInvalidValue;
   cudaStream_t st = static_cast<cudaStream_t>(stream_v);
-  for (ShardScratch* s : P->scr) rows_touched(*s);   // the row copies of the other entry points are replaced
+  cudaError_t e = pop_rows(*P);
+  if (e != cudaSuccess) return (int32_t)e;
   auto key = std::make_tuple(tpg, P->sched.lanes_per_neuron, P->sched.update_blocks_per_sm,
                              P->sched.aux_blocks_per_sm * 1000 + std::min(g_pop_fix_cap(), kFixCap) % 1000);
   cudaGraphExec_t exec = nullptr;
   auto it = P->graphs.find(key);
-  cudaError_t e = cudaSuccess;
   if (it != P->graphs.end()) {
     exec = it->second;
   } else {
@@ -817,11 +850,12 @@ int32_t axc_population_tune(void* handle, uint32_t tick0, uint32_t trial_ticks, 
     for (uint32_t ub : {2u, 3u, 4u})
       for (uint32_t ab : {1u, 2u}) cands.push_back(AxcPopSchedule{lanes, ub, ab});
   if (!pop_ticks_ok(*P, tick0, (uint64_t)trial_ticks * cands.size())) return (int32_t)cudaErrorInvalidValue;
-  for (ShardScratch* s : P->scr) rows_touched(*s);   // as in a run
+  cudaError_t e = pop_rows(*P);
+  if (e != cudaSuccess) return (int32_t)e;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  cudaError_t e = pop_begin(*P, st);
+  e = pop_begin(*P, st);
   float best = 1e30f;
   uint32_t tick = tick0;
   for (size_t i = 0; i < cands.size() && e == cudaSuccess; i++) {

@@ -88,6 +88,12 @@ def population(steps):
         S.upload_lut(W.default_lut())
 
 
+def test_a_brains_own_batches_between_population_runs(gpu):
+    """A brain's first own batch replaces the row buffers that the population made (a batch keeps a list of deferred
+    slots beside them): the population takes the new ones."""
+    population("create run" + 4 * " alone" + " run tune alone alone run")
+
+
 @pytest.mark.parametrize("batches", [3, 4, 5, 6, 7, 8])   # between two layouts of the batch path, or not
 def test_batches_around_a_population_tuning(gpu, batches):
     """The tuner's trial ticks move weights and use the rows' buffers."""
