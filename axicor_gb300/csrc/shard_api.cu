@@ -93,6 +93,7 @@ ShardScratch* scratch_for(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t
       if (s->state_base != vram->soma_voltage) {   // the same heads with another state allocation
         s->state_base = vram->soma_voltage;
         rows_touched(*s);
+        graph_cache_drop(s);   // the captured batches hold the old one's addresses
       }
       return s;
     }

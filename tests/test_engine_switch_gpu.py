@@ -98,3 +98,25 @@ def test_a_brains_own_batches_between_population_runs(gpu):
 def test_batches_around_a_population_tuning(gpu, batches):
     """The tuner's trial ticks move weights and use the rows' buffers."""
     population("alone create" + batches * " alone" + " tune alone run alone")
+
+
+def test_another_state_allocation_behind_the_same_heads(gpu):
+    """A captured batch holds its state's addresses; the shard is known by its heads."""
+    w = W.small(dims=(16, 16, 8), slots=40, inputs=64, p=0.2)
+    t = BatchTwin(w, frozen=False)
+    other = S.VramState(t.N, t.A)
+    first = N.ShardVramPtrs.from_buffer_copy(t.vram.ptrs)
+    try:
+        t.batch(10)
+        other.upload_state(t.h_state)
+        before = t.vram.download_state()
+        for f, _ in N.ShardVramPtrs._fields_[:-1]:
+            setattr(t.vram.ptrs, f, getattr(other.ptrs, f))
+        t.batch(10)
+        t.batch(10)
+        for f, _ in N.ShardVramPtrs._fields_:
+            setattr(t.vram.ptrs, f, getattr(first, f))
+        assert np.array_equal(t.vram.download_state(), before), "the first allocation is left as it was"
+    finally:
+        t.vram.free()
+        other.free()
