@@ -368,8 +368,9 @@ extern "C" int32_t axc_profile_ticks(const ShardVramPtrs* vram, uint32_t padded_
   if (!s) return (int32_t)e;
   const bool rows = engine == 1;
   cudaStream_t st = static_cast<cudaStream_t>(stream_v);
-  rows_touched(*s);
+  if (!rows) rows_touched(*s);   // the columnar kernels move the blob's weights
   if (rows) {
+    s->tick_rows_valid.store(false);   // as a batch
     bool realloc = false;
     e = ensure_counts(*s, ticks ? ticks : 1, &realloc, st);
     if (e == cudaSuccess) e = rows_alloc(*s, padded_n, total_axons, true, st);
@@ -380,10 +381,16 @@ extern "C" int32_t axc_profile_ticks(const ShardVramPtrs* vram, uint32_t padded_
       for (auto& kv : old->execs) cudaGraphExecDestroy(kv.second);
       old->execs.clear();
     }
+    const bool force = batch_rows_force(*s);
     cudaMemsetAsync(s->batch_counts, 0, (size_t)ticks * 4, st);
-    k_set_batch_ctl<<<1, 32, 0, st>>>(s->ctl, tick0, (int32_t)dopamine, 0u, 1u, ticks, nullptr, 0u);   // layouts its own
-    e = launch_rows_begin(*vram, *s, padded_n, total_axons, st);
-    if (e != cudaSuccess) return (int32_t)e;
+    // the rows that the next batch would run on
+    k_set_batch_ctl<<<1, 512, 0, st>>>(s->ctl, tick0, (int32_t)dopamine, 1u, force ? 1u : 0u, ticks, s->rows->alit,
+                                       total_axons);
+    e = launch_rows_begin(*vram, *s, padded_n, total_axons, st, false, true, true, true);
+    if (e != cudaSuccess) {
+      rows_touched(*s);
+      return (int32_t)e;
+    }
   }
   cudaEvent_t ev[kTickStages + 1];
   for (int i = 0; i <= kTickStages; i++) cudaEventCreate(&ev[i]);
@@ -421,6 +428,7 @@ extern "C" int32_t axc_profile_ticks(const ShardVramPtrs* vram, uint32_t padded_
   if (e == cudaSuccess)
     for (int i = 0; i < 7; i++) out_counts[i] = c1[i + 1] - c0[i + 1];
   for (int i = 0; i <= kTickStages; i++) cudaEventDestroy(ev[i]);
+  if (e != cudaSuccess) rows_touched(*s);
   return (int32_t)e;
 }
 

@@ -373,6 +373,7 @@ def run_gb300(args, dist: Dist) -> dict | None:
                      "algorithmic_bytes_per_launch": kb / prof_ticks,
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback"},
         "stage_ms_per_tick": {n: m / prof_ticks for n, m in zip(names, stage_ms)},
+        "stages_of": "kernel chain (the timed batches run in one launch)" if engine == 1 and small else "timed kernels",
         "tick_algorithmic_gbs": tick_bytes / (ms / 1e3) / 1e9,
         "per_tick": {"evaluated_slots": int(ctr[1]) / ticks_timed, "hits": int(ctr[2]) / ticks_timed,
                      "spikes": int(ctr[3]) / ticks_timed, "gsop_slots": int(ctr[4]) / ticks_timed,
@@ -846,6 +847,7 @@ def main():
             "roofline": r["roofline"],
             "tick_algorithmic_gbs": r["tick_algorithmic_gbs"],
             "stage_ms_per_tick": r["stage_ms_per_tick"],
+            "stages_of": r["stages_of"],
             "per_tick": r["per_tick"],
             "clocks": r["clocks"],
             "cpu_baseline": cpu,

@@ -343,8 +343,9 @@ void axc_io_pipeline_destroy(void* handle);
  * bitmask row k of the device array d_input_bitmask) without a graph, with
  * CUDA events recorded on `stream` around each stage.  engine 0: the
  * per-tick kernels of cu_step_day_phase; engine 1: the batch engine's
- * neuron-major kernels (the ticks then form one batch, rows built before and
- * weights written back after).  Sets out_ms[5] to the stage times in
+ * neuron-major kernels (the ticks then form one batch, on the rows that a batch
+ * would run on, weights written back after; as the kernel chain, also for a
+ * brain whose batches run in one launch).  Sets out_ms[5] to the stage times in
  * milliseconds: engine 0 network ids, axons, update, push, GSOP; engine 1
  * network ids, prologue, the 8-lane pass, the lit-sum pass (both with GSOP;
  * each returns at once on the other's ticks), fix-up and push; and out_counts[7] to

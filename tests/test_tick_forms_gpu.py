@@ -270,3 +270,24 @@ def test_learned_quiet_ticks_run_sparse(gpu, odd):
         N.lib().gpu_free(d_bits)
         vram.free()
         S.upload_lut(W.default_lut())
+
+
+def test_profiled_ticks_run_as_a_batch_does(gpu):
+    """axc_profile_ticks times the rows that a batch would run on: lit rows, not a layout of its own."""
+    r = Ring(600, 1024, 66)
+    ms, counts = (C.c_float * 5)(), (C.c_uint64 * 7)()
+    try:
+        for _ in range(8):
+            forms = r.run(False)
+        assert forms[LIT_ROWS] == 10, forms
+        r.vram.forms(reset=True)
+        err = N.lib().axc_profile_ticks(C.byref(r.vram.ptrs), r.n, r.A, 1, r.tick, 10, None, 0, 0, 0, 5, 1,
+                                        r.eng.stream, ms, counts)
+        assert err == 0 and ms[2] > 0
+        forms = r.vram.forms()
+        assert forms[LIT_ROWS] == 10 and forms[ONE_LAUNCH] == 0, forms
+        oracle.run_ticks(r.state, r.heads, r.lut, r.n, r.A, 1, r.tick, 10, None, 0, 0, 0, dopamine=5)
+        r.tick += 10
+        assert r.run(False)[LIT_ROWS] == 10
+    finally:
+        r.close()
