@@ -76,8 +76,9 @@ struct ShardCtl {
 // Inverted index of the row copy: per axon the row slots that target it
 // (n * 128 + row position), those of one segment together, for the sparse
 // form of a tick (row_engine.cuh).  The learned engine's: allocated when its
-// brain first turns quiet (4 bytes a slot; the batch and per-tick paths
-// allocate nothing beyond the row copy).
+// brain first turns quiet (576 bytes a neuron and axon, room for 128 slots a row
+// whatever it holds; the batch and per-tick paths allocate nothing beyond the row
+// copy).
 struct RowIndex {
   void* base = nullptr;
   uint32_t* off = nullptr;  // [A+1] first entry of an axon
@@ -85,7 +86,7 @@ struct RowIndex {
   uint32_t* bsum = nullptr; // scan block sums (build)
   uint16_t* seg = nullptr;  // [A][32] entries of an axon before segment s (s = 31: all segments >= 31);
                             // kSegUnsorted in [0]: too many entries, unsorted
-  uint32_t* ent = nullptr;  // [live slots]
+  uint32_t* ent = nullptr;  // [N * 128], the live slots first
 };
 
 // Neuron-major copy of the dendrites used by the batch engine for the length
@@ -295,7 +296,7 @@ cudaError_t launch_rows_end(const ShardVramPtrs& v, ShardScratch& s, uint32_t N,
 // so (as the chunk's own conditional layout would) and builds the index; else
 // nothing.
 cudaError_t rows_index_wish(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, uint32_t A, cudaStream_t stream,
-                            bool row_sum = false, bool with_posmap = true);
+                            bool row_sum, bool with_posmap);
 // The pinned word the device asks through.
 cudaError_t rows_wish_alloc(ShardScratch& s);
 

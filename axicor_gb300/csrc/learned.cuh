@@ -1055,7 +1055,7 @@ constexpr size_t kGateSnapBytes = offsetof(ShardCtl, slot_total) + sizeof(unsign
 static_assert(kGateSnapBytes == sizeof(GateSnap::before), "GateSnap mirrors ShardCtl::ctr .. slot_total");
 
 // Per chunk, before its graph: tick base, dopamine, and whether the chunk lays
-// its rows out anew (always on learned chunks: force).
+// its rows out anew (force: a call's first chunk, and after another path wrote the shard).
 __global__ void __launch_bounds__(512) k_learn_set_ctl(ShardCtl* ctl, uint32_t tick_base, int32_t dopamine,
                                                       uint32_t force, uint32_t ticks, const uint32_t* lit,
                                                       uint32_t A) {
@@ -1244,7 +1244,7 @@ static cudaError_t learned_tick(Learned& L, ShardScratch& s, uint32_t k, bool la
   const uint32_t G = std::max(A, N);
   const uint32_t raise = (bits_k && ((uint64_t)L.voff + L.nv > A)) ? AXC_ERR_VIRTUAL_RANGE : 0u;
   if (G)
-    k_rows_prologue<true><<<(G + 255) / 256, 256, 0, st>>>(L.v.axon_heads, A, L.v_seg, bits_k, L.voff,
+    k_rows_prologue<<<(G + 255) / 256, 256, 0, st>>>(L.v.axon_heads, A, L.v_seg, bits_k, L.voff,
                                                            bits_k ? L.nv : 0u, s.incoming, nullptr, k, r.mask2,
                                                            r.axw, L.v.soma_flags, L.v.timers, N, r.eval, s.ctl,
                                                            raise, r.lit, D, k > 0 ? s.pend : nullptr, r.xlit,
@@ -1254,8 +1254,7 @@ static cudaError_t learned_tick(Learned& L, ShardScratch& s, uint32_t k, bool la
                                         nullptr, nullptr, 0, ColWT{}, (volatile uint32_t*)s.h_counts_pinned);
   // soma pushes: by the next tick's prologue within a graph, here on its last tick
   if (last)
-    k_rows_push<<<2 * sms, 256, 0, st>>>(L.v.axon_heads, L.v.soma_to_axon, A, s.pend, r.eval, L.v.soma_flags, N,
-                                       nullptr, nullptr, 0, s.ctl, k);
+    k_rows_push<<<2 * sms, 256, 0, st>>>(L.v.axon_heads, L.v.soma_to_axon, A, s.pend, r.eval, L.v.soma_flags, s.ctl, k);
   if (features_on && L.T)
     k_learn_features<<<L.T, 128, 0, st>>>(D, L.v, N, r.cnt, L.fan, L.axn, L.hist, L.feat, L.pred, L.cap, L.part,
                                           L.wb, L.X, L.Y, L.nv ? L.stage + (size_t)(k + 1) * L.words : nullptr,

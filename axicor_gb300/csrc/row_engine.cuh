@@ -280,8 +280,10 @@ __device__ __forceinline__ bool sparse_tick(const ShardCtl* ctl, uint32_t k) {
 }
 
 // The inverted index matches the rows: it was built, from a layout with the
-// same targets at the same row positions.
-__device__ __forceinline__ bool index_ok(const ShardCtl* ctl) { return ctl->idx_ok && ctl->idx_sum == ctl->lay_sum; }
+// same targets at the same row positions (0: a layout without the checksum).
+__device__ __forceinline__ bool index_ok(const ShardCtl* ctl) {
+  return ctl->idx_ok && ctl->lay_sum != 0ull && ctl->idx_sum == ctl->lay_sum;
+}
 
 // Per-neuron GSOP constants (physics.cu:290-345).
 struct GsopConsts {
@@ -993,13 +995,12 @@ __device__ __forceinline__ uint32_t append_count(ShardCtl* ctl, uint32_t k, uint
 }
 
 // ---------------------------------------------------------------------------
-// per tick 1/4 of the learned engine (LEARN): axons (inject, network pushes,
+// per tick 1/4 of the learned engine's own graphs: axons (inject, network pushes,
 // propagate, split masks) and somas (refractory countdown, list of neurons to
 // evaluate), with learn_axons' per-tile activity and, on sparse ticks, the
 // compaction of the active axons.  The list entry positions are reserved once
 // per block.  The plain engine runs k_rows_prologue_plain.
 // ---------------------------------------------------------------------------
-template <bool LEARN>
 __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__ heads, uint32_t A, uint32_t v_seg,
                                                        const uint32_t* __restrict__ bitmask, uint32_t voff,
                                                        uint32_t nv, uint32_t* __restrict__ incoming,
@@ -1045,7 +1046,7 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     ctl->fix_overflow = 0;
   }
   bool lit = false, on = false;
-  uint32_t fan = 0, inflight = 0;   // LEARN: active synapses and heads in flight of axon i
+  uint32_t fan = 0, inflight = 0;   // active synapses and heads in flight of axon i
   if (i < A) {
     uint32_t h[8] = {hx.x, hx.y, hx.z, hx.w, hy.x, hy.y, hy.z, hy.w};
     uint32_t npush = ibit + pc;
@@ -1067,15 +1068,13 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
     // most one soma owns the axon, so for those segments the hit is 1 and one
     // push cannot change it
     lit = (m.x & own & kAxSegs) == (own & kAxSegs) && !(m.y >> 31);
-    if (LEARN) {
-      // active: some head covers a segment that a slot of the batch uses
-      on = ((m.x | (m.y & 0x7FFFFFFFu)) & act) != 0u;
-      if (on) fan = __ldg(L.inv_off + i + 1) - __ldg(L.inv_off + i);
+    // active: some head covers a segment that a slot of the batch uses
+    on = ((m.x | (m.y & 0x7FFFFFFFu)) & act) != 0u;
+    if (on) fan = __ldg(L.inv_off + i + 1) - __ldg(L.inv_off + i);
 #pragma unroll
-      for (int j = 0; j < 8; j++) inflight += h[j] < 255u + pmax ? 1u : 0u;
-    }
+    for (int j = 0; j < 8; j++) inflight += h[j] < 255u + pmax ? 1u : 0u;
   }
-  if (LEARN) learn_axons(L, i, A, fan, inflight);
+  learn_axons(L, i, A, fan, inflight);
   if (lit_bits) {
     const uint32_t lb = __ballot_sync(kFull, lit);
     if ((threadIdx.x & 31) == 0 && i < A) {
@@ -1096,8 +1095,8 @@ __global__ void __launch_bounds__(256) k_rows_prologue(BurstHeads8* __restrict__
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t ballot = __ballot_sync(kFull, ev), onb = __ballot_sync(kFull, on);
   if (lane == 0) {
-    if (LEARN && i < N) L.evbits[i >> 5] = evb[i >> 5] = ballot;
-    if (LEARN && i < A) live[i >> 5] = onb;
+    if (i < N) L.evbits[i >> 5] = evb[i >> 5] = ballot;
+    if (i < A) live[i >> 5] = onb;
     s_warp[w] = __popc(ballot);
     s_act[w] = __popc(onb);
   }
@@ -2713,8 +2712,7 @@ __global__ void __launch_bounds__(256) k_rows_fixup(ShardVramPtrs P, uint32_t N,
 // own-axon pushes (physics.cu:257-261), found in the evaluated list; on the
 // other ticks the next prologue applies them.
 __device__ __forceinline__ void rows_push(BurstHeads8* heads, const uint32_t* s2a, uint32_t A, uint32_t* pend,
-                                          const uint32_t* eval, const uint8_t* flags, uint32_t N, const uint32_t* ids,
-                                          uint8_t* out, uint32_t num_outputs, ShardCtl* ctl, uint32_t k) {
+                                          const uint32_t* eval, const uint8_t* flags, ShardCtl* ctl, uint32_t k) {
   const uint32_t ecount = ctl->eval_act[k & 1][0];
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2737,28 +2735,15 @@ __device__ __forceinline__ void rows_push(BurstHeads8* heads, const uint32_t* s2
     p[0] = make_uint4(h[0], h[1], h[2], h[3]);
     p[1] = make_uint4(h[4], h[5], h[6], h[7]);
   }
-  uint32_t err = 0;
-  for (uint32_t j = tid; j < num_outputs; j += stride) {
-    const uint32_t id = ids[j];
-    uint8_t v = 0;
-    if (id != AXC_NO_AXON) {
-      if (id < N) v = flags[id] & 0x01;
-      else err = AXC_ERR_READOUT_RANGE;
-    }
-    out[j] = v;
-  }
-  if (err) atomicOr(&ctl->err, err);
 }
 
 __global__ void __launch_bounds__(256) k_rows_push(BurstHeads8* __restrict__ heads, const uint32_t* __restrict__ s2a,
                                                    uint32_t A, uint32_t* __restrict__ pend,
                                                    const uint32_t* __restrict__ eval, const uint8_t* __restrict__ flags,
-                                                   uint32_t N, const uint32_t* __restrict__ ids,
-                                                   uint8_t* __restrict__ out, uint32_t num_outputs,
                                                    ShardCtl* __restrict__ ctl, uint32_t k) {
   chain_wait();
   chain_open();
-  rows_push(heads, s2a, A, pend, eval, flags, N, ids, out, num_outputs, ctl, k);
+  rows_push(heads, s2a, A, pend, eval, flags, ctl, k);
 }
 
 __global__ void k_rows_reset_lists(ShardCtl* ctl) {
@@ -3162,8 +3147,7 @@ __global__ void __launch_bounds__(1024, 1) k_rows_small(const __grid_constant__ 
     if ((nfix || spikes) && !small_barrier<CLUSTER>(ctl, target, tries, &s_ok)) return;
   }
   // the last tick's soma pushes
-  rows_push(b.P.axon_heads, b.P.soma_to_axon, b.A, b.pend, b.eval, b.P.soma_flags, b.N, nullptr, nullptr, 0u, ctl,
-            b.k0 + b.ticks - 1u);
+  rows_push(b.P.axon_heads, b.P.soma_to_axon, b.A, b.pend, b.eval, b.P.soma_flags, ctl, b.k0 + b.ticks - 1u);
 }
 
 }  // namespace
@@ -3458,7 +3442,7 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
   // the soma pushes: by the next tick's prologue within a batch, here on its last tick
   if (!a.defer_push)
     launch_chain(k_rows_push, dim3(8 * sms), dim3(256), 0, stream, pdl, v.axon_heads, v.soma_to_axon, A, s.pend,
-                 r.eval, v.soma_flags, N, (const uint32_t*)nullptr, (uint8_t*)nullptr, 0u, s.ctl, a.k);
+                 r.eval, v.soma_flags, s.ctl, a.k);
   if (ev) cudaEventRecord(ev[5], stream);
   return cudaGetLastError();
 }
