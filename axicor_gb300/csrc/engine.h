@@ -96,7 +96,7 @@ struct RowCache {
   void* base = nullptr;
   uint32_t* rt = nullptr;   // [N][128] targets, neuron-major
   int16_t* rw = nullptr;    // [N][128] weights, neuron-major
-  uint16_t* cnt = nullptr;  // [N] slots before the first empty target; bit 15: an invalid target
+  uint16_t* cnt = nullptr;  // [N] slots before the first empty target; bit 15: an invalid target, 14: split (kRowSplit)
   uint2* mask2 = nullptr;   // [A+1] split segment-hit masks (heads 0..6 | head 7); [A] dummy
   uint32_t* axw = nullptr;  // [A] owners and used segments of the axon (kAxOwned); population: somas that own it
   uint32_t* eval = nullptr; // [N] non-refractory neurons of the tick

@@ -99,6 +99,7 @@ __device__ __forceinline__ uint32_t used_segs(const ShardCtl* ctl, uint32_t cond
 }
 __device__ __forceinline__ uint32_t ax_owners(uint32_t axw) { return (axw & kAxOwned) + (axw >> 31); }
 constexpr uint32_t kRowBad = 0x8000u;    // cnt flag: the row holds an invalid target
+constexpr uint32_t kRowSplit = 0x4000u;  // cnt flag: its movable slots are in two groups (build_row), not in slot order
 
 // Bytes of the fully-lit bitmap of A axons as staged in shared memory (one
 // bit per axon and a spare word, rounded up to the bulk copy's 16 bytes; the
@@ -658,7 +659,7 @@ __device__ __forceinline__ RowBuilt build_row(const SlotStage& st, uint32_t j, u
     am[ch] = permute ? (lf >= lo + 32u ? kFull : (lf > lo ? (1u << (lf - lo)) - 1u : 0u)) : mv[ch];
   }
   if (lane == 0) {
-    cnt[n] = (uint16_t)(c | (bad ? kRowBad : 0u));
+    cnt[n] = (uint16_t)(c | (bad ? kRowBad : 0u) | (lm > 0u && lm < lf ? kRowSplit : 0u));
     amask[n] = make_uint4(am[0], am[1], am[2], am[3]);
     omask[n] = permute ? make_uint4(mv[0], mv[1], mv[2], mv[3]) : make_uint4(all[0], all[1], all[2], all[3]);
     if (lmask) lmask[n] = permute ? make_uint4(g0[0], g0[1], g0[2], g0[3]) : make_uint4(all[0], all[1], all[2], all[3]);
@@ -717,7 +718,7 @@ __device__ __forceinline__ void writeback_tile(int16_t* __restrict__ weights, ui
 // an invalid target) is movable; weights only freeze, so the marks hold for the whole
 // batch.  The dendrite sum (a wrapping i32 sum) and GSOP (per slot) do not depend on the
 // order of a row.
-// Per neuron: cnt = used slots (| kRowBad), lfz = movable slots, amask = their
+// Per neuron: cnt = used slots (| kRowBad | kRowSplit), lfz = movable slots, amask = their
 // row positions, omask = the columnar slots placed first (read by the
 // write-back; every used slot when the row keeps the columnar order).
 constexpr int kBuildBlocks = 4;
@@ -852,25 +853,30 @@ __global__ void __launch_bounds__(256) k_rows_mult(const uint32_t* __restrict__ 
 // then the others of omask[n] are the row's first positions, the only slots
 // whose weights GSOP can have changed.  Two kernels, one of which returns at once: a
 // thread per neuron where the rows have few such slots (a neuron without any, every
-// one of a frozen row, costs one 16-byte load; 8M settled neurons: 66 us, 176 through
-// the tiles' registers and shared memory), else tiles of 32 neurons: rows read whole,
-// columns written 64 bytes a warp (512k plastic neurons: 100 us against 228).
+// one of a frozen row, costs one 16-byte load and two bytes of cnt, and lmask is read
+// of split rows only; 8M settled neurons: 76 us, 88 with lmask read of every row that
+// moves, 176 through the tiles' registers and shared memory), else tiles of 32
+// neurons: rows read whole, columns written 64 bytes a warp (512k plastic neurons: 100
+// us against 228).
 __device__ __forceinline__ bool writeback_tiled(const ShardCtl* ctl, uint32_t N) {
   return ctl->mov_total + ctl->pfx_total > 24ull * N;
 }
 
 __global__ void __launch_bounds__(256) k_rows_writeback(int16_t* __restrict__ weights, uint32_t N,
                                                         const int16_t* __restrict__ rw,
+                                                        const uint16_t* __restrict__ cnt,
                                                         const uint4* __restrict__ omask,
                                                         const uint4* __restrict__ lmask,
                                                         const ShardCtl* __restrict__ ctl, uint32_t* __restrict__ pend,
                                                         uint32_t* __restrict__ incoming, uint32_t A) {
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint4 om = n < N ? omask[n] : make_uint4(0, 0, 0, 0);   // asked for beside the control block
+  const uint32_t cw = n < N ? cnt[n] : 0u;
+  const bool tiled = writeback_tiled(ctl, N);
   if (ctl->gave_up)   // pushes of ticks that never ended
     for (uint32_t a = n; a < A; a += gridDim.x * blockDim.x) pend[a] = incoming[a] = 0u;
-  const uint4 om = n < N ? omask[n] : make_uint4(0, 0, 0, 0);   // asked for beside the control block
-  if (writeback_tiled(ctl, N) || !(om.x | om.y | om.z | om.w)) return;
-  const uint4 lm = lmask[n];
+  if (tiled || !(om.x | om.y | om.z | om.w)) return;
+  const uint4 lm = cw & kRowSplit ? lmask[n] : make_uint4(0, 0, 0, 0);   // else one run, in slot order
   const uint32_t o[4] = {om.x, om.y, om.z, om.w}, x[4] = {lm.x, lm.y, lm.z, lm.w};
   const int16_t* row = rw + (size_t)n * kRowStride;
   uint32_t k = 0;
@@ -3752,8 +3758,8 @@ cudaError_t rows_index_wish(const ShardVramPtrs& v, ShardScratch& s, uint32_t N,
 cudaError_t launch_rows_end(const ShardVramPtrs& v, ShardScratch& s, uint32_t N, cudaStream_t stream) {
   RowCache& r = *s.rows;
   const uint32_t blocks = std::max(1u, (N + 255) / 256), tiles = std::max(1u, (N + 31) / 32);
-  k_rows_writeback<<<blocks, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.omask, r.lmask, s.ctl, s.pend, s.incoming,
-                                               s.total_axons);
+  k_rows_writeback<<<blocks, 256, 0, stream>>>(v.dendrite_weights, N, r.rw, r.cnt, r.omask, r.lmask, s.ctl, s.pend,
+                                               s.incoming, s.total_axons);
   k_rows_writeback_tiles<<<std::min(tiles, 4u * (uint32_t)sm_count()), 256, 0, stream>>>(v.dendrite_weights, N, r.rw,
                                                                                          r.omask, r.lmask, s.ctl);
   return cudaGetLastError();

@@ -291,3 +291,18 @@ def test_profiled_ticks_run_as_a_batch_does(gpu):
         assert r.run(False)[LIT_ROWS] == 10
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("slots", [21, 23, 60])   # write-back by a thread a neuron (two), in tiles
+def test_write_back_of_split_rows(gpu, slots):
+    """Movable slots on lit axons laid before one on a dark axon, in every second row: each weight back in its slot."""
+    r = Ring(608, 704, slots)
+    try:
+        sv = StateView(r.state, r.n)
+        sv.targets[7, ::2] = (2 << 24) | 700   # an axon that no soma owns
+        r.vram.upload_state(r.state)
+        for _ in range(8):
+            forms = r.run(False)
+        assert forms[LIT_ROWS] > 0, forms
+    finally:
+        r.close()
