@@ -194,11 +194,13 @@ namespace axc {
 // Prepares one shard for a batch (shard.rs:40-71): scratch and row cache, then
 // on `stream` the bulk H2D of the batch's inputs, the batch's tick base and
 // dopamine, and the burst-counter reset.  *out_rows: the kernels the batch runs
-// (1 the neuron-major row engine, 0 the columnar per-tick kernels).
+// (1 the neuron-major row engine, 0 the columnar per-tick kernels).  *out_s is set
+// on an error too: the caller marks the rows out of date (batch_undone).
 cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* out_rows, cudaStream_t stream) {
   cudaError_t e;
   ShardScratch* s = scratch_for(b.vram, b.padded_n, b.total_axons, &e);
   if (!s) return e;
+  *out_s = s;
   s->tick_rows_valid.store(false);   // the batch's row copy replaces the per-tick entry point's
   // Captured graphs hold the addresses of the scratch buffers: any
   // reallocation below drops them.
@@ -240,7 +242,6 @@ cudaError_t batch_prepare(const BatchArgs& b, ShardScratch** out_s, uint32_t* ou
   // burst-counter reset before the batch (shard.rs:71)
   e = launch_reset_burst(*b.vram, b.padded_n, stream);
   if (e != cudaSuccess) return e;
-  *out_s = s;
   *out_rows = rows;
   return cudaSuccess;
 }
@@ -288,33 +289,22 @@ cudaError_t batch_capture(const BatchArgs& b, ShardScratch& s, uint32_t rows, ui
   return le;
 }
 
-}  // namespace axc
-
-extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t total_axons,
-                                            uint32_t sync_batch_ticks, const AxcIoBuffers* io,
-                                            const uint32_t* h_input_bitmask, const uint32_t* h_incoming_spikes,
-                                            const uint32_t* h_spike_counts, uint32_t virtual_offset,
-                                            uint32_t num_virtual_axons, const uint32_t* mapped_soma_ids_device,
-                                            uint32_t v_seg, int16_t dopamine, uint32_t tick_base,
-                                            uint8_t* h_output_history, void* stream_v) {
-  if (!vram || !io) return (int32_t)cudaErrorInvalidValue;
-  if (sync_batch_ticks == 0) return 0;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  const BatchArgs b{vram, padded_n, total_axons, sync_batch_ticks, io, h_input_bitmask, h_incoming_spikes,
-                    h_spike_counts, virtual_offset, num_virtual_axons, mapped_soma_ids_device, v_seg, dopamine,
-                    tick_base};
-  ShardScratch* s = nullptr;
+// The batch; *out_s the shard's scratch, on an error too.
+static cudaError_t batch_step(const BatchArgs& b, uint8_t* h_output_history, ShardScratch** out_s,
+                              cudaStream_t stream) {
+  const AxcIoBuffers* io = b.io;
   uint32_t rows = 0;
-  cudaError_t e = batch_prepare(b, &s, &rows, stream);
-  if (e != cudaSuccess) return (int32_t)e;
+  cudaError_t e = batch_prepare(b, out_s, &rows, stream);
+  if (e != cudaSuccess) return e;
+  ShardScratch* s = *out_s;
 
   // the tick loop, as one graph (shard.rs:75-120), captured once per shape
   const uint32_t words = io->input_words_per_tick;
   // a cluster leaves the other SMs free: one shape of those sizes
-  const uint32_t whole = !rows || rows_small(padded_n, total_axons, false, true) || !others_running(*s, stream);
-  GraphKey key{padded_n, total_axons, sync_batch_ticks, virtual_offset, num_virtual_axons, v_seg,
+  const uint32_t whole = !rows || rows_small(b.padded_n, b.total_axons, false, true) || !others_running(*s, stream);
+  GraphKey key{b.padded_n, b.total_axons, b.ticks, b.voff, b.nv, b.v_seg,
                io->max_spikes_per_tick, words, io->num_outputs, rows, g_fix_cap.load(), whole, io->d_input_bitmask,
-               io->d_incoming_spikes, io->d_output_history, mapped_soma_ids_device};
+               io->d_incoming_spikes, io->d_output_history, b.ids};
   if (!s->graph_cache) s->graph_cache = new GraphCache();
   GraphCache* gc = static_cast<GraphCache*>(s->graph_cache);
   cudaGraphExec_t exec = nullptr;
@@ -326,11 +316,11 @@ extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t 
     } else {
       if (!gc->capture) {
         e = cudaStreamCreateWithFlags(&gc->capture, cudaStreamNonBlocking);
-        if (e != cudaSuccess) return (int32_t)e;
+        if (e != cudaSuccess) return e;
       }
       for (const bool one_launch : {true, false}) {
         e = cudaStreamBeginCapture(gc->capture, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return (int32_t)e;
+        if (e != cudaSuccess) return e;
         const cudaError_t le = batch_capture(b, *s, rows, key.fix_cap, gc->capture, whole != 0u, one_launch);
         cudaGraph_t graph = nullptr;
         e = cudaStreamEndCapture(gc->capture, &graph);
@@ -340,20 +330,40 @@ extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t 
         if (!launch_refused(e)) break;
         cudaGetLastError();   // not the second capture's
       }
-      if (e != cudaSuccess) return (int32_t)e;
+      if (e != cudaSuccess) return e;
       gc->execs[key] = exec;
     }
   }
   e = cudaGraphLaunch(exec, stream);
-  if (e != cudaSuccess) return (int32_t)e;
+  if (e != cudaSuccess) return e;
   work_started(*s, stream);
 
   // outputs (shard_thread.rs:208-227)
   if (h_output_history && io->d_output_history && io->num_outputs) {
-    e = cudaMemcpyAsync(h_output_history, io->d_output_history, (size_t)io->num_outputs * sync_batch_ticks,
+    e = cudaMemcpyAsync(h_output_history, io->d_output_history, (size_t)io->num_outputs * b.ticks,
                         cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
   }
+  return e;
+}
+
+}  // namespace axc
+
+extern "C" int32_t axc_step_day_phase_batch(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t total_axons,
+                                            uint32_t sync_batch_ticks, const AxcIoBuffers* io,
+                                            const uint32_t* h_input_bitmask, const uint32_t* h_incoming_spikes,
+                                            const uint32_t* h_spike_counts, uint32_t virtual_offset,
+                                            uint32_t num_virtual_axons, const uint32_t* mapped_soma_ids_device,
+                                            uint32_t v_seg, int16_t dopamine, uint32_t tick_base,
+                                            uint8_t* h_output_history, void* stream_v) {
+  if (!vram || !io) return (int32_t)cudaErrorInvalidValue;
+  if (sync_batch_ticks == 0) return 0;
+  const BatchArgs b{vram, padded_n, total_axons, sync_batch_ticks, io, h_input_bitmask, h_incoming_spikes,
+                    h_spike_counts, virtual_offset, num_virtual_axons, mapped_soma_ids_device, v_seg, dopamine,
+                    tick_base};
+  ShardScratch* s = nullptr;
+  const cudaError_t e = batch_step(b, h_output_history, &s, static_cast<cudaStream_t>(stream_v));
+  if (e != cudaSuccess) batch_undone(s);
   return (int32_t)e;
 }
 

@@ -319,6 +319,11 @@ inline void rows_touched(ShardScratch& s) {
   s.tick_rows_valid.store(false);
   s.batch_rows_valid.store(false);
 }
+// A batch or run that returned an error may not have made the layout that it was to
+// make (batch_rows_force counts it as made): the next one makes it.
+inline void batch_undone(ShardScratch* s) {
+  if (s) rows_touched(*s);
+}
 // Marks every shard whose .state allocation overlaps [dst, dst + size).
 void invalidate_overlapping(const void* dst, size_t size);
 // Looks up a shard's scratch without creating it (nullptr if none).

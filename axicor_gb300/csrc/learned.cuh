@@ -1560,6 +1560,7 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
     if (e != cudaSuccess) break;
     if (picked1 == picked0) L->gate_left = kGateChunks;
   }
+  if (e != cudaSuccess) batch_undone(s);
   return (int32_t)e;
 }
 

@@ -65,27 +65,14 @@ constexpr size_t kMaxZoneGraphs = 64;
 }  // namespace
 }  // namespace axc
 
-using namespace axc;
+namespace axc {
 
-extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nshards, const AxcGhostRoute* routes,
-                                       uint32_t nroutes, uint32_t sync_batch_ticks, uint32_t tick_base,
-                                       void* stream_v) {
-  if ((!shards && nshards) || (!routes && nroutes)) return (int32_t)cudaErrorInvalidValue;
-  if (nshards == 0 || sync_batch_ticks == 0) return 0;
-  for (uint32_t i = 0; i < nshards; i++) {
-    if (!shards[i].vram.axon_heads) return (int32_t)cudaErrorInvalidValue;
-    for (uint32_t j = 0; j < i; j++)
-      if (shards[j].vram.axon_heads == shards[i].vram.axon_heads) return (int32_t)cudaErrorInvalidValue;
-  }
-  for (uint32_t r = 0; r < nroutes; r++)
-    if (routes[r].src_shard >= nshards || routes[r].dst_shard >= nshards ||
-        (routes[r].count && (!routes[r].d_src_indices || !routes[r].d_dst_indices)))
-      return (int32_t)cudaErrorInvalidValue;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-
+// The zone's batch; scr: the shards' scratch, on an error too.
+static cudaError_t zone_step(const AxcZoneShard* shards, uint32_t nshards, const AxcGhostRoute* routes,
+                             uint32_t nroutes, uint32_t sync_batch_ticks, uint32_t tick_base,
+                             std::vector<ShardScratch*>& scr, cudaStream_t stream) {
   // per-batch inputs of every shard, on the caller's stream
   std::vector<BatchArgs> args(nshards);
-  std::vector<ShardScratch*> scr(nshards);
   std::vector<uint32_t> rows(nshards);
   for (uint32_t i = 0; i < nshards; i++) {
     const AxcZoneShard& z = shards[i];
@@ -93,7 +80,7 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
                         z.h_incoming_spikes, z.h_spike_counts, z.virtual_offset, z.num_virtual_axons,
                         z.mapped_soma_ids_device, z.v_seg, z.dopamine, tick_base};
     cudaError_t e = batch_prepare(args[i], &scr[i], &rows[i], stream);
-    if (e != cudaSuccess) return (int32_t)e;
+    if (e != cudaSuccess) return e;
   }
 
   // the graph of this zone shape: every pointer a captured node holds is in the key
@@ -133,10 +120,10 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
       c.execs.clear();
     }
     e = ensure_streams(c, nshards);
-    if (e != cudaSuccess) return (int32_t)e;
+    if (e != cudaSuccess) return e;
     for (const bool one_launch : {true, false}) {
       e = cudaStreamBeginCapture(c.root, cudaStreamCaptureModeThreadLocal);
-      if (e != cudaSuccess) return (int32_t)e;
+      if (e != cudaSuccess) return e;
       cudaError_t le = cudaEventRecord(c.events[0], c.root);
       // fork: every shard's tick loop on its own branch
       for (uint32_t i = 0; i < nshards && le == cudaSuccess; i++) {
@@ -160,11 +147,11 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
       if (!launch_refused(e)) break;
       cudaGetLastError();   // not the second capture's
     }
-    if (e != cudaSuccess) return (int32_t)e;
+    if (e != cudaSuccess) return e;
     c.execs[key] = exec;
   }
   e = cudaGraphLaunch(exec, stream);
-  if (e != cudaSuccess) return (int32_t)e;
+  if (e != cudaSuccess) return e;
   work_started(*scr[0], stream);
 
   // outputs (shard_thread.rs:208-227)
@@ -178,5 +165,31 @@ extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nsha
     }
   }
   if (e == cudaSuccess && wait) e = cudaStreamSynchronize(stream);
+  return e;
+}
+
+}  // namespace axc
+
+using namespace axc;
+
+extern "C" int32_t axc_step_zone_batch(const AxcZoneShard* shards, uint32_t nshards, const AxcGhostRoute* routes,
+                                       uint32_t nroutes, uint32_t sync_batch_ticks, uint32_t tick_base,
+                                       void* stream_v) {
+  if ((!shards && nshards) || (!routes && nroutes)) return (int32_t)cudaErrorInvalidValue;
+  if (nshards == 0 || sync_batch_ticks == 0) return 0;
+  for (uint32_t i = 0; i < nshards; i++) {
+    if (!shards[i].vram.axon_heads) return (int32_t)cudaErrorInvalidValue;
+    for (uint32_t j = 0; j < i; j++)
+      if (shards[j].vram.axon_heads == shards[i].vram.axon_heads) return (int32_t)cudaErrorInvalidValue;
+  }
+  for (uint32_t r = 0; r < nroutes; r++)
+    if (routes[r].src_shard >= nshards || routes[r].dst_shard >= nshards ||
+        (routes[r].count && (!routes[r].d_src_indices || !routes[r].d_dst_indices)))
+      return (int32_t)cudaErrorInvalidValue;
+  std::vector<ShardScratch*> scr(nshards, nullptr);
+  const cudaError_t e =
+      zone_step(shards, nshards, routes, nroutes, sync_batch_ticks, tick_base, scr, static_cast<cudaStream_t>(stream_v));
+  if (e != cudaSuccess)
+    for (ShardScratch* s : scr) batch_undone(s);
   return (int32_t)e;
 }

@@ -4,6 +4,8 @@ The columnar kernels (axc_batch_engine_mode(0), axc_tick_engine_mode(0)) move th
 (physics.cu:281-373), so a row copy that the batch path or the per-tick entry point kept is out of date after
 them.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -120,3 +122,52 @@ def test_another_state_allocation_behind_the_same_heads(gpu):
     finally:
         t.vram.free()
         other.free()
+
+
+@pytest.mark.parametrize("zone", [False, True])
+def test_a_batch_that_returned_an_error(gpu, zone):
+    """The layout that a batch was to make is made by the next one when the batch failed before its ticks: here it is
+    refused because its stream is being captured and it is to wait for its readout."""
+    lib, cu = N.lib(), C.CDLL("libcuda.so.1")
+    w = W.small(dims=(16, 16, 8), slots=40, inputs=64, p=0.2)
+    t = BatchTwin(w, frozen=False)
+    io, out = S.IoDeviceBuffers(t.words, 0, 32, 10), np.zeros(320, np.uint8)
+    d_ids = S.device_array(np.arange(32, dtype=np.uint32))
+    bm = S.input_bitmask(w.seed, 0, 10, w.num_inputs, w.rate_q32)
+    stream, graph = C.c_void_p(), C.c_void_p()
+    args = (t.N, t.A, io.as_struct(), N.ptr(bm), t.lay.virtual_offset, w.num_inputs)
+    try:
+        t.batch(10)
+        rng = np.random.default_rng(3)   # other targets: the rows are out of date
+        sv = StateView(t.h_state, t.N)
+        sv.targets[:40] = sv.targets[:40][:, rng.permutation(t.N)]
+        t.vram.upload_state(t.h_state)
+        lib.gpu_device_synchronize()
+        assert cu.cuStreamCreate(C.byref(stream), 1) == 0
+        assert cu.cuStreamBeginCapture_v2(stream, 2) == 0
+        if zone:
+            z = N.AxcZoneShard()
+            z.vram, z.padded_n, z.total_axons, z.io, z.h_input_bitmask, z.virtual_offset, z.num_virtual_axons = (
+                t.vram.ptrs, *args)
+            z.mapped_soma_ids_device, z.v_seg, z.h_output_history = d_ids, 1, N.ptr(out)
+            err = lib.axc_step_zone_batch(C.byref(z), 1, None, 0, 10, t.tick, stream)
+        else:
+            err = lib.axc_step_day_phase_batch(C.byref(t.vram.ptrs), t.N, t.A, 10, C.byref(args[2]), N.ptr(bm), None,
+                                               None, t.lay.virtual_offset, w.num_inputs, d_ids, 1, 0, t.tick,
+                                               N.ptr(out), stream)
+        assert err != 0
+        cu.cuStreamEndCapture(stream, C.byref(graph))   # (an error: the capture is void)
+        assert np.array_equal(t.vram.download_state(), t.h_state), "nothing ran"
+        try:
+            t.batch(10)
+        except RuntimeError:
+            pass   # the runtime hands the error out once more
+        t.batch(10)
+        t.batch(10)
+    finally:
+        if graph:
+            cu.cuGraphDestroy(graph)
+        if stream:
+            cu.cuStreamDestroy_v2(stream)
+        lib.gpu_free(d_ids)
+        t.vram.free()
