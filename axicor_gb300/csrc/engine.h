@@ -65,7 +65,9 @@ struct ShardCtl {
   uint32_t mixed_len;     // row engine: a neuron with slots has another signal_propagation_length than pmax
   uint32_t streak;        // row engine: consecutive ticks that the sparse form could have run (sparse_tick)
   uint32_t idx_ok;        // row engine: an inverted index was built (it holds while idx_sum == lay_sum)
-  uint32_t pad3;
+  uint32_t busy;          // row engine: consecutive ticks that it could not have run, up to kBusyStreak
+  uint32_t ix_run;        // row engine: the graph that runs has the sparse form's kernels
+  uint32_t busy_told;     // row engine: the host's pinned word says that busy reached kBusyStreak
   unsigned long long lay_sum, idx_sum;  // row engine: checksum of the rows' targets by position; the index's rows'
   const uint32_t* ix_off; // inverted index of the rows (RowIndex)
   const uint16_t* ix_seg;
@@ -133,7 +135,8 @@ struct ShardScratch {
   ShardCtl* ctl = nullptr;
   uint32_t* batch_counts = nullptr;  // [batch_cap] per-tick network spike counts
   uint32_t batch_cap = 0;
-  uint32_t* h_counts_pinned = nullptr;  // pinned: [0] the device asks for an inverted index (RowIndex)
+  uint32_t* h_counts_pinned = nullptr;  // pinned: [0] the device asks for an inverted index (RowIndex), [1] busy_told
+  bool ix_run = false;                  // ShardCtl::ix_run as last set
   void* graph_cache = nullptr;          // batch engine graphs (batch_engine.cu)
   RowCache* rows = nullptr;             // batch engine neuron-major dendrites
   // Per-tick entry point (cu_step_day_phase): its row cache lives across calls.
@@ -349,7 +352,8 @@ struct TickArgs {
   uint32_t fix_cap;           // row engine: deferred-GSOP list capacity (<= kFixCap)
   bool lit_new;               // row engine: the window of always-lit axons (RowCache::alit) starts at this tick
   bool shared_gpu;            // row engine: other shards' ticks run beside this one's
-  bool index;                 // row engine: the tick may run its sparse form (the learned engine's plain graph)
+  bool index;                 // row engine: count active axons, for the sparse form (the learned engine's plain graph)
+  bool sparse;                // row engine: and launch its kernels
   bool defer_push;            // row engine: leave this tick's soma pushes to the next tick's prologue
                               // (never on the last tick of a batch)
 };

@@ -1114,7 +1114,7 @@ struct Learned {
   cudaEvent_t gate_ev[2] = {nullptr, nullptr};
   bool gate_pend[2] = {false, false};
   const void* rows_base = nullptr;   // the row cache the graphs were captured with
-  std::map<std::tuple<uint32_t, uint32_t>, cudaGraphExec_t> graphs;
+  std::map<std::tuple<uint32_t, uint32_t, bool>, cudaGraphExec_t> graphs;
   cudaStream_t capture = nullptr;
 
   LearnDev dev() const {
@@ -1221,7 +1221,8 @@ static void learned_update_forms(Learned& L, ShardScratch& s, uint32_t k, cudaSt
   // (the 8-lane pass, or the lit-sum form when its lit set held)
   launch_rows_update(L.v, s, N, A, k, fix_cap, L.ctl, st, ColWT{}, false, true);
   launch_rows_lsum(L.v, s, A, k, fix_cap, L.ctl, st);
-  launch_rows_sparse(L.v, s, N, A, k, fix_cap, L.ctl, st);
+  // the sparse form, where an index was built
+  if (r.ix.base) launch_rows_sparse(L.v, s, N, A, k, fix_cap, L.ctl, st);
   // sparse: the axon-driven gather, GLIF, and GSOP of the spikers it listed
   k_learn_scatter<<<8 * sms, 256, ((size_t)L.T + 1) * 4, st>>>(D, L.T, L.inv, L.inv_seg, r.mask2, r.rw, r.posmap,
                                                                 L.v.soma_flags, L.v.axon_heads, A, L.acc, s.ctl);
@@ -1451,9 +1452,10 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
   }
   const bool features_on = L->policy < 0 || L->collect;
   // graph kinds: 0/1 learned (features off/on), 2 plain (the gate); the row
-  // layout of each chunk follows the device's decision (layout_decide)
-  auto graph_of = [&](uint32_t kind, cudaGraphExec_t* out) -> cudaError_t {
-    const auto key = std::make_tuple(tpg, kind);
+  // layout of each chunk follows the device's decision (layout_decide).  sparse: with
+  // the sparse form's kernels
+  auto graph_of = [&](uint32_t kind, bool sparse, cudaGraphExec_t* out) -> cudaError_t {
+    const auto key = std::make_tuple(tpg, kind, sparse);
     auto it = L->graphs.find(key);
     if (it != L->graphs.end()) {
       *out = it->second;
@@ -1479,6 +1481,7 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
         a.defer_push = k + 1 < tpg;
         a.fix_cap = kFixCap;
         a.index = true;
+        a.sparse = sparse;
         a.lit_new = k == (tpg > kLitWindow ? tpg - kLitWindow : 0u);
         le = launch_tick(L->v, *s, a, L->capture);
       } else {
@@ -1518,9 +1521,6 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
     // them out without the position map since); later chunks keep them as the
     // batch path does
     const bool force = batch_rows_force(*s) || c == 0;
-    cudaGraphExec_t exec = nullptr;
-    e = graph_of(gated ? 2u : (features_on ? 1u : 0u), &exec);
-    if (e != cudaSuccess) break;
     if (L->bits) {
       const uint32_t have = std::min(tpg + 1, L->bits_ticks - t0);
       e = cudaMemcpyAsync(L->stage, L->bits + (size_t)t0 * L->words, (size_t)have * L->words * 4,
@@ -1532,6 +1532,16 @@ int32_t axc_learned_run(void* handle, uint32_t tick0, uint32_t ticks, uint32_t t
     k_learn_set_ctl<<<1, 512, 0, st>>>(s->ctl, L->tick_base + t0, (int32_t)L->dopamine, force ? 1u : 0u, tpg,
                                        s->rows->alit, L->A);
     e = rows_index_wish(L->v, *s, L->N, L->A, st, true, true);
+    cudaGraphExec_t exec = nullptr;
+    // The sparse form's kernels need the index; the gate's graphs go without them while
+    // the brain is busy (kBusyStreak).  The device is told, so that no tick takes a form
+    // whose kernels are not there.
+    const bool sparse = s->rows->ix.base && !(gated && ((volatile uint32_t*)s->h_counts_pinned)[1]);
+    if (e == cudaSuccess) e = graph_of(gated ? 2u : (features_on ? 1u : 0u), sparse, &exec);
+    if (e == cudaSuccess && sparse != s->ix_run) {
+      e = cudaMemsetAsync(&s->ctl->ix_run, sparse ? 1 : 0, 4, st);
+      if (e == cudaSuccess) s->ix_run = sparse;
+    }
     if (e == cudaSuccess) e = launch_reset_burst(L->v, L->N, st);
     unsigned long long picked0 = 0, picked1 = 0;
     const size_t picked_at = offsetof(LearnCtl, stat) + kStSparsePicked * sizeof(unsigned long long);

@@ -258,17 +258,13 @@ struct ColRun {
 // oldest heads on) the rows are checked slot by slot (kFormVerify), with many, or in
 // rows of up to 32 slots, by the dense pass (504,000 plastic neurons, 32 slots: 31.7 us
 // a tick against 36.8 checked; tick_form has the other sizes).  Every thread
-// of both update kernels asks at its start; the three words were written by
-// earlier kernels and no kernel that asks writes them, so plain loads (cached
-// in L1 after the first warp of an SM) serve it: uncached loads sent every
+// of both update kernels asks at its start; the words were written by
+// earlier kernels and no kernel that asks writes them, so cached loads (in
+// L1 after the first warp of an SM) serve it: uncached loads sent every
 // warp's request to the one L2 slice that holds the control block, a few
 // microseconds per launch.
-__device__ __forceinline__ bool lit_layout(const ShardCtl* ctl) {
-  const unsigned long long p = ctl->pfx_total, c = ctl->slot_total;
-  return c > 0 && p * 8ull <= c;
-}
-__device__ __forceinline__ bool lsum_tick(const ShardCtl* ctl, uint32_t k) {
-  return lit_layout(ctl) && ctl->dense[k & 1] == 0u;
+__device__ __forceinline__ bool lit_layout(unsigned long long tested, unsigned long long slots) {
+  return slots > 0 && tested * 8ull <= slots;
 }
 
 // The sparse form can run tick k: fewer than half as many axons have a head on
@@ -276,15 +272,15 @@ __device__ __forceinline__ bool lsum_tick(const ShardCtl* ctl, uint32_t k) {
 // slot of the evaluated neurons (~4.5 ns a thousand slots at 1.5M neurons), the
 // sparse form walks the hit segments' entries of the active axons.  The two
 // words were written by the prologue.
-__device__ __forceinline__ bool sparse_tick(const ShardCtl* ctl, uint32_t k) {
-  return ctl->eval_act[k & 1][1] * 2u < ctl->eval_act[k & 1][0];
-}
+__device__ __forceinline__ bool sparse_tick(uint32_t eval, uint32_t active) { return active * 2u < eval; }
 
 // The inverted index matches the rows: it was built, from a layout with the
 // same targets at the same row positions (0: a layout without the checksum).
-__device__ __forceinline__ bool index_ok(const ShardCtl* ctl) {
+__device__ __forceinline__ bool index_built(const ShardCtl* ctl) {
   return ctl->idx_ok && ctl->lay_sum != 0ull && ctl->idx_sum == ctl->lay_sum;
 }
+// And this graph can use it.
+__device__ __forceinline__ bool index_ok(const ShardCtl* ctl) { return ctl->ix_run && index_built(ctl); }
 
 // Per-neuron GSOP constants (physics.cu:290-345).
 struct GsopConsts {
@@ -405,7 +401,7 @@ constexpr int kCountSmall = 6, kCountLayout = 7;   // forms[]: ticks inside k_ro
 __device__ __forceinline__ void count_form(ShardCtl* ctl, int form) { atomicAdd(&ctl->forms[form], 1ull); }
 
 // The control words are read at once (volatile, so that no load waits behind the
-// branch on another) through L1, as lsum_tick's comment says.
+// branch on another) through L1, as lit_layout's comment says.
 __device__ __forceinline__ unsigned long long ctl_ld64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(v) : "l"(p));
@@ -431,11 +427,11 @@ __device__ __forceinline__ TickForm tick_form(const ShardCtl* ctl, uint32_t k, u
   const unsigned long long p = ctl_ld64(&ctl->pfx_total), c = ctl_ld64(&ctl->slot_total), m = ctl_ld64(&ctl->mov_total);
   const uint32_t dark = ctl_ld32(&ctl->dense[k & 1]), smax = ctl_ld32(&ctl->row_smax);
   if (lc && lc->mode == 1u && !lc->overflow) return index_ok(ctl) ? kFormSparse : kFormScatter;
-  if (c > 0 && p * 8ull <= c) {
+  if (lit_layout(p, c)) {
     if (!dark) return (m + p) * 16ull > c ? kFormLitRows : kFormLitSum;
     return smax > 32u && (unsigned long long)dark * smax * kDarkRows <= A ? kFormVerify : kFormDense;
   }
-  return index && index_ok(ctl) && sparse_tick(ctl, k) ? kFormSparse : kFormDense;
+  return index && index_ok(ctl) && sparse_tick(ctl->eval_act[k & 1][0], ctl->eval_act[k & 1][1]) ? kFormSparse : kFormDense;
 }
 
 // 64-bit mix of one live slot for the targets checksum (order-independent sum).
@@ -649,7 +645,7 @@ __device__ __forceinline__ RowBuilt build_row(const SlotStage& st, uint32_t j, u
       p3 += __popc(g3);
     }
     if (q < c) {
-      if (want_sum) psum += slot_mix(t[ch], n * kRowStride + pos);
+      if (want_sum && moved) psum += slot_mix(t[ch], n * kRowStride + pos);
       rt[(size_t)n * kRowStride + pos] = t[ch];
       rw[(size_t)n * kRowStride + pos] = w[ch];
       if (posmap) posmap[(size_t)n * kRowStride + q] = (uint8_t)pos;
@@ -666,7 +662,7 @@ __device__ __forceinline__ RowBuilt build_row(const SlotStage& st, uint32_t j, u
     lfz[n] = (uint8_t)lf;
     if (rec) rec[n] = make_int2((int32_t)rsum, (int32_t)(lm | (lf << 8) | (end << 16)));
   }
-  if (want_sum) psum = warp_sum(psum);
+  if (want_sum) psum = moved ? warp_sum(psum) : hsum;   // the same slots at the same places
   return RowBuilt{smx, hsum, end - lm, lf, psum};
 }
 
@@ -2303,7 +2299,7 @@ __global__ void __launch_bounds__(256, kNeuronBlocks)
 }
 
 // ---------------------------------------------------------------------------
-// per tick 2/4, lit-sum form (lsum_tick: few tested slots, and every axon the row
+// per tick 2/4, lit-sum form (tick_form: few tested slots, and every axon the row
 // layout took as fully lit is fully lit).  An evaluated neuron's input current is
 // the row's lit-sum (frozen slots on fully-lit axons with segments 1..30: hits
 // whatever the tick, their weights summed once per layout; the dendrite sum is a
@@ -2624,6 +2620,11 @@ __device__ __forceinline__ void fixup_slot(const ShardVramPtrs& P, const Variant
 // Sparse-form ticks in a row before the index is asked for: building it costs
 // what the dense pass loses to the sparse form in ~20 ticks (1.5M neurons).
 constexpr uint32_t kIndexStreak = 16;
+// Dense ticks in a row after which the gate's plain graphs go without the sparse form's
+// kernels (two launches that return at once, 4 us of a saturated tick), longer than the
+// bursts of a quiet brain: one whose bursts follow a cycle of 100 ticks lost 8 % when the
+// graphs had them only while the last 16 ticks were quiet.
+constexpr uint32_t kBusyStreak = 256;
 
 // The next tick's lists (last used two ticks ago).
 __device__ __forceinline__ void rows_next_lists(ShardCtl* ctl, uint32_t k) {
@@ -2644,9 +2645,17 @@ __device__ __forceinline__ void rows_fixup(const ShardVramPtrs& P, uint32_t N, u
     if (tid == 0) {
       // ticks in a row that the sparse form would take: ask for its index
       if (wish) {
-        const uint32_t streak = !lsum_tick(ctl, k) && sparse_tick(ctl, k) ? ctl->streak + 1u : 0u;
-        ctl->streak = streak;
-        if (!index_ok(ctl) && streak >= kIndexStreak) *wish = 1u;
+        // (the words are read at once: one after another they were the kernel's end)
+        const unsigned long long p = ctl_ld64(&ctl->pfx_total), c = ctl_ld64(&ctl->slot_total);
+        const uint32_t dark = ctl_ld32(&ctl->dense[k & 1]), was = ctl_ld32(&ctl->streak);
+        const uint32_t busy0 = ctl_ld32(&ctl->busy), told = ctl_ld32(&ctl->busy_told);
+        const uint32_t eval = ctl_ld32(&ctl->eval_act[k & 1][0]), act = ctl_ld32(&ctl->eval_act[k & 1][1]);
+        const bool sparse = !(lit_layout(p, c) && dark == 0u) && sparse_tick(eval, act);
+        const uint32_t streak = sparse ? was + 1u : 0u, busy = sparse ? 0u : min(busy0 + 1u, kBusyStreak);
+        if (streak != was) ctl->streak = streak;
+        if (busy != busy0) ctl->busy = busy;
+        if (streak >= kIndexStreak && !index_built(ctl)) wish[0] = 1u;
+        if ((busy == kBusyStreak) != (told != 0u)) wish[1] = ctl->busy_told = busy == kBusyStreak;
       }
     }
     // readout of the tick (physics.cu:378-395): flags are final once the update pass is done
@@ -2781,8 +2790,8 @@ __device__ __forceinline__ void push_few(uint32_t h[8], uint32_t c) {
   }
 }
 
-// INDEX: also the live axons' and evaluated neurons' bits and the active axons'
-// count, for the sparse form (the learned engine's plain graph).
+// INDEX: also the active axons' count and, where live is given, the live axons' and
+// evaluated neurons' bits, for the sparse form (the learned engine's plain graph).
 // The flags that a refractory neuron's tick clears (physics.cu:168-174): stored here,
 // or with SMALL (one item) returned with bit 8 set for the caller to store; the listed
 // neurons stay in s_list, their count and place in the tick's list in s_place.
@@ -2876,7 +2885,7 @@ __device__ __forceinline__ uint32_t rows_prologue(uint32_t i0, BurstHeads8* head
     if (lane == 0 && i < A) {
       lit_bits[i >> 5] = lb;
       always_lit(alit + (i >> 5), lb, alit_new);
-      if (INDEX) live[i >> 5] = onb;
+      if (INDEX && live) live[i >> 5] = onb;
       // an axon the row layout summed as fully lit is not: this tick takes the full pass
       if (xw[r] & ~lb) atomicAdd(&ctl->dense[k & 1], (uint32_t)__popc(xw[r] & ~lb));
     }
@@ -2896,7 +2905,7 @@ __device__ __forceinline__ uint32_t rows_prologue(uint32_t i0, BurstHeads8* head
     }
     ebal[r] = __ballot_sync(kFull, ev);
     if (lane == 0) {
-      if (INDEX && i < N) evb[i >> 5] = ebal[r];
+      if (INDEX && live && i < N) evb[i >> 5] = ebal[r];
       s_warp[r][w] = __popc(ebal[r]) | (INDEX ? __popc(onb) << 16 : 0);
     }
   }
@@ -3175,7 +3184,7 @@ uint32_t set_barrier_limit(uint32_t tries) {
 cudaError_t rows_wish_alloc(ShardScratch& s) {
   if (s.h_counts_pinned) return cudaSuccess;
   const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&s.h_counts_pinned), 64, cudaHostAllocDefault);
-  if (e == cudaSuccess) *s.h_counts_pinned = 0u;
+  if (e == cudaSuccess) s.h_counts_pinned[0] = s.h_counts_pinned[1] = 0u;
   return e;
 }
 
@@ -3422,7 +3431,7 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
                  (have_incoming && !per_tick) ? s.batch_counts : nullptr, a.k, r.mask2, r.axw, v.soma_flags,
                  v.timers, N, r.eval, s.ctl, raise, r.lit, (a.k > 0 && !per_tick) ? s.pend : nullptr,
                  (have_incoming && per_tick) ? 1u : 0u, per_tick ? 1u : 0u, a.tick - a.k, (int32_t)a.dopamine,
-                 r.xlit, r.live, r.evb, r.alit, a.lit_new ? 1u : 0u);
+                 r.xlit, a.sparse ? r.live : nullptr, r.evb, r.alit, a.lit_new ? 1u : 0u);
   }
   if (ev) cudaEventRecord(ev[2], stream);
   ColWT wt{};
@@ -3436,10 +3445,10 @@ cudaError_t launch_tick_rows(const ShardVramPtrs& v, ShardScratch& s, const Tick
   // with GSOP; both are launched and each returns at once on the other's
   // ticks), ev[4]..ev[5] fix-up and push.
   const uint32_t fix_cap = min(a.fix_cap, kFixCap);
-  launch_rows_update(v, s, N, A, a.k, fix_cap, nullptr, stream, wt, pdl && G, a.index, a.shared_gpu);
+  launch_rows_update(v, s, N, A, a.k, fix_cap, nullptr, stream, wt, pdl && G, a.sparse, a.shared_gpu);
   if (ev) cudaEventRecord(ev[3], stream);
   launch_rows_lsum(v, s, A, a.k, fix_cap, nullptr, stream, wt, pdl, a.shared_gpu);
-  if (a.index) launch_rows_sparse(v, s, N, A, a.k, fix_cap, nullptr, stream);
+  if (a.sparse) launch_rows_sparse(v, s, N, A, a.k, fix_cap, nullptr, stream);
   if (ev) cudaEventRecord(ev[4], stream);
   const bool readout = a.num_outputs > 0 && a.mapped_soma_ids && a.output_history;
   launch_chain(k_rows_fixup, dim3(2 * sms), dim3(256), 0, stream, pdl, v, N, A, r.rt, r.rw, r.cnt, r.mask2, s.pend,
