@@ -72,6 +72,8 @@ struct ShardCtl {
   const uint32_t* ix_off; // inverted index of the rows (RowIndex)
   const uint16_t* ix_seg;
   const uint32_t* ix_ent;
+  uint32_t lay_segs;      // row engine: layouts since the last forced one, up to 2 (keep_segs)
+  uint32_t pad3;
   unsigned long long forms[8];   // row engine: ticks per form, one-launch ticks, layouts (axc_shard_forms)
 };
 
@@ -245,7 +247,10 @@ AXC_HD inline void layout_decision(ShardCtl* c, uint32_t force, uint32_t ticks, 
     c->lay_work = c->pfx_total + c->mov_total;
     c->lay_since = 0;
   }
-  if (build) c->lay_forced = force;
+  if (build) {
+    c->lay_forced = force;
+    c->lay_segs = force ? 0u : c->lay_segs < 2u ? c->lay_segs + 1u : 2u;
+  }
   c->gsop_same[0] = c->gsop_same[1] = 0;
   c->lit_seen = c->ctr[6];
   c->dec_ticks = ticks;

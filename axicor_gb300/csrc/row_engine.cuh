@@ -92,11 +92,13 @@ constexpr uint32_t kAxOwned = 1u, kAxShared = 0x80000000u, kAxSegs = 0x7FFFFFFEu
 // Seven heads one tick apart reach segment 7, two ticks apart 13: an axon lit on its
 // own segments at every tick is lit on those too.  A forced layout takes the larger
 // number: it is the one that a write, a LUT or a change of path makes a program wait
-// for, and the next layout, if it pays, marks the rest.
+// for, and the next layout, if it pays, marks the rest.  The layouts after that keep
+// the marks: the targets are the same until something forces a layout (keep_segs).
 constexpr uint32_t kUsedSegs = 7, kUsedSegsForced = 12;
 __device__ __forceinline__ uint32_t used_segs(const ShardCtl* ctl, uint32_t cond) {
   return cond && !ctl->lay_forced ? kUsedSegs : kUsedSegsForced;
 }
+__device__ __forceinline__ bool keep_segs(const ShardCtl* ctl, uint32_t cond) { return cond && ctl->lay_segs == 2u; }
 __device__ __forceinline__ uint32_t ax_owners(uint32_t axw) { return (axw & kAxOwned) + (axw >> 31); }
 constexpr uint32_t kRowBad = 0x8000u;    // cnt flag: the row holds an invalid target
 constexpr uint32_t kRowSplit = 0x4000u;  // cnt flag: its movable slots are in two groups (build_row), not in slot order
@@ -732,6 +734,7 @@ __global__ void __launch_bounds__(256, kBuildBlocks) k_rows_build(const uint32_t
                                                     uint8_t* __restrict__ posmap, uint32_t* axw, uint32_t cond,
                                                     uint32_t per) {
   if (cond && !ctl->lay_now) return;   // the batch keeps the last layout
+  if (keep_segs(ctl, cond)) axw = nullptr;
   __shared__ SlotStage st;
   const uint32_t pmax = lut_pmax(), used = used_segs(ctl, cond);
   // movable slots join the lit groups (no cooling step up to length 16), except in
@@ -816,8 +819,9 @@ __global__ void __launch_bounds__(256) k_rows_prep(const ShardCtl* __restrict__ 
                                                    uint32_t* __restrict__ xlit, uint32_t cond) {
   if (cond && !ctl->lay_now) return;
   const uint32_t words = A / 32 + 1, used = (2u << used_segs(ctl, cond)) - 2u;
+  const bool keep = keep_segs(ctl, cond);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < A; i += gridDim.x * blockDim.x) {
-    axw[i] = used;
+    axw[i] = keep ? axw[i] & kAxSegs : used;
     if (xlit && i < words) xlit[i] = alit[i];
   }
 }

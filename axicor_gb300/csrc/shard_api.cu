@@ -292,7 +292,10 @@ int32_t cu_step_day_phase(const ShardVramPtrs* vram, uint32_t padded_n, uint32_t
     if (force || s->tick_since_build >= kTickRelayout) {
       err = launch_rows_decide(*s, total_axons, force, kTickRelayout, st);
       if (err == cudaSuccess) err = launch_rows_begin(*vram, *s, padded_n, total_axons, st, false, true, true, true);
-      if (err != cudaSuccess) return (int32_t)err;
+      if (err != cudaSuccess) {
+        batch_undone(s);
+        return (int32_t)err;
+      }
       s->tick_rows_valid.store(true);
       s->tick_rows_lut = gen;
       s->tick_parity = 0;

@@ -225,6 +225,21 @@ def test_layout_tiles(gpu, tiles):
         r.close()
 
 
+def test_later_layouts_keep_the_used_segments(gpu):
+    """Forced, first and later layouts of the same targets, a new write (other targets), and the same again."""
+    r = Ring(600, 704, 40, segs=23)
+    try:
+        for shift in (0, 5):
+            sv = StateView(r.state, r.n)
+            sv.targets[:40] = np.roll(sv.targets[:40], shift, axis=1)
+            sv.targets[3] = ((24 + shift % 4) << 24) | (sv.targets[3] & np.uint32(0xFFFFFF))
+            r.vram.upload_state(r.state)
+            layouts = sum(int(r.run(False)[LAYOUTS]) for _ in range(60))
+            assert layouts >= 4, layouts
+    finally:
+        r.close()
+
+
 @pytest.mark.parametrize("per_tick", [False, True])
 def test_many_dark_axons_take_the_dense_pass(gpu, per_tick):
     """Checking rows slot by slot pays while few have a slot on a dark axon."""
